@@ -48,24 +48,24 @@ def listed():
         dict(name="moves 3000 trees 127x64", kind="moves", genes=127,
              cells=64, trees=3000),
         # the small command-line job from random trees: 8 chains, few blocks
-        dict(name="job 63x64, 8 chains", kind="job", genes=63, cells=64,
+        dict(name="job 63x64 8 chains", kind="job", genes=63, cells=64,
              chains=8, steps=2000, score="max", move="none"),
         # the largest size of the reference's FPGA build: fixed rates
-        dict(name="plain 95x96, 1024 chains", kind="plain", genes=95,
+        dict(name="plain 95x96 1024 chains", kind="plain", genes=95,
              cells=96, chains=1024, steps=8000, score="max", move="none",
              warm=20000, tune=True),
         # the same data with the sum score, learning both rates
-        dict(name="langevin 95x96, 1024 chains", kind="batch", genes=95,
+        dict(name="langevin 95x96 1024 chains", kind="batch", genes=95,
              cells=96, chains=1024, steps=8000, score="sum", move="langevin",
              warm=20000, tune=True),
         # many uneven datasets in one launch
         dict(name="mix of 128 datasets", kind="mix", datasets=128, sizes=512,
              chains=32, steps=2000, warm=2000, tune=True),
         # beyond the FPGA's caps
-        dict(name="plain 255x512, 1024 chains", kind="plain", genes=255,
+        dict(name="plain 255x512 1024 chains", kind="plain", genes=255,
              cells=512, chains=1024, steps=1000, score="max", move="none",
              warm=4000, tune=True),
-        dict(name="langevin 255x512, 1024 chains", kind="batch", genes=255,
+        dict(name="langevin 255x512 1024 chains", kind="batch", genes=255,
              cells=512, chains=1024, steps=1000, score="sum",
              move="langevin", warm=4000, tune=True),
     ]
