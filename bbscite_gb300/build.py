@@ -38,9 +38,15 @@ NVCC_FLAGS = ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC",
               "-Xcompiler", "-ffp-contract=off",
               "-Xcompiler", "-fvisibility=hidden", "-I" + INCLUDE,
               "-I" + CSRC]
-UNITS = ["bbs_mcmc_lo.cu", "bbs_mcmc_lo_rec.cu", "bbs_mcmc_hi.cu",
-         "bbs_mcmc_hi_rec.cu", "bbs_aux.cu", "bbs_api.cu",
-         "bbs_batch.cu", "bbs_batch_multi.cu"]
+# (source, object, defines): the chain kernels are compiled per row width,
+# so that the build is spread over the cores.
+UNITS = ([("bbs_batch.cu", f"bbs_batch_w{w}_m{m}.o",
+           [f"-DBBS_W={w}", f"-DBBS_MULTI={m}"])
+          for w in (4, 3, 2, 1, 8, 7, 6, 5) for m in (0, 1)]
+         + [("bbs_mcmc.cu", f"bbs_mcmc_w{w}_r{r}.o",
+             [f"-DBBS_W={w}", f"-DBBS_REC={r}"])
+            for w in (4, 3, 2, 1, 8, 7, 6, 5) for r in (0, 1)]
+         + [("bbs_aux.cu", "bbs_aux.o", []), ("bbs_api.cu", "bbs_api.o", [])])
 
 
 def nvcc() -> str:
@@ -72,21 +78,21 @@ def _deps() -> float:
     return max(os.path.getmtime(f) for f in files)
 
 
-def _compile(unit: str, newest: float, verbose: bool,
+def _compile(unit: tuple, newest: float, verbose: bool,
              checked: bool = False) -> str:
-    src = os.path.join(CSRC, unit)
-    obj = os.path.join(BUILD_CHECKED if checked else BUILD,
-                       unit.replace(".cu", ".o"))
+    name, out, defines = unit
+    src = os.path.join(CSRC, name)
+    obj = os.path.join(BUILD_CHECKED if checked else BUILD, out)
     if (os.path.exists(obj) and os.path.getmtime(obj) >= newest
             and elf_matches_host(obj)):
         return obj
-    cmd = [nvcc(), *ARCH, *NVCC_FLAGS, *(["-DBBS_CHECKED"] if checked else []),
-           "-c", src, "-o", obj]
+    cmd = [nvcc(), *ARCH, *NVCC_FLAGS, *defines,
+           *(["-DBBS_CHECKED"] if checked else []), "-c", src, "-o", obj]
     if verbose:
         cmd.insert(1, "-Xptxas=-v")
     r = subprocess.run(cmd, capture_output=True, text=True)
     if r.returncode != 0:
-        raise RuntimeError(f"nvcc failed for {unit}:\n{r.stderr}")
+        raise RuntimeError(f"nvcc failed for {out}:\n{r.stderr}")
     if verbose:
         sys.stderr.write(r.stderr)
     return obj
@@ -97,10 +103,9 @@ def build_checked(verbose: bool = False, jobs: int | None = None) -> str:
     debugging; the CLI is not rebuilt."""
     os.makedirs(BUILD_CHECKED, exist_ok=True)
     newest = _deps()
-    units = [u for u in UNITS if os.path.exists(os.path.join(CSRC, u))]
-    jobs = jobs or min(len(units), os.cpu_count() or 4)
+    jobs = jobs or min(len(UNITS), os.cpu_count() or 4)
     with cf.ThreadPoolExecutor(jobs) as ex:
-        objs = list(ex.map(lambda u: _compile(u, newest, verbose, True), units))
+        objs = list(ex.map(lambda u: _compile(u, newest, verbose, True), UNITS))
     if not elf_matches_host(LIB_CHECKED) or os.path.getmtime(LIB_CHECKED) < max(
             os.path.getmtime(o) for o in objs):
         r = subprocess.run([nvcc(), *ARCH, "-shared", "-o", LIB_CHECKED, *objs,
@@ -114,10 +119,9 @@ def build(verbose: bool = False, jobs: int | None = None) -> str:
     os.makedirs(BUILD, exist_ok=True)
     os.makedirs(os.path.dirname(CLI), exist_ok=True)
     newest = _deps()
-    units = [u for u in UNITS if os.path.exists(os.path.join(CSRC, u))]
-    jobs = jobs or min(len(units), os.cpu_count() or 4)
+    jobs = jobs or min(len(UNITS), os.cpu_count() or 4)
     with cf.ThreadPoolExecutor(jobs) as ex:
-        objs = list(ex.map(lambda u: _compile(u, newest, verbose), units))
+        objs = list(ex.map(lambda u: _compile(u, newest, verbose), UNITS))
     if not elf_matches_host(LIB) or os.path.getmtime(LIB) < max(
             os.path.getmtime(o) for o in objs):
         r = subprocess.run([nvcc(), *ARCH, "-shared", "-o", LIB, *objs,

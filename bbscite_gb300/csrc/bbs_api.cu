@@ -327,7 +327,9 @@ void prepare_dataset(const bbs_params *params, uint32_t n_cells,
   h.K.assign((size_t)n_cells * W64, 0);
   h.M.assign(h.K.size(), 0);
   int64_t sum_k = 0, sum_m = 0;
-  for (uint32_t cell = 0; cell < n_cells; cell++)
+  int max_d = 0, max_m = 0;
+  for (uint32_t cell = 0; cell < n_cells; cell++) {
+    int cell_k = 0, cell_m = 0;
     for (uint32_t k = 0; k < W64; k++) {
       uint64_t mask = ~0ull;
       const uint32_t lo = 64 * k;
@@ -336,9 +338,14 @@ void prepare_dataset(const bbs_params *params, uint32_t n_cells,
       const size_t i = (size_t)cell * W64 + k;
       h.K[i] = is_known[i] & mask;
       h.M[i] = is_mutated[i] & h.K[i];
-      sum_k += __builtin_popcountll(h.K[i]);
-      sum_m += __builtin_popcountll(h.M[i]);
+      cell_k += __builtin_popcountll(h.K[i]);
+      cell_m += __builtin_popcountll(h.M[i]);
     }
+    sum_k += cell_k;
+    sum_m += cell_m;
+    max_d = std::max(max_d, cell_k - cell_m);
+    max_m = std::max(max_m, cell_m);
+  }
   const float alpha = params->alpha_mean, bm = params->beta_mean,
               sd = params->beta_sd;
   DatasetDev &ds = h.ds;
@@ -346,6 +353,8 @@ void prepare_dataset(const bbs_params *params, uint32_t n_cells,
   ds.n_nodes = (int)n_nodes;
   ds.sum_k = (int)sum_k;
   ds.sum_m = (int)sum_m;
+  ds.max_d = max_d;
+  ds.max_m = max_m;
   ds.l00 = (float)std::log(1.0 - (double)alpha);
   ds.l10 = logf(alpha);
   ds.bpa = (float)(((double)(1.0f - bm) * std::pow((double)bm, 2.0) /
@@ -827,12 +836,17 @@ namespace {
 
 // One-warp chains per block (1-8; they share the block's increment table)
 // that keep the most warps resident on an SM; ties keep the smaller block.
+int chain_smem(const bbs_ctx *c, int q, int wpc, int cpb) {
+  return plan_tables((int)c->n_nodes, w32_of_nodes((int)c->n_nodes),
+                     (int)c->n_cells, q, wpc, cpb, c->md.score_mode != 0, true,
+                     c->smem_block)
+      .smem;
+}
+
 int pick_chains_per_block(const bbs_ctx *c, int q) {
-  const bool sum = c->md.score_mode != 0;
   int best = 1, best_warps = 0;
   for (int cpb = 1; cpb * 32 <= chain_max_threads(q); cpb++) {
-    const int smem = chain_launch_smem((int)c->n_nodes, (int)c->n_cells, q, 1,
-                                       cpb, sum);
+    const int smem = chain_smem(c, q, 1, cpb);
     const int w = chain_resident_warps(smem, cpb, q, c->smem_sm, c->smem_block,
                                        c->smem_reserved);
     if (w > best_warps) {
@@ -953,8 +967,7 @@ int start_run(bbs_ctx *c, uint32_t n_steps, const bbs_raw_move *d_moves,
               bbs_step_trace *d_trace) {
   {
     const int cpb = c->wpc > 1 ? 1 : c->cpb;
-    const int smem = chain_launch_smem((int)c->n_nodes, (int)c->n_cells, c->q,
-                                       c->wpc, cpb, c->md.score_mode != 0);
+    const int smem = chain_smem(c, c->q, c->wpc, cpb);
     if (32 * c->wpc * cpb > chain_max_threads(c->q) || smem > c->smem_block)
       return fail(BBS_ERR_SIZE,
                   "launch shape (%d cells per lane, %d warps per chain, %d "
@@ -982,7 +995,8 @@ int start_run(bbs_ctx *c, uint32_t n_steps, const bbs_raw_move *d_moves,
   BBS_CUDA(cudaMemsetAsync(c->d_status, 0, sizeof(int) * kStatusWords, c->stream),
            "cudaMemset");
   BBS_CUDA(cudaEventRecord(c->ev0, c->stream), "cudaEventRecord");
-  const int e = launch_mcmc(a, c->q, c->cpb, c->n_sms, c->stream);
+  const int e = launch_mcmc(a, c->q, c->cpb, c->n_sms, c->smem_block,
+                            c->stream);
   if (e != 0) return cuda_fail(e, "chain kernel launch");
   BBS_CUDA(cudaEventRecord(c->ev1, c->stream), "cudaEventRecord");
   return BBS_OK;
@@ -1132,8 +1146,7 @@ int bbs_autotune(bbs_ctx *c, uint32_t probe_steps, float *best_ms) {
         for (int cpb : {1, 2, 4, 7, 8}) {
           if (wpc > 1 && cpb > 1) continue;
           if (32 * wpc * cpb > chain_max_threads(q)) continue;
-          if (chain_launch_smem((int)c->n_nodes, (int)c->n_cells, q, wpc, cpb,
-                                c->md.score_mode != 0) > c->smem_block)
+          if (chain_smem(c, q, wpc, cpb) > c->smem_block)
             continue;  // too large a block
           c->q = q;
           c->wpc = wpc;
@@ -1803,7 +1816,7 @@ struct bbs_batch {
   uint64_t *d_chain_off = nullptr;
   // launch groups (row width), rebuilt when the shape changes
   struct Group {
-    int w32 = 0, max_nodes = 0;
+    int w32 = 0, max_nodes = 0, max_cells = 0;
     int only_ds = -1;  // the group's dataset when it has only one
     std::vector<uint32_t> units;
     uint32_t *d_units = nullptr;
@@ -1919,6 +1932,7 @@ int batch_build_groups(bbs_batch *b) {
       const double nodes = b->n_genes[d] + 1.0;
       cost.push_back({groups * nodes * w + 4.0 * nodes, c});
       g.max_nodes = std::max(g.max_nodes, (int)nodes);
+      g.max_cells = std::max(g.max_cells, (int)b->n_cells[d]);
     }
     if (cost.empty()) continue;
     std::stable_sort(cost.begin(), cost.end(),
@@ -1957,29 +1971,16 @@ int group_wpb(const bbs_batch *b, const bbs_batch::Group &grp) {
   return std::min(b->wpb, chain_max_threads(group_q(b, grp)) / 32);
 }
 
-// Whether the chains of a launch group inherit counts: rows of up to four
-// words when the group has one dataset whose cells stay in registers (the
-// block's increment tables hold that dataset's cells); wider rows always
-// (each warp builds its gene table from the cells it scores).
-bool group_counts(const bbs_batch *b, const bbs_batch::Group &grp) {
-  if (grp.w32 > 4) return true;
-  return grp.only_ds >= 0 &&
-         inherits_counts(grp.w32, (int)b->n_cells[grp.only_ds],
-                         32 * b->wpc * group_q(b, grp));
-}
-
 // Whether every launch group of the current shape fits a block: its shared
 // memory within the device's limit (threads are clamped to the kernel's
 // bounds by group_wpb).  Checked before a run launches anything.
 bool batch_shape_fits(const bbs_batch *b) {
   for (const auto &grp : b->groups) {
-    const int q = group_q(b, grp);
-    const int slots = group_wpb(b, grp) / b->wpc;
-    const bool counts = group_counts(b, grp);
     const int smem =
-        slots * slot_bytes(grp.max_nodes, rs_of_w32(grp.w32), b->wpc,
-                           b->sum || counts, grp.w32, q, counts) +
-        table_bytes(grp.max_nodes, grp.w32, q, b->wpc, counts);
+        plan_tables(grp.max_nodes, grp.w32, grp.max_cells, group_q(b, grp),
+                    b->wpc, group_wpb(b, grp) / b->wpc, b->sum,
+                    grp.only_ds >= 0, b->smem_block)
+            .smem;
     if (smem > b->smem_block) return false;
   }
   return true;
@@ -2026,10 +2027,10 @@ int batch_issue(bbs_batch *b, uint32_t n_steps) {
     a.max_nodes = grp.max_nodes;
     a.table_ds = grp.only_ds;
     const int q = group_q(b, grp);
-    a.with_counts = group_counts(b, grp) ? 1 : 0;
     a.wpc = b->wpc;
-    const int e = launch_batch(a, grp.w32, q, b->sum, group_wpb(b, grp),
-                               b->n_sms, b->side[g]);
+    const int e = launch_batch(a, grp.w32, grp.max_cells, q, b->sum,
+                               group_wpb(b, grp), b->n_sms, b->smem_block,
+                               b->side[g]);
     if (e != 0) return cuda_fail(e, "batch kernel launch");
     BBS_CUDA(cudaEventRecord(b->side_ev[g], b->side[g]), "event");
     BBS_CUDA(cudaStreamWaitEvent(b->stream, b->side_ev[g], 0), "wait");

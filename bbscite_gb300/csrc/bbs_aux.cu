@@ -10,27 +10,53 @@ int pick_q(int n_cells) {
   return std::min(kMaxQ, std::max(1, (n_cells + 31) / 32));
 }
 
-int launch_mcmc(const RunArgs &a, int q, int cpb, int n_sms, void *stream) {
+int launch_mcmc(const RunArgs &a, int q, int cpb, int n_sms, int smem_block,
+                void *stream) {
   const int w32 = w32_of_nodes(a.ds.n_nodes);
   cudaStream_t s = (cudaStream_t)stream;
   const bool sum = a.md.score_mode == 1;
   if (w32 > 4) q = std::min(q, 2);
   const bool rec = a.moves != nullptr || a.trace != nullptr;
-  if (w32 <= 4)
-    return rec ? launch_mcmc_lo_rec(a, w32, q, sum, cpb, n_sms, s)
-               : launch_mcmc_lo(a, w32, q, sum, cpb, n_sms, s);
-  return rec ? launch_mcmc_hi_rec(a, w32, q, sum, cpb, n_sms, s)
-             : launch_mcmc_hi(a, w32, q, sum, cpb, n_sms, s);
+  switch (w32) {
+#define BBS_MCMC_CASE(W)                                            \
+  case W:                                                           \
+    return rec ? launch_mcmc_w<W, true>(a, q, sum, cpb, n_sms, smem_block, s) \
+               : launch_mcmc_w<W, false>(a, q, sum, cpb, n_sms, smem_block, s);
+    BBS_MCMC_CASE(1)
+    BBS_MCMC_CASE(2)
+    BBS_MCMC_CASE(3)
+    BBS_MCMC_CASE(4)
+    BBS_MCMC_CASE(5)
+    BBS_MCMC_CASE(6)
+    BBS_MCMC_CASE(7)
+    BBS_MCMC_CASE(8)
+#undef BBS_MCMC_CASE
+    default: return (int)cudaErrorInvalidValue;
+  }
 }
 
-int launch_batch(const BatchArgs &b, int w32, int q, bool sum, int wpb,
-                 int n_sms, void *stream) {
+int launch_batch(const BatchArgs &b, int w32, int max_cells, int q, bool sum,
+                 int wpb, int n_sms, int smem_block, void *stream) {
   cudaStream_t s = (cudaStream_t)stream;
-  if (b.wpc > 1)
-    return w32 <= 4 ? launch_batch_lo_multi(b, w32, q, sum, wpb, n_sms, s)
-                    : launch_batch_hi_multi(b, w32, q, sum, wpb, n_sms, s);
-  if (w32 <= 4) return launch_batch_lo(b, w32, q, sum, wpb, n_sms, s);
-  return launch_batch_hi(b, w32, q, sum, wpb, n_sms, s);
+  switch (w32) {
+#define BBS_BATCH_CASE(W)                                                   \
+  case W:                                                                   \
+    return b.wpc > 1                                                        \
+               ? launch_batch_w<W, true>(b, max_cells, q, sum, wpb, n_sms,  \
+                                         smem_block, s)                     \
+               : launch_batch_w<W, false>(b, max_cells, q, sum, wpb, n_sms, \
+                                          smem_block, s);
+    BBS_BATCH_CASE(1)
+    BBS_BATCH_CASE(2)
+    BBS_BATCH_CASE(3)
+    BBS_BATCH_CASE(4)
+    BBS_BATCH_CASE(5)
+    BBS_BATCH_CASE(6)
+    BBS_BATCH_CASE(7)
+    BBS_BATCH_CASE(8)
+#undef BBS_BATCH_CASE
+    default: return (int)cudaErrorInvalidValue;
+  }
 }
 
 template <int W32, bool SUM>

@@ -1,58 +1,34 @@
-// Work-list kernels for many datasets in one launch, one instantiation per
-// row width W32 (trees of up to 32 W32 nodes) and cells per lane.
+// Work-list kernels for many datasets in one launch, for one row width BBS_W
+// (trees of up to 32 BBS_W nodes), with one-warp chains or (BBS_MULTI 1)
+// chains of several warps.  The build compiles this unit once per row width
+// and kind.
 #include "bbs_launch.cuh"
-
-// This unit builds the launches of one-warp chains; bbs_batch_multi.cu
-// includes it again for chains of several warps.
-#ifndef BBS_MULTI
-#define BBS_MULTI false
-#define BBS_BATCH_LO launch_batch_lo
-#define BBS_BATCH_HI launch_batch_hi
-#endif
 
 namespace bbs {
 
-#define BBS_BCASE(W, QQ)                                                  \
-  case W * 10 + QQ:                                                       \
-    return sum ? launch_batch_t<W, QQ, true, BBS_MULTI>(b, wpb, n_sms, s) \
-               : launch_batch_t<W, QQ, false, BBS_MULTI>(b, wpb, n_sms, s);
-
-int BBS_BATCH_LO(const BatchArgs &b, int w32, int q, bool sum, int wpb,
-                 int n_sms, cudaStream_t s) {
-  switch (w32 * 10 + q) {
-    BBS_BCASE(1, 1)
-    BBS_BCASE(1, 2)
-    BBS_BCASE(1, 3)
-    BBS_BCASE(1, 4)
-    BBS_BCASE(2, 1)
-    BBS_BCASE(2, 2)
-    BBS_BCASE(2, 3)
-    BBS_BCASE(2, 4)
-    BBS_BCASE(3, 1)
-    BBS_BCASE(3, 2)
-    BBS_BCASE(3, 3)
-    BBS_BCASE(3, 4)
-    BBS_BCASE(4, 1)
-    BBS_BCASE(4, 2)
-    BBS_BCASE(4, 3)
-    BBS_BCASE(4, 4)
+template <int W, bool MULTI>
+int launch_batch_w(const BatchArgs &b, int max_cells, int q, bool sum, int wpb,
+                   int n_sms, int smem_block, cudaStream_t s) {
+#define BBS_CASE(QQ)                                                   \
+  case QQ:                                                                   \
+    return sum ? launch_batch_t<W, QQ, true, MULTI>(b, max_cells, wpb, n_sms, \
+                                                    smem_block, s)           \
+               : launch_batch_t<W, QQ, false, MULTI>(b, max_cells, wpb,      \
+                                                     n_sms, smem_block, s);
+  switch (q) {
+    BBS_CASE(1)
+    BBS_CASE(2)
+#if BBS_W <= 4
+    BBS_CASE(3)
+    BBS_CASE(4)
+#endif
     default: return (int)cudaErrorInvalidValue;
   }
+#undef BBS_CASE
 }
 
-int BBS_BATCH_HI(const BatchArgs &b, int w32, int q, bool sum, int wpb,
-                 int n_sms, cudaStream_t s) {
-  switch (w32 * 10 + q) {
-    BBS_BCASE(5, 1)
-    BBS_BCASE(5, 2)
-    BBS_BCASE(6, 1)
-    BBS_BCASE(6, 2)
-    BBS_BCASE(7, 1)
-    BBS_BCASE(7, 2)
-    BBS_BCASE(8, 1)
-    BBS_BCASE(8, 2)
-    default: return (int)cudaErrorInvalidValue;
-  }
-}
+template int launch_batch_w<BBS_W, BBS_MULTI != 0>(const BatchArgs &, int,
+                                                   int, bool, int, int, int,
+                                                   cudaStream_t);
 
 }  // namespace bbs

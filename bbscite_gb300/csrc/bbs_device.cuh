@@ -808,20 +808,21 @@ __device__ __forceinline__ float ex2_approx(float t) {
 // the root first, every node after its parent -- and in the same pairs, so
 // that a cell's sum does not depend on where it is computed (cells held in
 // registers or streamed, any launch shape, batched or alone) nor on how its
-// counts are found.  Two count sources give the same integers:
-//   - masked popcounts of the node's ancestor row (any tree);
+// counts are found.  Three count sources give the same integers:
+//   - masked popcounts of the node's ancestor row (any tree, any cells);
+//   - a table of every node's counts of the current tree, brought to the
+//     proposal by what the move changes (bbs_incr.cuh; rows of up to four
+//     words);
 //   - inherited counts: a node's ancestors are its parent's plus itself,
-//     so (d, m) of node j = (d, m) of its parent + (D, M) bits of gene j.
-//     This needs the tree's parent vector, a per-warp table of every
-//     node's packed counts and a block table of per-gene increments, and
-//     issues no POPC; it serves cells held in registers with rows of up to
-//     four words.
+//     so (d, m) of node j = (d, m) of its parent + (D, M) bits of gene j
+//     (the ring below; rows of five to eight words with a known parent
+//     vector).
 // ------------------------------------------------------------------------
 struct SumCtx {
   uint16_t *ord;        // [n]: node | parent << 8, in canonical order
   int *hist;            // [32 * ceil(n / 32)]: depth histogram, scratch
-  uint32_t *cnt;        // [n][32][NW]: every node's packed counts of the
-                        // lane's cells, or null
+  uint32_t *cnt;        // [chunks][n][32][NW]: the table of every node for
+                        // the lane's cells (bbs_incr.cuh), or null
   const uint32_t *inc;  // [n][32][NW]: per-gene packed increments of the
                         // warp's cells, or null
   const uint8_t *par;   // parent vector of the evaluated tree, or null
@@ -1132,52 +1133,11 @@ __device__ __noinline__ bool parents_match_rows(const uint32_t *rows, int n,
   return __all_sync(BBS_FULL_MASK, ok);
 }
 
-// Inherited counts of the nodes at order positions i and i + 1, all Q
-// cells at once (packed), stored in the count table.  All four loads come
-// first; when node i + 1 is node i's child, its parent's counts are taken
-// from the register instead of the table (whose entry is not stored yet).
-template <int Q, int NW = kPackWords<Q>>
-__device__ __forceinline__ void inherit_pair(const SumCtx &sx, int i, int lane,
-                                             uint32_t (&k0)[NW],
-                                             uint32_t (&k1)[NW], int &j0,
-                                             int &j1) {
-  const uint32_t o0 = sx.ord[i], o1 = sx.ord[i + 1];
-  j0 = (int)(o0 & 0xFF);
-  j1 = (int)(o1 & 0xFF);
-  const int p0 = (int)(o0 >> 8), p1 = (int)(o1 >> 8);
-  uint32_t a0[NW], a1[NW], g0[NW], g1[NW];
-  ld_pack<Q>(sx.cnt, p0 * 32 + lane, a0);
-  ld_pack<Q>(sx.cnt, p1 * 32 + lane, a1);
-  ld_pack<Q>(sx.inc, j0 * 32 + lane, g0);
-  ld_pack<Q>(sx.inc, j1 * 32 + lane, g1);
-#pragma unroll
-  for (int w = 0; w < NW; w++) {
-    k0[w] = a0[w] + g0[w];
-    k1[w] = (p1 == j0 ? k0[w] : a1[w]) + g1[w];
-  }
-  st_pack<Q>(sx.cnt, j0 * 32 + lane, k0);
-  st_pack<Q>(sx.cnt, j1 * 32 + lane, k1);
-}
-
-// The same for the node at order position i alone.
-template <int Q, int NW = kPackWords<Q>>
-__device__ __forceinline__ void inherit_one(const SumCtx &sx, int i, int lane,
-                                            uint32_t (&k)[NW], int &j) {
-  const uint32_t o = sx.ord[i];
-  j = (int)(o & 0xFF);
-  const int p = (int)(o >> 8);
-  uint32_t a[NW], g[NW];
-  ld_pack<Q>(sx.cnt, p * 32 + lane, a);
-  ld_pack<Q>(sx.inc, j * 32 + lane, g);
-#pragma unroll
-  for (int w = 0; w < NW; w++) k[w] = a[w] + g[w];
-  st_pack<Q>(sx.cnt, j * 32 + lane, k);
-}
-
-// inherit_pair for rows of five to eight words: the parents' counts come
-// from the ring (entries hold the parents' order positions, ring_order),
-// the increments from the gene table, and positions i and i + 1 are stored
-// in the ring.  Why no load reads an overwritten entry: when the loads run,
+// Inherited counts of the nodes at order positions i and i + 1, all Q cells
+// at once (packed), for rows of five to eight words: the parents' counts
+// come from the ring (entries hold the parents' order positions,
+// ring_order), the increments from the gene table, and positions i and i + 1
+// are stored in the ring.  All four loads come first.  Why no load reads an overwritten entry: when the loads run,
 // positions up to i - 1 are stored (each lane reads and writes only its own
 // column, in program order).  A parent at position p < i was stored at
 // entry p % kRing, and the positions stored since, p + 1 .. i - 1, are
@@ -1223,38 +1183,13 @@ __device__ __forceinline__ void inherit_one_ring(const SumCtx &sx, int i,
   st_pack<Q>(sx.ring, (i & (kRing - 1)) * 32 + lane, k);
 }
 
-// The two count sources by inheritance: the table of every node (rows of
-// up to four words) or the ring.
-template <int Q, bool RING, int NW = kPackWords<Q>>
-__device__ __forceinline__ void inherit2(const SumCtx &sx, int i, int lane,
-                                         uint32_t (&k0)[NW],
-                                         uint32_t (&k1)[NW], int &j0,
-                                         int &j1) {
-  if constexpr (RING)
-    inherit_pair_ring<Q>(sx, i, lane, k0, k1, j0, j1);
-  else
-    inherit_pair<Q>(sx, i, lane, k0, k1, j0, j1);
-}
-
-template <int Q, bool RING, int NW = kPackWords<Q>>
-__device__ __forceinline__ void inherit1(const SumCtx &sx, int i, int lane,
-                                         uint32_t (&k)[NW], int &j) {
-  if constexpr (RING)
-    inherit_one_ring<Q>(sx, i, lane, k, j);
-  else
-    inherit_one<Q>(sx, i, lane, k, j);
-}
-
 // The root's zero counts, at order position 0.
-template <int Q, bool RING, int NW = kPackWords<Q>>
+template <int Q, int NW = kPackWords<Q>>
 __device__ __forceinline__ void store_root(const SumCtx &sx, int lane) {
   uint32_t zero[NW];
 #pragma unroll
   for (int w = 0; w < NW; w++) zero[w] = 0u;
-  if constexpr (RING)
-    st_pack<Q>(sx.ring, lane, zero);
-  else
-    st_pack<Q>(sx.cnt, (int)(sx.ord[0] & 0xFF) * 32 + lane, zero);
+  st_pack<Q>(sx.ring, lane, zero);
 }
 
 // The sum score's float work of two nodes, side by side in the halves of
@@ -1330,34 +1265,28 @@ struct Resum {
 // its own maximum (base already shifted), one node at a time in the
 // canonical order.  Rarely taken, so kept out of line: the node loop's code
 // stays small, and the cells come by value.
-template <int W32, int Q, bool INHERIT>
+template <int W32, int Q>
 __device__ __noinline__ Resum<Q> resum_cells(const uint32_t *rows, int n,
                                              const Cells<W32, Q> cb,
                                              const SumCtx sx, int lane,
                                              float c1, float c2,
                                              const QF<Q> base, unsigned bad) {
   constexpr int RS = rs_of_w32(W32);
-  constexpr int NW = kPackWords<Q>;
   Resum<Q> o;
 #pragma unroll
   for (int q = 0; q < Q; q++) o.z.v[q] = o.ed.v[q] = o.em.v[q] = 0.0f;
 #pragma unroll 1
   for (int i2 = 0; i2 < n; i2++) {
     const int j = (int)(sx.ord[i2] & 0xFF);
-    uint32_t a[W32], k[NW];
-    if constexpr (!INHERIT) ld_row<W32>(rows + j * RS, a);
-    if constexpr (INHERIT) ld_pack<Q>(sx.cnt, j * 32 + lane, k);
+    uint32_t a[W32];
+    ld_row<W32>(rows + j * RS, a);
 #pragma unroll
     for (int q = 0; q < Q; q++) {
       if (!((bad >> q) & 1u)) continue;
-      float fd, fm;
-      if constexpr (INHERIT) {
-        fd = pack_d_biased(k[q >> 1], q) - 8388608.0f;
-        fm = pack_m_biased(k[q >> 1], q) - 8388608.0f;
-      } else {
-        fd = __int_as_float(0x4B000000 + masked_popc<W32>(cb.D[q], a)) - 8388608.0f;
-        fm = __int_as_float(0x4B000000 + masked_popc<W32>(cb.M[q], a)) - 8388608.0f;
-      }
+      const float fd =
+          __int_as_float(0x4B000000 + masked_popc<W32>(cb.D[q], a)) - 8388608.0f;
+      const float fm =
+          __int_as_float(0x4B000000 + masked_popc<W32>(cb.M[q], a)) - 8388608.0f;
       const float e = ex2_approx(fmaf(fd, c1, fmaf(fm, c2, base.v[q])));
       o.z.v[q] += e;
       o.ed.v[q] = fmaf(e, fd, o.ed.v[q]);
@@ -1380,7 +1309,7 @@ __device__ __noinline__ Resum<Q> resum_cells_ring(int n, const SumCtx sx,
   Resum<Q> o;
 #pragma unroll
   for (int q = 0; q < Q; q++) o.z.v[q] = o.ed.v[q] = o.em.v[q] = 0.0f;
-  store_root<Q, true>(sx, lane);
+  store_root<Q>(sx, lane);
 #pragma unroll 1
   for (int i2 = 0; i2 < n; i2++) {
     uint32_t k[NW];
@@ -1418,7 +1347,7 @@ __device__ __noinline__ int2 counts_at_reload(const uint32_t *rows,
   return make_int2(k, m);
 }
 
-template <int W32, int Q, bool INHERIT, bool RING = false>
+template <int W32, int Q, bool RING>
 __device__ __forceinline__ void sum_cells(const uint32_t *rows, int n,
                                           const Cells<W32, Q> &cb,
                                           const LogTable &L, int c0, int stride,
@@ -1441,7 +1370,7 @@ __device__ __forceinline__ void sum_cells(const uint32_t *rows, int n,
     base2[q] = dup2(base[q]);
   }
   // the root (ord[0]) has no counted bits: t = base
-  if constexpr (INHERIT) store_root<Q, RING>(sx, lane);
+  if constexpr (RING) store_root<Q>(sx, lane);
 #pragma unroll
   for (int q = 0; q < Q; q++) {
     mx[q] = base[q];
@@ -1450,23 +1379,23 @@ __device__ __forceinline__ void sum_cells(const uint32_t *rows, int n,
   }
   // the other nodes two at a time, in the two halves of paired registers
   int i = 1;
-  if constexpr (INHERIT) {
+  if constexpr (RING) {
     // counts one pair ahead of the float work, which hides the table's
     // load latency behind the previous pair's arithmetic; two pairs per
     // iteration, alternating between two register sets
     if (i + 1 < n) {
       uint32_t kA0[NW], kA1[NW], kB0[NW], kB1[NW];
       int jA0, jA1, jB0, jB1;  // node numbers (the max score uses them)
-      inherit2<Q, RING>(sx, i, lane, kA0, kA1, jA0, jA1);
+      inherit_pair_ring<Q>(sx, i, lane, kA0, kA1, jA0, jA1);
 #pragma unroll 1
       for (; i + 5 < n; i += 4) {
-        inherit2<Q, RING>(sx, i + 2, lane, kB0, kB1, jB0, jB1);
+        inherit_pair_ring<Q>(sx, i + 2, lane, kB0, kB1, jB0, jB1);
         sum_counts2<Q, NW>(kA0, kA1, c1p, c2p, base2, mx, z2, ed2, em2);
-        inherit2<Q, RING>(sx, i + 4, lane, kA0, kA1, jA0, jA1);
+        inherit_pair_ring<Q>(sx, i + 4, lane, kA0, kA1, jA0, jA1);
         sum_counts2<Q, NW>(kB0, kB1, c1p, c2p, base2, mx, z2, ed2, em2);
       }
       if (i + 3 < n) {
-        inherit2<Q, RING>(sx, i + 2, lane, kB0, kB1, jB0, jB1);
+        inherit_pair_ring<Q>(sx, i + 2, lane, kB0, kB1, jB0, jB1);
         sum_counts2<Q, NW>(kA0, kA1, c1p, c2p, base2, mx, z2, ed2, em2);
         sum_counts2<Q, NW>(kB0, kB1, c1p, c2p, base2, mx, z2, ed2, em2);
         i += 4;
@@ -1508,10 +1437,10 @@ __device__ __forceinline__ void sum_cells(const uint32_t *rows, int n,
   }
   if (i < n) {
     float fd[Q], fm[Q];
-    if constexpr (INHERIT) {
+    if constexpr (RING) {
       uint32_t k[NW];
       int j;
-      inherit1<Q, RING>(sx, i, lane, k, j);
+      inherit_one_ring<Q>(sx, i, lane, k, j);
 #pragma unroll
       for (int q = 0; q < Q; q++) {
         fd[q] = pack_d_biased(k[q >> 1], q) - 8388608.0f;
@@ -1568,8 +1497,7 @@ __device__ __forceinline__ void sum_cells(const uint32_t *rows, int n,
     if constexpr (RING)
       o = resum_cells_ring<Q>(n, sx, lane, c1, c2, b2, badm);
     else
-      o = resum_cells<W32, Q, INHERIT>(rows, n, cb, sx, lane, c1, c2, b2,
-                                       badm);
+      o = resum_cells<W32, Q>(rows, n, cb, sx, lane, c1, c2, b2, badm);
 #pragma unroll
     for (int q = 0; q < Q; q++)
       if (bad[q]) {
@@ -1622,7 +1550,6 @@ __device__ __noinline__ Acc6 sum_cells_popc(const uint32_t *rows, int n,
 template <int W32, int Q>
 __device__ __forceinline__ void sum_part(const uint32_t *rows, int n,
                                          const DatasetDev &ds,
-                                         Cells<W32, Q> &cb, bool resident,
                                          const LogTable &L, int wpc, int wic,
                                          int lane, long long (&acc)[6],
                                          const SumCtx &sx) {
@@ -1643,7 +1570,7 @@ __device__ __forceinline__ void sum_part(const uint32_t *rows, int n,
         Cells<W32, Q> cc;
         load_cells<W32, Q>(cc, ds, c0 + 32 * wic, 32 * wpc, lane);
         build_gene_table<W32, Q>(cc, sx.gt, n, lane);
-        sum_cells<W32, Q, true, true>(rows, n, cc, L, c0 + 32 * wic, 32 * wpc,
+        sum_cells<W32, Q, true>(rows, n, cc, L, c0 + 32 * wic, 32 * wpc,
                                       lane, ds.n_cells, acc, sx);
       }
       acc[0] = warp_sum_ll(acc[0]);
@@ -1655,29 +1582,14 @@ __device__ __forceinline__ void sum_part(const uint32_t *rows, int n,
   } else {
     canonical_order<W32>(rows, n, sx.par, sx.ord, sx.hist, lane);
   }
-  if (resident) {
-    bool inherit = false;
-    if constexpr (W32 <= 4)
-      inherit = sx.cnt != nullptr && sx.inc != nullptr && sx.par != nullptr;
-    if (inherit) {
-      if constexpr (W32 <= 4)
-        sum_cells<W32, Q, true>(rows, n, cb, L, 32 * wic, 32 * wpc, lane,
-                                ds.n_cells, acc, sx);
-    } else {
-      const Acc6 o = sum_cells_popc<W32, Q>(rows, n, cb, L, 32 * wic,
-                                            32 * wpc, lane, ds.n_cells, sx);
+  const int span = 32 * wpc * Q;
+  for (int c0 = 0; c0 < ds.n_cells; c0 += span) {
+    Cells<W32, Q> cb;
+    load_cells<W32, Q>(cb, ds, c0 + 32 * wic, 32 * wpc, lane);
+    const Acc6 o = sum_cells_popc<W32, Q>(rows, n, cb, L, c0 + 32 * wic,
+                                          32 * wpc, lane, ds.n_cells, sx);
 #pragma unroll
-      for (int k = 0; k < 6; k++) acc[k] += o.v[k];
-    }
-  } else {
-    const int span = 32 * wpc * Q;
-    for (int c0 = 0; c0 < ds.n_cells; c0 += span) {
-      load_cells<W32, Q>(cb, ds, c0 + 32 * wic, 32 * wpc, lane);
-      const Acc6 o = sum_cells_popc<W32, Q>(rows, n, cb, L, c0 + 32 * wic,
-                                            32 * wpc, lane, ds.n_cells, sx);
-#pragma unroll
-      for (int k = 0; k < 6; k++) acc[k] += o.v[k];
-    }
+    for (int k = 0; k < 6; k++) acc[k] += o.v[k];
   }
   acc[0] = warp_sum_ll(acc[0]);
   acc[2] = warp_sum_ll(acc[2]);
@@ -1685,13 +1597,13 @@ __device__ __forceinline__ void sum_part(const uint32_t *rows, int n,
   acc[5] = warp_sum_ll(acc[5]);
 }
 
-// Max score with inherited counts (rows of up to four words, cells in
-// registers): the nodes in the canonical order with their counts found one
-// pair ahead as for the sum score, each node's score in the reference's
+// Max score with counts through the ring: the nodes in the canonical order
+// with their counts found one pair ahead as for the sum score, each node's score in the reference's
 // order, and the first maximum in node-index order -- an equal score at a
 // lower index wins, which is what std::max over the nodes in index order
-// keeps (src/TreeScorer.hpp:187-193) -- so the chosen nodes, and the class
-// counts at them, are those of best_nodes.
+// keeps (src/TreeScorer.hpp:187-193) -- so the chosen nodes are those of
+// best_nodes.  The ring no longer holds every node at the end: the class
+// counts at the chosen nodes are the caller's masked popcounts.
 __device__ __forceinline__ void max_select(float s, int j, float &best,
                                            int &bj) {
   const bool up = s > best || (s == best && j < bj);
@@ -1720,13 +1632,11 @@ __device__ __forceinline__ void max_update2(const uint32_t (&k0)[NW], int j0,
   }
 }
 
-template <int W32, int Q, bool RING = false>
-__device__ __forceinline__ void max_cells_inherit(const uint32_t *rows, int n,
-                                                  const Cells<W32, Q> &cb,
-                                                  const LogTable &L, float nz,
-                                                  int lane, const SumCtx &sx,
-                                                  int &k, int &m,
-                                                  QI<Q> *chosen = nullptr) {
+template <int W32, int Q>
+__device__ __forceinline__ void max_cells_ring(int n, const Cells<W32, Q> &cb,
+                                               const LogTable &L, float nz,
+                                               int lane, const SumCtx &sx,
+                                               QI<Q> &chosen) {
   constexpr int NW = kPackWords<Q>;
   const LogTable2 L2 = log_table2(L, nz);
   float best[Q];
@@ -1734,7 +1644,7 @@ __device__ __forceinline__ void max_cells_inherit(const uint32_t *rows, int n,
   float2 pdb[Q], pmb[Q];
   {
     const int root = (int)(sx.ord[0] & 0xFF);
-    store_root<Q, RING>(sx, lane);
+    store_root<Q>(sx, lane);
 #pragma unroll
     for (int q = 0; q < Q; q++) {
       best[q] = pair_score(0, 0, cb.pdb[q], cb.pmb[q], L.l00, L.l01, L.l10,
@@ -1748,16 +1658,16 @@ __device__ __forceinline__ void max_cells_inherit(const uint32_t *rows, int n,
   if (i + 1 < n) {
     uint32_t kA0[NW], kA1[NW], kB0[NW], kB1[NW];
     int jA0, jA1, jB0, jB1;
-    inherit2<Q, RING>(sx, i, lane, kA0, kA1, jA0, jA1);
+    inherit_pair_ring<Q>(sx, i, lane, kA0, kA1, jA0, jA1);
 #pragma unroll 1
     for (; i + 5 < n; i += 4) {
-      inherit2<Q, RING>(sx, i + 2, lane, kB0, kB1, jB0, jB1);
+      inherit_pair_ring<Q>(sx, i + 2, lane, kB0, kB1, jB0, jB1);
       max_update2<Q, NW>(kA0, jA0, kA1, jA1, pdb, pmb, L2, best, bj);
-      inherit2<Q, RING>(sx, i + 4, lane, kA0, kA1, jA0, jA1);
+      inherit_pair_ring<Q>(sx, i + 4, lane, kA0, kA1, jA0, jA1);
       max_update2<Q, NW>(kB0, jB0, kB1, jB1, pdb, pmb, L2, best, bj);
     }
     if (i + 3 < n) {
-      inherit2<Q, RING>(sx, i + 2, lane, kB0, kB1, jB0, jB1);
+      inherit_pair_ring<Q>(sx, i + 2, lane, kB0, kB1, jB0, jB1);
       max_update2<Q, NW>(kA0, jA0, kA1, jA1, pdb, pmb, L2, best, bj);
       max_update2<Q, NW>(kB0, jB0, kB1, jB1, pdb, pmb, L2, best, bj);
       i += 4;
@@ -1769,7 +1679,7 @@ __device__ __forceinline__ void max_cells_inherit(const uint32_t *rows, int n,
   if (i < n) {
     uint32_t kk[NW];
     int j;
-    inherit1<Q, RING>(sx, i, lane, kk, j);
+    inherit_one_ring<Q>(sx, i, lane, kk, j);
 #pragma unroll
     for (int q = 0; q < Q; q++) {
       const float s = pair_score_b(pack_d_biased(kk[q >> 1], q),
@@ -1778,21 +1688,8 @@ __device__ __forceinline__ void max_cells_inherit(const uint32_t *rows, int n,
       max_select(s, j, best[q], bj[q]);
     }
   }
-  // the counts at the chosen nodes: k = popc(K & A) = d + m (the ring no
-  // longer holds every node: the caller takes masked popcounts then)
-  if constexpr (RING) {
 #pragma unroll
-    for (int q = 0; q < Q; q++) chosen->v[q] = bj[q];
-  } else {
-#pragma unroll
-    for (int q = 0; q < Q; q++) {
-      uint32_t c[NW];
-      ld_pack<Q>(sx.cnt, bj[q] * 32 + lane, c);
-      const uint32_t f = pack_field<NW>(c, q);
-      k += (int)(f & 0xFFu) + (int)(f >> 8);
-      m += (int)(f >> 8);
-    }
-  }
+  for (int q = 0; q < Q; q++) chosen.v[q] = bj[q];
 }
 
 // The max score's masked-popcount pass over one chunk of cells it loads
@@ -1813,15 +1710,14 @@ __device__ __noinline__ int2 max_chunk_popc(const uint32_t *rows, int n,
 
 // This warp's part of the class sums over its cells (max score).  Cells
 // are split over the `wpc` warps of a chain: cell = c0 + 32*wpc*q +
-// 32*wic + lane.  With `resident`, cb already holds the warp's cells.
+// 32*wic + lane.
 template <int W32, int Q>
 __device__ __forceinline__ void score_part(const uint32_t *rows, int n,
                                            const DatasetDev &ds,
-                                           Cells<W32, Q> &cb, bool resident,
                                            const LogTable &L, int wpc,
                                            int wic, int lane, int &sk,
                                            int &sm, const SumCtx &sx) {
-  int k = 0, m = 0, bj[Q];
+  int k = 0, m = 0;
   if constexpr (W32 > 4) {
     // rows of five to eight words: counts through the ring, as for the sum
     // score
@@ -1834,8 +1730,7 @@ __device__ __forceinline__ void score_part(const uint32_t *rows, int n,
           Cells<W32, Q> cc;
           load_cells<W32, Q>(cc, ds, c0 + 32 * wic, 32 * wpc, lane);
           build_gene_table<W32, Q>(cc, sx.gt, n, lane);
-          max_cells_inherit<W32, Q, true>(rows, n, cc, L, ds.neg_zero, lane,
-                                          sx, k, m, &chosen);
+          max_cells_ring<W32, Q>(n, cc, L, ds.neg_zero, lane, sx, chosen);
         }
         const int2 km = counts_at_reload<W32, Q>(rows, &ds, c0 + 32 * wic,
                                                  32 * wpc, chosen, lane);
@@ -1847,34 +1742,21 @@ __device__ __forceinline__ void score_part(const uint32_t *rows, int n,
       return;
     }
   }
-  bool inherit = false;
-  if constexpr (W32 <= 4)
-    inherit = resident && sx.cnt != nullptr && sx.inc != nullptr &&
-              sx.par != nullptr;
-  if (inherit) {
-    if constexpr (W32 <= 4) {
-      canonical_order<W32>(rows, n, sx.par, sx.ord, sx.hist, lane);
-      max_cells_inherit<W32, Q>(rows, n, cb, L, ds.neg_zero, lane, sx, k,
-                                  m);
-    }
-  } else if (resident) {
-    best_nodes<W32, Q>(rows, n, cb, L.l00, L.l01, L.l10, L.l11, ds.neg_zero, bj);
-    counts_at<W32, Q>(rows, cb, bj, k, m);
-  } else {
-    const int span = 32 * wpc * Q;
-    for (int c0 = 0; c0 < ds.n_cells; c0 += span) {
-      if constexpr (W32 > 4) {
-        // (out of line: wider rows take their counts through the ring)
-        const int2 km = max_chunk_popc<W32, Q>(rows, n, &ds, c0 + 32 * wic,
-                                               32 * wpc, L, lane);
-        k += km.x;
-        m += km.y;
-      } else {
-        load_cells<W32, Q>(cb, ds, c0 + 32 * wic, 32 * wpc, lane);
-        best_nodes<W32, Q>(rows, n, cb, L.l00, L.l01, L.l10, L.l11,
-                           ds.neg_zero, bj);
-        counts_at<W32, Q>(rows, cb, bj, k, m);
-      }
+  const int span = 32 * wpc * Q;
+  for (int c0 = 0; c0 < ds.n_cells; c0 += span) {
+    if constexpr (W32 > 4) {
+      // (out of line: wider rows take their counts through the ring)
+      const int2 km = max_chunk_popc<W32, Q>(rows, n, &ds, c0 + 32 * wic,
+                                             32 * wpc, L, lane);
+      k += km.x;
+      m += km.y;
+    } else {
+      Cells<W32, Q> cb;
+      int bj[Q];
+      load_cells<W32, Q>(cb, ds, c0 + 32 * wic, 32 * wpc, lane);
+      best_nodes<W32, Q>(rows, n, cb, L.l00, L.l01, L.l10, L.l11, ds.neg_zero,
+                         bj);
+      counts_at<W32, Q>(rows, cb, bj, k, m);
     }
   }
   sk = (int)__reduce_add_sync(BBS_FULL_MASK, (uint32_t)k);
@@ -1916,25 +1798,6 @@ __device__ __forceinline__ void beta_terms(const DatasetDev &ds, float beta,
   prior = __fsub_rn(r, ds.lg_b);
 }
 
-// The same entries in single precision for the learned error moves (no
-// reference counterpart to match, so no double-precision logs): the log
-// table of a proposed (alpha, beta) and logscore_beta.
-__device__ __forceinline__ void alpha_terms_f(float alpha, float &l00,
-                                              float &l10) {
-  l00 = log1pf(-alpha);
-  l10 = logf(alpha);
-}
-__device__ __forceinline__ void beta_terms_f(const DatasetDev &ds, float beta,
-                                             float &l01, float &l11,
-                                             float &prior) {
-  l01 = logf(beta);
-  l11 = log1pf(-beta);
-  float r = __fadd_rn(ds.lg_ab, __fmul_rn(__fsub_rn(ds.bpa, 1.0f), l01));
-  r = __fadd_rn(r, __fmul_rn(__fsub_rn(ds.bpb, 1.0f), logf(__fsub_rn(1.0f, beta))));
-  r = __fsub_rn(r, ds.lg_a);
-  prior = __fsub_rn(r, ds.lg_b);
-}
-
 // ------------------------------------------------------------------------
 // Error-rate moves in (a, b) = (logit alpha, logit beta).  The target is
 //   gamma * S(alpha, beta) + log(alpha (1-alpha)) + log(beta (1-beta)),
@@ -1943,53 +1806,123 @@ __device__ __forceinline__ void beta_terms_f(const DatasetDev &ds, float beta,
 // e[4] = (n00, n01, n10, n11) give the gradient and a diagonal
 // preconditioner M = 1 / (1 + curvature) from the same counts.
 // ------------------------------------------------------------------------
-struct ErrorGeom {
-  float grad_a, grad_b, prec_a, prec_b;
+// One lane works on each side: lane 0 on alpha, lane 1 on beta, and the
+// functions -- logs, the square root, the sigmoid, quotients -- are issued
+// once for all their arguments, one per lane.  Written per scalar they were
+// some 1,500 instructions that a chain runs through once in ten steps, and
+// fetching those cost several times their execution.  All lanes but the first
+// compute with beta's arguments where no other is named.
+struct RateProposal {
+  float palpha, pbeta, pprior;  // the proposal (in every lane)
+  LogTable PL;
+  float from, to, grad, prec;   // this lane's side: logits, the gradient and
+                                // preconditioner at the current rates
 };
 
-__device__ __forceinline__ ErrorGeom error_geometry(const DatasetDev &ds,
-                                                    float alpha, float beta,
-                                                    float gamma,
-                                                    const float (&e)[4]) {
-  ErrorGeom g;
-  const float va = alpha * (1.0f - alpha), vb = beta * (1.0f - beta);
-  const float dS_da = -e[0] / (1.0f - alpha) + e[2] / alpha;
-  const float dS_db = e[1] / beta - e[3] / (1.0f - beta) +
-                      (ds.bpa - 1.0f) / beta - (ds.bpb - 1.0f) / (1.0f - beta);
-  g.grad_a = gamma * va * dS_da + (1.0f - 2.0f * alpha);
-  g.grad_b = gamma * vb * dS_db + (1.0f - 2.0f * beta);
-  g.prec_a = 1.0f / (1.0f + gamma * (e[0] + e[2]) * va);
-  g.prec_b = 1.0f / (1.0f + gamma * (e[1] + e[3] + fmaxf(ds.bpa + ds.bpb - 2.0f, 0.0f)) * vb);
-  return g;
+inline __device__ __noinline__ float log_lane(float x) { return logf(x); }
+inline __device__ __noinline__ float log1p_lane(float x) { return log1pf(x); }
+
+__device__ __forceinline__ float lane_of(float x, int l) {
+  return __shfl_sync(BBS_FULL_MASK, x, l);
 }
 
-__device__ __forceinline__ float logit(float p) { return logf(p) - log1pf(-p); }
-__device__ __forceinline__ float sigmoid(float x) { return 1.0f / (1.0f + __expf(-x)); }
-
-// log q(to | from) of the (preconditioned, optionally gradient-drifted)
-// Gaussian proposal, up to the constant shared by both directions.
-__device__ __forceinline__ float log_q(float ta, float tb, float fa, float fb,
-                                       const ErrorGeom &g, float eps,
-                                       bool drift) {
-  const float h = drift ? 0.5f * eps * eps : 0.0f;
-  const float ra = ta - fa - h * g.prec_a * g.grad_a;
-  const float rb = tb - fb - h * g.prec_b * g.grad_b;
-  const float e2 = eps * eps;
-  return -(ra * ra) / (2.0f * e2 * g.prec_a) - (rb * rb) / (2.0f * e2 * g.prec_b) -
-         0.5f * (logf(g.prec_a) + logf(g.prec_b));
+// The gradient and the preconditioner of this lane's side.
+__device__ __forceinline__ void rate_geometry(const DatasetDev &ds,
+                                              float alpha, float beta,
+                                              float gamma,
+                                              const float (&e)[4], int lane,
+                                              float &grad, float &prec) {
+  const bool a = lane == 0;
+  const float p = a ? alpha : beta, q = 1.0f - p, v = p * q;
+  const float hit = a ? e[2] : e[1], miss = a ? e[0] : e[3];
+  const float p1 = a ? 0.0f : ds.bpa - 1.0f, p2 = a ? 0.0f : ds.bpb - 1.0f;
+  const float more = a ? 0.0f : fmaxf(ds.bpa + ds.bpb - 2.0f, 0.0f);
+  const float dS = hit / p - miss / q + p1 / p - p2 / q;
+  grad = gamma * v * dS + (1.0f - 2.0f * p);
+  prec = 1.0f / (1.0f + gamma * (hit + miss + more) * v);
 }
 
-// Two standard normals from the move's two uniforms (Box-Muller); the
-// record's raw_descendant_of_v / raw_nondescendant_of_v are unused by
-// error moves, so recorded streams fix these draws too.
-__device__ __forceinline__ void error_normals(const bbs_raw_move &raw,
-                                              float &z0, float &z1) {
+// A (preconditioned) random walk or, with drift, a Langevin step in logit
+// space from the move's two uniforms (Box-Muller; the record's
+// raw_descendant_of_v / raw_nondescendant_of_v are unused by error moves, so
+// recorded streams fix these draws too), and the log table and Beta prior of
+// the proposed rates in single precision (no reference counterpart to match).
+__device__ __forceinline__ RateProposal
+propose_rates(const DatasetDev &ds, const ModelDev &md, float alpha,
+              float beta, const float (&ec)[4], const bbs_raw_move &raw,
+              int lane) {
+  RateProposal o;
+  rate_geometry(ds, alpha, beta, md.gamma, ec, lane, o.grad, o.prec);
+  const float eps = md.error_step;
+  const float h = md.error_move == 2 ? 0.5f * eps * eps : 0.0f;
+  const float p = lane == 0 ? alpha : beta;
   const float u1 = fmaxf(1.0f - raw.raw_descendant_of_v, 1.0e-30f);
-  const float r = sqrtf(-2.0f * logf(u1));
+  const float l = log_lane(lane == 2 ? u1 : p);
+  o.from = l - log1p_lane(-p);
+  const float root =
+      sqrtf(lane == 2 ? -2.0f * l : o.prec);  // lane 2: the normals' radius
+  const float radius = lane_of(root, 2);
   float s, c;
   sincospif(2.0f * raw.raw_nondescendant_of_v, &s, &c);
-  z0 = r * c;
-  z1 = r * s;
+  const float z = lane == 0 ? radius * c : radius * s;
+  const float to = o.from + h * o.prec * o.grad + eps * root * z;
+  const float pp =
+      fminf(fmaxf(1.0f / (1.0f + __expf(-to)), 1.0e-7f), 1.0f - 1.0e-7f);
+  o.palpha = lane_of(pp, 0);
+  o.pbeta = lane_of(pp, 1);
+  const float lp = log_lane(lane == 2 ? 1.0f - o.pbeta : pp);
+  const float l1 = log1p_lane(-pp);
+  o.to = lp - l1;
+  o.PL.l00 = lane_of(l1, 0);
+  o.PL.l10 = lane_of(lp, 0);
+  o.PL.l01 = lane_of(lp, 1);
+  o.PL.l11 = lane_of(l1, 1);
+  float r = __fadd_rn(ds.lg_ab, __fmul_rn(__fsub_rn(ds.bpa, 1.0f), o.PL.l01));
+  r = __fadd_rn(r, __fmul_rn(__fsub_rn(ds.bpb, 1.0f), lane_of(lp, 2)));
+  r = __fsub_rn(r, ds.lg_a);
+  o.pprior = __fsub_rn(r, ds.lg_b);
+  return o;
+}
+
+// Whether the proposed rates are accepted: the exact Metropolis-Hastings
+// ratio with the densities of the (preconditioned, optionally
+// gradient-drifted) Gaussian proposal both ways, up to their common constant.
+__device__ __forceinline__ bool accept_rates(const DatasetDev &ds,
+                                             const ModelDev &md,
+                                             const RateProposal &o,
+                                             float alpha, float beta,
+                                             float score, float pscore,
+                                             const float (&pe)[4], float u,
+                                             int lane) {
+  float pgrad, pprec;
+  rate_geometry(ds, o.palpha, o.pbeta, md.gamma, pe, lane, pgrad, pprec);
+  const float eps = md.error_step, e2 = eps * eps;
+  const float h = md.error_move == 2 ? 0.5f * eps * eps : 0.0f;
+  // squared distances over twice the variances, back and forth
+  const float rb = o.from - o.to - h * pprec * pgrad;
+  const float rf = o.to - o.from - h * o.prec * o.grad;
+  const float qb = (rb * rb) / (2.0f * e2 * pprec);
+  const float qf = (rf * rf) / (2.0f * e2 * o.prec);
+  // every logarithm at once: lanes 0-3 the Jacobian terms, 4-7 the
+  // preconditioners, 8 the acceptance level
+  const int side = lane & 1;
+  const float prec_s = lane_of(o.prec, side), pprec_s = lane_of(pprec, side);
+  const float pr = (lane & 2) ? (side ? o.pbeta : o.palpha)
+                              : (side ? beta : alpha);
+  const float x = lane < 4   ? pr * (1.0f - pr)
+                  : lane < 6 ? prec_s
+                  : lane < 8 ? pprec_s
+                             : u;
+  const float l = log_lane(x);
+  const float logj = lane_of(l, 0) + lane_of(l, 1);
+  const float plogj = lane_of(l, 2) + lane_of(l, 3);
+  const float log_qb = -lane_of(qb, 0) - lane_of(qb, 1) -
+                       0.5f * (lane_of(l, 6) + lane_of(l, 7));
+  const float log_qf = -lane_of(qf, 0) - lane_of(qf, 1) -
+                       0.5f * (lane_of(l, 4) + lane_of(l, 5));
+  const float logr =
+      md.gamma * (pscore - score) + plogj - logj + log_qb - log_qf;
+  return logr > lane_of(l, 8);
 }
 
 }  // namespace bbs

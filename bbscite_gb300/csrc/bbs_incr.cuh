@@ -1,0 +1,763 @@
+// bbs_incr.cuh -- proposals evaluated from what they change (rows of up to
+// four words).
+//
+// A tree move leaves most nodes' ancestor sets as they are; the others, two
+// disjoint classes of nodes, all change by the same genes, so every cell's
+// counts (d, m) change there by one constant per class and cell.  A chain
+// therefore keeps a table of every node and cell of its current tree in
+// shared memory and reads a proposal off it:
+//   - max score: the table holds integer codes that order a cell's nodes as
+//     their scores do (MaxCode), 16 bits per cell; a proposal's best nodes
+//     are the maxima over the unchanged nodes and the two shifted classes;
+//   - sum score: the table holds the counts.  A proposal is first bounded
+//     from above by the terms that move (two exponentials per class and
+//     cell); only one that the bound does not reject is summed, over the
+//     proposal's canonical order, term by term as everywhere else.
+// The rows, the parent vector and the table follow accepted moves only.
+// Decisions, scores and trees are those of an evaluation of every node.
+//
+// Measured against evaluating every node of every proposal (GB300, 1024
+// chains at 95 x 96 after 20,000 steps; 10-20 % of the proposals accepted):
+// max score 98 -> 307 M chain-steps/s, sum score with Langevin error moves
+// 121 -> 168 M; 128 uneven datasets of 32 chains 3.5 times as fast; 8 chains
+// at 63 x 64 6.4 -> 3.4 us a step.
+#pragma once
+#include "bbs_device.cuh"
+
+namespace bbs {
+
+// ------------------------------------------------------------------------
+// Integer codes of the max score
+// ------------------------------------------------------------------------
+// With fixed rates a cell's score at a node is, but for rounding, affine in
+// its counts: const + c1 d + c2 m with c1 = l01 - l00 and c2 = l11 - l10 of
+// opposite signs.  Two nodes compare as the ratio |c1| / |c2| compares with
+// a fraction (difference of m) / (difference of d), of which only finitely
+// many can occur.  Any weights with a ratio between the same two
+// neighbouring fractions al/bl < |c1|/|c2| < au/bu order all nodes alike;
+// their mediant P/Q is the smallest: T = s (Q m - P d) + off fits 16 bits
+// (P <= 2 mmax, Q <= 2 dmax, dmax and mmax the largest counts of a cell; at
+// most 4 x 127 x 127).  Different (d, m) give different T, and au Q - bu P =
+// 1 turns T back into (d, m).
+//   exact: no two counts of a cell lie so close that the rounding of the
+//          reference-order float score could tie or swap them, so the
+//          largest T is the reference's choice.  Otherwise its score is
+//          within `margin` of it, and only decides what `margin` leaves no
+//          doubt about.
+//   usable: the codes exist at all (rates with alpha + beta = 1 or
+//          non-finite logs have none).
+struct MaxCode {
+  int P, Q, s, au, bu, off;
+  uint32_t invP, invQ;  // floor(2^32 / P) + 1: exact quotients of x < 2^23
+  float margin;
+  bool usable, exact;
+};
+
+inline __device__ __noinline__ MaxCode make_code(float l00, float l01, float l10,
+                                          float l11, int dmax, int mmax,
+                                          int lane) {
+  MaxCode k;
+  const float c1 = l01 - l00, c2 = l11 - l10;
+  const float a1 = fabsf(c1), a2 = fabsf(c2);
+  k.s = c1 < 0.0f && c2 > 0.0f ? 1 : -1;
+  // rounding of two scores (four products and three sums each, all within
+  // `big`), of c1 and c2 and of the gaps below: 16 units of 2^-24 big
+  const float big = dmax * fmaxf(fabsf(l00), fabsf(l01)) +
+                    mmax * fmaxf(fabsf(l10), fabsf(l11));
+  k.margin = big * 1.9073486e-06f;  // 2^-19: twice that
+  k.usable = c1 * c2 < 0.0f && a1 > 1.0e-6f && a2 > 1.0e-6f && big < 1.0e6f;
+  bool exact = a1 > k.margin && a2 > k.margin;
+  // neighbours of a1 / a2 among the fractions a / b, b <= dmax, a <= mmax
+  int al = 0, bl = 1, au = 1, bu = 0;
+  if (k.usable) {
+    const float ratio = a1 / a2;
+    for (int b = lane + 1; b <= dmax; b += 32) {
+      int a = (int)fminf(floorf((float)b * ratio), (float)mmax);
+      const float x = (float)b * a1;
+      if (a < mmax && (float)(a + 1) * a2 - x <= k.margin) a++;
+      exact = exact && fabsf(x - (float)a * a2) > k.margin;
+      if (a * bl > al * b) {
+        al = a;
+        bl = b;
+      }
+      if (a < mmax && (a + 1) * bu < au * b) {
+        au = a + 1;
+        bu = b;
+      }
+    }
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    const int xa = __shfl_xor_sync(BBS_FULL_MASK, al, o),
+              xb = __shfl_xor_sync(BBS_FULL_MASK, bl, o),
+              ya = __shfl_xor_sync(BBS_FULL_MASK, au, o),
+              yb = __shfl_xor_sync(BBS_FULL_MASK, bu, o);
+    if (xa * bl > al * xb || (xa * bl == al * xb && xb < bl)) {
+      al = xa;
+      bl = xb;
+    }
+    if (ya * bu < au * yb || (ya * bu == au * yb && yb < bu)) {
+      au = ya;
+      bu = yb;
+    }
+  }
+  k.P = al + au;
+  k.Q = bl + bu;
+  if (k.P == 1) {  // decode divides by P > 1: the next weights in between
+    k.P += au;
+    k.Q += bu;
+  }
+  k.au = au;
+  k.bu = bu;
+  k.off = k.s > 0 ? k.P * dmax : k.Q * mmax;
+  // neighbours in lowest terms; near-ties sorted inconsistently are not
+  k.usable = k.usable && au * bl - al * bu == 1 &&
+             k.P * dmax + k.Q * mmax <= 65535;
+  k.exact = __all_sync(BBS_FULL_MASK, exact);
+  k.invP = 0xFFFFFFFFu / (uint32_t)k.P + 1u;
+  k.invQ = 0xFFFFFFFFu / (uint32_t)k.Q + 1u;
+  return k;
+}
+
+// (d, m) of a code: T0 = Q m - P d.  The solutions are (bu T0 - Q t,
+// au T0 - P t); with T0 >= 0 the smallest d >= 0 gives m >= 0, with T0 < 0
+// the smallest m >= 0 gives d > 0, and the next ones exceed the cell's bits.
+__device__ __forceinline__ void decode(const MaxCode &k, uint32_t T, int &d,
+                                       int &m) {
+  const int T0 = k.s * ((int)T - k.off);
+  const uint32_t a = (uint32_t)abs(T0);
+  const int t = T0 >= 0 ? (int)__umulhi((uint32_t)k.bu * a, k.invQ)
+                        : -(int)__umulhi((uint32_t)(k.au * (int)a + k.P - 1), k.invP);
+  d = k.bu * T0 - k.Q * t;
+  m = k.au * T0 - k.P * t;
+}
+
+// ------------------------------------------------------------------------
+// The table: entry [chunk][node][lane] of (Q + 1) / 2 words, 16 bits per
+// cell: off + wd d + wm m of the cell at the node.  Counts are off = 0, wd
+// = 1, wm = 256.  Chunk c holds the warp's cells from 32 wpc Q c on, as
+// load_cells takes them.
+// ------------------------------------------------------------------------
+// From the ancestor rows by masked popcounts (any rows): at the start of a
+// launch and after the rare moves that are not followed node by node.
+template <int W32, int Q>
+__device__ __noinline__ void fill_table(const uint32_t *rows,
+                                        const DatasetDev *ds, uint32_t *tab,
+                                        int chunks, int wpc, int wic,
+                                        int lane, int off, int wd, int wm) {
+  constexpr int RS = rs_of_w32(W32);
+  constexpr int NW = kPackWords<Q>;
+  const int n = ds->n_nodes;
+  for (int c = 0; c < chunks; c++) {
+    Cells<W32, Q> cb;
+    load_cells<W32, Q>(cb, *ds, 32 * (wpc * Q * c + wic), 32 * wpc, lane);
+#pragma unroll 1
+    for (int j = 0; j < n; j++) {
+      uint32_t a[W32], k[NW];
+      ld_row<W32>(rows + j * RS, a);
+#pragma unroll
+      for (int w = 0; w < NW; w++) k[w] = 0u;
+#pragma unroll
+      for (int q = 0; q < Q; q++)
+        k[q >> 1] += (uint32_t)(off + wd * masked_popc<W32>(cb.D[q], a) +
+                                wm * masked_popc<W32>(cb.M[q], a))
+                     << (16 * (q & 1));
+      st_pack<Q>(tab, (c * n + j) * 32 + lane, k);
+    }
+  }
+  __syncwarp();
+}
+
+// The same from the block's increment table, along a parents-first order
+// (canonical_order with the tree's parent vector): one chunk, each lane its
+// own column.
+template <int Q>
+__device__ __noinline__ void fill_table_inherit(const SumCtx sx, int n,
+                                                int lane, int off, int wd,
+                                                int wm) {
+  constexpr int NW = kPackWords<Q>;
+  {
+    uint32_t k[NW];
+#pragma unroll
+    for (int w = 0; w < NW; w++) k[w] = (uint32_t)off * 0x10001u;
+    st_pack<Q>(sx.cnt, (int)(sx.ord[0] & 0xFF) * 32 + lane, k);
+  }
+#pragma unroll 2
+  for (int i = 1; i < n; i++) {
+    const uint32_t o = sx.ord[i];
+    const int j = (int)(o & 0xFF), p = (int)(o >> 8);
+    uint32_t a[NW], g[NW];
+    ld_pack<Q>(sx.cnt, p * 32 + lane, a);
+    ld_pack<Q>(sx.inc, j * 32 + lane, g);
+#pragma unroll
+    for (int w = 0; w < NW; w++)
+      a[w] += (g[w] & 0x00010001u) * (uint32_t)wd +
+              ((g[w] >> 8) & 0x00010001u) * (uint32_t)wm;
+    st_pack<Q>(sx.cnt, j * 32 + lane, a);
+  }
+}
+
+// ------------------------------------------------------------------------
+// A realised tree move as two classes of changed nodes
+// ------------------------------------------------------------------------
+// Entries of class v change by T[a0] - T[b0], those of class w by T[a1] -
+// T[b1].  SwapNodes(v, w) changes the two classes by opposite amounts, +-
+// (T[a0] - T[b0] - T[a1] + T[b1]) with a1, b1 = v and its parent, a0, b0 = w
+// and its parent, and then exchanges the entries of v and w.
+struct Delta {
+  uint32_t v, w, a0, b0, a1, b1;
+  bool swap;
+};
+
+// select_bit without its branches: each lane ranks its own nodes.
+template <int W32>
+__device__ __forceinline__ uint32_t kth_bit(const uint32_t (&S)[W32],
+                                            uint32_t k, int lane) {
+  const uint32_t below = (1u << lane) - 1u;
+  uint32_t before = 0, result = 0;
+#pragma unroll
+  for (int r = 0; r < W32; r++) {
+    const bool hit = ((S[r] >> lane) & 1u) &&
+                     before + (uint32_t)__popc(S[r] & below) == k;
+    const uint32_t b = __ballot_sync(BBS_FULL_MASK, hit);
+    if (b) result = 32u * r + (uint32_t)(__ffs(b) - 1);
+    before += (uint32_t)__popc(S[r]);
+  }
+  return result;
+}
+
+// realize_move for a tree whose parent vector is known; what the move does
+// not use is not drawn.  `general`: a k-th (non)descendant beyond the count
+// (the reference's node-0 rule), a move of the root or of one node onto
+// itself: not expressed as classes.
+template <int W32>
+__device__ __forceinline__ bbs_move_params realize_classes(
+    const uint32_t *rows, const uint8_t *par, int n, const bbs_raw_move &raw,
+    int lane, uint32_t (&Dv)[W32], uint32_t (&Dw)[W32], bool &related,
+    bool &general, float &corr) {
+  constexpr int RS = rs_of_w32(W32);
+  bbs_move_params p;
+  uint32_t v = min(raw.raw_v, (uint32_t)(n - 1));
+  uint32_t w = min(raw.raw_w, (uint32_t)(n - 1));
+  // every load before the first use: is_ancestor(v, w), both parents and
+  // both descendant sets, exchanged afterwards where v is above w
+  const bool above = (rows[w * RS + (v >> 5)] >> (v & 31u)) & 1u;
+  const uint32_t pv = par[v], pw = par[w];
+  descendant_sets<W32>(rows, n, v, w, lane, Dv, Dw);
+  if (above) {
+    const uint32_t t = v;
+    v = w;
+    w = t;
+#pragma unroll
+    for (int r = 0; r < W32; r++) {
+      const uint32_t d = Dv[r];
+      Dv[r] = Dw[r];
+      Dw[r] = d;
+    }
+  }
+  p.parent_of_v = above ? pw : pv;
+  p.parent_of_w = above ? pv : pw;
+  p.move_type = raw.move_type;
+  p.v = v;
+  p.w = w;
+  p.descendant_of_v = p.nondescendant_of_v = 0;
+  p.new_beta = 0.0f;
+  related = has_bit<W32>(Dw, v);
+  general = v == w || w == (uint32_t)(n - 1) || v == (uint32_t)(n - 1);
+  int ndv = 0;
+#pragma unroll
+  for (int r = 0; r < W32; r++) ndv += __popc(Dv[r]);
+  if (raw.move_type == BBS_MOVE_PRUNE_REATTACH) {
+    const int nnd = n - ndv;
+    const uint32_t k = __float2uint_rz(
+        floorf(__fmul_rn(raw.raw_nondescendant_of_v, (float)nnd)));
+    uint32_t ND[W32];
+#pragma unroll
+    for (int r = 0; r < W32; r++) ND[r] = ~Dv[r] & group_mask(r, n);
+    p.nondescendant_of_v = kth_bit<W32>(ND, k, lane);
+    general = general || k >= (uint32_t)nnd;
+  } else if (raw.move_type == BBS_MOVE_SWAP_SUBTREES && related) {
+    int ndw = 0;
+#pragma unroll
+    for (int r = 0; r < W32; r++) ndw += __popc(Dw[r]);
+    const uint32_t k = __float2uint_rz(
+        floorf(__fmul_rn(raw.raw_descendant_of_v, (float)ndv)));
+    p.descendant_of_v = kth_bit<W32>(Dv, k, lane);
+    general = general || k >= (uint32_t)ndv;
+    corr = __fdiv_rn((float)ndv, (float)ndw);  // src/Application.hpp:443-450
+  }
+  return p;
+}
+
+// Two sets of nodes: the descendants of v and of w, or the two classes.
+template <int W32>
+struct NodeSets {
+  uint32_t v[W32], w[W32];
+};
+
+// The classes of a realised move (not a general one).
+template <int W32>
+__device__ __forceinline__ Delta move_classes(const bbs_move_params &p,
+                                              bool related,
+                                              const NodeSets<W32> &D,
+                                              NodeSets<W32> &C) {
+  Delta x;
+  const bool prune = p.move_type == BBS_MOVE_PRUNE_REATTACH;
+  x.swap = p.move_type == BBS_MOVE_SWAP_NODES;
+  x.v = p.v;
+  x.w = p.w;
+  x.b0 = x.b1 = p.parent_of_v;
+  x.a0 = prune ? p.nondescendant_of_v : p.parent_of_w;
+  x.a1 = p.descendant_of_v;
+  if (x.swap) {
+    x.a0 = p.w;
+    x.b0 = p.parent_of_w;
+    x.a1 = p.v;
+  } else if (!related) {
+    x.a1 = p.parent_of_v;
+    x.b1 = p.parent_of_w;
+  }
+#pragma unroll
+  for (int r = 0; r < W32; r++) {
+    C.v[r] = x.swap ? D.v[r] & ~D.w[r] : D.v[r];
+    C.w[r] = prune ? 0u : D.w[r] & ~D.v[r];
+  }
+  return x;
+}
+
+// The changed nodes as a list in shared memory, class v first: a loop over
+// it is one copy of its body, whatever the row width (the chain kernels are
+// bound by instruction fetch before anything else when their step code is
+// unrolled per row word).  nv: nodes of class v; returns the total.
+template <int W32>
+__device__ __forceinline__ int list_nodes(const NodeSets<W32> &C,
+                                          uint8_t *list, int lane, int &nv) {
+  const uint32_t below = (1u << lane) - 1u;
+  int at = 0;
+#pragma unroll
+  for (int r = 0; r < W32; r++) {
+    if ((C.v[r] >> lane) & 1u)
+      list[at + __popc(C.v[r] & below)] = (uint8_t)(32 * r + lane);
+    at += __popc(C.v[r]);
+  }
+  nv = at;
+#pragma unroll
+  for (int r = 0; r < W32; r++) {
+    if ((C.w[r] >> lane) & 1u)
+      list[at + __popc(C.w[r] & below)] = (uint8_t)(32 * r + lane);
+    at += __popc(C.w[r]);
+  }
+  __syncwarp();
+  return at;
+}
+
+// Packed differences by value.
+template <int NW>
+struct Packed {
+  uint32_t k[NW];
+};
+
+// The classes' changes as packed differences (their sum with an entry is the
+// new entry, field borrows included).
+template <int Q, int NW = kPackWords<Q>>
+__device__ __forceinline__ void class_deltas(const uint32_t *tab,
+                                             const Delta &x, int lane,
+                                             Packed<NW> &dv, Packed<NW> &dw) {
+  uint32_t a[NW], b[NW], c[NW], e[NW];
+  ld_pack<Q>(tab, (int)x.a0 * 32 + lane, a);
+  ld_pack<Q>(tab, (int)x.b0 * 32 + lane, b);
+  ld_pack<Q>(tab, (int)x.a1 * 32 + lane, c);
+  ld_pack<Q>(tab, (int)x.b1 * 32 + lane, e);
+#pragma unroll
+  for (int i = 0; i < NW; i++) {
+    dv.k[i] = a[i] - b[i];
+    dw.k[i] = c[i] - e[i];
+    if (x.swap) {
+      dv.k[i] -= dw.k[i];
+      dw.k[i] = 0u - dv.k[i];
+    }
+  }
+}
+
+// Adds the classes' changes to the table, or takes them back.
+template <int W32, int Q, int NW = kPackWords<Q>>
+__device__ __noinline__ void apply_classes(uint32_t *tab, uint8_t *list,
+                                           const Delta x,
+                                           const NodeSets<W32> C,
+                                           Packed<NW> dv, Packed<NW> dw,
+                                           bool back, int lane) {
+  auto swap_entries = [&]() {
+    uint32_t a[NW], b[NW];
+    ld_pack<Q>(tab, (int)x.v * 32 + lane, a);
+    ld_pack<Q>(tab, (int)x.w * 32 + lane, b);
+    st_pack<Q>(tab, (int)x.v * 32 + lane, b);
+    st_pack<Q>(tab, (int)x.w * 32 + lane, a);
+  };
+  if (back && x.swap) swap_entries();
+  int nv;
+  const int nc = list_nodes<W32>(C, list, lane, nv);
+  if (back) {
+#pragma unroll
+    for (int i = 0; i < NW; i++) {
+      dv.k[i] = 0u - dv.k[i];
+      dw.k[i] = 0u - dw.k[i];
+    }
+  }
+#pragma unroll 2
+  for (int c = 0; c < nc; c++) {
+    const int j = list[c];
+    uint32_t k[NW];
+    ld_pack<Q>(tab, j * 32 + lane, k);
+#pragma unroll
+    for (int i = 0; i < NW; i++) k[i] += c < nv ? dv.k[i] : dw.k[i];
+    st_pack<Q>(tab, j * 32 + lane, k);
+  }
+  if (!back && x.swap) swap_entries();
+  __syncwarp();  // the list has been read
+}
+
+// ------------------------------------------------------------------------
+// Max score: a proposal's largest codes
+// ------------------------------------------------------------------------
+// The largest code of each cell over the proposal's nodes: the unchanged
+// ones (the root is always one) and each class's largest, shifted.  list
+// holds the nc changed nodes, the first nv of class v.
+template <int W32, int Q, int NW = kPackWords<Q>>
+__device__ __forceinline__ void scan_codes(const uint32_t *tab, int n,
+                                           const NodeSets<W32> &C,
+                                           const uint8_t *list, int nv, int nc,
+                                           const Packed<NW> &dv,
+                                           const Packed<NW> &dw, int lane,
+                                           uint32_t (&best)[NW]) {
+  uint32_t un[W32], tv[NW], tw[NW];
+#pragma unroll
+  for (int r = 0; r < W32; r++) un[r] = ~(C.v[r] | C.w[r]) & group_mask(r, n);
+#pragma unroll
+  for (int i = 0; i < NW; i++) best[i] = tv[i] = tw[i] = 0u;
+#pragma unroll 1
+  for (int j = 0; j < n; j += 8) {
+    const uint32_t u = pick<W32>(un, (uint32_t)j >> 5) >> (j & 31);
+    const uint32_t *t = tab + j * 32 * NW;
+    uint32_t k[8][NW];
+    if (j + 8 <= n) {
+#pragma unroll
+      for (int b = 0; b < 8; b++) ld_pack<Q>(t, b * 32 + lane, k[b]);
+    } else {  // the last nodes: entry 0 of the group in place of the missing
+#pragma unroll
+      for (int b = 0; b < 8; b++)
+        ld_pack<Q>(t, (j + b < n ? b : 0) * 32 + lane, k[b]);
+    }
+#pragma unroll
+    for (int b = 0; b < 8; b++)
+      if ((u >> b) & 1u) {
+#pragma unroll
+        for (int i = 0; i < NW; i++) best[i] = __vmaxu2(best[i], k[b][i]);
+      }
+  }
+#pragma unroll 2
+  for (int c = 0; c < nv; c++) {
+    uint32_t k[NW];
+    ld_pack<Q>(tab, (int)list[c] * 32 + lane, k);
+#pragma unroll
+    for (int i = 0; i < NW; i++) tv[i] = __vmaxu2(tv[i], k[i]);
+  }
+#pragma unroll 2
+  for (int c = nv; c < nc; c++) {
+    uint32_t k[NW];
+    ld_pack<Q>(tab, (int)list[c] * 32 + lane, k);
+#pragma unroll
+    for (int i = 0; i < NW; i++) tw[i] = __vmaxu2(tw[i], k[i]);
+  }
+#pragma unroll
+  for (int i = 0; i < NW; i++) {
+    if (nv > 0) best[i] = __vmaxu2(best[i], tv[i] + dv.k[i]);
+    if (nc > nv) best[i] = __vmaxu2(best[i], tw[i] + dw.k[i]);
+  }
+}
+
+// ------------------------------------------------------------------------
+// Sum score
+// ------------------------------------------------------------------------
+// What the bound keeps of the current tree, for the lane's Q cells: the
+// exponents' offset, the sum of the terms and its reciprocal, and the
+// largest exponent (all against the reference the sum was taken against).
+template <int Q>
+struct CellSums {
+  float base[Q], z[Q], rz[Q], mx[Q];
+};
+
+// The second pass over the far-off cells of one cell slot (resum_cells'
+// terms in the same order), counts from the table.  One slot at a time, four
+// nodes' loads and exponentials in flight: what is left is the chain of
+// additions (a dataset whose rates leave one cell far below its bound takes
+// this pass in every evaluation).
+struct Resum1 {
+  float z, ed, em;
+};
+
+template <int Q>
+__device__ __noinline__ Resum1 resum_slot_table(const uint32_t *tab,
+                                                const uint16_t *ord, int n,
+                                                int lane, float c1, float c2,
+                                                float base, int q) {
+  constexpr int NW = kPackWords<Q>;
+  const uint32_t *t = tab + lane * NW + (q >> 1);
+  const uint32_t sd = (q & 1) ? 0x7542u : 0x7540u;
+  Resum1 o{0.0f, 0.0f, 0.0f};
+#pragma unroll 4
+  for (int i = 0; i < n; i++) {
+    const uint32_t k = t[(int)(ord[i] & 0xFF) * 32 * NW];
+    const float fd =
+        __int_as_float((int)__byte_perm(k, 0x4B000000u, sd)) - 8388608.0f;
+    const float fm =
+        __int_as_float((int)__byte_perm(k, 0x4B000000u, sd + 1u)) - 8388608.0f;
+    const float e = ex2_approx(fmaf(fd, c1, fmaf(fm, c2, base)));
+    o.z += e;
+    o.ed = fmaf(e, fd, o.ed);
+    o.em = fmaf(e, fm, o.em);
+  }
+  return o;
+}
+
+// sum_cells with the counts of every node in the table (sx.cnt) and the
+// tree's canonical order (sx.ord): the same terms in the same pairs and
+// order, so the same sums.  The table's entries are all in place before the
+// loop, so its loads wait for nothing but the order.
+template <int Q>
+__device__ __forceinline__ void sum_cells_table(
+    int n, const float (&pd)[Q], const float (&pm)[Q], const LogTable &L,
+    int c0, int stride, int lane, int n_cells, long long (&acc)[6],
+    const SumCtx &sx, CellSums<Q> &cs) {
+  constexpr int NW = kPackWords<Q>;
+  const float c1 = (L.l01 - L.l00) * kLog2E;
+  const float c2 = (L.l11 - L.l10) * kLog2E;
+  const float2 c1p = dup2(c1), c2p = dup2(c2);
+  const float u0 = fmaxf(L.l00, L.l01), u1 = fmaxf(L.l10, L.l11);
+  float r[Q], base[Q], mx[Q];
+  float2 base2[Q], z2[Q], ed2[Q], em2[Q];
+#pragma unroll
+  for (int q = 0; q < Q; q++) {
+    r[q] = fmaf(pd[q], u0, pm[q] * u1) - 72.0f;
+    base[q] = (fmaf(pd[q], L.l00, pm[q] * L.l10) - r[q]) * kLog2E;
+    base2[q] = dup2(base[q]);
+    mx[q] = base[q];  // the root has no counted bits
+    z2[q] = make_float2(ex2_approx(base[q]), 0.0f);
+    ed2[q] = em2[q] = make_float2(0.0f, 0.0f);
+  }
+  auto entry = [&](uint32_t o, uint32_t (&k)[NW]) {
+    ld_pack<Q>(sx.cnt, (int)(o & 0xFF) * 32 + lane, k);
+  };
+  int i = 1;
+  if (i + 1 < n) {
+    // the table's loads one pair ahead of the float work, the order's two
+    uint32_t kA0[NW], kA1[NW], kB0[NW], kB1[NW];
+    const uint16_t *ord = sx.ord;
+    const int last = n - 1;
+    entry(ord[i], kA0);
+    entry(ord[i + 1], kA1);
+    uint32_t o0 = ord[min(i + 2, last)], o1 = ord[min(i + 3, last)];
+#pragma unroll 1
+    for (; i + 5 < n; i += 4) {
+      entry(o0, kB0);
+      entry(o1, kB1);
+      o0 = ord[i + 4];
+      o1 = ord[i + 5];
+      sum_counts2<Q, NW>(kA0, kA1, c1p, c2p, base2, mx, z2, ed2, em2);
+      entry(o0, kA0);
+      entry(o1, kA1);
+      o0 = ord[min(i + 6, last)];
+      o1 = ord[min(i + 7, last)];
+      sum_counts2<Q, NW>(kB0, kB1, c1p, c2p, base2, mx, z2, ed2, em2);
+    }
+    sum_counts2<Q, NW>(kA0, kA1, c1p, c2p, base2, mx, z2, ed2, em2);
+    i += 2;
+    if (i + 1 < n) {
+      entry(o0, kB0);
+      entry(o1, kB1);
+      sum_counts2<Q, NW>(kB0, kB1, c1p, c2p, base2, mx, z2, ed2, em2);
+      i += 2;
+    }
+  }
+  if (i < n) {
+    uint32_t k[NW];
+    entry(sx.ord[i], k);
+#pragma unroll
+    for (int q = 0; q < Q; q++) {
+      const float fd = pack_d_biased(k[q >> 1], q) - 8388608.0f;
+      const float fm = pack_m_biased(k[q >> 1], q) - 8388608.0f;
+      const float t = fmaf(fd, c1, fmaf(fm, c2, base[q]));
+      const float e = ex2_approx(t);
+      mx[q] = fmaxf(mx[q], t);
+      z2[q].x += e;
+      ed2[q].x = fmaf(e, fd, ed2[q].x);
+      em2[q].x = fmaf(e, fm, em2[q].x);
+    }
+  }
+  float z[Q], ed[Q], em[Q];
+  bool bad[Q], any = false;
+#pragma unroll
+  for (int q = 0; q < Q; q++) {
+    z[q] = z2[q].x + z2[q].y;
+    ed[q] = ed2[q].x + ed2[q].y;
+    em[q] = em2[q].x + em2[q].y;
+    bad[q] = !(mx[q] >= -80.0f * kLog2E);
+    any |= bad[q];
+  }
+  if (__any_sync(BBS_FULL_MASK, any)) {
+#pragma unroll
+    for (int q = 0; q < Q; q++) {
+      if (!__any_sync(BBS_FULL_MASK, bad[q])) continue;
+      const Resum1 o = resum_slot_table<Q>(
+          sx.cnt, sx.ord, n, lane, c1, c2,
+          bad[q] ? base[q] - mx[q] : base[q], q);
+      if (bad[q]) {
+        r[q] = fmaf(mx[q], kLn2, r[q]);
+        base[q] -= mx[q];
+        mx[q] = 0.0f;
+        z[q] = o.z;
+        ed[q] = o.ed;
+        em[q] = o.em;
+      }
+    }
+  }
+#pragma unroll
+  for (int q = 0; q < Q; q++) {
+    const float inv = __frcp_rn(z[q]);
+    cs.base[q] = base[q];
+    cs.z[q] = z[q];
+    cs.rz[q] = inv;
+    cs.mx[q] = mx[q];
+    const int c = c0 + stride * q + lane;
+    if (c >= n_cells) continue;
+    const float Ed = ed[q] * inv, Em = em[q] * inv;
+    acc[0] += (long long)__float2int_rn((r[q] + logf(z[q])) * kScoreScale);
+    acc[2] += (long long)__float2int_rn(Ed * kFixScale);
+    acc[4] += (long long)__float2int_rn(Em * kFixScale);
+    acc[5] += (long long)__float2int_rn(fmaf(mx[q], kLn2, r[q]) * kScoreScale);
+  }
+}
+
+// The current tree's terms at the listed nodes: their sum and largest
+// exponent per cell, two nodes at a time.
+template <int Q, int NW = kPackWords<Q>>
+__device__ __forceinline__ void class_terms(const uint32_t *tab,
+                                            const uint8_t *list, int n_list,
+                                            float c1, float c2,
+                                            const float (&base)[Q], int lane,
+                                            float (&zo)[Q], float (&mo)[Q]) {
+  const float2 c1p = dup2(c1), c2p = dup2(c2);
+  float2 z2[Q];
+#pragma unroll
+  for (int q = 0; q < Q; q++) {
+    z2[q] = make_float2(0.0f, 0.0f);
+    mo[q] = -INFINITY;
+  }
+  uint32_t a0[NW], a1[NW];
+  ld_pack<Q>(tab, (int)list[0] * 32 + lane, a0);
+  ld_pack<Q>(tab, (int)list[n_list > 1 ? 1 : 0] * 32 + lane, a1);
+#pragma unroll 1
+  for (int c = 0; c < n_list; c += 2) {
+    // an odd last node is paired with itself; its copy's term is dropped
+    const bool two = c + 1 < n_list;
+    float2 fd[Q], fm[Q];
+    pack_to_float2<Q, NW>(a0, a1, fd, fm);
+    // the next pair's entries (the last loads again past the end)
+    ld_pack<Q>(tab, (int)list[min(c + 2, n_list - 1)] * 32 + lane, a0);
+    ld_pack<Q>(tab, (int)list[min(c + 3, n_list - 1)] * 32 + lane, a1);
+#pragma unroll
+    for (int q = 0; q < Q; q++) {
+      const float2 t = ffma2(fd[q], c1p, ffma2(fm[q], c2p, dup2(base[q])));
+      const float e1 = ex2_approx(t.y);
+      z2[q] = fadd2(z2[q], make_float2(ex2_approx(t.x), two ? e1 : 0.0f));
+      mo[q] = fmax3(mo[q], t.x, t.y);
+    }
+  }
+#pragma unroll
+  for (int q = 0; q < Q; q++) zo[q] = z2[q].x + z2[q].y;
+}
+
+// Exponent shift of cell slot q between two table entries a and b (their
+// signed count differences times c1 and c2).
+template <int NW>
+__device__ __forceinline__ float entry_shift(const uint32_t (&a)[NW],
+                                             const uint32_t (&b)[NW], int q,
+                                             float c1, float c2) {
+  const float dd = pack_d_biased(a[q >> 1], q) - pack_d_biased(b[q >> 1], q);
+  const float dm = pack_m_biased(a[q >> 1], q) - pack_m_biased(b[q >> 1], q);
+  return fmaf(dd, c1, dm * c2);
+}
+
+inline constexpr float kBoundUnit = 4096.0f;  // 2^-12 of a base-2 log
+
+// Upper bounds of a proposal's sum score and max score over this warp's
+// cells, relative to the current tree: up[0] bounds sum_c log2(z'_c / z_c),
+// up[1] bounds sum_c (largest exponent' - largest exponent), in units of
+// 1 / kBoundUnit.  eps bounds the relative rounding of a term against its
+// shifted form.  Sums of up to 128 terms are good to 2^-17 of the largest
+// partial sum, so a cell's remainder z - zo is taken with 2^-15 z on top.
+template <int Q, int NW = kPackWords<Q>>
+__device__ __forceinline__ void bound_proposal(
+    const uint32_t *tab, const Delta &x, const uint8_t *list, int nv, int nc,
+    const CellSums<Q> &cs, const LogTable &L, float eps, int c0, int stride,
+    int n_cells, int lane, int (&up)[2]) {
+  const float c1 = (L.l01 - L.l00) * kLog2E;
+  const float c2 = (L.l11 - L.l10) * kLog2E;
+  float hv[Q], hw[Q], z1[Q], gain[Q], rest[Q];
+  {
+    uint32_t a[NW], b[NW], c[NW], e[NW];
+    ld_pack<Q>(tab, (int)x.a0 * 32 + lane, a);
+    ld_pack<Q>(tab, (int)x.b0 * 32 + lane, b);
+    ld_pack<Q>(tab, (int)x.a1 * 32 + lane, c);
+    ld_pack<Q>(tab, (int)x.b1 * 32 + lane, e);
+#pragma unroll
+    for (int q = 0; q < Q; q++) {
+      hv[q] = entry_shift<NW>(a, b, q, c1, c2);
+      hw[q] = entry_shift<NW>(c, e, q, c1, c2);
+      if (x.swap) {
+        hv[q] -= hw[q];
+        hw[q] = -hv[q];
+      }
+      z1[q] = 0.0f;
+      gain[q] = -INFINITY;
+      rest[q] = cs.z[q];
+    }
+  }
+#pragma unroll 1
+  for (int cls = 0; cls < 2; cls++) {
+    const int at = cls ? nv : 0, count = cls ? nc - nv : nv;
+    if (count > 0) {
+      float zo[Q], mo[Q];
+      class_terms<Q>(tab, list + at, count, c1, c2, cs.base, lane, zo, mo);
+#pragma unroll
+      for (int q = 0; q < Q; q++) {
+        rest[q] -= zo[q];
+        // terms below 2^-126 were flushed to zero: at most 2^-118 together
+        z1[q] = fmaf(zo[q] + 3.0092655e-36f, ex2_approx(hv[q]), z1[q]);
+        gain[q] = fmaxf(gain[q], mo[q] + hv[q]);
+      }
+    }
+#pragma unroll
+    for (int q = 0; q < Q; q++) hv[q] = hw[q];
+  }
+  float s = 0.0f, g = 0.0f;
+#pragma unroll
+  for (int q = 0; q < Q; q++) {
+    const float left = fmaxf(rest[q], 0.0f) + 3.0517578e-05f * cs.z[q];
+    const float zu = fmaf(z1[q], 1.0f + eps, left);
+    // the largest exponent left is at most the current one and at most the
+    // logarithm of what is left of the sum
+    const float top = fmaxf(fminf(cs.mx[q], __log2f(left) + eps), gain[q] + eps);
+    if (c0 + stride * q + lane < n_cells) {
+      s += __log2f(zu * cs.rz[q]);
+      g += top - cs.mx[q];
+    }
+  }
+  // rounded up; beyond +-8000 per lane the sum saturates upwards (inf and
+  // NaN end there too: such a proposal is not rejected)
+  s = s < 8000.0f && g < 8000.0f ? fmaxf(s, -8000.0f) : 8000.0f;
+  g = g < 8000.0f ? fmaxf(g, -8000.0f) : 8000.0f;
+  up[0] = __reduce_add_sync(BBS_FULL_MASK, __float2int_ru(s * kBoundUnit) + 1);
+  up[1] = __reduce_add_sync(BBS_FULL_MASK, __float2int_ru(g * kBoundUnit) + 1);
+}
+
+}  // namespace bbs

@@ -21,15 +21,13 @@ __host__ __device__ constexpr int rs_of_w32(int w32) {
   return 2 * ((w32 + 1) / 2);
 }
 __host__ __device__ constexpr int w32_of_nodes(int n) { return (n + 31) / 32; }
-// Chains inherit counts from the parent (max or sum score):
-//   - rows of up to four words, when all their cells stay in registers (at
-//     most cells_per_pass = 32 x cells per lane x warps per chain): the
-//     block's increment tables and each warp's count table of every node
-//     exist then;
-//   - rows of five to eight words, always: each warp keeps a ring of the
-//     counts of the last kRing nodes in the canonical order and a gene
-//     table of the cells it is scoring, rebuilt per chunk of streamed
-//     cells.
+// Rows of five to eight words inherit counts from the parent: each warp
+// keeps a ring of the counts of the last kRing nodes in the canonical order
+// and a gene table of the cells it is scoring, rebuilt per chunk of streamed
+// cells.  Rows of up to four words keep a table of every node where it fits
+// (TablePlan in bbs_layout.h), with the block's increment tables when a
+// chain's cells take one pass (at most cells_per_pass = 32 x cells per lane
+// x warps per chain).
 inline constexpr int kRing = 64;
 __host__ __device__ constexpr bool inherits_counts(int w32, int n_cells,
                                                    int cells_per_pass) {
@@ -49,6 +47,7 @@ struct DatasetDev {
   const uint32_t *M;  // mutated rows [n_cells][RS], pre-masked with K
   int n_cells, n_nodes;
   int sum_k, sum_m;   // sum over cells of popc(K), popc(M)
+  int max_d, max_m;   // largest popc(K & ~M) and popc(M) of a cell
   float l00, l10;     // log(1-alpha), log(alpha) of alpha_mean
                       // (src/TreeScorer.hpp:99-106)
   float bpa, bpb;     // Beta prior parameters (src/TreeScorer.hpp:108-111)
@@ -106,6 +105,8 @@ struct RunArgs {
   const volatile int *cancel; // host-writable flag (mapped) or null
   int *status;                // device status word (0 = ok, 1 = cancelled)
   int wpc;                    // warps per chain (cells split over them)
+  int chunks;                 // table of every node (TablePlan); 0: none
+  int with_inc;               // 1: increment tables after the slots
 };
 
 // Many datasets in one launch: chains are listed by unit (chain index in
@@ -126,11 +127,8 @@ struct BatchArgs {
   int *status;
   int max_nodes;             // shared memory is sized for this
   int table_ds;              // the launch's only dataset, or -1
-  int with_counts;           // 1: the chains inherit counts (rows of up to
-                             // four words, one dataset whose cells stay in
-                             // registers; wider rows always); shared memory
-                             // holds the count and increment tables, or
-                             // the rings and gene tables, only then
+  int chunks;                // table of every node (TablePlan); 0: none
+  int with_inc;              // 1: increment tables (one dataset only)
   int wpc;                   // warps per chain: 1 (blocks of one-warp
                              // chains), or 2-4 (a block is one chain)
 };
@@ -197,12 +195,15 @@ struct GradArgs {
   float *posterior;  // [n_trees][n_cells][n_nodes] or null
 };
 
-// Host launchers (bbs_aux.cu, bbs_mcmc_*.cu).  Return a cudaError_t as int.
+// Host launchers (bbs_aux.cu, bbs_mcmc.cu, bbs_batch.cu).  Return a cudaError_t as int.
 // chains_per_block must be 1 when a.wpc > 1 (the block is one chain).
+// smem_block: the dynamic shared memory a block may have; max_cells: the
+// cells of the launch's largest dataset.  The plan of the table (chunks,
+// with_inc) is made here.
 int launch_mcmc(const RunArgs &a, int q, int chains_per_block, int n_sms,
-                void *stream);
-int launch_batch(const BatchArgs &b, int w32, int q, bool sum,
-                 int warps_per_block, int n_sms, void *stream);
+                int smem_block, void *stream);
+int launch_batch(const BatchArgs &b, int w32, int max_cells, int q, bool sum,
+                 int warps_per_block, int n_sms, int smem_block, void *stream);
 // Launch groups: every chain of a launch must store its rows with the
 // stride rs_of_w32(w32) of the launch (w32 at least the chains' own).
 int launch_init(const InitArgs &a, int w32, bool sum, void *stream);

@@ -15,6 +15,7 @@
 #include <cmath>
 
 #include "bbs_device.cuh"
+#include "bbs_incr.cuh"
 
 namespace bbs {
 
@@ -68,6 +69,17 @@ __host__ __device__ __forceinline__ SlotSum slot_sum(uint8_t *slot, int n,
   return o;
 }
 
+// Warp wic's part of the table of a slot without increments
+// (table_slot_bytes).
+__host__ __device__ __forceinline__ uint32_t *table_part(uint8_t *slot, int n,
+                                                         int rs, int wpc,
+                                                         int wic, int w32,
+                                                         int q, int chunks) {
+  return reinterpret_cast<uint32_t *>(
+      slot + slot_bytes(n, rs, wpc, true, w32, q, false) +
+      wic * table_part_bytes(n, q, chunks));
+}
+
 // The block's increment tables: for warp part wic of wpc and lane l, the
 // cells c = 32 wic + 32 wpc q + l (q < Q; zero past the dataset's cells),
 // as load_cells takes them; gene j's entry packs D bit | M bit << 8 of each
@@ -102,62 +114,87 @@ __device__ __forceinline__ void build_increments(uint8_t *table, int wpc,
   }
 }
 
-// Evaluates a tree for the whole chain (all wpc warps): returns the score
-// S = data term + prior and the (exact or expected) class counts e[4];
-// sk, sm are the class sums of the max score and smax the max score itself
-// (S for the max score; for the sum score, sum_c max_j s_cj + prior).
+// An evaluated tree: the score S = data term + prior, the (exact or
+// expected) class counts e[4], the class sums sk and sm of the max score and
+// the max score itself (S for the max score; for the sum score, sum_c max_j
+// s_cj + prior).
+struct Evaluated {
+  float score, smax;
+  float e[4];
+  int sk, sm;
+};
+
+// The chain's class sums from its warps' (one block barrier when wpc > 1).
+__device__ __forceinline__ Evaluated finish_max(const DatasetDev &ds,
+                                                const LogTable &L, float prior,
+                                                int a, int b, int wpc, int wic,
+                                                int lane, int *part,
+                                                int parity) {
+  if (wpc > 1) {
+    int *pp = part + parity * 12 * wpc;
+    if (lane == 0) {
+      pp[12 * wic] = a;
+      pp[12 * wic + 1] = b;
+    }
+    __syncthreads();
+    a = b = 0;
+    for (int w = 0; w < wpc; w++) {
+      a += pp[12 * w];
+      b += pp[12 * w + 1];
+    }
+  }
+  Evaluated o;
+  o.sk = a;
+  o.sm = b;
+  int N[4];
+  class_totals(ds, a, b, N);
+#pragma unroll
+  for (int i = 0; i < 4; i++) o.e[i] = (float)N[i];
+  o.score = o.smax = tree_score(ds, a, b, L, prior);
+  return o;
+}
+
+// The same for the sum score's fixed-point sums.
+__device__ __forceinline__ Evaluated finish_sum(const DatasetDev &ds,
+                                                float prior,
+                                                long long (&acc)[6], int wpc,
+                                                int wic, int lane, int *part,
+                                                int parity) {
+  if (wpc > 1) {
+    long long *pp = reinterpret_cast<long long *>(part) + parity * 6 * wpc;
+    if (lane == 0)
+      for (int i = 0; i < 6; i++) pp[6 * wic + i] = acc[i];
+    __syncthreads();
+    for (int i = 0; i < 6; i++) acc[i] = 0;
+    for (int w = 0; w < wpc; w++)
+      for (int i = 0; i < 6; i++) acc[i] += pp[6 * w + i];
+  }
+  complete_expected_counts(ds, acc);
+  Evaluated o;
+  o.sk = o.sm = 0;
+#pragma unroll
+  for (int i = 0; i < 4; i++) o.e[i] = ll_to_float(acc[i + 1]) * (1.0f / kFixScale);
+  o.smax = __fadd_rn(ll_to_float(acc[5]) * (1.0f / kScoreScale), prior);
+  o.score = __fadd_rn(ll_to_float(acc[0]) * (1.0f / kScoreScale), prior);
+  return o;
+}
+
+// Evaluates a tree for the whole chain (all wpc warps) from its rows.
 template <int W32, int Q, bool SUM>
-__device__ __forceinline__ float evaluate(const uint32_t *rows, int n,
-                                          const DatasetDev &ds,
-                                          Cells<W32, Q> &cb, bool resident,
-                                          const LogTable &L, float prior,
-                                          int wpc, int wic, int lane,
-                                          int *part, int parity,
-                                          const SumCtx &sx,
-                                          float (&e)[4], int &sk, int &sm,
-                                          float &smax) {
+__device__ __forceinline__ Evaluated evaluate(const uint32_t *rows, int n,
+                                              const DatasetDev &ds,
+                                              const LogTable &L, float prior,
+                                              int wpc, int wic, int lane,
+                                              int *part, int parity,
+                                              const SumCtx &sx) {
   if constexpr (!SUM) {
     int a, b;
-    score_part<W32, Q>(rows, n, ds, cb, resident, L, wpc, wic, lane, a, b, sx);
-    if (wpc > 1) {
-      int *pp = part + parity * 12 * wpc;
-      if (lane == 0) {
-        pp[12 * wic] = a;
-        pp[12 * wic + 1] = b;
-      }
-      __syncthreads();
-      a = b = 0;
-      for (int w = 0; w < wpc; w++) {
-        a += pp[12 * w];
-        b += pp[12 * w + 1];
-      }
-    }
-    sk = a;
-    sm = b;
-    int N[4];
-    class_totals(ds, sk, sm, N);
-#pragma unroll
-    for (int i = 0; i < 4; i++) e[i] = (float)N[i];
-    smax = tree_score(ds, sk, sm, L, prior);
-    return smax;
+    score_part<W32, Q>(rows, n, ds, L, wpc, wic, lane, a, b, sx);
+    return finish_max(ds, L, prior, a, b, wpc, wic, lane, part, parity);
   } else {
     long long acc[6];
-    sum_part<W32, Q>(rows, n, ds, cb, resident, L, wpc, wic, lane, acc, sx);
-    if (wpc > 1) {
-      long long *pp = reinterpret_cast<long long *>(part) + parity * 6 * wpc;
-      if (lane == 0)
-        for (int i = 0; i < 6; i++) pp[6 * wic + i] = acc[i];
-      __syncthreads();
-      for (int i = 0; i < 6; i++) acc[i] = 0;
-      for (int w = 0; w < wpc; w++)
-        for (int i = 0; i < 6; i++) acc[i] += pp[6 * w + i];
-    }
-    complete_expected_counts(ds, acc);
-    sk = sm = 0;
-#pragma unroll
-    for (int i = 0; i < 4; i++) e[i] = ll_to_float(acc[i + 1]) * (1.0f / kFixScale);
-    smax = __fadd_rn(ll_to_float(acc[5]) * (1.0f / kScoreScale), prior);
-    return __fadd_rn(ll_to_float(acc[0]) * (1.0f / kScoreScale), prior);
+    sum_part<W32, Q>(rows, n, ds, L, wpc, wic, lane, acc, sx);
+    return finish_sum(ds, prior, acc, wpc, wic, lane, part, parity);
   }
 }
 
@@ -172,26 +209,24 @@ __device__ __forceinline__ void run_chain(
     const bbs_raw_move *moves, bbs_step_trace *trace, int n_steps,
     const volatile int *cancel, int *status, uint32_t *buf0, uint32_t *buf1,
     int *part, volatile int *sflag, uint4 *pbuf, const SlotSum &ss,
-    Cells<W32, Q> &cb, bool resident, int wpc, int wic, int lane) {
+    int wpc, int wic, int lane) {
   const int n = ds.n_nodes;
   const bool multi = wpc > 1;
   const ChainState st = *gstate;
   copy_rows_part<W32>(g, buf0, n, wpc, wic, lane);
   if (multi) __syncthreads(); else __syncwarp();
   uint32_t *cur = buf0, *prop = buf1;
-  // Inherited counts (rows of up to four words): the parent vectors of the
-  // current tree and of the proposal follow the rows.  A parent vector is
-  // used only after it has been checked against its rows: a realised move
-  // whose k-th (non)descendant fell back to node 0 (the reference's rule
-  // when floor(u * count) reaches the count) changes the rows in a way the
-  // parent-vector form does not follow, and may leave rows that are no tree.
-  // Such trees are scored with masked popcounts, which take any rows.
-  // Rows of five to eight words inherit through the ring, which needs the
-  // parent vectors too (any cells, resident or streamed).
+  // Rows of five to eight words inherit their counts through the ring, which
+  // needs the parent vectors of the current tree and of the proposal.  A
+  // parent vector is used only after it has been checked against its rows: a
+  // realised move whose k-th (non)descendant fell back to node 0 (the
+  // reference's rule when floor(u * count) reaches the count) changes the
+  // rows in a way the parent-vector form does not follow, and may leave rows
+  // that are no tree.  Such trees, and streamed cells of narrower rows, are
+  // scored with masked popcounts, which take any rows.
   uint8_t *cpar = nullptr, *ppar = nullptr;
   bool cur_par_ok = false;  // cpar describes cur
-  const bool track = W32 <= 4 ? ss.sx.inc != nullptr && resident
-                              : ss.sx.ring != nullptr;
+  const bool track = W32 > 4 && ss.sx.ring != nullptr;
   if (track) {
     cpar = ss.par0;
     ppar = ss.par1;
@@ -241,8 +276,7 @@ __device__ __forceinline__ void run_chain(
     LogTable PL = L;
     const uint32_t *scored = cur;
     float corr = 1.0f;
-    float fa = 0.0f, fb = 0.0f, ta = 0.0f, tb = 0.0f;
-    ErrorGeom geo{};  // of the current state, on learned error moves
+    RateProposal rates{};  // learned error moves
     bool fallback_move = false;  // the realised move took node 0 by fallback
     uint32_t Dv[W32], Dw[W32];
     if (!err_move) {
@@ -273,21 +307,11 @@ __device__ __forceinline__ void run_chain(
     } else {
       // (preconditioned) random walk or Langevin step in logit space, with
       // the geometry of the current state from its class counts
-      geo = error_geometry(ds, alpha, beta, md.gamma, ec);
-      float z0, z1;
-      error_normals(raw, z0, z1);
-      const float eps = md.error_step;
-      const float h = md.error_move == 2 ? 0.5f * eps * eps : 0.0f;
-      fa = logit(alpha);
-      fb = logit(beta);
-      ta = fa + h * geo.prec_a * geo.grad_a + eps * sqrtf(geo.prec_a) * z0;
-      tb = fb + h * geo.prec_b * geo.grad_b + eps * sqrtf(geo.prec_b) * z1;
-      palpha = fminf(fmaxf(sigmoid(ta), 1.0e-7f), 1.0f - 1.0e-7f);
-      pbeta = fminf(fmaxf(sigmoid(tb), 1.0e-7f), 1.0f - 1.0e-7f);
-      ta = logit(palpha);
-      tb = logit(pbeta);
-      alpha_terms_f(palpha, PL.l00, PL.l10);
-      beta_terms_f(ds, pbeta, PL.l01, PL.l11, pprior);
+      rates = propose_rates(ds, md, alpha, beta, ec, raw, lane);
+      palpha = rates.palpha;
+      pbeta = rates.pbeta;
+      pprior = rates.pprior;
+      PL = rates.PL;
     }
     if (multi) __syncthreads(); else __syncwarp();
     // The evaluated tree's parent vector.  It is checked against the rows
@@ -315,22 +339,15 @@ __device__ __forceinline__ void run_chain(
     }
     sx.par = par_ok ? (scored == cur ? cpar : ppar) : nullptr;
     const bool prop_par_ok = par_ok && scored != cur;
-    float e[4], psmax;
-    int sk, sm;
-    const float pscore = evaluate<W32, Q, SUM>(scored, n, ds, cb, resident, PL,
-                                               pprior, wpc, wic, lane, part,
-                                               i & 1, sx, e, sk, sm, psmax);
+    const Evaluated ev = evaluate<W32, Q, SUM>(scored, n, ds, PL, pprior, wpc,
+                                               wic, lane, part, i & 1, sx);
+    const float pscore = ev.score, psmax = ev.smax;
+    const float (&e)[4] = ev.e;
+    const int sk = ev.sk, sm = ev.sm;
     bool accept;
     if (err_move && learn) {
-      const ErrorGeom pgeo = error_geometry(ds, palpha, pbeta, md.gamma, e);
-      const float logj = logf(alpha * (1.0f - alpha)) + logf(beta * (1.0f - beta));
-      const float plogj =
-          logf(palpha * (1.0f - palpha)) + logf(pbeta * (1.0f - pbeta));
-      const bool drift = md.error_move == 2;
-      const float logr = md.gamma * (pscore - score) + plogj - logj +
-                         log_q(fa, fb, ta, tb, pgeo, md.error_step, drift) -
-                         log_q(ta, tb, fa, fb, geo, md.error_step, drift);
-      accept = logr > logf(raw.acceptance_level);
+      accept = accept_rates(ds, md, rates, alpha, beta, score, pscore, e,
+                            raw.acceptance_level, lane);
       err_prop++;
       if (accept) err_acc++;
     } else {
@@ -452,6 +469,471 @@ __device__ __forceinline__ void run_chain(
   if (multi) __syncthreads(); else __syncwarp();
 }
 
+// A tree scored from its rows, off the hot path: proposals that are not
+// followed node by node, and error moves of the max score.
+template <int W32, int Q, bool SUM>
+__device__ __noinline__ Evaluated evaluate_rows(const uint32_t *rows,
+                                                const DatasetDev *ds,
+                                                const LogTable L, float prior,
+                                                int wpc, int wic, int lane,
+                                                int *part, int parity,
+                                                SumCtx sx) {
+  sx.par = nullptr;
+  return evaluate<W32, Q, SUM>(rows, ds->n_nodes, *ds, L, prior, wpc, wic,
+                               lane, part, parity, sx);
+}
+
+// A proposal's rows and, for a tree whose parent vector is known, its parent
+// vector: off the path of rejected proposals.
+template <int W32>
+__device__ __noinline__ void propose_tree(const uint32_t *cur, uint32_t *prop,
+                                          const uint8_t *cpar, uint8_t *ppar,
+                                          int n, const bbs_move_params p,
+                                          const NodeSets<W32> D, bool related,
+                                          bool tree_ok, int wpc, int wic,
+                                          int lane) {
+  build_proposal<W32>(cur, prop, n, p, D.v, D.w, related, wpc, wic, lane);
+  if (tree_ok && wic == 0) propose_parents(cpar, ppar, n, p, related, lane);
+  if (wpc > 1) __syncthreads(); else __syncwarp();
+}
+
+// run_chain with the table of bbs_incr.cuh in ss.sx.cnt (rows of up to four
+// words; `chunks` chunks of the warp's cells, one for the sum score).
+// Bound at 95 x 96 (1024 one-warp chains, 1.8 warps per scheduler) by the
+// latency of one step's serial chain -- draw, descendant sets, table loads,
+// reductions -- no longer by the node loop's instructions.
+template <int W32, int Q, bool SUM>
+__device__ __forceinline__ void run_chain_table(
+    const DatasetDev &ds, const ModelDev &md, uint32_t chain_id,
+    uint32_t *g, uint32_t *gbest, uint64_t *lhash, float *lbeta, int K,
+    ChainState *gstate, const bbs_raw_move *moves, bbs_step_trace *trace,
+    int n_steps, const volatile int *cancel, int *status, uint32_t *buf0,
+    uint32_t *buf1, int *part, volatile int *sflag, uint4 *pbuf,
+    const SlotSum &ss, int chunks, int wpc, int wic, int lane) {
+  constexpr int NW = kPackWords<Q>;
+  const int n = ds.n_nodes;
+  const bool multi = wpc > 1;
+  const int stride = 32 * wpc, c0 = 32 * wic;
+  const ChainState st = *gstate;
+  copy_rows_part<W32>(g, buf0, n, wpc, wic, lane);
+  if (multi) __syncthreads(); else __syncwarp();
+  uint32_t *cur = buf0, *prop = buf1;
+  uint8_t *cpar = ss.par0, *ppar = ss.par1;
+  uint32_t *const tab = ss.sx.cnt;
+  float alpha = st.alpha, beta = st.beta, score = st.score, prior = st.prior;
+  LogTable L{st.l00, st.l10, st.l01, st.l11};
+  float ec[4] = {st.ec[0], st.ec[1], st.ec[2], st.ec[3]};
+  int csk = st.sk, csm = st.sm;
+  bool has_best = st.has_best != 0;
+  float best_score = st.best_score, best_alpha = st.best_alpha,
+        best_beta = st.best_beta;
+  int bsk = st.best_sk, bsm = st.best_sm;
+  uint32_t err_prop = st.err_proposed, err_acc = st.err_accepted;
+  uint32_t lcount = st.list_count;
+  const bool learn = md.error_move != 0;
+  // the current tree's parent vector holds (its rows are a tree, and the
+  // table and, for the sum score, the order and cell sums follow it)
+  bool tree_ok = false;
+  bool ord_ok = false;  // ss.sx.ord is the current tree's order
+  MaxCode code{};
+  CellSums<Q> cs;
+  float pd[Q], pm[Q];
+  float smax = 0.0f, eps = 0.0f, slack = 0.0f;  // of the sum score's bound
+  if constexpr (SUM) {
+    Cells<W32, Q> cb;
+    load_cells<W32, Q>(cb, ds, c0, stride, lane);
+#pragma unroll
+    for (int q = 0; q < Q; q++) {
+      pd[q] = cb.pdb[q] - 8388608.0f;
+      pm[q] = cb.pmb[q] - 8388608.0f;
+    }
+  }
+  // The bound's tolerances for the current rates.  Exponents lie within
+  // 1.45 n_genes max|l| + 105 in size and carry a few roundings each; a
+  // cell's stored terms are rounded to 2^-16 and at their own size.
+  auto tolerances = [&]() {
+    const float big =
+        (float)n * fmaxf(fmaxf(fabsf(L.l00), fabsf(L.l01)),
+                         fmaxf(fabsf(L.l10), fabsf(L.l11))) + 73.0f;
+    eps = big * 2.3841858e-06f;  // 10 roundings of twice 2^-24 big / ln 2
+    slack = (float)ds.n_cells * fmaf(big, 4.7683716e-07f, 3.0517578e-05f);
+  };
+  // Set at the start and after an accepted tree that was not followed node
+  // by node: the parent vector (where the rows are a tree), the codes and the
+  // table anew from the rows; and, for the max score, after accepted rates
+  // (the codes and the table).
+  bool fresh_rows = true, fresh_table = true;
+  uint8_t *const list = reinterpret_cast<uint8_t *>(ss.sx.hist);
+  int i = 0;
+  bool cancelled = false;
+  while (i < n_steps) {
+    const bool fresh = fresh_table;
+    bool err_move = false;
+    bbs_raw_move raw{};
+    if (!fresh) {
+      if (cancel != nullptr && (i & 255) == 0) {
+        if (wic == 0 && lane == 0) *sflag = *cancel;
+        if (multi) __syncthreads(); else __syncwarp();
+        const int c = *sflag;
+        if (multi) __syncthreads(); else __syncwarp();
+        if (c) {
+          cancelled = true;
+          break;
+        }
+      }
+      if (moves == nullptr && (i & 15) == 0) {
+        philox_fill(pbuf, md.seed, chain_id, st.steps_done + (uint64_t)i, lane);
+        __syncwarp();
+      }
+      raw = moves != nullptr
+                ? moves[i]
+                : move_from_words(md.mp, (uint32_t)n, pbuf[2 * (i & 15)],
+                                  pbuf[2 * (i & 15) + 1], trace != nullptr);
+      err_move = raw.move_type == BBS_MOVE_CHANGE_BETA;
+    }
+    float palpha = alpha, pbeta = beta, pprior = prior;
+    LogTable PL = L;
+    float corr = 1.0f;
+    RateProposal rates{};  // learned error moves
+    Evaluated ev;
+    CellSums<Q> pcs;
+    NodeSets<W32> D, C;
+    Packed<NW> dv{}, dw{};
+    Delta delta{};
+    bbs_move_params mp{};
+    bool related = false;
+    bool classes = false;    // the proposal is described by classes
+    bool built = false;      // prop holds the proposal's rows
+    bool applied = false;    // the table holds the proposal's counts
+    bool from_rows = false;  // scored from its rows
+    bool from_table = false; // summed over the table in the order of
+    const uint32_t *order = nullptr;  // these rows (null: sx.ord holds it)
+    if (fresh) {
+      if (fresh_rows) {
+        if (multi) __syncthreads(); else __syncwarp();
+        if (wic == 0) derive_parents<W32>(cur, n, cpar, ss.sx.hist, lane);
+        if (multi) __syncthreads(); else __syncwarp();
+        tree_ok = parents_match_rows<W32>(cur, n, cpar, lane);
+      }
+      fresh_rows = fresh_table = false;
+      if constexpr (!SUM)
+        code = make_code(L.l00, L.l01, L.l10, L.l11, ds.max_d, ds.max_m, lane);
+      else
+        tolerances();
+      if (!tree_ok || (!SUM && !code.usable)) continue;
+      from_table = SUM;
+      order = cur;
+    } else if (!err_move) {
+      bool general = true;
+      if (tree_ok) {
+        mp = realize_classes<W32>(cur, cpar, n, raw, lane, D.v, D.w, related,
+                                  general, corr);
+      }
+      if constexpr (!SUM) general = general || !code.usable;
+      if (general) {
+        corr = 1.0f;
+        const Realized R = realize_move<W32>(cur, n, beta, raw, lane, D.v, D.w);
+        mp = R.p;
+        related = R.related;
+        if (raw.move_type == BBS_MOVE_SWAP_SUBTREES && R.related)
+          corr = __fdiv_rn((float)R.ndv, (float)R.ndw);
+      }
+      const uint32_t top = max(max(max(mp.v, mp.w), max(mp.parent_of_v, mp.parent_of_w)),
+                               max(mp.descendant_of_v, mp.nondescendant_of_v));
+      if (!device_check(top < (uint32_t)n, status, kCheckMoveNode, top, (uint32_t)n)) {
+        cancelled = true;  // the chain stops where it is
+        break;
+      }
+      classes = !general;
+      from_rows = general;
+    } else if (!learn) {
+      // reference ChangeBeta (src/MutationTree.hpp:345-351)
+      float nb = __fadd_rn(beta, raw.beta_jump);
+      if (nb < 0.0f) nb = fabsf(nb);
+      if (nb > 1.0f) nb = __fsub_rn(nb, __fmul_rn(2.0f, __fsub_rn(nb, 1.0f)));
+      pbeta = nb;
+      beta_terms(ds, pbeta, PL.l01, PL.l11, pprior);
+    } else {
+      rates = propose_rates(ds, md, alpha, beta, ec, raw, lane);
+      palpha = rates.palpha;
+      pbeta = rates.pbeta;
+      pprior = rates.pprior;
+      PL = rates.PL;
+    }
+    if (classes) {
+      delta = move_classes<W32>(mp, related, D, C);
+      class_deltas<Q>(tab, delta, lane, dv, dw);
+      int nv;
+      const int nc = list_nodes<W32>(C, list, lane, nv);
+      if constexpr (!SUM) {
+        int sk = 0, sm = 0;
+        for (int c = 0; c < chunks; c++) {
+          const uint32_t *t = tab + c * n * 32 * NW;
+          uint32_t best[NW];
+          if (c > 0) class_deltas<Q>(t, delta, lane, dv, dw);
+          scan_codes<W32, Q>(t, n, C, list, nv, nc, dv, dw, lane, best);
+#pragma unroll
+          for (int q = 0; q < Q; q++) {
+            int d, m;
+            decode(code, pack_field<NW>(best, q), d, m);
+            sk += d + m;
+            sm += m;
+          }
+        }
+        sk = __reduce_add_sync(BBS_FULL_MASK, sk);
+        sm = __reduce_add_sync(BBS_FULL_MASK, sm);
+        ev = finish_max(ds, L, prior, sk, sm, wpc, wic, lane, part, i & 1);
+        if (!code.exact) {
+          // the codes' choice is within the margin per cell of the
+          // reference's: enough to reject, otherwise score the rows
+          const float tol = fmaf((float)ds.n_cells, code.margin,
+                                 fabsf(ev.score) * 1.0e-6f + 1.0e-3f);
+          const float up = ev.score + tol;
+          from_rows = !(trace == nullptr && md.gamma > 0.0f && has_best &&
+                        up < best_score &&
+                        corr * expf((up - score) * md.gamma) * 1.001f <
+                            raw.acceptance_level);
+        }
+      } else {
+        if (trace == nullptr && md.gamma > 0.0f && has_best) {
+          int up[2];
+          bound_proposal<Q>(tab, delta, list, nv, nc, cs, L, eps, c0, stride,
+                            ds.n_cells, lane, up);
+          if (multi) {
+            int *pp = part + (i & 1) * 12 * wpc;
+            if (lane == 0) {
+              pp[12 * wic] = up[0];
+              pp[12 * wic + 1] = up[1];
+            }
+            __syncthreads();
+            up[0] = up[1] = 0;
+            for (int w = 0; w < wpc; w++) {
+              up[0] += pp[12 * w];
+              up[1] += pp[12 * w + 1];
+            }
+          }
+          const float tol = slack + fabsf(score) * 4.8e-07f +
+                            fabsf(smax) * 4.8e-07f + 1.0e-3f;
+          const float ds_up = fmaf((float)up[0], kLn2 / kBoundUnit, tol);
+          const float dm_up = fmaf((float)up[1], kLn2 / kBoundUnit, tol);
+          if (smax + dm_up < best_score &&
+              corr * expf(ds_up * md.gamma) * 1.001f < raw.acceptance_level) {
+            __syncwarp();
+            i++;
+            continue;  // rejected: the chain's state stays as it is
+          }
+        }
+        __syncwarp();  // the list is written again
+        from_table = true;
+        order = prop;
+      }
+    } else if (SUM && err_move && tree_ok) {
+      from_table = true;
+      if (!ord_ok) order = cur;
+    } else if (!fresh) {
+      from_rows = true;
+    }
+    if (classes ? (SUM || from_rows) : (from_rows && !err_move)) {
+      propose_tree<W32>(cur, prop, cpar, ppar, n, mp, D, related, tree_ok, wpc,
+                        wic, lane);
+      built = true;
+    }
+    if constexpr (SUM) {
+      if (classes) {
+        apply_classes<W32, Q>(tab, list, delta, C, dv, dw, false, lane);
+        applied = true;
+      }
+    }
+    if (order != nullptr && (SUM || ss.sx.inc != nullptr))
+      canonical_order<W32>(order, n, fresh ? cpar : nullptr, ss.sx.ord,
+                           ss.sx.hist, lane);
+    if (fresh) {
+      const int off = SUM ? 0 : code.off, wd = SUM ? 1 : -code.s * code.P,
+                wm = SUM ? 256 : code.s * code.Q;
+      if (ss.sx.inc != nullptr)
+        fill_table_inherit<Q>(ss.sx, n, lane, off, wd, wm);
+      else
+        fill_table<W32, Q>(cur, &ds, tab, chunks, wpc, wic, lane, off, wd, wm);
+    }
+    if constexpr (SUM) {
+      if (from_table) {
+        long long acc[6] = {0, 0, 0, 0, 0, 0};
+        sum_cells_table<Q>(n, pd, pm, PL, c0, stride, lane, ds.n_cells, acc,
+                           ss.sx, pcs);
+        acc[0] = warp_sum_ll(acc[0]);
+        acc[2] = warp_sum_ll(acc[2]);
+        acc[4] = warp_sum_ll(acc[4]);
+        acc[5] = warp_sum_ll(acc[5]);
+        ev = finish_sum(ds, pprior, acc, wpc, wic, lane, part, i & 1);
+      }
+    }
+    if (fresh) {
+      ord_ok = true;
+      if constexpr (SUM) {
+        cs = pcs;
+        smax = ev.smax;
+        if (multi) __syncthreads();  // step i writes the same partial sums
+      }
+      continue;
+    }
+    if (from_rows)
+      ev = evaluate_rows<W32, Q, SUM>(err_move ? cur : prop, &ds, PL, pprior,
+                                      wpc, wic, lane, part, i & 1, ss.sx);
+    if (order != nullptr || from_rows) ord_ok = order == cur && !from_rows;
+    const float pscore = ev.score, psmax = ev.smax;
+    bool accept;
+    if (err_move && learn) {
+      accept = accept_rates(ds, md, rates, alpha, beta, score, pscore, ev.e,
+                            raw.acceptance_level, lane);
+      err_prop++;
+      if (accept) err_acc++;
+    } else {
+      // src/Application.hpp:452-455
+      const float ratio = __fmul_rn(
+          corr, expf(__fmul_rn(__fsub_rn(pscore, score), md.gamma)));
+      accept = ratio > raw.acceptance_level;
+      if (err_move) {
+        err_prop++;
+        if (accept) err_acc++;
+      }
+    }
+    // src/Application.hpp:456 and the co-optimal list, as in run_chain
+    const bool better = !has_best || psmax > best_score;
+    const bool tie = !better && K > 1 && psmax == best_score &&
+                     lcount < (uint32_t)K;
+    if (!err_move && !built && (accept || better || tie))
+      propose_tree<W32>(cur, prop, cpar, ppar, n, mp, D, related, tree_ok, wpc,
+                        wic, lane);
+    const uint32_t *scored_rows = err_move ? cur : prop;
+    if (better) {
+      has_best = true;
+      best_score = psmax;
+      best_alpha = palpha;
+      best_beta = pbeta;
+      bsk = ev.sk;
+      bsm = ev.sm;
+      copy_rows_part<W32>(scored_rows, gbest, n, wpc, wic, lane);
+      if (K > 1) {
+        const uint64_t h = tree_hash<W32>(scored_rows, n, lane);
+        if (multi) __syncthreads();  // before the rows are written again
+        if (wic == 0 && lane == 0) {
+          lhash[0] = h;
+          lbeta[0] = pbeta;
+        }
+        lcount = 1;
+      }
+    } else if (tie) {
+      const uint64_t h = tree_hash<W32>(scored_rows, n, lane);
+      const bool seen =
+          __any_sync(BBS_FULL_MASK, lane < (int)lcount && lhash[lane] == h);
+      if (multi) __syncthreads();  // before rows or list are written again
+      if (!seen) {
+        copy_rows_part<W32>(scored_rows,
+                            gbest + (size_t)lcount * n * rs_of_w32(W32), n, wpc,
+                            wic, lane);
+        if (wic == 0 && lane == 0) {
+          lhash[lcount] = h;
+          lbeta[lcount] = pbeta;
+        }
+        lcount++;
+      }
+    }
+    if (trace != nullptr && wic == 0 && lane == 0) {
+      bbs_step_trace *t = trace + i;
+      t->move = raw;
+      t->proposed_score = pscore;
+      t->current_score = accept ? pscore : score;
+      t->proposed_beta = pbeta;
+      t->accepted = accept ? 1u : 0u;
+      t->proposed_alpha = palpha;
+      t->proposed_max_score = psmax;
+#pragma unroll
+      for (int k = 0; k < 2; k++) t->reserved[k] = 0;
+#pragma unroll
+      for (int k = 0; k < 4; k++)
+        t->proposed_counts[k] = SUM ? 0ull : (uint64_t)ev.e[k];
+    }
+    if (accept) {
+      alpha = palpha;
+      beta = pbeta;
+      score = pscore;
+      prior = pprior;
+      L = PL;
+#pragma unroll
+      for (int k = 0; k < 4; k++) ec[k] = ev.e[k];
+      csk = ev.sk;
+      csm = ev.sm;
+      smax = psmax;
+      if (!err_move) {
+        uint32_t *t = cur;
+        cur = prop;
+        prop = t;
+        uint8_t *tp = cpar;
+        cpar = ppar;
+        ppar = tp;
+        if (classes) {
+          if constexpr (!SUM) {
+            for (int c = 0; c < chunks; c++) {
+              uint32_t *tc = tab + c * n * 32 * NW;
+              if (chunks > 1) class_deltas<Q>(tc, delta, lane, dv, dw);
+              apply_classes<W32, Q>(tc, list, delta, C, dv, dw, false, lane);
+            }
+          } else {
+            cs = pcs;
+            ord_ok = true;
+          }
+#ifdef BBS_CHECKED
+          device_check(parents_match_rows<W32>(cur, n, cpar, lane), status,
+                       kCheckParent, (uint32_t)raw.move_type, 4u);
+#endif
+        } else {
+          fresh_rows = fresh_table = true;
+        }
+      } else if (tree_ok) {
+        if constexpr (SUM) {
+          cs = pcs;
+          tolerances();
+        } else {
+          fresh_table = true;
+        }
+      }
+    } else if (applied) {
+      apply_classes<W32, Q>(tab, list, delta, C, dv, dw, true, lane);
+    }
+    __syncwarp();
+    i++;
+  }
+  copy_rows_part<W32>(cur, g, n, wpc, wic, lane);
+  if (wic == 0 && lane == 0) {
+    ChainState o = st;
+    o.alpha = alpha;
+    o.beta = beta;
+    o.score = score;
+    o.prior = prior;
+    o.l00 = L.l00;
+    o.l10 = L.l10;
+    o.l01 = L.l01;
+    o.l11 = L.l11;
+#pragma unroll
+    for (int k = 0; k < 4; k++) o.ec[k] = ec[k];
+    o.sk = csk;
+    o.sm = csm;
+    o.has_best = has_best ? 1u : 0u;
+    o.best_alpha = best_alpha;
+    o.best_beta = best_beta;
+    o.best_score = best_score;
+    o.best_sk = bsk;
+    o.best_sm = bsm;
+    o.steps_done = st.steps_done + (uint64_t)i;
+    o.err_proposed = err_prop;
+    o.err_accepted = err_acc;
+    o.list_count = lcount;
+    *gstate = o;
+    if (cancelled && status != nullptr) atomicOr(status, 1);
+  }
+  if (multi) __syncthreads(); else __syncwarp();
+}
+
 // Launch bounds of each cells-per-lane variant (bbs_layout.h).
 template <int Q>
 struct ChainBounds {
@@ -476,13 +958,12 @@ __global__ void __launch_bounds__(ChainBounds<Q>::threads,
   const int cpb = wpb / wpc;
   const int slot = wib / wpc, wic = wib - slot * wpc;
   const int n = a.ds.n_nodes;
-  // rows of five to eight words stream their cells per evaluation (their
-  // counts come through the ring and a gene table built per chunk)
-  const bool resident = W32 <= 4 && a.ds.n_cells <= 32 * wpc * Q;
-  // the same decisions as the launcher's, for the whole block
-  const bool counts = inherits_counts(W32, a.ds.n_cells, 32 * wpc * Q);
-  const bool scratch = SUM || counts;
-  const int sb = slot_bytes(n, RS, wpc, scratch, W32, Q, counts);
+  // the launcher's plan, for the whole block
+  const bool inc = a.with_inc != 0, ring = W32 > 4;
+  const bool scratch = SUM || ring || a.chunks > 0;
+  const int sb = a.chunks > 0 && !inc
+                     ? table_slot_bytes(n, RS, wpc, W32, Q, a.chunks)
+                     : slot_bytes(n, RS, wpc, scratch, W32, Q, inc || ring);
   uint8_t *slot_base = reinterpret_cast<uint8_t *>(smem) + (size_t)slot * sb;
   uint32_t *buf0 = reinterpret_cast<uint32_t *>(slot_base);
   uint32_t *buf1 = buf0 + n * RS;
@@ -490,18 +971,18 @@ __global__ void __launch_bounds__(ChainBounds<Q>::threads,
   volatile int *sflag = part + 24 * wpc;
   uint4 *pbuf = reinterpret_cast<uint4 *>(
       slot_base + 4 * (2 * n * RS + 24 * wpc + 4) + kPhiloxBytes * wic);
-  Cells<W32, Q> cb;
-  if (resident) load_cells<W32, Q>(cb, a.ds, 32 * wic, 32 * wpc, lane);
   SlotSum ss{};
   if (scratch) {
-    ss = slot_sum(slot_base, n, RS, wpc, wic, W32, Q, counts);
+    ss = slot_sum(slot_base, n, RS, wpc, wic, W32, Q, inc || ring);
     if constexpr (W32 <= 4) {
-      if (counts) {
+      if (inc) {
         uint8_t *table = reinterpret_cast<uint8_t *>(smem) + (size_t)cpb * sb;
         build_increments<Q>(table, wpc, a.ds, RS);
         __syncthreads();
         ss.sx.inc = reinterpret_cast<const uint32_t *>(
             table + (size_t)wic * inc_table_bytes(n, Q));
+      } else if (a.chunks > 0) {
+        ss.sx.cnt = table_part(slot_base, n, RS, wpc, wic, W32, Q, a.chunks);
       }
     }
   }
@@ -514,14 +995,23 @@ __global__ void __launch_bounds__(ChainBounds<Q>::threads,
       if (a.trace != nullptr) trace = a.trace + (size_t)chain * a.n_steps;
     }
     const int K = a.list_hash != nullptr ? a.md.treelist : 1;
-    run_chain<W32, Q, SUM>(
-        a.ds, a.md, (uint32_t)chain, a.rows + (size_t)chain * n * RS,
-        a.best_rows + (size_t)chain * K * n * RS,
-        K > 1 ? a.list_hash + (size_t)chain * K : nullptr,
-        K > 1 ? a.list_beta + (size_t)chain * K : nullptr, K, a.states + chain,
-        moves, trace,
-        a.n_steps, a.cancel, a.status, buf0, buf1, part, sflag, pbuf, ss, cb,
-        resident, wpc, wic, lane);
+    uint32_t *rows = a.rows + (size_t)chain * n * RS;
+    uint32_t *best = a.best_rows + (size_t)chain * K * n * RS;
+    uint64_t *lhash = K > 1 ? a.list_hash + (size_t)chain * K : nullptr;
+    float *lbeta = K > 1 ? a.list_beta + (size_t)chain * K : nullptr;
+    if constexpr (W32 <= 4) {
+      if (a.chunks > 0) {
+        run_chain_table<W32, Q, SUM>(
+            a.ds, a.md, (uint32_t)chain, rows, best, lhash, lbeta, K,
+            a.states + chain, moves, trace, a.n_steps, a.cancel, a.status,
+            buf0, buf1, part, sflag, pbuf, ss, a.chunks, wpc, wic, lane);
+        continue;
+      }
+    }
+    run_chain<W32, Q, SUM>(a.ds, a.md, (uint32_t)chain, rows, best, lhash,
+                           lbeta, K, a.states + chain, moves, trace,
+                           a.n_steps, a.cancel, a.status, buf0, buf1, part,
+                           sflag, pbuf, ss, wpc, wic, lane);
   }
 }
 
@@ -533,27 +1023,31 @@ __device__ __forceinline__ void batch_unit(const BatchArgs &b,
                                            const ModelDev &md, uint32_t chain,
                                            uint32_t d, uint32_t *buf0,
                                            int *part, volatile int *sflag,
-                                           uint4 *pbuf, const SlotSum &ss_in,
-                                           Cells<W32, Q> &cb, int wpc,
-                                           int wic, int lane) {
+                                           uint4 *pbuf, const SlotSum &ss,
+                                           int wpc, int wic, int lane) {
   constexpr int RS = rs_of_w32(W32);
   // the dataset's node count is within this launch's row width
   uint32_t *buf1 = buf0 + ds.n_nodes * RS;
-  // rows of five to eight words stream their cells per evaluation (their
-  // counts come through the ring and a gene table built per chunk)
-  const bool resident = W32 <= 4 && ds.n_cells <= 32 * wpc * Q;
-  if (resident) load_cells<W32, Q>(cb, ds, 32 * wic, 32 * wpc, lane);
   const uint64_t off = b.chain_off[chain];
   // Philox key: the chain's number within its dataset, so a dataset's
   // chains draw the same moves here as in a one-dataset run.
   const uint32_t local = chain - d * (uint32_t)b.chains_per_dataset;
-  // the increment table holds the cells of dataset b.table_ds only
-  SlotSum ss = ss_in;
-  if ((int)d != b.table_ds) ss.sx.inc = nullptr;
+  if constexpr (W32 <= 4) {
+    if (b.chunks > 0) {
+      // (this dataset's chunks: a launch's largest dataset sizes the slots)
+      const int span = 32 * wpc * Q;
+      run_chain_table<W32, Q, SUM>(
+          ds, md, local, b.rows + off, b.best_rows + off, nullptr, nullptr, 1,
+          b.states + chain, nullptr, nullptr, b.n_steps, b.cancel, b.status,
+          buf0, buf1, part, sflag, pbuf, ss, (ds.n_cells + span - 1) / span,
+          wpc, wic, lane);
+      return;
+    }
+  }
   run_chain<W32, Q, SUM>(ds, md, local, b.rows + off, b.best_rows + off,
                          nullptr, nullptr, 1, b.states + chain, nullptr,
                          nullptr, b.n_steps, b.cancel, b.status, buf0, buf1,
-                         part, sflag, pbuf, ss, cb, resident, wpc, wic, lane);
+                         part, sflag, pbuf, ss, wpc, wic, lane);
 }
 
 // Many datasets: warps take chains from a shared work list (costliest
@@ -577,10 +1071,13 @@ __global__ void __launch_bounds__(ChainBounds<Q>::threads,
   const int wib = threadIdx.x >> 5;
   const int wpc = MULTI ? b.wpc : 1;
   const int slot = wib / wpc, wic = wib - slot * wpc;
-  // inherited counts (the host's decision, the same in every thread)
-  const bool counts = b.with_counts != 0;
-  const bool scratch = SUM || counts;
-  const int sb = slot_bytes(b.max_nodes, RS, wpc, scratch, W32, Q, counts);
+  // the host's plan, the same in every thread
+  const bool inc = b.with_inc != 0, ring = W32 > 4;
+  const bool scratch = SUM || ring || b.chunks > 0;
+  const int sb =
+      b.chunks > 0 && !inc
+          ? table_slot_bytes(b.max_nodes, RS, wpc, W32, Q, b.chunks)
+          : slot_bytes(b.max_nodes, RS, wpc, scratch, W32, Q, inc || ring);
   uint8_t *slot_base = reinterpret_cast<uint8_t *>(smem) + (size_t)slot * sb;
   uint32_t *buf0 = reinterpret_cast<uint32_t *>(slot_base);
   int *part = reinterpret_cast<int *>(buf0 + 2 * b.max_nodes * RS);
@@ -593,11 +1090,10 @@ __global__ void __launch_bounds__(ChainBounds<Q>::threads,
       kPhiloxBytes * wic);
   SlotSum ss{};
   if (scratch) {
-    ss = slot_sum(slot_base, b.max_nodes, RS, wpc, wic, W32, Q, counts);
+    ss = slot_sum(slot_base, b.max_nodes, RS, wpc, wic, W32, Q, inc || ring);
     if constexpr (W32 <= 4) {
-      if (counts) {
-        // one increment table per warp part of a chain (the launch's one
-        // dataset)
+      if (inc) {
+        // the increment table of the launch's one dataset
         uint8_t *table = reinterpret_cast<uint8_t *>(smem) +
                          (size_t)((blockDim.x >> 5) / wpc) * sb;
         const DatasetDev &tds = b.ds[b.table_ds];
@@ -605,10 +1101,12 @@ __global__ void __launch_bounds__(ChainBounds<Q>::threads,
         __syncthreads();
         ss.sx.inc = reinterpret_cast<const uint32_t *>(
             table + (size_t)wic * inc_table_bytes(tds.n_nodes, Q));
+      } else if (b.chunks > 0) {
+        ss.sx.cnt = table_part(slot_base, b.max_nodes, RS, wpc, wic, W32, Q,
+                               b.chunks);
       }
     }
   }
-  Cells<W32, Q> cb;
   for (;;) {
     unsigned int unit = 0;
     if constexpr (!MULTI) {
@@ -636,12 +1134,12 @@ __global__ void __launch_bounds__(ChainBounds<Q>::threads,
     // (measured faster there).
     if constexpr (SUM) {
       batch_unit<W32, Q, SUM>(b, b.ds[d], b.md[d], chain, d, buf0, part,
-                              sflag, pbuf, ss, cb, wpc, wic, lane);
+                              sflag, pbuf, ss, wpc, wic, lane);
     } else {
       const DatasetDev ds = b.ds[d];
       const ModelDev md = b.md[d];
       batch_unit<W32, Q, SUM>(b, ds, md, chain, d, buf0, part, sflag, pbuf,
-                              ss, cb, wpc, wic, lane);
+                              ss, wpc, wic, lane);
     }
   }
 }
@@ -679,25 +1177,22 @@ __global__ void __launch_bounds__(128) init_kernel(const InitArgs a) {
   const float *tm = a.terms + 8 * (size_t)d;
   const LogTable L{tm[2], tm[3], tm[4], tm[5]};
   const float alpha = tm[0], beta = tm[1], prior = tm[6];
-  Cells<W32, Q> cb;
-  float e[4], smax;
-  int sk, sm;
-  const float S = evaluate<W32, Q, SUM>(rows, n, ds, cb, false, L, prior, 1, 0,
-                                        lane, nullptr, 0, sx, e, sk, sm, smax);
+  const Evaluated ev = evaluate<W32, Q, SUM>(rows, n, ds, L, prior, 1, 0, lane,
+                                             nullptr, 0, sx);
   if (lane == 0) {
     ChainState o;
     o.alpha = alpha;
     o.beta = beta;
-    o.score = S;
+    o.score = ev.score;
     o.prior = prior;
     o.l00 = L.l00;
     o.l10 = L.l10;
     o.l01 = L.l01;
     o.l11 = L.l11;
 #pragma unroll
-    for (int k = 0; k < 4; k++) o.ec[k] = e[k];
-    o.sk = sk;
-    o.sm = sm;
+    for (int k = 0; k < 4; k++) o.ec[k] = ev.e[k];
+    o.sk = ev.sk;
+    o.sm = ev.sm;
     o.has_best = 0;
     o.best_alpha = alpha;
     o.best_beta = beta;

@@ -19,16 +19,16 @@ inline cudaError_t prepare_smem(K kernel, size_t smem) {
 // blocks of one chain of wpc warps.  As many blocks as chains need, capped
 // at what stays resident; each block then walks its chain slots.
 template <int W32, int Q, bool SUM, bool REC>
-int launch_mcmc_t(const RunArgs &a, int cpb, int n_sms, cudaStream_t s) {
-  constexpr int RS = rs_of_w32(W32);
+int launch_mcmc_t(RunArgs a, int cpb, int n_sms, int smem_block,
+                  cudaStream_t s) {
   if (a.wpc > 1) cpb = 1;
   const int threads = 32 * a.wpc * cpb;
   if (threads > chain_max_threads(Q)) return (int)cudaErrorInvalidConfiguration;
-  const bool counts = inherits_counts(W32, a.ds.n_cells, 32 * a.wpc * Q);
-  const size_t smem =
-      (size_t)cpb * slot_bytes(a.ds.n_nodes, RS, a.wpc, SUM || counts, W32, Q,
-                               counts) +
-      table_bytes(a.ds.n_nodes, W32, Q, a.wpc, counts);
+  const TablePlan p = plan_tables(a.ds.n_nodes, W32, a.ds.n_cells, Q, a.wpc,
+                                  cpb, SUM, true, smem_block);
+  a.chunks = p.chunks;
+  a.with_inc = p.inc ? 1 : 0;
+  const size_t smem = (size_t)p.smem;
   auto kern = mcmc_kernel<W32, Q, SUM, REC>;
   cudaError_t e = prepare_smem(kern, smem);
   if (e != cudaSuccess) return (int)e;
@@ -46,21 +46,19 @@ int launch_mcmc_t(const RunArgs &a, int cpb, int n_sms, cudaStream_t s) {
 // there are units.  Blocks of wpb one-warp slots (b.wpc == 1), or of one
 // slot of wpb == b.wpc warps.
 template <int W32, int Q, bool SUM, bool MULTI>
-int launch_batch_t(const BatchArgs &b, int wpb, int n_sms, cudaStream_t s) {
-  constexpr int RS = rs_of_w32(W32);
+int launch_batch_t(BatchArgs b, int max_cells, int wpb, int n_sms,
+                   int smem_block, cudaStream_t s) {
   const int threads = 32 * wpb;
   if (threads > chain_max_threads(Q)) return (int)cudaErrorInvalidConfiguration;
   if (b.wpc < 1 || b.wpc > 4 || (b.wpc > 1) != MULTI ||
       (MULTI && wpb != b.wpc))
     return (int)cudaErrorInvalidValue;
   const int slots = wpb / b.wpc;
-  const bool counts = b.with_counts != 0;
-  if (counts && W32 <= 4 && b.table_ds < 0)
-    return (int)cudaErrorInvalidValue;  // count tables need one dataset's rows
-  const size_t smem =
-      (size_t)slots * slot_bytes(b.max_nodes, RS, b.wpc, SUM || counts, W32,
-                                 Q, counts) +
-      table_bytes(b.max_nodes, W32, Q, b.wpc, counts);
+  const TablePlan p = plan_tables(b.max_nodes, W32, max_cells, Q, b.wpc, slots,
+                                  SUM, b.table_ds >= 0, smem_block);
+  b.chunks = p.chunks;
+  b.with_inc = p.inc ? 1 : 0;
+  const size_t smem = (size_t)p.smem;
   auto kern = batch_kernel<W32, Q, SUM, MULTI>;
   cudaError_t e = prepare_smem(kern, smem);
   if (e != cudaSuccess) return (int)e;
@@ -74,23 +72,14 @@ int launch_batch_t(const BatchArgs &b, int wpb, int n_sms, cudaStream_t s) {
   return (int)cudaGetLastError();
 }
 
-// Recording launches (recorded moves or a trace) go to the _rec units.
-int launch_mcmc_lo(const RunArgs &a, int w32, int q, bool sum, int cpb,
-                   int n_sms, cudaStream_t s);
-int launch_mcmc_hi(const RunArgs &a, int w32, int q, bool sum, int cpb,
-                   int n_sms, cudaStream_t s);
-int launch_mcmc_lo_rec(const RunArgs &a, int w32, int q, bool sum, int cpb,
-                       int n_sms, cudaStream_t s);
-int launch_mcmc_hi_rec(const RunArgs &a, int w32, int q, bool sum, int cpb,
-                       int n_sms, cudaStream_t s);
-int launch_batch_lo(const BatchArgs &b, int w32, int q, bool sum, int wpb,
-                    int n_sms, cudaStream_t s);
-int launch_batch_hi(const BatchArgs &b, int w32, int q, bool sum, int wpb,
-                    int n_sms, cudaStream_t s);
-// (chains of several warps: their own units)
-int launch_batch_lo_multi(const BatchArgs &b, int w32, int q, bool sum,
-                          int wpb, int n_sms, cudaStream_t s);
-int launch_batch_hi_multi(const BatchArgs &b, int w32, int q, bool sum,
-                          int wpb, int n_sms, cudaStream_t s);
+// One unit per row width: launches with recorded moves or a trace (REC) or
+// without, and work-list launches of one-warp chains or chains of several
+// warps (MULTI).
+template <int W, bool REC>
+int launch_mcmc_w(const RunArgs &a, int q, bool sum, int cpb, int n_sms,
+                  int smem_block, cudaStream_t s);
+template <int W, bool MULTI>
+int launch_batch_w(const BatchArgs &b, int max_cells, int q, bool sum, int wpb,
+                   int n_sms, int smem_block, cudaStream_t s);
 
 }  // namespace bbs

@@ -101,6 +101,54 @@ __host__ __device__ inline int chain_launch_smem(int n, int n_cells, int q,
          table_bytes(n, w32, q, wpc, counts);
 }
 
+// Rows of up to four words: the table of every node that proposals are read
+// off (bbs_incr.cuh).
+//   chunks  chunks of 32 wpc q cells the table holds (0: no table, the cells
+//           are streamed); the sum score takes one.
+//   inc     the block's increment tables come with it, which refill the table
+//           after the rates of a chain change: one-warp chains of one dataset
+//           in one chunk share one (the layout with `counts` above).  Other
+//           launches fill their tables from the rows and keep the room.
+struct TablePlan {
+  int chunks;
+  bool inc;
+  int smem;  // dynamic shared memory of the launch
+};
+
+__host__ __device__ inline int table_part_bytes(int n, int q, int chunks) {
+  return chunks * align16(pack_table_bytes(n, q));
+}
+// A slot with its table but without increments: the slot with the scratch,
+// then each warp's part of the table.
+__host__ __device__ inline int table_slot_bytes(int n, int rs, int wpc,
+                                                int w32, int q, int chunks) {
+  return slot_bytes(n, rs, wpc, true, w32, q, false) +
+         wpc * table_part_bytes(n, q, chunks);
+}
+
+// The plan of a launch of `slots` chain slots per block, its largest dataset
+// of n nodes and n_cells cells.  Where the tables do not fit a block, or a
+// sum-score chain's cells do not fit one chunk, the cells are streamed as
+// before (such launches are bound by their masked popcounts).
+inline TablePlan plan_tables(int n, int w32, int n_cells, int q, int wpc,
+                             int slots, bool sum, bool one_dataset,
+                             int smem_block) {
+  const int rs = rs_of_w32(w32), span = 32 * wpc * q;
+  if (w32 > 4)
+    return TablePlan{0, false,
+                     chain_launch_smem(n, n_cells, q, wpc, slots, sum)};
+  const TablePlan p{0, false,
+                    slots * slot_bytes(n, rs, wpc, sum, w32, q, false)};
+  const int chunks = (n_cells + span - 1) / span;
+  if (sum && chunks > 1) return p;
+  const bool inc = wpc == 1 && one_dataset && chunks == 1;
+  const int smem =
+      inc ? chain_launch_smem(n, n_cells, q, wpc, slots, sum)
+          : slots * table_slot_bytes(n, rs, wpc, w32, q, chunks);
+  if (smem > smem_block) return p;
+  return TablePlan{chunks, inc, smem};
+}
+
 // Resident warps per SM of such a launch (blocks of warps_per_block
 // warps), from the SM's shared memory (smem_sm bytes, reserved_per_block
 // of them taken by each block, at most smem_block per block) and registers.

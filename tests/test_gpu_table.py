@@ -1,0 +1,126 @@
+"""Chains that read proposals off a table of every node (rows of up to four
+words): exact counts, scores and trees at the edges of the table's groups and
+chunks, at rates whose integer codes tie, are near their margin or do not
+exist, and without a trace (proposals rejected by a bound) as with one."""
+import os
+import subprocess
+
+import numpy as np
+import pytest
+
+from bbscite_gb300 import data as D
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+
+
+def _setup(G, Cn, seed=3):
+    m, _, _ = D.generate_dataset(seed * 1000 + G * 7 + Cn, G, Cn, 2e-3, 0.2,
+                                 0.1, 0.02)
+    return D.matrix_to_bits(m)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("G,Cn,launch,alpha,beta", [
+    (2, 1, (1, 1, 1), 1e-3, 0.2),       # the smallest problem
+    (7, 40, (2, 1, 2), 1e-3, 0.2),      # one group of eight nodes
+    (8, 33, (1, 2, 1), 1e-5, 0.4),      # a ragged group, two warps
+    (32, 129, (1, 1, 4), 1e-3, 0.2),    # five chunks, the last of one cell
+    (95, 200, (3, 1, 2), 6e-5, 0.43),   # three chunks of 96
+    (127, 256, (2, 4, 1), 1e-3, 0.2),   # the widest table, four warps
+    (40, 64, (2, 1, 2), 0.2, 0.2),      # every fraction ties: ratio 1
+    (40, 64, (2, 1, 2), 0.125, 0.5),    # few distinct logs
+    (40, 64, (2, 1, 2), 0.7, 0.6),      # alpha + beta above 1: signs turn
+    (30, 40, (2, 1, 2), 0.5, 0.5),      # no codes: every node scores alike
+])
+def test_max_chains_match_the_oracle(native, orc, G, Cn, launch, alpha, beta):
+    mut, known = _setup(G, Cn)
+    chains, steps = 3, 120
+    p = native.default_params(alpha_mean=alpha, beta_mean=beta, seed=11)
+    rng = np.random.default_rng(G)
+    starts = np.stack([D.random_parent_vector(rng, G) for _ in range(chains)])
+    out = []
+    for trace in (True, False):
+        with native.Context(mut, known, Cn, G, p) as c:
+            c.init_chains(chains, starts)
+            c.set_launch(*launch)
+            tr = c.run(steps, trace=trace)
+            out.append((c.chains(), c.best()))
+            if trace:
+                t = tr
+    (a, ab), (b, bb) = out
+    for k in ("dm", "score", "counts", "beta"):
+        np.testing.assert_array_equal(a[k], b[k])
+    assert ab["score"] == bb["score"] and (ab["dm"] == bb["dm"]).all()
+    for ch in range(chains):
+        raws = np.zeros(steps, dtype=orc.RAW_MOVE)
+        raws.view(np.uint8)[:] = np.frombuffer(t["move"][ch].tobytes(),
+                                               dtype=np.uint8)
+        res = orc.run_chain(alpha, beta, 0.1, 1.0, starts[ch], mut, known,
+                            raws, score_mode=1, forced=t["accepted"][ch],
+                            ambiguity=1e-5)
+        np.testing.assert_array_equal(res["trace"]["counts"],
+                                      t["proposed_counts"][ch])
+        assert (res["dm"] == a["dm"][ch]).all()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("score", ["max", "sum"])
+@pytest.mark.parametrize("move", ["beta_walk", "langevin"])
+@pytest.mark.parametrize("G,Cn,q", [(2, 3, 1), (31, 32, 1), (64, 70, 3),
+                                    (95, 96, 3), (127, 128, 4)])
+def test_untraced_chains_equal_traced_ones(native, score, move, G, Cn, q):
+    """The sum score's bound and the near-tie margin of the max score reject
+    proposals without evaluating them; a traced chain evaluates every one."""
+    mut, known = _setup(G, Cn, 5)
+    p = native.default_params(
+        alpha_mean=1e-2, beta_mean=0.3, seed=29, prob_beta_change=0.15,
+        score_mode=getattr(native, "SCORE_" + score.upper()),
+        error_move=getattr(native, "ERROR_" + move.upper()))
+    got = []
+    for trace in (False, True):
+        with native.Context(mut, known, Cn, G, p) as c:
+            c.init_chains(8)
+            c.set_launch(q, 1, 1)
+            for steps in (1, 37, 400):
+                c.run(steps, trace=trace)
+            got.append((c.chains(), c.best(), c.save_chains()))
+    assert got[0][2] == got[1][2]
+    assert got[0][1]["score"] == got[1][1]["score"]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("shape", [(1, 4, 0, 1), (4, 2, 1, 1), (2, 4, 0, 4)])
+def test_mixed_batches_equal_their_datasets_alone(native, shape):
+    """Datasets of one launch with one to eight chunks of cells."""
+    sizes = [(33, 17), (40, 250), (63, 64), (60, 129), (20, 31), (127, 200)]
+    data = [_setup(G, Cn, 9 + i) + (Cn, G) for i, (G, Cn) in enumerate(sizes)]
+    params = [native.default_params(alpha_mean=1e-3 * (i + 1), beta_mean=0.2,
+                                    seed=70 + i) for i in range(len(sizes))]
+    q, wpb, merge, wpc = shape
+    with native.Batch(data, params) as b:
+        b.init_chains(5)
+        b.set_launch(q, wpb, merge)
+        b.set_chain_warps(wpc)
+        b.run(150)
+        best = [b.best(d) for d in range(len(sizes))]
+    for d, (G, Cn) in enumerate(sizes):
+        with native.Context(*data[d], params[d]) as c:
+            c.init_chains(5)
+            c.run(150)
+            one = c.best()
+        assert one["score"] == best[d]["score"]
+        assert (one["dm"] == best[d]["dm"]).all()
+
+
+def test_layout_of_slots_with_tables(tmp_path):
+    """Every piece of a slot with a table but no increments lies inside its
+    slot, apart from the others and aligned, and the plan asks for the room."""
+    from bbscite_gb300 import build as B
+    exe = str(tmp_path / "table_probe")
+    subprocess.run([B.nvcc(), *B.ARCH, "-std=c++17", "-I" + B.INCLUDE,
+                    "-I" + B.CSRC,
+                    os.path.join(ROOT, "tests", "cpp", "table_probe.cu"),
+                    "-o", exe], check=True, capture_output=True)
+    r = subprocess.run([exe], capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stdout
+    assert r.stdout.startswith("tables ok "), r.stdout
