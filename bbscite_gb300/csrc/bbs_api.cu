@@ -247,10 +247,11 @@ struct bbs_ctx {
   bool running = false;
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
   float last_ms = 0.0f;
-  // scratch of the host-buffer scoring calls and its pinned host mirror,
-  // scratch_cap bytes each; grows, never shrinks
+  // scratch of the host-buffer scoring calls (scratch_cap bytes) and the
+  // pinned host mirror of its small pieces (mirror_cap); both grow, neither
+  // shrinks
   uint8_t *d_scratch = nullptr, *h_scratch = nullptr;
-  size_t scratch_cap = 0;
+  size_t scratch_cap = 0, mirror_cap = 0;
   uint64_t fingerprint = 0;  // of the dataset and parameters (checkpoints)
 };
 
@@ -401,68 +402,124 @@ struct DevBuf {
   cudaError_t alloc(size_t n) { return cudaMalloc((void **)&p, sizeof(T) * std::max<size_t>(n, 1)); }
 };
 
-// A piece of the context's scratch: its device address and the same
-// offset in the pinned host mirror.
+// A piece of the context's scratch: its device address and, for a small
+// piece, the same offset in the pinned host mirror (null for a large one).
 template <typename T>
 struct Piece {
   T *d;
   T *h;
 };
 
+// Arrays above this go straight between the caller's memory and the device;
+// smaller ones of a call share one copy each way through the pinned mirror.
+// On GB300 the copy engines read and write pageable memory through the host's
+// page tables: 6.3 MB take 48 us in and 42 us out (38 and 41 us pinned),
+// while the memcpy into or out of the mirror alone runs at 19 GB/s, 320 us.
+// A copy of its own costs some microseconds whatever its size, the memcpy of
+// 64 KB about three.
+constexpr size_t kDirectBytes = 64 * 1024;
+
 // Pieces of the context's scratch for one call of a host-buffer entry point
 // (bbs_score_trees, bbs_apply_moves, bbs_sumscore_grad).  The call adds up
 // its pieces with add(), reserves once, then takes them in the same order
-// with take(); inputs come first and outputs last, so that each call moves
-// one contiguous range each way between the pinned mirror and the device.
-// The scratch only moves while nothing is taken, and a caller that scores
-// one tree at a time allocates on its first call only.
+// with take().  Small pieces come first in the scratch, inputs before
+// outputs, and have a pinned mirror: one contiguous copy each way moves them
+// all.  Large ones follow and are copied from and to the caller's arrays by
+// in() and out().  The scratch only moves while nothing is taken, and a
+// caller that scores one tree at a time allocates on its first call only.
 class ScratchPlan {
  public:
   template <typename T>
-  void add(size_t n) { bytes_ += piece(sizeof(T) * n); }
+  void add(size_t n) {
+    const size_t b = sizeof(T) * n;
+    (b > kDirectBytes ? large_ : small_) += piece(b);
+  }
   int reserve(bbs_ctx *c) {
     c_ = c;
-    off_ = 0;
-    if (bytes_ <= c->scratch_cap) return BBS_OK;
-    // every entry point drains the stream before it returns, so no copy or
-    // kernel of an earlier call still uses the old scratch
-    cudaFree(c->d_scratch);
-    if (c->h_scratch) cudaFreeHost(c->h_scratch);
-    c->d_scratch = c->h_scratch = nullptr;
-    c->scratch_cap = 0;
-    // half again as much, so that a slowly growing caller reallocates
-    // rarely; the exact size when that much is not free
-    for (const size_t cap : {bytes_ + bytes_ / 2, bytes_}) {
-      cudaError_t e = cudaMalloc(&c->d_scratch, cap);
-      if (e == cudaSuccess) e = cudaHostAlloc(&c->h_scratch, cap, cudaHostAllocDefault);
-      if (e == cudaSuccess) {
-        c->scratch_cap = cap;
-        return BBS_OK;
-      }
-      (void)cudaGetLastError();
+    small_off_ = 0;
+    large_off_ = small_;
+    const size_t bytes = small_ + large_;
+    if (bytes > c->scratch_cap) {
+      // every entry point drains the stream before it returns, so no copy or
+      // kernel of an earlier call still uses the old scratch
       cudaFree(c->d_scratch);
+      c->d_scratch = nullptr;
+      c->scratch_cap = 0;
+      // half again as much, so that a slowly growing caller reallocates
+      // rarely; the exact size when that much is not free
+      for (const size_t cap : {bytes + bytes / 2, bytes}) {
+        const cudaError_t e = cudaMalloc(&c->d_scratch, cap);
+        if (e == cudaSuccess) {
+          c->scratch_cap = cap;
+          break;
+        }
+        (void)cudaGetLastError();
+        c->d_scratch = nullptr;
+        if (cap == bytes) return cuda_fail((int)e, "scratch allocation");
+      }
+    }
+    if (small_ > c->mirror_cap) {
       if (c->h_scratch) cudaFreeHost(c->h_scratch);
-      c->d_scratch = c->h_scratch = nullptr;
-      if (cap == bytes_) return cuda_fail((int)e, "scratch allocation");
+      c->h_scratch = nullptr;
+      c->mirror_cap = 0;
+      const size_t cap = small_ + small_ / 2;
+      const cudaError_t e =
+          cudaHostAlloc(&c->h_scratch, cap, cudaHostAllocDefault);
+      if (e != cudaSuccess) {
+        (void)cudaGetLastError();
+        c->h_scratch = nullptr;
+        return cuda_fail((int)e, "scratch allocation");
+      }
+      c->mirror_cap = cap;
     }
     return BBS_OK;
   }
   template <typename T>
   Piece<T> take(size_t n) {
-    Piece<T> p{reinterpret_cast<T *>(c_->d_scratch + off_),
-               reinterpret_cast<T *>(c_->h_scratch + off_)};
-    off_ += piece(sizeof(T) * n);
+    const size_t b = sizeof(T) * n;
+    const bool direct = b > kDirectBytes;
+    size_t &off = direct ? large_off_ : small_off_;
+    Piece<T> p{reinterpret_cast<T *>(c_->d_scratch + off),
+               direct ? nullptr : reinterpret_cast<T *>(c_->h_scratch + off)};
+    off += piece(b);
     return p;
   }
-  // Offset of the next piece: the end of the inputs, the start of the outputs.
-  size_t mark() const { return off_; }
+  // An input array: into the mirror, or to the device at once.
+  template <typename T>
+  cudaError_t in(const Piece<T> &p, const T *src, size_t n) const {
+    if (n == 0) return cudaSuccess;
+    if (p.h != nullptr) {
+      std::memcpy(p.h, src, sizeof(T) * n);
+      return cudaSuccess;
+    }
+    return cudaMemcpyAsync(p.d, src, sizeof(T) * n, cudaMemcpyHostToDevice,
+                           c_->stream);
+  }
+  // A large output array, after the kernel; a small one by finish().
+  template <typename T>
+  cudaError_t out(const Piece<T> &p, T *dst, size_t n) const {
+    if (n == 0 || p.h != nullptr || dst == nullptr) return cudaSuccess;
+    return cudaMemcpyAsync(dst, p.d, sizeof(T) * n, cudaMemcpyDeviceToHost,
+                           c_->stream);
+  }
+  // A small output array, after the stream has been drained.
+  template <typename T>
+  static void finish(const Piece<T> &p, T *dst, size_t n) {
+    if (n != 0 && p.h != nullptr && dst != nullptr)
+      std::memcpy(dst, p.h, sizeof(T) * n);
+  }
+  // Offset of the next small piece: the end of the inputs, the start of the
+  // outputs.
+  size_t mark() const { return small_off_; }
   // One copy of the mirror's bytes [from, to) to the device or back, on the
   // context's stream.
   cudaError_t to_device(size_t from, size_t to) const {
+    if (to == from) return cudaSuccess;
     return cudaMemcpyAsync(c_->d_scratch + from, c_->h_scratch + from, to - from,
                            cudaMemcpyHostToDevice, c_->stream);
   }
   cudaError_t to_host(size_t from, size_t to) const {
+    if (to == from) return cudaSuccess;
     return cudaMemcpyAsync(c_->h_scratch + from, c_->d_scratch + from, to - from,
                            cudaMemcpyDeviceToHost, c_->stream);
   }
@@ -472,9 +529,28 @@ class ScratchPlan {
   // left out may still be taken with n = 0
   static size_t piece(size_t bytes) { return (bytes + 255) & ~size_t(255); }
   bbs_ctx *c_ = nullptr;
-  size_t bytes_ = 0;
-  size_t off_ = 0;
+  size_t small_ = 0, large_ = 0;
+  size_t small_off_ = 0, large_off_ = 0;
 };
+
+// Drains the stream when a call returns early, while copies from or to the
+// caller's arrays may be under way.
+struct Drain {
+  cudaStream_t stream;
+  bool armed = true;
+  ~Drain() {
+    if (armed) cudaStreamSynchronize(stream);
+  }
+};
+
+// A host array of `n` values that is sent as it is when small pieces are
+// mirrored (p.h), or staged in `own` when it is large: what in() copies.
+template <typename T>
+T *staging(const Piece<T> &p, std::vector<T> &own, size_t n) {
+  if (p.h != nullptr) return p.h;
+  own.resize(n);
+  return own.data();
+}
 
 // FNV-1a, 64 bit.
 uint64_t fnv1a(uint64_t h, const void *p, size_t n) {
@@ -1489,12 +1565,18 @@ int bbs_score_trees(bbs_ctx *c, const uint64_t *dm, const float *betas,
     const auto d_attach = plan.take<uint32_t>(attach ? n_attach : 0);
     const size_t out_end = plan.mark();
     // inputs: the ancestor rows and the host log-table terms of each beta
-    std::memcpy(rows.h, dm, sizeof(uint64_t) * words);
+    // (computed while the rows are on their way)
+    std::vector<float> own;
+    Drain drain{c->stream};
+    BBS_CUDA(plan.in(rows, dm, words), "scratch upload");
+    float *ht = staging(terms, own, 4 * (size_t)n_trees);
     for (uint32_t t = 0; t < n_trees; t++) {
-      float *tt = terms.h + 4 * (size_t)t;
+      float *tt = ht + 4 * (size_t)t;
       tt[0] = betas[t];
       host_beta_terms(c->ds, betas[t], &tt[1], &tt[2], &tt[3]);
     }
+    if (!own.empty())
+      BBS_CUDA(plan.in(terms, own.data(), own.size()), "scratch upload");
     BBS_CUDA(plan.to_device(0, out_begin), "scratch upload");
     ScoreArgs a{};
     a.ds = c->ds;
@@ -1507,12 +1589,17 @@ int bbs_score_trees(bbs_ctx *c, const uint64_t *dm, const float *betas,
     a.states = nullptr;
     const int e = launch_score(a, c->q, c->stream);
     if (e != 0) return cuda_fail(e, "score kernel launch");
+    const size_t n_counts = counts ? 4 * (size_t)n_trees : 0;
     BBS_CUDA(plan.to_host(out_begin, out_end), "result copy");
+    BBS_CUDA(plan.out(d_scores, scores, n_trees), "result copy");
+    BBS_CUDA(plan.out(d_counts, counts, n_counts), "result copy");
+    BBS_CUDA(plan.out(d_attach, attach, attach ? n_attach : 0), "result copy");
     r = sync_stream(c, "score kernel");
+    drain.armed = false;
     if (r != BBS_OK) return r;
-    std::memcpy(scores, d_scores.h, sizeof(float) * n_trees);
-    if (counts) std::memcpy(counts, d_counts.h, sizeof(uint64_t) * 4 * n_trees);
-    if (attach) std::memcpy(attach, d_attach.h, sizeof(uint32_t) * n_attach);
+    plan.finish(d_scores, scores, n_trees);
+    plan.finish(d_counts, counts, n_counts);
+    plan.finish(d_attach, attach, attach ? n_attach : 0);
     return BBS_OK;
   } catch (...) {
     return fail(BBS_ERR_ALLOC, "allocation failed in bbs_score_trees");
@@ -1570,12 +1657,11 @@ int bbs_apply_moves(bbs_ctx *c, const uint64_t *dm, const float *betas,
     const auto out_beta = plan.take<float>(n_trees);
     const auto out_par = plan.take<bbs_move_params>(n_trees);
     const size_t out_end = plan.mark();
-    std::memcpy(rows.h, dm, sizeof(uint64_t) * words);
-    std::memcpy(in_betas.h, betas, sizeof(float) * n_trees);
-    if (raw)
-      std::memcpy(in_raw.h, raw, sizeof(bbs_raw_move) * n_trees);
-    else
-      std::memcpy(in_par.h, params, sizeof(bbs_move_params) * n_trees);
+    Drain drain{c->stream};
+    BBS_CUDA(plan.in(rows, dm, words), "scratch upload");
+    BBS_CUDA(plan.in(in_betas, betas, n_trees), "scratch upload");
+    BBS_CUDA(plan.in(in_raw, raw, raw ? n_trees : 0), "scratch upload");
+    BBS_CUDA(plan.in(in_par, params, raw ? 0 : n_trees), "scratch upload");
     BBS_CUDA(plan.to_device(0, out_begin), "scratch upload");
     BBS_CUDA(cudaMemsetAsync(out_rows.d, 0, sizeof(uint64_t) * words, c->stream), "memset");
     ApplyArgs a{};
@@ -1591,12 +1677,15 @@ int bbs_apply_moves(bbs_ctx *c, const uint64_t *dm, const float *betas,
     const int e = launch_apply(a, c->stream);
     if (e != 0) return cuda_fail(e, "apply kernel launch");
     BBS_CUDA(plan.to_host(out_begin, out_end), "result copy");
+    BBS_CUDA(plan.out(out_rows, dm_out, words), "result copy");
+    BBS_CUDA(plan.out(out_beta, beta_out, n_trees), "result copy");
+    BBS_CUDA(plan.out(out_par, params_out, n_trees), "result copy");
     r = sync_stream(c, "apply kernel");
+    drain.armed = false;
     if (r != BBS_OK) return r;
-    std::memcpy(dm_out, out_rows.h, sizeof(uint64_t) * words);
-    if (beta_out) std::memcpy(beta_out, out_beta.h, sizeof(float) * n_trees);
-    if (params_out)
-      std::memcpy(params_out, out_par.h, sizeof(bbs_move_params) * n_trees);
+    plan.finish(out_rows, dm_out, words);
+    plan.finish(out_beta, beta_out, n_trees);
+    plan.finish(out_par, params_out, n_trees);
     return BBS_OK;
   } catch (...) {
     return fail(BBS_ERR_ALLOC, "allocation failed in bbs_apply_moves");
@@ -1620,21 +1709,26 @@ int bbs_sumscore_grad(bbs_ctx *c, const uint64_t *dm, const float *alphas,
     ScratchPlan plan;
     plan.add<uint64_t>(words);
     plan.add<float>(6 * (size_t)n_trees);
-    plan.add<float>(3 * (size_t)n_trees);
+    for (int k = 0; k < 3; k++) plan.add<float>(n_trees);
     if (posterior) plan.add<float>(n_post);
     int r = plan.reserve(c);
     if (r != BBS_OK) return r;
     const auto rows = plan.take<uint64_t>(words);
     const auto tab = plan.take<float>(6 * (size_t)n_trees);
     const size_t out_begin = plan.mark();
-    const auto out = plan.take<float>(3 * (size_t)n_trees);
+    const auto d_logl = plan.take<float>(n_trees);
+    const auto d_da = plan.take<float>(n_trees);
+    const auto d_db = plan.take<float>(n_trees);
     const auto post = plan.take<float>(posterior ? n_post : 0);
     const size_t out_end = plan.mark();
-    std::memcpy(rows.h, dm, sizeof(uint64_t) * words);
+    std::vector<float> own;
+    Drain drain{c->stream};
+    BBS_CUDA(plan.in(rows, dm, words), "scratch upload");
     // per tree: alpha, beta, log(1-alpha), log beta, log alpha, log(1-beta)
+    float *ht = staging(tab, own, 6 * (size_t)n_trees);
     for (uint32_t t = 0; t < n_trees; t++) {
       const double a = alphas[t], b = betas[t];
-      float *tt = tab.h + 6 * (size_t)t;
+      float *tt = ht + 6 * (size_t)t;
       tt[0] = alphas[t];
       tt[1] = betas[t];
       tt[2] = (float)std::log1p(-a);
@@ -1642,25 +1736,32 @@ int bbs_sumscore_grad(bbs_ctx *c, const uint64_t *dm, const float *alphas,
       tt[4] = (float)std::log(a);
       tt[5] = (float)std::log1p(-b);
     }
+    if (!own.empty())
+      BBS_CUDA(plan.in(tab, own.data(), own.size()), "scratch upload");
     BBS_CUDA(plan.to_device(0, out_begin), "scratch upload");
     GradArgs a{};
     a.ds = c->ds;
     a.rows = reinterpret_cast<const uint32_t *>(rows.d);
     a.tables = tab.d;
     a.n_trees = (int)n_trees;
-    a.logl = out.d;
-    a.dalpha = out.d + n_trees;
-    a.dbeta = out.d + 2 * (size_t)n_trees;
+    a.logl = d_logl.d;
+    a.dalpha = d_da.d;
+    a.dbeta = d_db.d;
     a.posterior = posterior ? post.d : nullptr;
     const int e = launch_grad(a, c->q, c->stream);
     if (e != 0) return cuda_fail(e, "adjoint kernel launch");
     BBS_CUDA(plan.to_host(out_begin, out_end), "result copy");
+    BBS_CUDA(plan.out(d_logl, logl, n_trees), "result copy");
+    BBS_CUDA(plan.out(d_da, dalpha, n_trees), "result copy");
+    BBS_CUDA(plan.out(d_db, dbeta, n_trees), "result copy");
+    BBS_CUDA(plan.out(post, posterior, posterior ? n_post : 0), "result copy");
     r = sync_stream(c, "adjoint kernel");
+    drain.armed = false;
     if (r != BBS_OK) return r;
-    std::memcpy(logl, out.h, sizeof(float) * n_trees);
-    if (dalpha) std::memcpy(dalpha, out.h + n_trees, sizeof(float) * n_trees);
-    if (dbeta) std::memcpy(dbeta, out.h + 2 * (size_t)n_trees, sizeof(float) * n_trees);
-    if (posterior) std::memcpy(posterior, post.h, sizeof(float) * n_post);
+    plan.finish(d_logl, logl, n_trees);
+    plan.finish(d_da, dalpha, n_trees);
+    plan.finish(d_db, dbeta, n_trees);
+    plan.finish(post, posterior, posterior ? n_post : 0);
     return BBS_OK;
   } catch (...) {
     return fail(BBS_ERR_ALLOC, "allocation failed in bbs_sumscore_grad");
