@@ -17,6 +17,7 @@
 
 #include "bbs_internal.h"
 #include "bbs_layout.h"
+#include "bbs_incr.cuh"
 
 using namespace bbs;
 
@@ -221,6 +222,29 @@ int put_string(const std::string &s, char *buf, size_t cap, size_t *len) {
 // ------------------------------------------------------------------------
 // Context
 // ------------------------------------------------------------------------
+// Device memory that grows to the largest launch so far and is freed with
+// its owner.
+struct TableBuf {
+  uint32_t *p = nullptr;
+  size_t cap = 0;
+  ~TableBuf() { cudaFree(p); }
+  // (no launch that uses the old memory is in flight: runs are synchronous,
+  // an asynchronous one refuses the next until it is done)
+  bool reserve(size_t bytes) {
+    if (bytes <= cap) return true;
+    cudaFree(p);
+    p = nullptr;
+    cap = 0;
+    if (cudaMalloc(&p, bytes) != cudaSuccess) {
+      (void)cudaGetLastError();
+      p = nullptr;
+      return false;
+    }
+    cap = bytes;
+    return true;
+  }
+};
+
 struct bbs_ctx {
   int device = 0, n_sms = 0;
   int smem_sm = 0, smem_block = 0, smem_reserved = 0;  // per SM / block
@@ -253,6 +277,7 @@ struct bbs_ctx {
   uint8_t *d_scratch = nullptr, *h_scratch = nullptr;
   size_t scratch_cap = 0, mirror_cap = 0;
   uint64_t fingerprint = 0;  // of the dataset and parameters (checkpoints)
+  TableBuf table;            // global tables of wide rows (TablePlan)
 };
 
 namespace {
@@ -565,6 +590,25 @@ uint64_t fnv1a(uint64_t h, const void *p, size_t n) {
 template <typename T>
 uint64_t fnv1a_of(uint64_t h, const T &v) {
   return fnv1a(h, &v, sizeof(T));
+}
+
+// Whether chains with rows of five to eight words may take a table
+// (plan_tables): the max score at fixed rates that have codes.
+bool wide_tables(const DatasetDev &ds, const ModelDev &md, const float *terms) {
+  return md.score_mode == 0 && md.mp.cum_beta == 0.0f &&
+         make_code_host(terms[2], terms[4], terms[3], terms[5], ds.max_d,
+                        ds.max_m)
+             .usable;
+}
+
+// Device bytes of the global tables of a launch: its blocks are at most what
+// the chains need and what is resident.
+size_t table_bytes(const TablePlan &p, int slots, size_t n_chains, int n_sms,
+                   int smem_sm) {
+  const size_t want = (n_chains + slots - 1) / slots;
+  const size_t resident =
+      (size_t)std::max(1, smem_sm / std::max(1, p.smem)) * n_sms;
+  return std::min(want, resident) * slots * p.global;
 }
 
 // The dataset as the kernels see it and every parameter field (not the
@@ -912,17 +956,17 @@ namespace {
 
 // One-warp chains per block (1-8; they share the block's increment table)
 // that keep the most warps resident on an SM; ties keep the smaller block.
-int chain_smem(const bbs_ctx *c, int q, int wpc, int cpb) {
+TablePlan chain_plan(const bbs_ctx *c, int q, int wpc, int cpb) {
   return plan_tables((int)c->n_nodes, w32_of_nodes((int)c->n_nodes),
                      (int)c->n_cells, q, wpc, cpb, c->md.score_mode != 0, true,
-                     c->smem_block)
-      .smem;
+                     wide_tables(c->ds, c->md, c->terms), c->smem_block,
+                     c->smem_sm);
 }
 
 int pick_chains_per_block(const bbs_ctx *c, int q) {
   int best = 1, best_warps = 0;
   for (int cpb = 1; cpb * 32 <= chain_max_threads(q); cpb++) {
-    const int smem = chain_smem(c, q, 1, cpb);
+    const int smem = chain_plan(c, q, 1, cpb).smem;
     const int w = chain_resident_warps(smem, cpb, q, c->smem_sm, c->smem_block,
                                        c->smem_reserved);
     if (w > best_warps) {
@@ -1043,7 +1087,7 @@ int start_run(bbs_ctx *c, uint32_t n_steps, const bbs_raw_move *d_moves,
               bbs_step_trace *d_trace) {
   {
     const int cpb = c->wpc > 1 ? 1 : c->cpb;
-    const int smem = chain_smem(c, c->q, c->wpc, cpb);
+    const int smem = chain_plan(c, c->q, c->wpc, cpb).smem;
     if (32 * c->wpc * cpb > chain_max_threads(c->q) || smem > c->smem_block)
       return fail(BBS_ERR_SIZE,
                   "launch shape (%d cells per lane, %d warps per chain, %d "
@@ -1067,12 +1111,28 @@ int start_run(bbs_ctx *c, uint32_t n_steps, const bbs_raw_move *d_moves,
   a.cancel = c->d_cancel;
   a.status = c->d_status;
   a.wpc = c->wpc;
+  {
+    const int cpb = c->wpc > 1 ? 1 : c->cpb;
+    TablePlan p = chain_plan(c, c->q, c->wpc, cpb);
+    // replays and traces of rows of five to eight words go through the ring
+    const bool rec = d_moves != nullptr || d_trace != nullptr;
+    if ((rec && c->n_nodes > 128) ||
+        !c->table.reserve(table_bytes(p, cpb, c->n_chains, c->n_sms,
+                                      c->smem_sm)))
+      p = TablePlan{0, false,
+                    chain_launch_smem((int)c->n_nodes, (int)c->n_cells, c->q,
+                                      c->wpc, cpb, c->md.score_mode != 0), 0, 0};
+    a.chunks = p.chunks;
+    a.with_inc = p.inc ? 1 : 0;
+    a.smem = p.smem;
+    a.ns = p.ns;
+    a.table = c->table.p;
+  }
   *c->h_cancel = 0;
   BBS_CUDA(cudaMemsetAsync(c->d_status, 0, sizeof(int) * kStatusWords, c->stream),
            "cudaMemset");
   BBS_CUDA(cudaEventRecord(c->ev0, c->stream), "cudaEventRecord");
-  const int e = launch_mcmc(a, c->q, c->cpb, c->n_sms, c->smem_block,
-                            c->stream);
+  const int e = launch_mcmc(a, c->q, c->cpb, c->n_sms, c->stream);
   if (e != 0) return cuda_fail(e, "chain kernel launch");
   BBS_CUDA(cudaEventRecord(c->ev1, c->stream), "cudaEventRecord");
   return BBS_OK;
@@ -1222,7 +1282,7 @@ int bbs_autotune(bbs_ctx *c, uint32_t probe_steps, float *best_ms) {
         for (int cpb : {1, 2, 4, 7, 8}) {
           if (wpc > 1 && cpb > 1) continue;
           if (32 * wpc * cpb > chain_max_threads(q)) continue;
-          if (chain_smem(c, q, wpc, cpb) > c->smem_block)
+          if (chain_plan(c, q, wpc, cpb).smem > c->smem_block)
             continue;  // too large a block
           c->q = q;
           c->wpc = wpc;
@@ -1919,6 +1979,7 @@ struct bbs_batch {
   struct Group {
     int w32 = 0, max_nodes = 0, max_cells = 0;
     int only_ds = -1;  // the group's dataset when it has only one
+    bool wide = true;  // every dataset may take tables of wide rows
     std::vector<uint32_t> units;
     uint32_t *d_units = nullptr;
   };
@@ -1932,6 +1993,8 @@ struct bbs_batch {
   uint32_t graph_steps = 0;
   float last_ms = 0.0f;
   uint64_t fingerprint = 0;  // of all datasets and parameters (checkpoints)
+  TableBuf table;            // global tables of wide rows (TablePlan)
+  int smem_sm = 0;
 };
 
 namespace {
@@ -2042,6 +2105,9 @@ int batch_build_groups(bbs_batch *b) {
     g.only_ds = (int)b->chain_ds[g.units[0]];
     for (const uint32_t u : g.units)
       if ((int)b->chain_ds[u] != g.only_ds) g.only_ds = -1;
+    for (uint32_t d = 0; d < b->n_datasets && w > 4; d++)
+      if (key[d] == w)
+        g.wide = g.wide && wide_tables(b->ds[d], b->md[d], &b->terms[8 * d]);
     BBS_CUDA(cudaMalloc(&g.d_units, sizeof(uint32_t) * g.units.size()), "cudaMalloc");
     BBS_CUDA(cudaMemcpy(g.d_units, g.units.data(), sizeof(uint32_t) * g.units.size(),
                         cudaMemcpyHostToDevice), "cudaMemcpy");
@@ -2072,16 +2138,32 @@ int group_wpb(const bbs_batch *b, const bbs_batch::Group &grp) {
   return std::min(b->wpb, chain_max_threads(group_q(b, grp)) / 32);
 }
 
+TablePlan group_plan(const bbs_batch *b, const bbs_batch::Group &grp) {
+  return plan_tables(grp.max_nodes, grp.w32, grp.max_cells, group_q(b, grp),
+                     b->wpc, group_wpb(b, grp) / b->wpc, b->sum,
+                     grp.only_ds >= 0, grp.wide, b->smem_block, b->smem_sm);
+}
+
+// The groups' global tables, one after the other in b->table; before a
+// capture, which may not allocate.  False: not enough memory (the groups that
+// would need it take the ring).
+bool batch_reserve_tables(bbs_batch *b) {
+  size_t bytes = 0;
+  for (const auto &grp : b->groups) {
+    const TablePlan p = group_plan(b, grp);
+    if (p.global)
+      bytes += table_bytes(p, group_wpb(b, grp) / b->wpc, grp.units.size(),
+                           b->n_sms, b->smem_sm);
+  }
+  return b->table.reserve(bytes);
+}
+
 // Whether every launch group of the current shape fits a block: its shared
 // memory within the device's limit (threads are clamped to the kernel's
 // bounds by group_wpb).  Checked before a run launches anything.
 bool batch_shape_fits(const bbs_batch *b) {
   for (const auto &grp : b->groups) {
-    const int smem =
-        plan_tables(grp.max_nodes, grp.w32, grp.max_cells, group_q(b, grp),
-                    b->wpc, group_wpb(b, grp) / b->wpc, b->sum,
-                    grp.only_ds >= 0, b->smem_block)
-            .smem;
+    const int smem = group_plan(b, grp).smem;
     if (smem > b->smem_block) return false;
   }
   return true;
@@ -2100,6 +2182,7 @@ int batch_issue(bbs_batch *b, uint32_t n_steps) {
   if (b->groups.size() > (size_t)kMaxW32)
     return fail(BBS_ERR_STATE, "%zu launch groups, at most %d", b->groups.size(),
                 kMaxW32);
+  size_t table_at = 0;
   BBS_CUDA(cudaMemsetAsync(b->d_counters, 0, sizeof(unsigned int) * kMaxW32,
                            b->stream), "memset");
   BBS_CUDA(cudaMemsetAsync(b->d_status, 0, sizeof(int) * kStatusWords, b->stream),
@@ -2129,9 +2212,22 @@ int batch_issue(bbs_batch *b, uint32_t n_steps) {
     a.table_ds = grp.only_ds;
     const int q = group_q(b, grp);
     a.wpc = b->wpc;
-    const int e = launch_batch(a, grp.w32, grp.max_cells, q, b->sum,
-                               group_wpb(b, grp), b->n_sms, b->smem_block,
-                               b->side[g]);
+    TablePlan p = group_plan(b, grp);
+    const int slots = group_wpb(b, grp) / b->wpc;
+    const size_t tb = p.global ? table_bytes(p, slots, grp.units.size(),
+                                             b->n_sms, b->smem_sm)
+                               : 0;
+    if (table_at + tb > b->table.cap)
+      p = TablePlan{0, false, chain_launch_smem(grp.max_nodes, grp.max_cells, q,
+                                                b->wpc, slots, b->sum), 0, 0};
+    a.chunks = p.chunks;
+    a.with_inc = p.inc ? 1 : 0;
+    a.smem = p.smem;
+    a.ns = p.ns;
+    a.table = b->table.p + table_at / 4;
+    table_at += tb;
+    const int e = launch_batch(a, grp.w32, q, b->sum, group_wpb(b, grp),
+                               b->n_sms, b->side[g]);
     if (e != 0) return cuda_fail(e, "batch kernel launch");
     BBS_CUDA(cudaEventRecord(b->side_ev[g], b->side[g]), "event");
     BBS_CUDA(cudaStreamWaitEvent(b->stream, b->side_ev[g], 0), "wait");
@@ -2180,6 +2276,8 @@ int bbs_batch_create(bbs_batch **out, uint32_t n_datasets,
     b->sum = sum;
     cudaGetDevice(&b->device);
     cudaDeviceGetAttribute(&b->n_sms, cudaDevAttrMultiProcessorCount, b->device);
+    cudaDeviceGetAttribute(&b->smem_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor,
+                           b->device);
     cudaDeviceGetAttribute(&b->smem_block, cudaDevAttrMaxSharedMemoryPerBlockOptin,
                            b->device);
     cudaError_t e = cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking);
@@ -2328,6 +2426,7 @@ int bbs_batch_run(bbs_batch *b, uint32_t n_steps) {
     if (b->graph) cudaGraphExecDestroy(b->graph);
     b->graph = nullptr;
     cudaGraph_t g = nullptr;
+    (void)batch_reserve_tables(b);
     BBS_CUDA(cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal),
              "begin capture");
     const int r = batch_issue(b, n_steps);
@@ -2443,6 +2542,7 @@ int bbs_batch_autotune(bbs_batch *b, uint32_t probe_steps, float *best_ms) {
           r = bbs_batch_set_chain_warps(b, sh.wpc);
           if (r != BBS_OK) return r;
           if (!batch_shape_fits(b)) continue;  // too large a block
+          (void)batch_reserve_tables(b);
           BBS_CUDA(cudaEventRecord(b->ev0, b->stream), "event");
           r = batch_issue(b, probe_steps);
           if (r != BBS_OK) return r;

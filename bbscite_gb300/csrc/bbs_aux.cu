@@ -10,8 +10,7 @@ int pick_q(int n_cells) {
   return std::min(kMaxQ, std::max(1, (n_cells + 31) / 32));
 }
 
-int launch_mcmc(const RunArgs &a, int q, int cpb, int n_sms, int smem_block,
-                void *stream) {
+int launch_mcmc(const RunArgs &a, int q, int cpb, int n_sms, void *stream) {
   const int w32 = w32_of_nodes(a.ds.n_nodes);
   cudaStream_t s = (cudaStream_t)stream;
   const bool sum = a.md.score_mode == 1;
@@ -20,8 +19,8 @@ int launch_mcmc(const RunArgs &a, int q, int cpb, int n_sms, int smem_block,
   switch (w32) {
 #define BBS_MCMC_CASE(W)                                            \
   case W:                                                           \
-    return rec ? launch_mcmc_w<W, true>(a, q, sum, cpb, n_sms, smem_block, s) \
-               : launch_mcmc_w<W, false>(a, q, sum, cpb, n_sms, smem_block, s);
+    return rec ? launch_mcmc_w<W, true>(a, q, sum, cpb, n_sms, s)   \
+               : launch_mcmc_w<W, false>(a, q, sum, cpb, n_sms, s);
     BBS_MCMC_CASE(1)
     BBS_MCMC_CASE(2)
     BBS_MCMC_CASE(3)
@@ -35,17 +34,14 @@ int launch_mcmc(const RunArgs &a, int q, int cpb, int n_sms, int smem_block,
   }
 }
 
-int launch_batch(const BatchArgs &b, int w32, int max_cells, int q, bool sum,
-                 int wpb, int n_sms, int smem_block, void *stream) {
+int launch_batch(const BatchArgs &b, int w32, int q, bool sum, int wpb,
+                 int n_sms, void *stream) {
   cudaStream_t s = (cudaStream_t)stream;
   switch (w32) {
 #define BBS_BATCH_CASE(W)                                                   \
   case W:                                                                   \
-    return b.wpc > 1                                                        \
-               ? launch_batch_w<W, true>(b, max_cells, q, sum, wpb, n_sms,  \
-                                         smem_block, s)                     \
-               : launch_batch_w<W, false>(b, max_cells, q, sum, wpb, n_sms, \
-                                          smem_block, s);
+    return b.wpc > 1 ? launch_batch_w<W, true>(b, q, sum, wpb, n_sms, s)    \
+                     : launch_batch_w<W, false>(b, q, sum, wpb, n_sms, s);
     BBS_BATCH_CASE(1)
     BBS_BATCH_CASE(2)
     BBS_BATCH_CASE(3)

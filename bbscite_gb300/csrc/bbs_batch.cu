@@ -7,14 +7,12 @@
 namespace bbs {
 
 template <int W, bool MULTI>
-int launch_batch_w(const BatchArgs &b, int max_cells, int q, bool sum, int wpb,
-                   int n_sms, int smem_block, cudaStream_t s) {
+int launch_batch_w(const BatchArgs &b, int q, bool sum, int wpb, int n_sms,
+                   cudaStream_t s) {
 #define BBS_CASE(QQ)                                                   \
-  case QQ:                                                                   \
-    return sum ? launch_batch_t<W, QQ, true, MULTI>(b, max_cells, wpb, n_sms, \
-                                                    smem_block, s)           \
-               : launch_batch_t<W, QQ, false, MULTI>(b, max_cells, wpb,      \
-                                                     n_sms, smem_block, s);
+  case QQ:                                                             \
+    return sum ? launch_batch_t<W, QQ, true, MULTI>(b, wpb, n_sms, s)  \
+               : launch_batch_t<W, QQ, false, MULTI>(b, wpb, n_sms, s);
   switch (q) {
     BBS_CASE(1)
     BBS_CASE(2)
@@ -28,7 +26,7 @@ int launch_batch_w(const BatchArgs &b, int max_cells, int q, bool sum, int wpb,
 }
 
 template int launch_batch_w<BBS_W, BBS_MULTI != 0>(const BatchArgs &, int,
-                                                   int, bool, int, int, int,
+                                                   bool, int, int,
                                                    cudaStream_t);
 
 }  // namespace bbs

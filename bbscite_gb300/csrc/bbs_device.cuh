@@ -112,6 +112,34 @@ __device__ __forceinline__ void philox_fill(uint4 *buf, uint64_t seed,
                             key);
 }
 
+// The moves of 16 consecutive steps in place of their blocks (the same 512
+// bytes): a pair of lanes draws the two blocks of a step and its even lane
+// makes the move of them, so that a step reads its move whole.
+__device__ __forceinline__ void moves_fill(uint4 *buf, const ModelDev &md,
+                                           uint32_t n_nodes, uint32_t chain,
+                                           uint64_t step0, bool always_jump,
+                                           int lane) {
+  const uint2 key = make_uint2((uint32_t)md.seed, (uint32_t)(md.seed >> 32));
+  const uint64_t step = step0 + (uint64_t)(lane >> 1);
+  const uint4 a = philox4x32_10(make_uint4((uint32_t)step,
+                                           (uint32_t)(step >> 32), chain,
+                                           (uint32_t)(lane & 1)),
+                                key);
+  uint4 b;
+  b.x = __shfl_down_sync(BBS_FULL_MASK, a.x, 1);
+  b.y = __shfl_down_sync(BBS_FULL_MASK, a.y, 1);
+  b.z = __shfl_down_sync(BBS_FULL_MASK, a.z, 1);
+  b.w = __shfl_down_sync(BBS_FULL_MASK, a.w, 1);
+  if ((lane & 1) == 0) {
+    const bbs_raw_move m = move_from_words(md.mp, n_nodes, a, b, always_jump);
+    buf[lane] = make_uint4((uint32_t)m.move_type, m.raw_v, m.raw_w,
+                           __float_as_uint(m.raw_descendant_of_v));
+    buf[lane + 1] = make_uint4(__float_as_uint(m.raw_nondescendant_of_v),
+                               __float_as_uint(m.beta_jump),
+                               __float_as_uint(m.acceptance_level), 0u);
+  }
+}
+
 // ------------------------------------------------------------------------
 // Bit rows
 // ------------------------------------------------------------------------

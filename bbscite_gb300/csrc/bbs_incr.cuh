@@ -1,26 +1,31 @@
-// bbs_incr.cuh -- proposals evaluated from what they change (rows of up to
-// four words).
+// bbs_incr.cuh -- proposals evaluated from what they change.
 //
 // A tree move leaves most nodes' ancestor sets as they are; the others, two
 // disjoint classes of nodes, all change by the same genes, so every cell's
 // counts (d, m) change there by one constant per class and cell.  A chain
-// therefore keeps a table of every node and cell of its current tree in
-// shared memory and reads a proposal off it:
+// therefore keeps a table of every node and cell of its current tree and
+// reads a proposal off it:
 //   - max score: the table holds integer codes that order a cell's nodes as
 //     their scores do (MaxCode), 16 bits per cell; a proposal's best nodes
 //     are the maxima over the unchanged nodes and the two shifted classes;
-//   - sum score: the table holds the counts.  A proposal is first bounded
-//     from above by the terms that move (two exponentials per class and
-//     cell); only one that the bound does not reject is summed, over the
-//     proposal's canonical order, term by term as everywhere else.
+//   - sum score (rows of up to four words): the table holds the counts.  A
+//     proposal is first bounded from above by the terms that move (two
+//     exponentials per class and cell); only one that the bound does not
+//     reject is summed, over the proposal's canonical order, term by term as
+//     everywhere else.
 // The rows, the parent vector and the table follow accepted moves only.
 // Decisions, scores and trees are those of an evaluation of every node.
 //
-// Measured against evaluating every node of every proposal (GB300, 1024
-// chains at 95 x 96 after 20,000 steps; 10-20 % of the proposals accepted):
-// max score 98 -> 307 M chain-steps/s, sum score with Langevin error moves
-// 121 -> 168 M; 128 uneven datasets of 32 chains 3.5 times as fast; 8 chains
-// at 63 x 64 6.4 -> 3.4 us a step.
+// Measured against evaluating every node of every proposal (GB300, 10-30 % of
+// the proposals accepted): 1024 chains at 95 x 96 max score 98 -> 380 M
+// chain-steps/s, sum score with Langevin error moves 121 -> 188 M; at 255 x
+// 512 max score 8.0 -> 18.7 M; 128 uneven datasets of 32 chains 4.4 times as
+// fast; 8 chains at 63 x 64 6.3 -> 2.0 us a step.
+// What bounds it now is a step's serial chain of short dependent pieces (draw,
+// descendant sets, table loads, maxima, reductions: some 4 clocks for each of
+// 1,300 instructions at 1.8 warps per scheduler), and for the sum score the
+// special-function unit where a proposal is summed (six exponentials for two
+// nodes and three cells, 8 clocks each).
 #pragma once
 #include "bbs_device.cuh"
 
@@ -48,86 +53,133 @@ namespace bbs {
 //          non-finite logs have none).
 struct MaxCode {
   int P, Q, s, au, bu, off;
-  uint32_t invP, invQ;  // floor(2^32 / P) + 1: exact quotients of x < 2^23
+  uint32_t invP, invQ;  // floor(2^32 / P) + 1: quotients of x < 2^24
   float margin;
   bool usable, exact;
 };
 
-inline __device__ __noinline__ MaxCode make_code(float l00, float l01, float l10,
-                                          float l11, int dmax, int mmax,
-                                          int lane) {
+// Neighbouring fractions al / bl < |c1| / |c2| < au / bu, found so far.
+struct Neighbours {
+  int al = 0, bl = 1, au = 1, bu = 0;
+  bool exact = true;
+  __host__ __device__ void below(int a, int b) {
+    if (a * bl > al * b || (a * bl == al * b && b < bl)) {
+      al = a;
+      bl = b;
+    }
+  }
+  __host__ __device__ void above(int a, int b) {
+    if (a * bu < au * b || (a * bu == au * b && b < bu)) {
+      au = a;
+      bu = b;
+    }
+  }
+  // the fractions with denominator b; near-ties count as below
+  __host__ __device__ void denominator(int b, float a1, float a2,
+                                       float margin, int mmax) {
+    int a = (int)fminf(floorf((float)b * (a1 / a2)), (float)mmax);
+    const float x = (float)b * a1;
+    if (a < mmax && (float)(a + 1) * a2 - x <= margin) a++;
+    exact = exact && fabsf(x - (float)a * a2) > margin;
+    below(a, b);
+    if (a < mmax) above(a + 1, b);
+  }
+};
+
+// What the log table alone says: sign, margin, whether codes can exist.
+__host__ __device__ inline MaxCode code_begin(float l00, float l01, float l10,
+                                              float l11, int dmax, int mmax,
+                                              float &a1, float &a2) {
   MaxCode k;
   const float c1 = l01 - l00, c2 = l11 - l10;
-  const float a1 = fabsf(c1), a2 = fabsf(c2);
+  a1 = fabsf(c1);
+  a2 = fabsf(c2);
   k.s = c1 < 0.0f && c2 > 0.0f ? 1 : -1;
   // rounding of two scores (four products and three sums each, all within
-  // `big`), of c1 and c2 and of the gaps below: 16 units of 2^-24 big
+  // `big`), of c1 and c2 and of the gaps: 16 units of 2^-24 big
   const float big = dmax * fmaxf(fabsf(l00), fabsf(l01)) +
                     mmax * fmaxf(fabsf(l10), fabsf(l11));
   k.margin = big * 1.9073486e-06f;  // 2^-19: twice that
   k.usable = c1 * c2 < 0.0f && a1 > 1.0e-6f && a2 > 1.0e-6f && big < 1.0e6f;
-  bool exact = a1 > k.margin && a2 > k.margin;
-  // neighbours of a1 / a2 among the fractions a / b, b <= dmax, a <= mmax
-  int al = 0, bl = 1, au = 1, bu = 0;
-  if (k.usable) {
-    const float ratio = a1 / a2;
-    for (int b = lane + 1; b <= dmax; b += 32) {
-      int a = (int)fminf(floorf((float)b * ratio), (float)mmax);
-      const float x = (float)b * a1;
-      if (a < mmax && (float)(a + 1) * a2 - x <= k.margin) a++;
-      exact = exact && fabsf(x - (float)a * a2) > k.margin;
-      if (a * bl > al * b) {
-        al = a;
-        bl = b;
-      }
-      if (a < mmax && (a + 1) * bu < au * b) {
-        au = a + 1;
-        bu = b;
-      }
-    }
-  }
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    const int xa = __shfl_xor_sync(BBS_FULL_MASK, al, o),
-              xb = __shfl_xor_sync(BBS_FULL_MASK, bl, o),
-              ya = __shfl_xor_sync(BBS_FULL_MASK, au, o),
-              yb = __shfl_xor_sync(BBS_FULL_MASK, bu, o);
-    if (xa * bl > al * xb || (xa * bl == al * xb && xb < bl)) {
-      al = xa;
-      bl = xb;
-    }
-    if (ya * bu < au * yb || (ya * bu == au * yb && yb < bu)) {
-      au = ya;
-      bu = yb;
-    }
-  }
-  k.P = al + au;
-  k.Q = bl + bu;
+  k.exact = a1 > k.margin && a2 > k.margin;
+  return k;
+}
+
+__host__ __device__ inline void code_end(MaxCode &k, const Neighbours &f,
+                                         int dmax, int mmax) {
+  k.P = f.al + f.au;
+  k.Q = f.bl + f.bu;
   if (k.P == 1) {  // decode divides by P > 1: the next weights in between
-    k.P += au;
-    k.Q += bu;
+    k.P += f.au;
+    k.Q += f.bu;
   }
-  k.au = au;
-  k.bu = bu;
+  k.au = f.au;
+  k.bu = f.bu;
   k.off = k.s > 0 ? k.P * dmax : k.Q * mmax;
   // neighbours in lowest terms; near-ties sorted inconsistently are not
-  k.usable = k.usable && au * bl - al * bu == 1 &&
+  k.usable = k.usable && f.au * f.bl - f.al * f.bu == 1 &&
              k.P * dmax + k.Q * mmax <= 65535;
-  k.exact = __all_sync(BBS_FULL_MASK, exact);
+  k.exact = k.exact && f.exact;
   k.invP = 0xFFFFFFFFu / (uint32_t)k.P + 1u;
   k.invQ = 0xFFFFFFFFu / (uint32_t)k.Q + 1u;
+}
+
+// The codes of a log table, the denominators spread over the lanes.
+inline __device__ __noinline__ MaxCode make_code(float l00, float l01,
+                                                 float l10, float l11,
+                                                 int dmax, int mmax,
+                                                 int lane) {
+  float a1, a2;
+  MaxCode k = code_begin(l00, l01, l10, l11, dmax, mmax, a1, a2);
+  Neighbours f;
+  if (k.usable)
+    for (int b = lane + 1; b <= dmax; b += 32)
+      f.denominator(b, a1, a2, k.margin, mmax);
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    const int xa = __shfl_xor_sync(BBS_FULL_MASK, f.al, o),
+              xb = __shfl_xor_sync(BBS_FULL_MASK, f.bl, o),
+              ya = __shfl_xor_sync(BBS_FULL_MASK, f.au, o),
+              yb = __shfl_xor_sync(BBS_FULL_MASK, f.bu, o);
+    f.below(xa, xb);
+    f.above(ya, yb);
+  }
+  f.exact = __all_sync(BBS_FULL_MASK, f.exact);
+  code_end(k, f, dmax, mmax);
+  return k;
+}
+
+// The same on the host: whether a launch plans for them.
+inline MaxCode make_code_host(float l00, float l01, float l10, float l11,
+                              int dmax, int mmax) {
+  float a1, a2;
+  MaxCode k = code_begin(l00, l01, l10, l11, dmax, mmax, a1, a2);
+  Neighbours f;
+  if (k.usable)
+    for (int b = 1; b <= dmax; b++) f.denominator(b, a1, a2, k.margin, mmax);
+  code_end(k, f, dmax, mmax);
   return k;
 }
 
 // (d, m) of a code: T0 = Q m - P d.  The solutions are (bu T0 - Q t,
 // au T0 - P t); with T0 >= 0 the smallest d >= 0 gives m >= 0, with T0 < 0
 // the smallest m >= 0 gives d > 0, and the next ones exceed the cell's bits.
+// The quotient t comes from a reciprocal, exact for dividends below 2^23 (at
+// most 128 nodes); WIDE dividends reach 2^24 and may give one too many.
+template <bool WIDE>
 __device__ __forceinline__ void decode(const MaxCode &k, uint32_t T, int &d,
                                        int &m) {
   const int T0 = k.s * ((int)T - k.off);
   const uint32_t a = (uint32_t)abs(T0);
-  const int t = T0 >= 0 ? (int)__umulhi((uint32_t)k.bu * a, k.invQ)
-                        : -(int)__umulhi((uint32_t)(k.au * (int)a + k.P - 1), k.invP);
+  const bool up = T0 >= 0;
+  const uint32_t x = up ? (uint32_t)k.bu * a
+                        : (uint32_t)(k.au * (int)a + k.P - 1);
+  uint32_t q = __umulhi(x, up ? k.invQ : k.invP);
+  if constexpr (WIDE) {
+    const uint32_t den = (uint32_t)(up ? k.Q : k.P);
+    if (q * den > x) q--;
+  }
+  const int t = up ? (int)q : -(int)q;
   d = k.bu * T0 - k.Q * t;
   m = k.au * T0 - k.P * t;
 }
@@ -138,11 +190,37 @@ __device__ __forceinline__ void decode(const MaxCode &k, uint32_t T, int &d,
 // = 1, wm = 256.  Chunk c holds the warp's cells from 32 wpc Q c on, as
 // load_cells takes them.
 // ------------------------------------------------------------------------
+// One chunk's part of it: nodes below ns in shared memory, the others (rows
+// of five to eight words only, where 256 nodes x 512 cells take 256 KB) in
+// global memory, which stays in L2 for the chains at work.
+template <int W32, int Q>
+struct Table {
+  static constexpr int NW = kPackWords<Q>;
+  uint32_t *s, *g;
+  int ns;
+  __device__ __forceinline__ uint32_t *at(int j) const {
+    if constexpr (W32 <= 4) return s + j * 32 * NW;
+    return j < ns ? s + j * 32 * NW : g + (j - ns) * 32 * NW;
+  }
+  __device__ __forceinline__ void ld(int j, int lane,
+                                     uint32_t (&k)[NW]) const {
+    ld_pack<Q>(at(j), lane, k);
+  }
+  __device__ __forceinline__ void st(int j, int lane,
+                                     const uint32_t (&k)[NW]) const {
+    st_pack<Q>(at(j), lane, k);
+  }
+  __device__ __forceinline__ Table chunk(int c, int n) const {
+    return Table{s + c * ns * 32 * NW, g + c * (n - ns) * 32 * NW, ns};
+  }
+};
+
 // From the ancestor rows by masked popcounts (any rows): at the start of a
 // launch and after the rare moves that are not followed node by node.
 template <int W32, int Q>
 __device__ __noinline__ void fill_table(const uint32_t *rows,
-                                        const DatasetDev *ds, uint32_t *tab,
+                                        const DatasetDev *ds,
+                                        const Table<W32, Q> tab,
                                         int chunks, int wpc, int wic,
                                         int lane, int off, int wd, int wm) {
   constexpr int RS = rs_of_w32(W32);
@@ -162,7 +240,7 @@ __device__ __noinline__ void fill_table(const uint32_t *rows,
         k[q >> 1] += (uint32_t)(off + wd * masked_popc<W32>(cb.D[q], a) +
                                 wm * masked_popc<W32>(cb.M[q], a))
                      << (16 * (q & 1));
-      st_pack<Q>(tab, (c * n + j) * 32 + lane, k);
+      tab.chunk(c, n).st(j, lane, k);
     }
   }
   __syncwarp();
@@ -359,15 +437,15 @@ struct Packed {
 
 // The classes' changes as packed differences (their sum with an entry is the
 // new entry, field borrows included).
-template <int Q, int NW = kPackWords<Q>>
-__device__ __forceinline__ void class_deltas(const uint32_t *tab,
+template <int W32, int Q, int NW = kPackWords<Q>>
+__device__ __forceinline__ void class_deltas(const Table<W32, Q> &tab,
                                              const Delta &x, int lane,
                                              Packed<NW> &dv, Packed<NW> &dw) {
   uint32_t a[NW], b[NW], c[NW], e[NW];
-  ld_pack<Q>(tab, (int)x.a0 * 32 + lane, a);
-  ld_pack<Q>(tab, (int)x.b0 * 32 + lane, b);
-  ld_pack<Q>(tab, (int)x.a1 * 32 + lane, c);
-  ld_pack<Q>(tab, (int)x.b1 * 32 + lane, e);
+  tab.ld((int)x.a0, lane, a);
+  tab.ld((int)x.b0, lane, b);
+  tab.ld((int)x.a1, lane, c);
+  tab.ld((int)x.b1, lane, e);
 #pragma unroll
   for (int i = 0; i < NW; i++) {
     dv.k[i] = a[i] - b[i];
@@ -381,17 +459,18 @@ __device__ __forceinline__ void class_deltas(const uint32_t *tab,
 
 // Adds the classes' changes to the table, or takes them back.
 template <int W32, int Q, int NW = kPackWords<Q>>
-__device__ __noinline__ void apply_classes(uint32_t *tab, uint8_t *list,
-                                           const Delta x,
-                                           const NodeSets<W32> C,
-                                           Packed<NW> dv, Packed<NW> dw,
-                                           bool back, int lane) {
+__device__ __forceinline__ void apply_classes(const Table<W32, Q> &tab,
+                                              uint8_t *list,
+                                              const Delta &x,
+                                              const NodeSets<W32> &C,
+                                              Packed<NW> dv, Packed<NW> dw,
+                                              bool back, int lane) {
   auto swap_entries = [&]() {
     uint32_t a[NW], b[NW];
-    ld_pack<Q>(tab, (int)x.v * 32 + lane, a);
-    ld_pack<Q>(tab, (int)x.w * 32 + lane, b);
-    st_pack<Q>(tab, (int)x.v * 32 + lane, b);
-    st_pack<Q>(tab, (int)x.w * 32 + lane, a);
+    tab.ld((int)x.v, lane, a);
+    tab.ld((int)x.w, lane, b);
+    tab.st((int)x.v, lane, b);
+    tab.st((int)x.w, lane, a);
   };
   if (back && x.swap) swap_entries();
   int nv;
@@ -403,76 +482,173 @@ __device__ __noinline__ void apply_classes(uint32_t *tab, uint8_t *list,
       dw.k[i] = 0u - dw.k[i];
     }
   }
-#pragma unroll 2
-  for (int c = 0; c < nc; c++) {
-    const int j = list[c];
-    uint32_t k[NW];
-    ld_pack<Q>(tab, j * 32 + lane, k);
+  // (every load of a batch before its stores: one node at a time waited some
+  // 100 clocks for each)
+  constexpr int B = W32 > 4 ? 8 : 4;
+#pragma unroll 1
+  for (int c0 = 0; c0 < nc; c0 += B) {
+    uint32_t k[B][NW];
+    int j[B];
 #pragma unroll
-    for (int i = 0; i < NW; i++) k[i] += c < nv ? dv.k[i] : dw.k[i];
-    st_pack<Q>(tab, j * 32 + lane, k);
+    for (int b = 0; b < B; b++) j[b] = (int)list[min(c0 + b, nc - 1)];
+#pragma unroll
+    for (int b = 0; b < B; b++) tab.ld(j[b], lane, k[b]);
+#pragma unroll
+    for (int b = 0; b < B; b++) {
+#pragma unroll
+      for (int i = 0; i < NW; i++) k[b][i] += c0 + b < nv ? dv.k[i] : dw.k[i];
+      if (c0 + b < nc) tab.st(j[b], lane, k[b]);
+    }
   }
   if (!back && x.swap) swap_entries();
   __syncwarp();  // the list has been read
 }
 
+// Taking a rejected proposal back, out of line: the bound leaves few of them.
+template <int W32, int Q, int NW = kPackWords<Q>>
+__device__ __noinline__ void take_back(const Table<W32, Q> tab, uint8_t *list,
+                                       const Delta x, const NodeSets<W32> C,
+                                       const Packed<NW> dv,
+                                       const Packed<NW> dw, int lane) {
+  apply_classes<W32, Q>(tab, list, x, C, dv, dw, true, lane);
+}
+
 // ------------------------------------------------------------------------
 // Max score: a proposal's largest codes
 // ------------------------------------------------------------------------
-// The largest code of each cell over the proposal's nodes: the unchanged
-// ones (the root is always one) and each class's largest, shifted.  list
-// holds the nc changed nodes, the first nv of class v.
-template <int W32, int Q, int NW = kPackWords<Q>>
-__device__ __forceinline__ void scan_codes(const uint32_t *tab, int n,
+// best = max(best, k) field by field over the nodes b < 8 whose bit of u is
+// set.  Codes are at least 0 and the root always counts, so the others are
+// masked to 0; as branches or predicated maxima a group of eight took 216 and
+// 144 clocks, masked 100 (one warp, two words an entry).
+template <int NW>
+__device__ __forceinline__ void max8(uint32_t (&best)[NW],
+                                     const uint32_t (&k)[8][NW], uint32_t u) {
+#pragma unroll
+  for (int b = 0; b < 8; b++) {
+    const uint32_t m = (uint32_t)((int)(u << (31 - b)) >> 31);
+#pragma unroll
+    for (int i = 0; i < NW; i++) best[i] = __vmaxu2(best[i], k[b][i] & m);
+  }
+}
+
+// A node's entries in CH chunks of a table, side by side.
+template <int Q, int CH, int NW = kPackWords<Q>>
+__device__ __forceinline__ void ld_chunks(const uint32_t *t, int chunk_words,
+                                          int idx, uint32_t (&k)[CH * NW]) {
+#pragma unroll
+  for (int c = 0; c < CH; c++) {
+    uint32_t e[NW];
+    ld_pack<Q>(t + c * chunk_words, idx, e);
+#pragma unroll
+    for (int i = 0; i < NW; i++) k[c * NW + i] = e[i];
+  }
+}
+
+// max8 over nodes first .. first + count - 1 (first a multiple of 8) at t:
+// whole groups, the next one's loads under the current one, then what is
+// left.
+template <int W32, int Q, int CH, int NW = kPackWords<Q>>
+__device__ __forceinline__ void max_nodes(uint32_t (&best)[CH * NW],
+                                          const uint32_t *t, int chunk_words,
+                                          const uint32_t (&un)[W32], int first,
+                                          int count, int lane) {
+  auto bits = [&](int j) {
+    return pick<W32>(un, (uint32_t)j >> 5) >> (j & 31);
+  };
+  int j = 0;
+#pragma unroll 2
+  for (; j + 8 <= count; j += 8) {
+    uint32_t k[8][CH * NW];
+#pragma unroll
+    for (int b = 0; b < 8; b++)
+      ld_chunks<Q, CH>(t, chunk_words, (j + b) * 32 + lane, k[b]);
+    max8<CH * NW>(best, k, bits(first + j));
+  }
+  if (j < count) {
+    uint32_t k[8][CH * NW];
+#pragma unroll
+    for (int b = 0; b < 8; b++)
+      ld_chunks<Q, CH>(t, chunk_words, min(j + b, count - 1) * 32 + lane, k[b]);
+    max8<CH * NW>(best, k, bits(first + j) & ((1u << (count - j)) - 1u));
+  }
+}
+
+// The largest code of each cell of CH chunks over the proposal's nodes: the
+// unchanged ones (the root is always one) and each class's largest, shifted.
+// list holds the nc changed nodes, the first nv of class v.  Two chunks at a
+// time share the masks and the list and have twice the loads in flight.
+template <int W32, int Q, int CH, int NW = kPackWords<Q>>
+__device__ __forceinline__ void scan_codes(const Table<W32, Q> &tab, int n,
                                            const NodeSets<W32> &C,
                                            const uint8_t *list, int nv, int nc,
-                                           const Packed<NW> &dv,
-                                           const Packed<NW> &dw, int lane,
-                                           uint32_t (&best)[NW]) {
-  uint32_t un[W32], tv[NW], tw[NW];
+                                           const Packed<NW> (&dv)[CH],
+                                           const Packed<NW> (&dw)[CH],
+                                           int lane,
+                                           uint32_t (&best)[CH * NW]) {
+  uint32_t un[W32], tv[CH * NW], tw[CH * NW];
 #pragma unroll
   for (int r = 0; r < W32; r++) un[r] = ~(C.v[r] | C.w[r]) & group_mask(r, n);
 #pragma unroll
-  for (int i = 0; i < NW; i++) best[i] = tv[i] = tw[i] = 0u;
+  for (int i = 0; i < CH * NW; i++) best[i] = tv[i] = tw[i] = 0u;
+  const int sw = tab.ns * 32 * NW;
+  if constexpr (W32 <= 4) {
+    max_nodes<W32, Q, CH>(best, tab.s, sw, un, 0, n, lane);
+  } else {
+    // the global part's loads, eight nodes at a time, each under its share of
+    // the nodes in shared memory (ns is a multiple of 8, or n)
+    const int ne = n - tab.ns, groups = (ne + 7) >> 3, gw = ne * 32 * NW;
+    const int share =
+        groups > 0 ? ((tab.ns + 8 * groups - 1) / (8 * groups)) * 8 : tab.ns;
+    int j = 0;
 #pragma unroll 1
-  for (int j = 0; j < n; j += 8) {
-    const uint32_t u = pick<W32>(un, (uint32_t)j >> 5) >> (j & 31);
-    const uint32_t *t = tab + j * 32 * NW;
-    uint32_t k[8][NW];
-    if (j + 8 <= n) {
+    for (int e = 0; j < tab.ns || e < ne; e += 8) {
+      uint32_t x[8][CH * NW];
+      if (e < ne) {
 #pragma unroll
-      for (int b = 0; b < 8; b++) ld_pack<Q>(t, b * 32 + lane, k[b]);
-    } else {  // the last nodes: entry 0 of the group in place of the missing
+        for (int b = 0; b < 8; b++)
+          ld_chunks<Q, CH>(tab.g, gw, min(e + b, ne - 1) * 32 + lane, x[b]);
+      }
+      const int count = min(share, tab.ns - j);
+      max_nodes<W32, Q, CH>(best, tab.s + j * 32 * NW, sw, un, j, count, lane);
+      j += count;
+      if (e < ne) {
+        uint32_t u = pick<W32>(un, (uint32_t)(tab.ns + e) >> 5) >> ((tab.ns + e) & 31);
+        if (ne - e < 8) u &= (1u << (ne - e)) - 1u;
+        max8<CH * NW>(best, x, u);
+      }
+    }
+  }
+  constexpr int B = W32 > 4 ? 8 : 4;
+#pragma unroll 1
+  for (int c0 = 0; c0 < nc; c0 += B) {
+    uint32_t k[B][CH * NW];
 #pragma unroll
-      for (int b = 0; b < 8; b++)
-        ld_pack<Q>(t, (j + b < n ? b : 0) * 32 + lane, k[b]);
+    for (int b = 0; b < B; b++) {
+      const int j = (int)list[min(c0 + b, nc - 1)];
+      if (W32 <= 4 || j < tab.ns)
+        ld_chunks<Q, CH>(tab.s, sw, j * 32 + lane, k[b]);
+      else
+        ld_chunks<Q, CH>(tab.g, (n - tab.ns) * 32 * NW,
+                         (j - tab.ns) * 32 + lane, k[b]);
     }
 #pragma unroll
-    for (int b = 0; b < 8; b++)
-      if ((u >> b) & 1u) {
+    for (int b = 0; b < B; b++) {
+      const bool in_v = min(c0 + b, nc - 1) < nv;
 #pragma unroll
-        for (int i = 0; i < NW; i++) best[i] = __vmaxu2(best[i], k[b][i]);
+      for (int i = 0; i < CH * NW; i++) {
+        tv[i] = __vmaxu2(tv[i], in_v ? k[b][i] : 0u);
+        tw[i] = __vmaxu2(tw[i], in_v ? 0u : k[b][i]);
       }
-  }
-#pragma unroll 2
-  for (int c = 0; c < nv; c++) {
-    uint32_t k[NW];
-    ld_pack<Q>(tab, (int)list[c] * 32 + lane, k);
-#pragma unroll
-    for (int i = 0; i < NW; i++) tv[i] = __vmaxu2(tv[i], k[i]);
-  }
-#pragma unroll 2
-  for (int c = nv; c < nc; c++) {
-    uint32_t k[NW];
-    ld_pack<Q>(tab, (int)list[c] * 32 + lane, k);
-#pragma unroll
-    for (int i = 0; i < NW; i++) tw[i] = __vmaxu2(tw[i], k[i]);
+    }
   }
 #pragma unroll
-  for (int i = 0; i < NW; i++) {
-    if (nv > 0) best[i] = __vmaxu2(best[i], tv[i] + dv.k[i]);
-    if (nc > nv) best[i] = __vmaxu2(best[i], tw[i] + dw.k[i]);
-  }
+  for (int c = 0; c < CH; c++)
+#pragma unroll
+    for (int i = 0; i < NW; i++) {
+      uint32_t &o = best[c * NW + i];
+      if (nv > 0) o = __vmaxu2(o, tv[c * NW + i] + dv[c].k[i]);
+      if (nc > nv) o = __vmaxu2(o, tw[c * NW + i] + dw[c].k[i]);
+    }
 }
 
 // ------------------------------------------------------------------------
@@ -487,7 +663,7 @@ struct CellSums {
 };
 
 // The second pass over the far-off cells of one cell slot (resum_cells'
-// terms in the same order), counts from the table.  One slot at a time, four
+// terms in the same order), counts from the table.  One slot at a time, eight
 // nodes' loads and exponentials in flight: what is left is the chain of
 // additions (a dataset whose rates leave one cell far below its bound takes
 // this pass in every evaluation).
@@ -495,18 +671,16 @@ struct Resum1 {
   float z, ed, em;
 };
 
-template <int Q>
-__device__ __noinline__ Resum1 resum_slot_table(const uint32_t *tab,
+template <int W32, int Q>
+__device__ __noinline__ Resum1 resum_slot_table(const Table<W32, Q> tab,
                                                 const uint16_t *ord, int n,
                                                 int lane, float c1, float c2,
                                                 float base, int q) {
   constexpr int NW = kPackWords<Q>;
-  const uint32_t *t = tab + lane * NW + (q >> 1);
+  const int word = lane * NW + (q >> 1);
   const uint32_t sd = (q & 1) ? 0x7542u : 0x7540u;
   Resum1 o{0.0f, 0.0f, 0.0f};
-#pragma unroll 4
-  for (int i = 0; i < n; i++) {
-    const uint32_t k = t[(int)(ord[i] & 0xFF) * 32 * NW];
+  auto term = [&](uint32_t k) {
     const float fd =
         __int_as_float((int)__byte_perm(k, 0x4B000000u, sd)) - 8388608.0f;
     const float fm =
@@ -515,19 +689,21 @@ __device__ __noinline__ Resum1 resum_slot_table(const uint32_t *tab,
     o.z += e;
     o.ed = fmaf(e, fd, o.ed);
     o.em = fmaf(e, fm, o.em);
-  }
+  };
+#pragma unroll 8
+  for (int i = 0; i < n; i++) term(tab.at((int)(ord[i] & 0xFF))[word]);
   return o;
 }
 
-// sum_cells with the counts of every node in the table (sx.cnt) and the
-// tree's canonical order (sx.ord): the same terms in the same pairs and
+// sum_cells with the counts of every node in the table and the tree's
+// canonical order (ord): the same terms in the same pairs and
 // order, so the same sums.  The table's entries are all in place before the
 // loop, so its loads wait for nothing but the order.
-template <int Q>
+template <int W32, int Q>
 __device__ __forceinline__ void sum_cells_table(
-    int n, const float (&pd)[Q], const float (&pm)[Q], const LogTable &L,
+    const Table<W32, Q> &tab, const uint16_t *ord, int n, const float (&pd)[Q], const float (&pm)[Q], const LogTable &L,
     int c0, int stride, int lane, int n_cells, long long (&acc)[6],
-    const SumCtx &sx, CellSums<Q> &cs) {
+    CellSums<Q> &cs) {
   constexpr int NW = kPackWords<Q>;
   const float c1 = (L.l01 - L.l00) * kLog2E;
   const float c2 = (L.l11 - L.l10) * kLog2E;
@@ -545,13 +721,12 @@ __device__ __forceinline__ void sum_cells_table(
     ed2[q] = em2[q] = make_float2(0.0f, 0.0f);
   }
   auto entry = [&](uint32_t o, uint32_t (&k)[NW]) {
-    ld_pack<Q>(sx.cnt, (int)(o & 0xFF) * 32 + lane, k);
+    tab.ld((int)(o & 0xFF), lane, k);
   };
   int i = 1;
   if (i + 1 < n) {
     // the table's loads one pair ahead of the float work, the order's two
     uint32_t kA0[NW], kA1[NW], kB0[NW], kB1[NW];
-    const uint16_t *ord = sx.ord;
     const int last = n - 1;
     entry(ord[i], kA0);
     entry(ord[i + 1], kA1);
@@ -580,7 +755,7 @@ __device__ __forceinline__ void sum_cells_table(
   }
   if (i < n) {
     uint32_t k[NW];
-    entry(sx.ord[i], k);
+    entry(ord[i], k);
 #pragma unroll
     for (int q = 0; q < Q; q++) {
       const float fd = pack_d_biased(k[q >> 1], q) - 8388608.0f;
@@ -607,9 +782,8 @@ __device__ __forceinline__ void sum_cells_table(
 #pragma unroll
     for (int q = 0; q < Q; q++) {
       if (!__any_sync(BBS_FULL_MASK, bad[q])) continue;
-      const Resum1 o = resum_slot_table<Q>(
-          sx.cnt, sx.ord, n, lane, c1, c2,
-          bad[q] ? base[q] - mx[q] : base[q], q);
+      const Resum1 o = resum_slot_table<W32, Q>(
+          tab, ord, n, lane, c1, c2, bad[q] ? base[q] - mx[q] : base[q], q);
       if (bad[q]) {
         r[q] = fmaf(mx[q], kLn2, r[q]);
         base[q] -= mx[q];
@@ -638,9 +812,9 @@ __device__ __forceinline__ void sum_cells_table(
 }
 
 // The current tree's terms at the listed nodes: their sum and largest
-// exponent per cell, two nodes at a time.
-template <int Q, int NW = kPackWords<Q>>
-__device__ __forceinline__ void class_terms(const uint32_t *tab,
+// exponent per cell.
+template <int W32, int Q, int NW = kPackWords<Q>>
+__device__ __forceinline__ void class_terms(const Table<W32, Q> &tab,
                                             const uint8_t *list, int n_list,
                                             float c1, float c2,
                                             const float (&base)[Q], int lane,
@@ -653,8 +827,8 @@ __device__ __forceinline__ void class_terms(const uint32_t *tab,
     mo[q] = -INFINITY;
   }
   uint32_t a0[NW], a1[NW];
-  ld_pack<Q>(tab, (int)list[0] * 32 + lane, a0);
-  ld_pack<Q>(tab, (int)list[n_list > 1 ? 1 : 0] * 32 + lane, a1);
+  tab.ld((int)list[0], lane, a0);
+  tab.ld((int)list[n_list > 1 ? 1 : 0], lane, a1);
 #pragma unroll 1
   for (int c = 0; c < n_list; c += 2) {
     // an odd last node is paired with itself; its copy's term is dropped
@@ -662,8 +836,8 @@ __device__ __forceinline__ void class_terms(const uint32_t *tab,
     float2 fd[Q], fm[Q];
     pack_to_float2<Q, NW>(a0, a1, fd, fm);
     // the next pair's entries (the last loads again past the end)
-    ld_pack<Q>(tab, (int)list[min(c + 2, n_list - 1)] * 32 + lane, a0);
-    ld_pack<Q>(tab, (int)list[min(c + 3, n_list - 1)] * 32 + lane, a1);
+    tab.ld((int)list[min(c + 2, n_list - 1)], lane, a0);
+    tab.ld((int)list[min(c + 3, n_list - 1)], lane, a1);
 #pragma unroll
     for (int q = 0; q < Q; q++) {
       const float2 t = ffma2(fd[q], c1p, ffma2(fm[q], c2p, dup2(base[q])));
@@ -689,26 +863,26 @@ __device__ __forceinline__ float entry_shift(const uint32_t (&a)[NW],
 
 inline constexpr float kBoundUnit = 4096.0f;  // 2^-12 of a base-2 log
 
-// Upper bounds of a proposal's sum score and max score over this warp's
-// cells, relative to the current tree: up[0] bounds sum_c log2(z'_c / z_c),
+// Adds upper bounds of a proposal's sum score and max score over one chunk of
+// this warp's cells, relative to the current tree, to up: up[0] bounds sum_c log2(z'_c / z_c),
 // up[1] bounds sum_c (largest exponent' - largest exponent), in units of
 // 1 / kBoundUnit.  eps bounds the relative rounding of a term against its
 // shifted form.  Sums of up to 128 terms are good to 2^-17 of the largest
 // partial sum, so a cell's remainder z - zo is taken with 2^-15 z on top.
-template <int Q, int NW = kPackWords<Q>>
+template <int W32, int Q, int NW = kPackWords<Q>>
 __device__ __forceinline__ void bound_proposal(
-    const uint32_t *tab, const Delta &x, const uint8_t *list, int nv, int nc,
+    const Table<W32, Q> &tab, const Delta &x, const uint8_t *list, int nv, int nc,
     const CellSums<Q> &cs, const LogTable &L, float eps, int c0, int stride,
-    int n_cells, int lane, int (&up)[2]) {
+    int n_cells, int lane, float (&up)[2]) {
   const float c1 = (L.l01 - L.l00) * kLog2E;
   const float c2 = (L.l11 - L.l10) * kLog2E;
   float hv[Q], hw[Q], z1[Q], gain[Q], rest[Q];
   {
     uint32_t a[NW], b[NW], c[NW], e[NW];
-    ld_pack<Q>(tab, (int)x.a0 * 32 + lane, a);
-    ld_pack<Q>(tab, (int)x.b0 * 32 + lane, b);
-    ld_pack<Q>(tab, (int)x.a1 * 32 + lane, c);
-    ld_pack<Q>(tab, (int)x.b1 * 32 + lane, e);
+    tab.ld((int)x.a0, lane, a);
+    tab.ld((int)x.b0, lane, b);
+    tab.ld((int)x.a1, lane, c);
+    tab.ld((int)x.b1, lane, e);
 #pragma unroll
     for (int q = 0; q < Q; q++) {
       hv[q] = entry_shift<NW>(a, b, q, c1, c2);
@@ -727,7 +901,7 @@ __device__ __forceinline__ void bound_proposal(
     const int at = cls ? nv : 0, count = cls ? nc - nv : nv;
     if (count > 0) {
       float zo[Q], mo[Q];
-      class_terms<Q>(tab, list + at, count, c1, c2, cs.base, lane, zo, mo);
+      class_terms<W32, Q>(tab, list + at, count, c1, c2, cs.base, lane, zo, mo);
 #pragma unroll
       for (int q = 0; q < Q; q++) {
         rest[q] -= zo[q];
@@ -756,8 +930,8 @@ __device__ __forceinline__ void bound_proposal(
   // NaN end there too: such a proposal is not rejected)
   s = s < 8000.0f && g < 8000.0f ? fmaxf(s, -8000.0f) : 8000.0f;
   g = g < 8000.0f ? fmaxf(g, -8000.0f) : 8000.0f;
-  up[0] = __reduce_add_sync(BBS_FULL_MASK, __float2int_ru(s * kBoundUnit) + 1);
-  up[1] = __reduce_add_sync(BBS_FULL_MASK, __float2int_ru(g * kBoundUnit) + 1);
+  up[0] += (float)__reduce_add_sync(BBS_FULL_MASK, __float2int_ru(s * kBoundUnit) + 1);
+  up[1] += (float)__reduce_add_sync(BBS_FULL_MASK, __float2int_ru(g * kBoundUnit) + 1);
 }
 
 }  // namespace bbs

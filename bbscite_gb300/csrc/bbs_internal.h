@@ -107,6 +107,9 @@ struct RunArgs {
   int wpc;                    // warps per chain (cells split over them)
   int chunks;                 // table of every node (TablePlan); 0: none
   int with_inc;               // 1: increment tables after the slots
+  int smem;                   // dynamic shared memory of the plan
+  int ns;                     // nodes of the table in shared memory
+  uint32_t *table;            // the others' entries, per slot of the launch
 };
 
 // Many datasets in one launch: chains are listed by unit (chain index in
@@ -129,6 +132,9 @@ struct BatchArgs {
   int table_ds;              // the launch's only dataset, or -1
   int chunks;                // table of every node (TablePlan); 0: none
   int with_inc;              // 1: increment tables (one dataset only)
+  int smem;                  // dynamic shared memory of the plan
+  int ns;                    // nodes of the table in shared memory
+  uint32_t *table;           // the others' entries, per slot of the launch
   int wpc;                   // warps per chain: 1 (blocks of one-warp
                              // chains), or 2-4 (a block is one chain)
 };
@@ -197,13 +203,11 @@ struct GradArgs {
 
 // Host launchers (bbs_aux.cu, bbs_mcmc.cu, bbs_batch.cu).  Return a cudaError_t as int.
 // chains_per_block must be 1 when a.wpc > 1 (the block is one chain).
-// smem_block: the dynamic shared memory a block may have; max_cells: the
-// cells of the launch's largest dataset.  The plan of the table (chunks,
-// with_inc) is made here.
+// The arguments carry the launch's plan (TablePlan).
 int launch_mcmc(const RunArgs &a, int q, int chains_per_block, int n_sms,
-                int smem_block, void *stream);
-int launch_batch(const BatchArgs &b, int w32, int max_cells, int q, bool sum,
-                 int warps_per_block, int n_sms, int smem_block, void *stream);
+                void *stream);
+int launch_batch(const BatchArgs &b, int w32, int q, bool sum,
+                 int warps_per_block, int n_sms, void *stream);
 // Launch groups: every chain of a launch must store its rows with the
 // stride rs_of_w32(w32) of the launch (w32 at least the chains' own).
 int launch_init(const InitArgs &a, int w32, bool sum, void *stream);

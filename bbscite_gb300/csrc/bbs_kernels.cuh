@@ -469,6 +469,11 @@ __device__ __forceinline__ void run_chain(
   if (multi) __syncthreads(); else __syncwarp();
 }
 
+template <int N>
+struct IntConst {
+  static constexpr int value = N;
+};
+
 // A tree scored from its rows, off the hot path: proposals that are not
 // followed node by node, and error moves of the max score.
 template <int W32, int Q, bool SUM>
@@ -484,17 +489,28 @@ __device__ __noinline__ Evaluated evaluate_rows(const uint32_t *rows,
 }
 
 // A proposal's rows and, for a tree whose parent vector is known, its parent
-// vector: off the path of rejected proposals.
+// vector.
 template <int W32>
-__device__ __noinline__ void propose_tree(const uint32_t *cur, uint32_t *prop,
-                                          const uint8_t *cpar, uint8_t *ppar,
-                                          int n, const bbs_move_params p,
-                                          const NodeSets<W32> D, bool related,
-                                          bool tree_ok, int wpc, int wic,
-                                          int lane) {
+__device__ __forceinline__ void propose_tree(
+    const uint32_t *cur, uint32_t *prop, const uint8_t *cpar, uint8_t *ppar,
+    int n, const bbs_move_params &p, const NodeSets<W32> &D, bool related,
+    bool tree_ok, int wpc, int wic, int lane) {
   build_proposal<W32>(cur, prop, n, p, D.v, D.w, related, wpc, wic, lane);
   if (tree_ok && wic == 0) propose_parents(cpar, ppar, n, p, related, lane);
   if (wpc > 1) __syncthreads(); else __syncwarp();
+}
+
+// The same out of line, for proposals that are not described by classes.
+// (Structures passed by value to functions that are not inlined go through
+// local memory: with this and the table's update called that way on every
+// proposal summed, 95 x 96 took 12.2 us a step, inlined 10.9.)
+template <int W32>
+__device__ __noinline__ void propose_tree_call(
+    const uint32_t *cur, uint32_t *prop, const uint8_t *cpar, uint8_t *ppar,
+    int n, const bbs_move_params p, const NodeSets<W32> D, bool related,
+    bool tree_ok, int wpc, int wic, int lane) {
+  propose_tree<W32>(cur, prop, cpar, ppar, n, p, D, related, tree_ok, wpc, wic,
+                    lane);
 }
 
 // run_chain with the table of bbs_incr.cuh in ss.sx.cnt (rows of up to four
@@ -509,7 +525,8 @@ __device__ __forceinline__ void run_chain_table(
     ChainState *gstate, const bbs_raw_move *moves, bbs_step_trace *trace,
     int n_steps, const volatile int *cancel, int *status, uint32_t *buf0,
     uint32_t *buf1, int *part, volatile int *sflag, uint4 *pbuf,
-    const SlotSum &ss, int chunks, int wpc, int wic, int lane) {
+    const SlotSum &ss, const Table<W32, Q> tab, int chunks, int wpc, int wic,
+    int lane) {
   constexpr int NW = kPackWords<Q>;
   const int n = ds.n_nodes;
   const bool multi = wpc > 1;
@@ -519,7 +536,6 @@ __device__ __forceinline__ void run_chain_table(
   if (multi) __syncthreads(); else __syncwarp();
   uint32_t *cur = buf0, *prop = buf1;
   uint8_t *cpar = ss.par0, *ppar = ss.par1;
-  uint32_t *const tab = ss.sx.cnt;
   float alpha = st.alpha, beta = st.beta, score = st.score, prior = st.prior;
   LogTable L{st.l00, st.l10, st.l01, st.l11};
   float ec[4] = {st.ec[0], st.ec[1], st.ec[2], st.ec[3]};
@@ -539,6 +555,7 @@ __device__ __forceinline__ void run_chain_table(
   CellSums<Q> cs;
   float pd[Q], pm[Q];
   float smax = 0.0f, eps = 0.0f, slack = 0.0f;  // of the sum score's bound
+  int bounded = 0, rejected = 0, skip = 0;      // proposals bounded, rejected
   if constexpr (SUM) {
     Cells<W32, Q> cb;
     load_cells<W32, Q>(cb, ds, c0, stride, lane);
@@ -582,13 +599,13 @@ __device__ __forceinline__ void run_chain_table(
         }
       }
       if (moves == nullptr && (i & 15) == 0) {
-        philox_fill(pbuf, md.seed, chain_id, st.steps_done + (uint64_t)i, lane);
+        moves_fill(pbuf, md, (uint32_t)n, chain_id, st.steps_done + (uint64_t)i,
+                   trace != nullptr, lane);
         __syncwarp();
       }
       raw = moves != nullptr
                 ? moves[i]
-                : move_from_words(md.mp, (uint32_t)n, pbuf[2 * (i & 15)],
-                                  pbuf[2 * (i & 15) + 1], trace != nullptr);
+                : reinterpret_cast<const bbs_raw_move *>(pbuf)[i & 15];
       err_move = raw.move_type == BBS_MOVE_CHANGE_BETA;
     }
     float palpha = alpha, pbeta = beta, pprior = prior;
@@ -662,24 +679,36 @@ __device__ __forceinline__ void run_chain_table(
     }
     if (classes) {
       delta = move_classes<W32>(mp, related, D, C);
-      class_deltas<Q>(tab, delta, lane, dv, dw);
       int nv;
       const int nc = list_nodes<W32>(C, list, lane, nv);
       if constexpr (!SUM) {
         int sk = 0, sm = 0;
-        for (int c = 0; c < chunks; c++) {
-          const uint32_t *t = tab + c * n * 32 * NW;
-          uint32_t best[NW];
-          if (c > 0) class_deltas<Q>(t, delta, lane, dv, dw);
-          scan_codes<W32, Q>(t, n, C, list, nv, nc, dv, dw, lane, best);
+        // CH chunks of cells from chunk c on
+        auto read_off = [&](auto CHT, int c) {
+          constexpr int CH = decltype(CHT)::value;
+          Packed<NW> pv[CH], pw[CH];
+          uint32_t best[CH * NW];
 #pragma unroll
-          for (int q = 0; q < Q; q++) {
-            int d, m;
-            decode(code, pack_field<NW>(best, q), d, m);
-            sk += d + m;
-            sm += m;
-          }
-        }
+          for (int k = 0; k < CH; k++)
+            class_deltas<W32, Q>(tab.chunk(c + k, n), delta, lane, pv[k], pw[k]);
+          scan_codes<W32, Q, CH>(tab.chunk(c, n), n, C, list, nv, nc, pv, pw,
+                                 lane, best);
+#pragma unroll
+          for (int k = 0; k < CH; k++)
+#pragma unroll
+            for (int q = 0; q < Q; q++) {
+              const uint32_t T = (best[k * NW + (q >> 1)] >> (16 * (q & 1))) & 0xFFFFu;
+              int d, m;
+              decode<(W32 > 4)>(code, T, d, m);
+              sk += d + m;
+              sm += m;
+            }
+          dv = pv[0];  // (kept for accepted proposals of one chunk)
+          dw = pw[0];
+        };
+        int c = 0;
+        for (; c + 2 <= chunks; c += 2) read_off(IntConst<2>{}, c);
+        if (c < chunks) read_off(IntConst<1>{}, c);
         sk = __reduce_add_sync(BBS_FULL_MASK, sk);
         sm = __reduce_add_sync(BBS_FULL_MASK, sm);
         ev = finish_max(ds, L, prior, sk, sm, wpc, wic, lane, part, i & 1);
@@ -695,18 +724,30 @@ __device__ __forceinline__ void run_chain_table(
                             raw.acceptance_level);
         }
       } else {
-        if (trace == nullptr && md.gamma > 0.0f && has_best) {
-          int up[2];
-          bound_proposal<Q>(tab, delta, list, nv, nc, cs, L, eps, c0, stride,
-                            ds.n_cells, lane, up);
+        // Where the bound rejects less than a third of the proposals it is
+        // left out for a while (few cells, flat likelihoods: at 67 x 9 most
+        // proposals are accepted, and bounding them all first cost 40 %).
+        const bool bound = trace == nullptr && md.gamma > 0.0f && has_best &&
+                           skip == 0;
+        if (skip > 0) skip--;
+        float up[2] = {0.0f, 0.0f};
+        class_deltas<W32, Q>(tab, delta, lane, dv, dw);
+        if (bound)
+          bound_proposal<W32, Q>(tab, delta, list, nv, nc, cs, L, eps, c0,
+                                 stride, ds.n_cells, lane, up);
+        if (bound) {
+          if ((++bounded & 31) == 0) {
+            if (rejected < 10) skip = 96;
+            rejected = 0;
+          }
           if (multi) {
-            int *pp = part + (i & 1) * 12 * wpc;
+            float *pp = reinterpret_cast<float *>(part + (i & 1) * 12 * wpc);
             if (lane == 0) {
               pp[12 * wic] = up[0];
               pp[12 * wic + 1] = up[1];
             }
             __syncthreads();
-            up[0] = up[1] = 0;
+            up[0] = up[1] = 0.0f;
             for (int w = 0; w < wpc; w++) {
               up[0] += pp[12 * w];
               up[1] += pp[12 * w + 1];
@@ -714,11 +755,12 @@ __device__ __forceinline__ void run_chain_table(
           }
           const float tol = slack + fabsf(score) * 4.8e-07f +
                             fabsf(smax) * 4.8e-07f + 1.0e-3f;
-          const float ds_up = fmaf((float)up[0], kLn2 / kBoundUnit, tol);
-          const float dm_up = fmaf((float)up[1], kLn2 / kBoundUnit, tol);
+          const float ds_up = fmaf(up[0], kLn2 / kBoundUnit, tol);
+          const float dm_up = fmaf(up[1], kLn2 / kBoundUnit, tol);
           if (smax + dm_up < best_score &&
               corr * expf(ds_up * md.gamma) * 1.001f < raw.acceptance_level) {
             __syncwarp();
+            rejected++;
             i++;
             continue;  // rejected: the chain's state stays as it is
           }
@@ -734,8 +776,12 @@ __device__ __forceinline__ void run_chain_table(
       from_rows = true;
     }
     if (classes ? (SUM || from_rows) : (from_rows && !err_move)) {
-      propose_tree<W32>(cur, prop, cpar, ppar, n, mp, D, related, tree_ok, wpc,
-                        wic, lane);
+      if constexpr (SUM)
+        propose_tree<W32>(cur, prop, cpar, ppar, n, mp, D, related, tree_ok,
+                          wpc, wic, lane);
+      else  // (rarely: out of line)
+        propose_tree_call<W32>(cur, prop, cpar, ppar, n, mp, D, related,
+                               tree_ok, wpc, wic, lane);
       built = true;
     }
     if constexpr (SUM) {
@@ -758,8 +804,8 @@ __device__ __forceinline__ void run_chain_table(
     if constexpr (SUM) {
       if (from_table) {
         long long acc[6] = {0, 0, 0, 0, 0, 0};
-        sum_cells_table<Q>(n, pd, pm, PL, c0, stride, lane, ds.n_cells, acc,
-                           ss.sx, pcs);
+        sum_cells_table<W32, Q>(tab, ss.sx.ord, n, pd, pm, PL, c0, stride, lane,
+                                ds.n_cells, acc, pcs);
         acc[0] = warp_sum_ll(acc[0]);
         acc[2] = warp_sum_ll(acc[2]);
         acc[4] = warp_sum_ll(acc[4]);
@@ -801,9 +847,10 @@ __device__ __forceinline__ void run_chain_table(
     const bool better = !has_best || psmax > best_score;
     const bool tie = !better && K > 1 && psmax == best_score &&
                      lcount < (uint32_t)K;
-    if (!err_move && !built && (accept || better || tie))
-      propose_tree<W32>(cur, prop, cpar, ppar, n, mp, D, related, tree_ok, wpc,
-                        wic, lane);
+    if constexpr (!SUM)
+      if (!err_move && !built && (accept || better || tie))
+        propose_tree<W32>(cur, prop, cpar, ppar, n, mp, D, related, tree_ok,
+                          wpc, wic, lane);
     const uint32_t *scored_rows = err_move ? cur : prop;
     if (better) {
       has_best = true;
@@ -874,13 +921,13 @@ __device__ __forceinline__ void run_chain_table(
         if (classes) {
           if constexpr (!SUM) {
             for (int c = 0; c < chunks; c++) {
-              uint32_t *tc = tab + c * n * 32 * NW;
-              if (chunks > 1) class_deltas<Q>(tc, delta, lane, dv, dw);
+              const Table<W32, Q> tc = tab.chunk(c, n);
+              if (chunks > 1) class_deltas<W32, Q>(tc, delta, lane, dv, dw);
               apply_classes<W32, Q>(tc, list, delta, C, dv, dw, false, lane);
             }
           } else {
             cs = pcs;
-            ord_ok = true;
+                ord_ok = true;
           }
 #ifdef BBS_CHECKED
           device_check(parents_match_rows<W32>(cur, n, cpar, lane), status,
@@ -892,13 +939,13 @@ __device__ __forceinline__ void run_chain_table(
       } else if (tree_ok) {
         if constexpr (SUM) {
           cs = pcs;
-          tolerances();
+            tolerances();
         } else {
           fresh_table = true;
         }
       }
     } else if (applied) {
-      apply_classes<W32, Q>(tab, list, delta, C, dv, dw, true, lane);
+      take_back<W32, Q>(tab, list, delta, C, dv, dw, lane);
     }
     __syncwarp();
     i++;
@@ -934,20 +981,39 @@ __device__ __forceinline__ void run_chain_table(
   if (multi) __syncthreads(); else __syncwarp();
 }
 
-// Launch bounds of each cells-per-lane variant (bbs_layout.h).
-template <int Q>
+// A warp's table in a slot of rows of five to eight words, its nodes from ns
+// on in global memory (`table`, a part per slot of the launch and warp).
+template <int W32, int Q>
+__device__ __forceinline__ Table<W32, Q> wide_table(uint8_t *slot_base, int n,
+                                                    int rs, int wpc, int wic,
+                                                    int chunks, int ns,
+                                                    uint32_t *table,
+                                                    int slot) {
+  uint8_t *p = slot_base + slot_bytes(n, rs, wpc, true, W32, Q, false) +
+               wic * wide_part_bytes(Q, chunks, ns);
+  return Table<W32, Q>{reinterpret_cast<uint32_t *>(p),
+                       table + (size_t)(slot * wpc + wic) * chunks *
+                                   (pack_table_bytes(n - ns, Q) / 4),
+                       ns};
+}
+
+// Launch bounds of each variant (bbs_layout.h).
+template <int W32, int Q, bool TAB>
 struct ChainBounds {
   static constexpr int threads = chain_max_threads(Q);
-  static constexpr int min_blocks = chain_min_blocks(Q);
+  static constexpr int min_blocks = chain_blocks(W32, Q, TAB);
 };
 
 // One dataset: chains 0..n_chains-1, one warp per chain (blocks of `cpb`
 // chains) or wpc warps per chain (the block is one chain).  REC: recorded
 // moves and/or a step trace (replays and tests); without them the move and
 // trace paths compile away.
-template <int W32, int Q, bool SUM, bool REC>
-__global__ void __launch_bounds__(ChainBounds<Q>::threads,
-                                  ChainBounds<Q>::min_blocks)
+// TAB: proposals are read off a table (a.chunks > 0), else every node is
+// evaluated; kernels of their own, so that neither carries the other's code
+// and registers.
+template <int W32, int Q, bool SUM, bool REC, bool TAB>
+__global__ void __launch_bounds__((ChainBounds<W32, Q, TAB>::threads),
+                                  (ChainBounds<W32, Q, TAB>::min_blocks))
     mcmc_kernel(const RunArgs a) {
   extern __shared__ __align__(16) uint32_t smem[];
   constexpr int RS = rs_of_w32(W32);
@@ -959,11 +1025,13 @@ __global__ void __launch_bounds__(ChainBounds<Q>::threads,
   const int slot = wib / wpc, wic = wib - slot * wpc;
   const int n = a.ds.n_nodes;
   // the launcher's plan, for the whole block
-  const bool inc = a.with_inc != 0, ring = W32 > 4;
-  const bool scratch = SUM || ring || a.chunks > 0;
-  const int sb = a.chunks > 0 && !inc
-                     ? table_slot_bytes(n, RS, wpc, W32, Q, a.chunks)
-                     : slot_bytes(n, RS, wpc, scratch, W32, Q, inc || ring);
+  const bool inc = a.with_inc != 0, ring = W32 > 4 && !TAB;
+  constexpr bool wide = W32 > 4 && TAB;
+  constexpr bool scratch = SUM || W32 > 4 || TAB;
+  const int sb =
+      wide ? wide_slot_bytes(n, RS, wpc, W32, Q, a.chunks, a.ns)
+      : TAB && !inc ? table_slot_bytes(n, RS, wpc, W32, Q, a.chunks)
+                    : slot_bytes(n, RS, wpc, scratch, W32, Q, inc || ring);
   uint8_t *slot_base = reinterpret_cast<uint8_t *>(smem) + (size_t)slot * sb;
   uint32_t *buf0 = reinterpret_cast<uint32_t *>(slot_base);
   uint32_t *buf1 = buf0 + n * RS;
@@ -972,18 +1040,23 @@ __global__ void __launch_bounds__(ChainBounds<Q>::threads,
   uint4 *pbuf = reinterpret_cast<uint4 *>(
       slot_base + 4 * (2 * n * RS + 24 * wpc + 4) + kPhiloxBytes * wic);
   SlotSum ss{};
-  if (scratch) {
-    ss = slot_sum(slot_base, n, RS, wpc, wic, W32, Q, inc || ring);
-    if constexpr (W32 <= 4) {
+  if (scratch) ss = slot_sum(slot_base, n, RS, wpc, wic, W32, Q, inc || ring);
+  Table<W32, Q> tab{};
+  if constexpr (TAB) {
+    if constexpr (wide) {
+      tab = wide_table<W32, Q>(slot_base, n, RS, wpc, wic, a.chunks, a.ns,
+                               a.table, blockIdx.x * cpb + slot);
+    } else {
       if (inc) {
         uint8_t *table = reinterpret_cast<uint8_t *>(smem) + (size_t)cpb * sb;
         build_increments<Q>(table, wpc, a.ds, RS);
         __syncthreads();
         ss.sx.inc = reinterpret_cast<const uint32_t *>(
             table + (size_t)wic * inc_table_bytes(n, Q));
-      } else if (a.chunks > 0) {
+      } else {
         ss.sx.cnt = table_part(slot_base, n, RS, wpc, wic, W32, Q, a.chunks);
       }
+      tab = Table<W32, Q>{ss.sx.cnt, nullptr, n};
     }
   }
   for (int chain = blockIdx.x * cpb + slot; chain < a.n_chains;
@@ -999,31 +1072,29 @@ __global__ void __launch_bounds__(ChainBounds<Q>::threads,
     uint32_t *best = a.best_rows + (size_t)chain * K * n * RS;
     uint64_t *lhash = K > 1 ? a.list_hash + (size_t)chain * K : nullptr;
     float *lbeta = K > 1 ? a.list_beta + (size_t)chain * K : nullptr;
-    if constexpr (W32 <= 4) {
-      if (a.chunks > 0) {
-        run_chain_table<W32, Q, SUM>(
-            a.ds, a.md, (uint32_t)chain, rows, best, lhash, lbeta, K,
-            a.states + chain, moves, trace, a.n_steps, a.cancel, a.status,
-            buf0, buf1, part, sflag, pbuf, ss, a.chunks, wpc, wic, lane);
-        continue;
-      }
-    }
-    run_chain<W32, Q, SUM>(a.ds, a.md, (uint32_t)chain, rows, best, lhash,
-                           lbeta, K, a.states + chain, moves, trace,
-                           a.n_steps, a.cancel, a.status, buf0, buf1, part,
-                           sflag, pbuf, ss, wpc, wic, lane);
+    if constexpr (TAB)
+      run_chain_table<W32, Q, SUM>(
+          a.ds, a.md, (uint32_t)chain, rows, best, lhash, lbeta, K,
+          a.states + chain, moves, trace, a.n_steps, a.cancel, a.status, buf0,
+          buf1, part, sflag, pbuf, ss, tab, a.chunks, wpc, wic, lane);
+    else
+      run_chain<W32, Q, SUM>(a.ds, a.md, (uint32_t)chain, rows, best, lhash,
+                             lbeta, K, a.states + chain, moves, trace,
+                             a.n_steps, a.cancel, a.status, buf0, buf1, part,
+                             sflag, pbuf, ss, wpc, wic, lane);
   }
 }
 
 // One work unit of the batched launch: chain `chain` of dataset `d`, run
 // by the wpc warps of its slot (warp wic of them).
-template <int W32, int Q, bool SUM>
+template <int W32, int Q, bool SUM, bool TAB>
 __device__ __forceinline__ void batch_unit(const BatchArgs &b,
                                            const DatasetDev &ds,
                                            const ModelDev &md, uint32_t chain,
                                            uint32_t d, uint32_t *buf0,
                                            int *part, volatile int *sflag,
                                            uint4 *pbuf, const SlotSum &ss,
+                                           const Table<W32, Q> &slot_tab,
                                            int wpc, int wic, int lane) {
   constexpr int RS = rs_of_w32(W32);
   // the dataset's node count is within this launch's row width
@@ -1032,38 +1103,35 @@ __device__ __forceinline__ void batch_unit(const BatchArgs &b,
   // Philox key: the chain's number within its dataset, so a dataset's
   // chains draw the same moves here as in a one-dataset run.
   const uint32_t local = chain - d * (uint32_t)b.chains_per_dataset;
-  if constexpr (W32 <= 4) {
-    if (b.chunks > 0) {
-      // (this dataset's chunks: a launch's largest dataset sizes the slots)
-      const int span = 32 * wpc * Q;
-      run_chain_table<W32, Q, SUM>(
-          ds, md, local, b.rows + off, b.best_rows + off, nullptr, nullptr, 1,
-          b.states + chain, nullptr, nullptr, b.n_steps, b.cancel, b.status,
-          buf0, buf1, part, sflag, pbuf, ss, (ds.n_cells + span - 1) / span,
-          wpc, wic, lane);
-      return;
-    }
+  if constexpr (TAB) {
+    // (this dataset's chunks and nodes: a launch's largest dataset sizes the
+    // slots)
+    const int span = 32 * wpc * Q;
+    Table<W32, Q> tab = slot_tab;
+    tab.ns = min(tab.ns, ds.n_nodes);
+    run_chain_table<W32, Q, SUM>(
+        ds, md, local, b.rows + off, b.best_rows + off, nullptr, nullptr, 1,
+        b.states + chain, nullptr, nullptr, b.n_steps, b.cancel, b.status, buf0,
+        buf1, part, sflag, pbuf, ss, tab, (ds.n_cells + span - 1) / span, wpc,
+        wic, lane);
+  } else {
+    run_chain<W32, Q, SUM>(ds, md, local, b.rows + off, b.best_rows + off,
+                           nullptr, nullptr, 1, b.states + chain, nullptr,
+                           nullptr, b.n_steps, b.cancel, b.status, buf0, buf1,
+                           part, sflag, pbuf, ss, wpc, wic, lane);
   }
-  run_chain<W32, Q, SUM>(ds, md, local, b.rows + off, b.best_rows + off,
-                         nullptr, nullptr, 1, b.states + chain, nullptr,
-                         nullptr, b.n_steps, b.cancel, b.status, buf0, buf1,
-                         part, sflag, pbuf, ss, wpc, wic, lane);
 }
 
 // Many datasets: warps take chains from a shared work list (costliest
 // first); each chain brings its own dataset and rules.  One warp per chain
 // (blocks of one-warp slots), or wpc warps per chain (the block is one
 // slot and takes its chains together).
-// Rows of five to eight words leave the register count free (up to 255):
-// a one-warp slot there takes about 31 KB of shared memory, so at most 7
-// such blocks fit an SM whatever their registers, and with the tighter
-// bound of two cells per lane (168) the sum score's kernel spilled
-// (measured at 255 x 512: 7.5 M against 6.7 M chain-steps/s).
 // MULTI: chains of b.wpc > 1 warps; without it every chain is one warp,
 // known at compile time.
-template <int W32, int Q, bool SUM, bool MULTI>
-__global__ void __launch_bounds__(ChainBounds<Q>::threads,
-                                  W32 > 4 ? 1 : ChainBounds<Q>::min_blocks)
+template <int W32, int Q, bool SUM, bool MULTI, bool TAB>
+__global__ void __launch_bounds__((ChainBounds<W32, Q, TAB>::threads),
+                                  (W32 > 4 ? 1
+                                           : ChainBounds<W32, Q, TAB>::min_blocks))
     batch_kernel(const BatchArgs b) {
   extern __shared__ __align__(16) uint32_t smem[];
   constexpr int RS = rs_of_w32(W32);
@@ -1072,10 +1140,12 @@ __global__ void __launch_bounds__(ChainBounds<Q>::threads,
   const int wpc = MULTI ? b.wpc : 1;
   const int slot = wib / wpc, wic = wib - slot * wpc;
   // the host's plan, the same in every thread
-  const bool inc = b.with_inc != 0, ring = W32 > 4;
-  const bool scratch = SUM || ring || b.chunks > 0;
+  const bool inc = b.with_inc != 0, ring = W32 > 4 && !TAB;
+  constexpr bool wide = W32 > 4 && TAB;
+  constexpr bool scratch = SUM || W32 > 4 || TAB;
   const int sb =
-      b.chunks > 0 && !inc
+      wide ? wide_slot_bytes(b.max_nodes, RS, wpc, W32, Q, b.chunks, b.ns)
+      : TAB && !inc
           ? table_slot_bytes(b.max_nodes, RS, wpc, W32, Q, b.chunks)
           : slot_bytes(b.max_nodes, RS, wpc, scratch, W32, Q, inc || ring);
   uint8_t *slot_base = reinterpret_cast<uint8_t *>(smem) + (size_t)slot * sb;
@@ -1089,9 +1159,15 @@ __global__ void __launch_bounds__(ChainBounds<Q>::threads,
       slot_base + 4 * (2 * b.max_nodes * RS + 24 * wpc + 4) +
       kPhiloxBytes * wic);
   SlotSum ss{};
-  if (scratch) {
+  if (scratch)
     ss = slot_sum(slot_base, b.max_nodes, RS, wpc, wic, W32, Q, inc || ring);
-    if constexpr (W32 <= 4) {
+  Table<W32, Q> tab{};
+  if constexpr (TAB) {
+    if constexpr (wide) {
+      tab = wide_table<W32, Q>(
+          slot_base, b.max_nodes, RS, wpc, wic, b.chunks, b.ns, b.table,
+          blockIdx.x * ((blockDim.x >> 5) / wpc) + slot);
+    } else {
       if (inc) {
         // the increment table of the launch's one dataset
         uint8_t *table = reinterpret_cast<uint8_t *>(smem) +
@@ -1101,10 +1177,11 @@ __global__ void __launch_bounds__(ChainBounds<Q>::threads,
         __syncthreads();
         ss.sx.inc = reinterpret_cast<const uint32_t *>(
             table + (size_t)wic * inc_table_bytes(tds.n_nodes, Q));
-      } else if (b.chunks > 0) {
+      } else {
         ss.sx.cnt = table_part(slot_base, b.max_nodes, RS, wpc, wic, W32, Q,
                                b.chunks);
       }
+      tab = Table<W32, Q>{ss.sx.cnt, nullptr, b.max_nodes};
     }
   }
   for (;;) {
@@ -1133,13 +1210,13 @@ __global__ void __launch_bounds__(ChainBounds<Q>::threads,
     // registers, measured faster); the max score keeps register copies
     // (measured faster there).
     if constexpr (SUM) {
-      batch_unit<W32, Q, SUM>(b, b.ds[d], b.md[d], chain, d, buf0, part,
-                              sflag, pbuf, ss, wpc, wic, lane);
+      batch_unit<W32, Q, SUM, TAB>(b, b.ds[d], b.md[d], chain, d, buf0, part,
+                              sflag, pbuf, ss, tab, wpc, wic, lane);
     } else {
       const DatasetDev ds = b.ds[d];
       const ModelDev md = b.md[d];
-      batch_unit<W32, Q, SUM>(b, ds, md, chain, d, buf0, part, sflag, pbuf,
-                              ss, wpc, wic, lane);
+      batch_unit<W32, Q, SUM, TAB>(b, ds, md, chain, d, buf0, part, sflag, pbuf,
+                              ss, tab, wpc, wic, lane);
     }
   }
 }

@@ -18,18 +18,13 @@ inline cudaError_t prepare_smem(K kernel, size_t smem) {
 // Persistent launch.  wpc == 1: blocks of `cpb` one-warp chains; wpc > 1:
 // blocks of one chain of wpc warps.  As many blocks as chains need, capped
 // at what stays resident; each block then walks its chain slots.
-template <int W32, int Q, bool SUM, bool REC>
-int launch_mcmc_t(RunArgs a, int cpb, int n_sms, int smem_block,
-                  cudaStream_t s) {
+template <int W32, int Q, bool SUM, bool REC, bool TAB>
+int launch_mcmc_k(const RunArgs &a, int cpb, int n_sms, cudaStream_t s) {
   if (a.wpc > 1) cpb = 1;
   const int threads = 32 * a.wpc * cpb;
   if (threads > chain_max_threads(Q)) return (int)cudaErrorInvalidConfiguration;
-  const TablePlan p = plan_tables(a.ds.n_nodes, W32, a.ds.n_cells, Q, a.wpc,
-                                  cpb, SUM, true, smem_block);
-  a.chunks = p.chunks;
-  a.with_inc = p.inc ? 1 : 0;
-  const size_t smem = (size_t)p.smem;
-  auto kern = mcmc_kernel<W32, Q, SUM, REC>;
+  const size_t smem = (size_t)a.smem;
+  auto kern = mcmc_kernel<W32, Q, SUM, REC, TAB>;
   cudaError_t e = prepare_smem(kern, smem);
   if (e != cudaSuccess) return (int)e;
   int per_sm = 0;
@@ -42,24 +37,29 @@ int launch_mcmc_t(RunArgs a, int cpb, int n_sms, int smem_block,
   return (int)cudaGetLastError();
 }
 
+template <int W32, int Q, bool SUM, bool REC>
+int launch_mcmc_t(const RunArgs &a, int cpb, int n_sms, cudaStream_t s) {
+  // (rows of five to eight words replay and trace through the ring)
+  // (and the sum score keeps it)
+  if constexpr (W32 <= 4 || (!REC && !SUM))
+    if (a.chunks > 0)
+      return launch_mcmc_k<W32, Q, SUM, REC, true>(a, cpb, n_sms, s);
+  return launch_mcmc_k<W32, Q, SUM, REC, false>(a, cpb, n_sms, s);
+}
+
 // Work-list launch: enough resident slots to fill the GPU, never more than
 // there are units.  Blocks of wpb one-warp slots (b.wpc == 1), or of one
 // slot of wpb == b.wpc warps.
-template <int W32, int Q, bool SUM, bool MULTI>
-int launch_batch_t(BatchArgs b, int max_cells, int wpb, int n_sms,
-                   int smem_block, cudaStream_t s) {
+template <int W32, int Q, bool SUM, bool MULTI, bool TAB>
+int launch_batch_k(const BatchArgs &b, int wpb, int n_sms, cudaStream_t s) {
   const int threads = 32 * wpb;
   if (threads > chain_max_threads(Q)) return (int)cudaErrorInvalidConfiguration;
   if (b.wpc < 1 || b.wpc > 4 || (b.wpc > 1) != MULTI ||
       (MULTI && wpb != b.wpc))
     return (int)cudaErrorInvalidValue;
   const int slots = wpb / b.wpc;
-  const TablePlan p = plan_tables(b.max_nodes, W32, max_cells, Q, b.wpc, slots,
-                                  SUM, b.table_ds >= 0, smem_block);
-  b.chunks = p.chunks;
-  b.with_inc = p.inc ? 1 : 0;
-  const size_t smem = (size_t)p.smem;
-  auto kern = batch_kernel<W32, Q, SUM, MULTI>;
+  const size_t smem = (size_t)b.smem;
+  auto kern = batch_kernel<W32, Q, SUM, MULTI, TAB>;
   cudaError_t e = prepare_smem(kern, smem);
   if (e != cudaSuccess) return (int)e;
   int per_sm = 0;
@@ -72,14 +72,22 @@ int launch_batch_t(BatchArgs b, int max_cells, int wpb, int n_sms,
   return (int)cudaGetLastError();
 }
 
+template <int W32, int Q, bool SUM, bool MULTI>
+int launch_batch_t(const BatchArgs &b, int wpb, int n_sms, cudaStream_t s) {
+  if constexpr (W32 <= 4 || !SUM)
+    if (b.chunks > 0)
+      return launch_batch_k<W32, Q, SUM, MULTI, true>(b, wpb, n_sms, s);
+  return launch_batch_k<W32, Q, SUM, MULTI, false>(b, wpb, n_sms, s);
+}
+
 // One unit per row width: launches with recorded moves or a trace (REC) or
 // without, and work-list launches of one-warp chains or chains of several
 // warps (MULTI).
 template <int W, bool REC>
 int launch_mcmc_w(const RunArgs &a, int q, bool sum, int cpb, int n_sms,
-                  int smem_block, cudaStream_t s);
+                  cudaStream_t s);
 template <int W, bool MULTI>
-int launch_batch_w(const BatchArgs &b, int max_cells, int q, bool sum, int wpb,
-                   int n_sms, int smem_block, cudaStream_t s);
+int launch_batch_w(const BatchArgs &b, int q, bool sum, int wpb, int n_sms,
+                   cudaStream_t s);
 
 }  // namespace bbs

@@ -82,7 +82,13 @@ inline constexpr int kMaxBlockThreads = 256;
 __host__ __device__ constexpr int chain_max_threads(int q) {
   return q >= 3 ? 256 : 128;
 }
-__host__ __device__ constexpr int chain_min_blocks(int q) {
+// Kernels that read proposals off a table (tab) get more registers: at 128 and
+// 168 for one and two cells per lane they spilled (20 x 12, sum score: 5.8 ms
+// against 4.6 ms per 1346 steps; 63 x 64, 8 chains: 3.4 against 2.1 us a step).
+// So do the batched kernels of wide rows, whose blocks shared memory limits
+// first.
+__host__ __device__ constexpr int chain_blocks(int w32, int q, bool tab) {
+  if (tab) return w32 > 4 ? 1 : (q == 1 ? 3 : (q == 2 ? 2 : 1));
   return q == 1 ? 4 : (q == 2 ? 3 : 1);
 }
 __host__ __device__ constexpr int chain_regs(int q) {
@@ -112,7 +118,9 @@ __host__ __device__ inline int chain_launch_smem(int n, int n_cells, int q,
 struct TablePlan {
   int chunks;
   bool inc;
-  int smem;  // dynamic shared memory of the launch
+  int smem;         // dynamic shared memory of the launch
+  int ns;           // nodes whose entries are in shared memory
+  size_t global;    // bytes of table per slot in global memory (the others')
 };
 
 __host__ __device__ inline int table_part_bytes(int n, int q, int chunks) {
@@ -126,27 +134,62 @@ __host__ __device__ inline int table_slot_bytes(int n, int rs, int wpc,
          wpc * table_part_bytes(n, q, chunks);
 }
 
+// Rows of five to eight words: a warp's part of a slot holds the table's
+// first ns nodes.
+__host__ __device__ inline int wide_part_bytes(int q, int chunks, int ns) {
+  return chunks * align16(pack_table_bytes(ns, q));
+}
+__host__ __device__ inline int wide_slot_bytes(int n, int rs, int wpc, int w32,
+                                               int q, int chunks, int ns) {
+  return slot_bytes(n, rs, wpc, true, w32, q, false) +
+         wpc * wide_part_bytes(q, chunks, ns);
+}
+
 // The plan of a launch of `slots` chain slots per block, its largest dataset
 // of n nodes and n_cells cells.  Where the tables do not fit a block, or a
-// sum-score chain's cells do not fit one chunk, the cells are streamed as
-// before (such launches are bound by their masked popcounts).
+// sum-score chain's cells of rows of up to four words do not fit one chunk,
+// the cells are streamed as before (such launches are bound by their masked
+// popcounts).
+// Rows of five to eight words take a table when `wide`: max-score chains at
+// fixed rates that have codes (after a change of rates the table would have to
+// be made again).  It is in shared memory where that leaves an SM four warps;
+// else one chain per SM keeps as many nodes there as fit (255 x 512: 216 of
+// 256), the others in global memory.  The sum score keeps the ring: half of
+// its proposals are accepted in the runs measured (255 x 512) and then summed
+// over every node, which with a table was slower (200 x 150: 17 M against
+// 22 M chain-steps/s).
 inline TablePlan plan_tables(int n, int w32, int n_cells, int q, int wpc,
-                             int slots, bool sum, bool one_dataset,
-                             int smem_block) {
+                             int slots, bool sum, bool one_dataset, bool wide,
+                             int smem_block, int smem_sm) {
   const int rs = rs_of_w32(w32), span = 32 * wpc * q;
-  if (w32 > 4)
-    return TablePlan{0, false,
-                     chain_launch_smem(n, n_cells, q, wpc, slots, sum)};
-  const TablePlan p{0, false,
-                    slots * slot_bytes(n, rs, wpc, sum, w32, q, false)};
   const int chunks = (n_cells + span - 1) / span;
+  if (w32 > 4) {
+    const TablePlan ring{0, false,
+                         chain_launch_smem(n, n_cells, q, wpc, slots, sum), 0, 0};
+    if (!wide || sum) return ring;
+    auto smem_of = [&](int ns) {
+      return slots * wide_slot_bytes(n, rs, wpc, w32, q, chunks, ns);
+    };
+    const int full = smem_of(n);
+    if (full <= smem_block &&
+        smem_sm / (full + 1024) * slots * wpc >= 4)
+      return TablePlan{chunks, false, full, n, 0};
+    if (slots > 1) return ring;
+    int ns = n & ~7;
+    while (ns > 0 && smem_of(ns) > smem_block) ns -= 8;
+    if (ns < n / 2) return ring;
+    return TablePlan{chunks, false, smem_of(ns), ns,
+                     (size_t)wpc * chunks * pack_table_bytes(n - ns, q)};
+  }
+  const TablePlan p{0, false, slots * slot_bytes(n, rs, wpc, sum, w32, q, false),
+                    n, 0};
   if (sum && chunks > 1) return p;
   const bool inc = wpc == 1 && one_dataset && chunks == 1;
   const int smem =
       inc ? chain_launch_smem(n, n_cells, q, wpc, slots, sum)
           : slots * table_slot_bytes(n, rs, wpc, w32, q, chunks);
   if (smem > smem_block) return p;
-  return TablePlan{chunks, inc, smem};
+  return TablePlan{chunks, inc, smem, n, 0};
 }
 
 // Resident warps per SM of such a launch (blocks of warps_per_block

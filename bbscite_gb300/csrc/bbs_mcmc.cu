@@ -7,12 +7,11 @@ namespace bbs {
 
 template <int W, bool REC>
 int launch_mcmc_w(const RunArgs &a, int q, bool sum, int cpb, int n_sms,
-                  int smem_block, cudaStream_t s) {
+                  cudaStream_t s) {
 #define BBS_CASE(QQ)                                                  \
-  case QQ:                                                                   \
-    return sum                                                               \
-               ? launch_mcmc_t<W, QQ, true, REC>(a, cpb, n_sms, smem_block, s) \
-               : launch_mcmc_t<W, QQ, false, REC>(a, cpb, n_sms, smem_block, s);
+  case QQ:                                                            \
+    return sum ? launch_mcmc_t<W, QQ, true, REC>(a, cpb, n_sms, s)    \
+               : launch_mcmc_t<W, QQ, false, REC>(a, cpb, n_sms, s);
   switch (q) {
     BBS_CASE(1)
     BBS_CASE(2)
@@ -26,6 +25,6 @@ int launch_mcmc_w(const RunArgs &a, int q, bool sum, int cpb, int n_sms,
 }
 
 template int launch_mcmc_w<BBS_W, BBS_REC != 0>(const RunArgs &, int, bool,
-                                                int, int, int, cudaStream_t);
+                                                int, int, cudaStream_t);
 
 }  // namespace bbs

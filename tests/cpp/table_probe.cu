@@ -48,7 +48,8 @@ int main() {
           for (int slots = 1; slots <= (wpc > 1 ? 1 : 4); slots++)
             for (int sum = 0; sum < 2; sum++) {
               const bbs::TablePlan p = bbs::plan_tables(
-                  n, w32, cells, q, wpc, slots, sum != 0, false, kBlock);
+                  n, w32, cells, q, wpc, slots, sum != 0, false, true, kBlock,
+                  kBlock + 1024);
               const bool fits = slots * sb <= kBlock && !(sum && chunks > 1);
               if (p.inc || p.chunks != (fits ? chunks : 0) ||
                   p.smem != slots * (fits ? sb
@@ -62,6 +63,33 @@ int main() {
               cases++;
             }
         }
+  // rows of five to eight words: plans that fit a block, the nodes that do not
+  // in global memory; the sum score takes none
+  for (int n = 129; n <= 256; n++)
+    for (int q = 1; q <= 2; q++)
+      for (int wpc = 1; wpc <= 4; wpc++)
+        for (int sum = 0; sum < 2; sum++)
+          for (int cells : {1, 33, 150, 512, 2049}) {
+            const int w32 = bbs::w32_of_nodes(n), rs = bbs::rs_of_w32(w32);
+            const int chunks = (cells + 32 * wpc * q - 1) / (32 * wpc * q);
+            const bbs::TablePlan p =
+                bbs::plan_tables(n, w32, cells, q, wpc, 1, sum != 0, true, true,
+                                 kBlock, kBlock + 1024);
+            bool ok = p.smem <= kBlock && !(sum && p.chunks > 0);
+            if (p.chunks > 0)
+              ok = ok && p.chunks == chunks && p.ns >= n / 2 && p.ns <= n &&
+                   (p.ns == n || p.ns % 8 == 0) &&
+                   p.smem == bbs::wide_slot_bytes(n, rs, wpc, w32, q, chunks,
+                                                  p.ns) &&
+                   p.global == (size_t)wpc * chunks *
+                                   bbs::pack_table_bytes(n - p.ns, q);
+            if (!ok) {
+              std::printf("FAIL wide n=%d q=%d wpc=%d sum=%d cells=%d\n", n, q,
+                          wpc, sum, cells);
+              return 1;
+            }
+            cases++;
+          }
   std::printf("tables ok %ld\n", cases);
   return 0;
 }

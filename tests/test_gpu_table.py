@@ -124,3 +124,28 @@ def test_layout_of_slots_with_tables(tmp_path):
     r = subprocess.run([exe], capture_output=True, text=True, timeout=300)
     assert r.returncode == 0, r.stdout
     assert r.stdout.startswith("tables ok "), r.stdout
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("G,Cn,launch", [
+    (128, 40, (2, 1, 2)),     # 129 nodes, the table in shared memory
+    (200, 150, (1, 3, 1)),    # two chunks
+    (191, 97, (2, 1, 1)),     # 192 nodes, an odd last chunk
+    (255, 512, (2, 4, 1)),    # nodes past the block's room in global memory
+    (255, 300, (1, 3, 1)),    # four chunks, some nodes in global memory
+])
+def test_wide_max_chains_equal_traced_ones(native, G, Cn, launch):
+    """Rows of five to eight words at fixed rates: chains on a table against
+    traced ones, which evaluate every node through the ring."""
+    mut, known = _setup(G, Cn, 7)
+    p = native.default_params(alpha_mean=1e-3, beta_mean=0.2, seed=31)
+    got = []
+    for trace in (False, True):
+        with native.Context(mut, known, Cn, G, p) as c:
+            c.init_chains(5)
+            c.set_launch(*launch)
+            for steps in (1, 60, 200):
+                c.run(steps, trace=trace)
+            got.append((c.chains(), c.best(), c.save_chains()))
+    assert got[0][2] == got[1][2]
+    assert got[0][1]["score"] == got[1][1]["score"]
