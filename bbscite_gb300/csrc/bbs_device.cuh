@@ -684,32 +684,32 @@ __device__ __forceinline__ void load_cells(Cells<W32, Q> &cb,
   }
 }
 
-// First-max attachment node of each of the lane's Q cells against all n
-// ancestor rows (ties keep the lower node: std::max in
-// src/TreeScorer.hpp:187-193; node 0 always initialises).  Nodes are taken
+// First-max attachment node of each of the lane's Q cells against ancestor
+// rows j0 .. j1 - 1, and its score (ties keep the lower node: std::max in
+// src/TreeScorer.hpp:187-193; node j0 always initialises).  Nodes are taken
 // two at a time for instruction-level parallelism, in order.
 template <int W32, int Q>
-__device__ __forceinline__ void best_nodes(const uint32_t *rows, int n,
-                                           const Cells<W32, Q> &cb, float l00,
-                                           float l01, float l10, float l11,
-                                           float nz, int (&bj)[Q]) {
+__device__ __forceinline__ void best_nodes_of(const uint32_t *rows, int j0,
+                                              int j1, const Cells<W32, Q> &cb,
+                                              float l00, float l01, float l10,
+                                              float l11, float nz,
+                                              float (&best)[Q], int (&bj)[Q]) {
   constexpr int RS = rs_of_w32(W32);
-  float best[Q];
   {
     uint32_t a[W32];
-    ld_row<W32>(rows, a);
+    ld_row<W32>(rows + j0 * RS, a);
 #pragma unroll
     for (int q = 0; q < Q; q++) {
       const int d = masked_popc<W32>(cb.D[q], a);
       const int m = masked_popc<W32>(cb.M[q], a);
       best[q] = pair_score(d, m, cb.pdb[q], cb.pmb[q], l00, l01, l10, l11);
-      bj[q] = 0;
+      bj[q] = j0;
     }
   }
-  int j = 1;
+  int j = j0 + 1;
   const LogTable2 L2{dup2(l00), dup2(l01), dup2(l10), dup2(l11), dup2(nz)};
 #pragma unroll 1
-  for (; j + 1 < n; j += 2) {
+  for (; j + 1 < j1; j += 2) {
     uint32_t a[W32], b[W32];
     ld_row<W32>(rows + j * RS, a);
     ld_row<W32>(rows + (j + 1) * RS, b);
@@ -732,7 +732,7 @@ __device__ __forceinline__ void best_nodes(const uint32_t *rows, int n,
       bj[q] = up1 ? j + 1 : bj[q];
     }
   }
-  if (j < n) {
+  if (j < j1) {
     uint32_t a[W32];
     ld_row<W32>(rows + j * RS, a);
 #pragma unroll
@@ -745,6 +745,16 @@ __device__ __forceinline__ void best_nodes(const uint32_t *rows, int n,
       bj[q] = up ? j : bj[q];
     }
   }
+}
+
+// The same against all n rows.
+template <int W32, int Q>
+__device__ __forceinline__ void best_nodes(const uint32_t *rows, int n,
+                                           const Cells<W32, Q> &cb, float l00,
+                                           float l01, float l10, float l11,
+                                           float nz, int (&bj)[Q]) {
+  float best[Q];
+  best_nodes_of<W32, Q>(rows, 0, n, cb, l00, l01, l10, l11, nz, best, bj);
 }
 
 // Lane sums of k and m at the chosen nodes.

@@ -1285,6 +1285,38 @@ __global__ void __launch_bounds__(128) init_kernel(const InitArgs a) {
   }
 }
 
+__device__ __forceinline__ void write_score(const ScoreArgs &a, int tree,
+                                            int sk, int sm, const LogTable &L,
+                                            float prior) {
+  const float s = tree_score(a.ds, sk, sm, L, prior);
+  if (a.scores) a.scores[tree] = s;
+  if (a.counts) {
+    int N[4];
+    class_totals(a.ds, sk, sm, N);
+    for (int q = 0; q < 4; q++) a.counts[4 * (size_t)tree + q] = (uint64_t)N[q];
+  }
+}
+
+// Shared memory of score_walk_kernel: the rows, parents, order and depth
+// histogram (n ints and the node -> position map fit it), then each warp's
+// ring and gene table.
+struct WalkLayout {
+  int par, ord, hist, warps, per_warp;
+  __host__ __device__ WalkLayout(int n, int rs) {
+    par = 4 * n * rs;
+    ord = par + align16(n);
+    hist = ord + align16(2 * n);
+    warps = hist + align16(4 * 32 * ((n + 31) / 32));
+    per_warp = align16(ring_bytes(2)) + align16(gene_table_bytes(n, 2));
+  }
+  __host__ __device__ int bytes(int n_warps) const {
+    return warps + n_warps * per_warp;
+  }
+};
+
+// Scores of a batch, one warp per tree: many trees of rows of up to four
+// words, whose trees' parent vectors and orders would cost as much as they
+// save (95 x 96: 65 us for 4096 trees).
 template <int W32, int Q, bool ATTACH>
 __global__ void __launch_bounds__(128) score_kernel(const ScoreArgs a) {
   extern __shared__ __align__(16) uint32_t smem[];
@@ -1320,14 +1352,241 @@ __global__ void __launch_bounds__(128) score_kernel(const ScoreArgs a) {
   const int sk = (int)__reduce_add_sync(BBS_FULL_MASK, (uint32_t)k);
   const int sm = (int)__reduce_add_sync(BBS_FULL_MASK, (uint32_t)m);
   if (lane == 0) {
-    const float s = tree_score(a.ds, sk, sm, L, prior);
-    if (a.scores) a.scores[tree] = s;
-    if (a.counts) {
-      int N[4];
-      class_totals(a.ds, sk, sm, N);
-      for (int q = 0; q < 4; q++) a.counts[4 * (size_t)tree + q] = (uint64_t)N[q];
+    write_score(a, tree, sk, sm, L, prior);
+  }
+}
+
+// Scores of few trees: one block per tree, its warps split the chunks of 32
+// cells and, four ways, the nodes, so that a call for one tree waits for some
+// 25 nodes' latency instead of all nodes of two chunks (kernel time of one tree
+// at 95 x 96: 20.5 -> 5.6 us; at 255 x 512 the call went from 434 to 98 us).
+inline constexpr int kFewRanges = 4, kFewGroups = 4;
+
+template <int W32, bool ATTACH>
+__global__ void __launch_bounds__(32 * kFewRanges * kFewGroups)
+    score_few_kernel(const ScoreArgs a) {
+  extern __shared__ __align__(16) uint32_t smem[];
+  constexpr int RS = rs_of_w32(W32);
+  __shared__ float part_s[kFewGroups][kFewRanges][32];
+  __shared__ int part_j[kFewGroups][kFewRanges][32];
+  __shared__ int sums[2];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int group = warp / kFewRanges, range = warp % kFewRanges;
+  const int n = a.ds.n_nodes, tree = blockIdx.x;
+  const uint32_t *src = a.rows + (size_t)tree * n * RS;
+  for (int i = threadIdx.x; i < n * RS; i += blockDim.x) smem[i] = src[i];
+  if (threadIdx.x < 2) sums[threadIdx.x] = 0;
+  __syncthreads();
+  const float *bt = a.beta_terms + 4 * (size_t)tree;
+  const LogTable L{a.ds.l00, a.ds.l10, bt[1], bt[2]};
+  const int j0 = n * range / kFewRanges, j1 = n * (range + 1) / kFewRanges;
+  int k = 0, m = 0;
+  for (int base = 0; base < a.ds.n_cells; base += 32 * kFewGroups) {
+    const int c0 = base + 32 * group;
+    Cells<W32, 1> cb;
+    load_cells<W32, 1>(cb, a.ds, c0, 32, lane);
+    if (j0 < j1) {
+      float best[1];
+      int bj[1];
+      best_nodes_of<W32, 1>(smem, j0, j1, cb, L.l00, L.l01, L.l10, L.l11,
+                            a.ds.neg_zero, best, bj);
+      part_s[group][range][lane] = best[0];
+      part_j[group][range][lane] = bj[0];
+    } else {
+      part_j[group][range][lane] = -1;  // fewer nodes than ranges
+    }
+    __syncthreads();
+    if (range == 0) {
+      // the first maximum: ranges are in node order, an equal score later on
+      // does not win
+      float best = 0.0f;
+      int bj[1] = {-1};
+#pragma unroll
+      for (int r = 0; r < kFewRanges; r++) {
+        const int j = part_j[group][r][lane];
+        const float s = part_s[group][r][lane];
+        if (j >= 0 && (bj[0] < 0 || s > best)) {
+          best = s;
+          bj[0] = j;
+        }
+      }
+      counts_at<W32, 1>(smem, cb, bj, k, m);
+      if constexpr (ATTACH) {
+        const int c = c0 + lane;
+        if (c < a.ds.n_cells)
+          a.attach[(size_t)tree * a.ds.n_cells + c] = (uint32_t)bj[0];
+      }
+    }
+    __syncthreads();  // the partial results are written again
+  }
+  k = (int)__reduce_add_sync(BBS_FULL_MASK, (uint32_t)k);
+  m = (int)__reduce_add_sync(BBS_FULL_MASK, (uint32_t)m);
+  if (range == 0 && lane == 0) {
+    atomicAdd(&sums[0], k);
+    atomicAdd(&sums[1], m);
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) write_score(a, tree, sums[0], sums[1], L, bt[3]);
+}
+
+// Scores of many trees with rows of five to eight words: one block per tree,
+// four warps over its chunks of 64 cells.  Where the rows are a tree whose
+// order fits the ring and its rates have exact codes (bbs_incr.cuh), each node
+// takes its parent's codes from the ring plus its gene's, some 20
+// instructions a node for 64 cells; otherwise masked popcounts, which run the
+// population-count pipe at its peak (255 x 512, 1500 trees: 735 us, now 230 us,
+// bound by the latency of the walk at three blocks per SM).
+template <int W32, bool ATTACH>
+__global__ void __launch_bounds__(128) score_walk_kernel(const ScoreArgs a) {
+  extern __shared__ __align__(16) uint32_t smem[];
+  constexpr int RS = rs_of_w32(W32), Q = 2, WARPS = 4;
+  __shared__ int sums[2], fits;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int n = a.ds.n_nodes, tree = blockIdx.x;
+  const WalkLayout w(n, RS);
+  uint8_t *base = reinterpret_cast<uint8_t *>(smem);
+  uint32_t *rows = smem;
+  uint8_t *par = base + w.par;
+  uint16_t *ord = reinterpret_cast<uint16_t *>(base + w.ord);
+  int *hist = reinterpret_cast<int *>(base + w.hist);
+  uint32_t *ring = reinterpret_cast<uint32_t *>(base + w.warps + warp * w.per_warp);
+  uint32_t *gt = ring + ring_bytes(Q) / 4;
+  copy_rows_part<W32>(a.rows + (size_t)tree * n * RS, rows, n, WARPS, warp, lane);
+  if (threadIdx.x < 2) sums[threadIdx.x] = 0;
+  __syncthreads();
+  const float *bt = a.beta_terms + 4 * (size_t)tree;
+  const LogTable L{a.ds.l00, a.ds.l10, bt[1], bt[2]};
+  // parents: the deepest proper ancestor, checked against the rows
+  for (int x = threadIdx.x; x < n; x += blockDim.x) {
+    uint32_t r[W32];
+    ld_row<W32>(rows + x * RS, r);
+    int pc = 0;
+#pragma unroll
+    for (int k = 0; k < W32; k++) pc += __popc(r[k]);
+    hist[x] = pc;
+  }
+  __syncthreads();
+  bool ok = true;
+  for (int x = threadIdx.x; x < n; x += blockDim.x) {
+    uint32_t r[W32], q[W32];
+    ld_row<W32>(rows + x * RS, r);
+    // a tree's parent has one ancestor less
+    int p = x == n - 1 ? x : -1;
+#pragma unroll
+    for (int k = 0; k < W32; k++) {
+      uint32_t v = k == (x >> 5) ? r[k] & ~(1u << (x & 31)) : r[k];
+      while (v != 0u && p < 0) {
+        const int y = 32 * k + __ffs(v) - 1;
+        v &= v - 1u;
+        if (y < n && hist[y] == hist[x] - 1) p = y;
+      }
+    }
+    if (p < 0) {
+      ok = false;
+      p = n - 1;
+    }
+    par[x] = (uint8_t)p;
+    ld_row<W32>(rows + p * RS, q);
+#pragma unroll
+    for (int k = 0; k < W32; k++) {
+      const uint32_t own = k == (x >> 5) ? 1u << (x & 31) : 0u;
+      ok = ok && (x == n - 1 ? r[k] == own
+                             : r[k] == (q[k] | own) && (q[k] & own) == 0u);
     }
   }
+  ok = __syncthreads_and(ok);
+  const MaxCode code =
+      make_code(L.l00, L.l01, L.l10, L.l11, a.ds.max_d, a.ds.max_m, lane);
+  ok = ok && code.usable && code.exact;
+  if (ok && warp == 0) {
+    const bool f = ring_order<W32>(rows, n, par, ord, hist, lane);
+    if (lane == 0) fits = f ? 1 : 0;
+  }
+  __syncthreads();
+  ok = ok && fits != 0;
+  const uint32_t wd = (uint32_t)(-code.s * code.P), wm = (uint32_t)(code.s * code.Q);
+  int k = 0, m = 0;
+  for (int c0 = 64 * warp; c0 < a.ds.n_cells; c0 += 64 * WARPS) {
+    Cells<W32, Q> cb;
+    load_cells<W32, Q>(cb, a.ds, c0, 32, lane);
+    int bj[Q];
+    if (ok) {
+      build_gene_table<W32, Q>(cb, gt, n, lane);
+      // T of both cells in one word; with attachments, keys T << 8 | 255 - j
+      uint32_t best = (uint32_t)code.off * 0x10001u;
+      uint32_t key0 = 0u, key1 = 0u;
+      auto see = [&](uint32_t t, int j) {
+        if constexpr (ATTACH) {
+          const uint32_t jj = 255u - (uint32_t)j;
+          key0 = max(key0, __byte_perm(t, jj, 0x5104u));
+          key1 = max(key1, __byte_perm(t, jj, 0x5324u));
+        } else {
+          best = __vmaxu2(best, t);
+        }
+      };
+      auto gene = [&](int j) {
+        uint32_t g[1];
+        gene_inc<Q>(gt, j, lane, g);
+        return (g[0] & 0x00010001u) * wd + ((g[0] >> 8) & 0x00010001u) * wm;
+      };
+      ring[lane] = best;
+      see(best, n - 1);
+      int i = 1;
+#pragma unroll 2
+      for (; i + 1 < n; i += 2) {
+        const uint32_t o0 = ord[i], o1 = ord[i + 1];
+        const int u0 = (int)(o0 & 0xFF), u1 = (int)(o1 & 0xFF);
+        const int p0 = (int)(o0 >> 8), p1 = (int)(o1 >> 8);
+        const uint32_t a0 = ring[(p0 & (kRing - 1)) * 32 + lane];
+        const uint32_t a1 = ring[(p1 & (kRing - 1)) * 32 + lane];
+        const uint32_t t0 = a0 + gene(u0);
+        const uint32_t t1 = (p1 == i ? t0 : a1) + gene(u1);
+        ring[(i & (kRing - 1)) * 32 + lane] = t0;
+        ring[((i + 1) & (kRing - 1)) * 32 + lane] = t1;
+        see(t0, u0);
+        see(t1, u1);
+      }
+      if (i < n) {
+        const uint32_t o = ord[i];
+        see(ring[((int)(o >> 8) & (kRing - 1)) * 32 + lane] + gene((int)(o & 0xFF)),
+            (int)(o & 0xFF));
+      }
+#pragma unroll
+      for (int q = 0; q < Q; q++) {
+        int d, mm;
+        if constexpr (ATTACH) {
+          const uint32_t key = q ? key1 : key0;
+          bj[q] = 255 - (int)(key & 0xFFu);
+          decode<true>(code, key >> 8, d, mm);
+        } else {
+          decode<true>(code, (best >> (16 * q)) & 0xFFFFu, d, mm);
+        }
+        k += d + mm;
+        m += mm;
+      }
+      __syncwarp();
+    } else {
+      best_nodes<W32, Q>(rows, n, cb, L.l00, L.l01, L.l10, L.l11,
+                         a.ds.neg_zero, bj);
+      counts_at<W32, Q>(rows, cb, bj, k, m);
+    }
+    if constexpr (ATTACH) {
+#pragma unroll
+      for (int q = 0; q < Q; q++) {
+        const int c = c0 + 32 * q + lane;
+        if (c < a.ds.n_cells)
+          a.attach[(size_t)tree * a.ds.n_cells + c] = (uint32_t)bj[q];
+      }
+    }
+  }
+  k = (int)__reduce_add_sync(BBS_FULL_MASK, (uint32_t)k);
+  m = (int)__reduce_add_sync(BBS_FULL_MASK, (uint32_t)m);
+  if (lane == 0) {
+    atomicAdd(&sums[0], k);
+    atomicAdd(&sums[1], m);
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) write_score(a, tree, sums[0], sums[1], L, bt[3]);
 }
 
 template <int W32>
@@ -1366,99 +1625,156 @@ __global__ void __launch_bounds__(128) apply_kernel(const ApplyArgs a) {
   }
 }
 
-// Sum-over-attachments score and adjoint.  Per cell an online logsumexp
-// over nodes carries the softmax-weighted sums of k = popc(K & A_j) and
-// m = popc(M & A_j); the expected class counts follow from the identity
-// above, and dlogL/dtheta = sum_c sum_k E_pi[n_k] dl_k/dtheta.
-template <int W32, int Q>
-__global__ void __launch_bounds__(128) grad_kernel(const GradArgs a) {
+// Sum-over-attachments score and adjoint: one block per tree, its warps over
+// the chunks of 32 cells.  Per cell exp(s_j - r) is summed against r = ub -
+// 72, ub >= every s_j (as in sum_cells: no term overflows), with the
+// softmax-weighted sums of d and m; a cell whose maximum lies more than 80
+// below r is summed again against its maximum.  An online maximum per term,
+// as before, took both sides of a branch and two exponentials for most nodes
+// (4096 trees at 95 x 96: 110 us, now 85 us, bound by instruction issue).  The expected class counts give dlogL /
+// dtheta = sum_c sum_k E_pi[n_k] dl_k / dtheta.
+// With posteriors a warp keeps its cells' scores in shared memory (`tile`
+// floats per cell) and writes the 32 cells' rows as one contiguous piece; a
+// store per lane and node went to 32 lines each (50 trees at 61 x 201: 83 ->
+// 15 us).
+template <int W32, bool POST>
+__global__ void __launch_bounds__(256) grad_kernel(const GradArgs a) {
   extern __shared__ __align__(16) uint32_t smem[];
   constexpr int RS = rs_of_w32(W32);
-  const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-  const int wpb = blockDim.x >> 5;
-  const int tree = blockIdx.x * wpb + wib;
-  if (tree >= a.n_trees) return;
-  const int n = a.ds.n_nodes;
-  uint32_t *rows = smem + (size_t)wib * n * RS;
-  copy_rows<W32>(a.rows + (size_t)tree * n * RS, rows, n, lane);
-  __syncwarp();
+  __shared__ float sums[8][5];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int warps = blockDim.x >> 5;
+  const int n = a.ds.n_nodes, tree = blockIdx.x;
+  const int tile = n | 1;  // odd: a node's 32 scores lie in 32 banks
+  float *mine = reinterpret_cast<float *>(smem + n * RS) + warp * 32 * tile;
+  const uint32_t *src = a.rows + (size_t)tree * n * RS;
+  for (int i = threadIdx.x; i < n * RS; i += blockDim.x) smem[i] = src[i];
+  __syncthreads();
   const float *tb = a.tables + 6 * (size_t)tree;
   const float l00 = tb[2], l01 = tb[3], l10 = tb[4], l11 = tb[5];
-  float acc_lse = 0.0f, acc_n00 = 0.0f, acc_n01 = 0.0f, acc_n10 = 0.0f,
-        acc_n11 = 0.0f;
-  Cells<W32, Q> cb;
-  for (int c0 = 0; c0 < a.ds.n_cells; c0 += 32 * Q) {
-    load_cells<W32, Q>(cb, a.ds, c0, 32, lane);
-    float mx[Q], z[Q], ek[Q], em[Q];
-#pragma unroll
-    for (int q = 0; q < Q; q++) {
-      mx[q] = -INFINITY;
-      z[q] = ek[q] = em[q] = 0.0f;
-    }
-    for (int j = 0; j < n; j++) {
-      uint32_t r[W32];
-      ld_row<W32>(rows + j * RS, r);
-#pragma unroll
-      for (int q = 0; q < Q; q++) {
-        const int d = masked_popc<W32>(cb.D[q], r);
-        const int m = masked_popc<W32>(cb.M[q], r);
-        const int k = d + m;
-        const float s = pair_score(d, m, cb.pdb[q], cb.pmb[q], l00, l01, l10, l11);
-        if (s > mx[q]) {
-          const float sc = expf(mx[q] - s);
-          z[q] = z[q] * sc + 1.0f;
-          ek[q] = ek[q] * sc + (float)k;
-          em[q] = em[q] * sc + (float)m;
-          mx[q] = s;
-        } else {
-          const float e = expf(s - mx[q]);
-          z[q] += e;
-          ek[q] += e * (float)k;
-          em[q] += e * (float)m;
+  const LogTable2 L2{dup2(l00), dup2(l01), dup2(l10), dup2(l11),
+                     dup2(a.ds.neg_zero)};
+  // Chunk c adds to sum c % 8, whichever warp takes it: the totals are the
+  // same with any number of warps (posteriors leave room for fewer).
+  for (int slot = warp; slot < 8; slot += warps) {
+    float acc[5] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f};  // lse, n00, n01, n10, n11
+    for (int c0 = 32 * slot; c0 < a.ds.n_cells; c0 += 32 * 8) {
+      Cells<W32, 1> cb;
+      load_cells<W32, 1>(cb, a.ds, c0, 32, lane);
+      const float pd = cb.pdb[0] - 8388608.0f, pm = cb.pmb[0] - 8388608.0f;
+      float r = fmaf(pd, fmaxf(l00, l01), pm * fmaxf(l10, l11)) - 72.0f;
+      float mx, z, ed, em;
+      auto sum = [&](bool first) {
+        mx = -INFINITY;
+        float2 z2 = dup2(0.0f), d2 = z2, m2 = z2;
+        int j = 0;
+#pragma unroll 2
+        for (; j + 1 < n; j += 2) {
+          uint32_t ra[W32], rb[W32];
+          ld_row<W32>(smem + j * RS, ra);
+          ld_row<W32>(smem + (j + 1) * RS, rb);
+          const float2 db = make_float2(
+              __int_as_float(0x4B000000 + masked_popc<W32>(cb.D[0], ra)),
+              __int_as_float(0x4B000000 + masked_popc<W32>(cb.D[0], rb)));
+          const float2 mb = make_float2(
+              __int_as_float(0x4B000000 + masked_popc<W32>(cb.M[0], ra)),
+              __int_as_float(0x4B000000 + masked_popc<W32>(cb.M[0], rb)));
+          const float2 s =
+              pair_score_b2(db, mb, dup2(cb.pdb[0]), dup2(cb.pmb[0]), L2);
+          mx = fmax3(mx, s.x, s.y);
+          if (POST && first) {
+            mine[lane * tile + j] = s.x;
+            mine[lane * tile + j + 1] = s.y;
+          }
+          const float2 e = make_float2(expf(s.x - r), expf(s.y - r));
+          const float2 bias = dup2(8388608.0f);
+          z2 = fadd2(z2, e);
+          d2 = ffma2(e, fsub2(db, bias), d2);
+          m2 = ffma2(e, fsub2(mb, bias), m2);
         }
+        z = z2.x + z2.y;
+        ed = d2.x + d2.y;
+        em = m2.x + m2.y;
+        if (j < n) {
+          uint32_t ra[W32];
+          ld_row<W32>(smem + j * RS, ra);
+          const int d = masked_popc<W32>(cb.D[0], ra);
+          const int m = masked_popc<W32>(cb.M[0], ra);
+          const float s =
+              pair_score(d, m, cb.pdb[0], cb.pmb[0], l00, l01, l10, l11);
+          mx = fmaxf(mx, s);
+          if (POST && first) mine[lane * tile + j] = s;
+          const float e = expf(s - r);
+          z += e;
+          ed = fmaf(e, (float)d, ed);
+          em = fmaf(e, (float)m, em);
+        }
+      };
+      sum(true);
+      const bool bad = !(mx - r >= -80.0f);
+      if (__any_sync(BBS_FULL_MASK, bad)) {
+        if (bad) r = mx;
+        sum(false);
       }
-    }
-#pragma unroll
-    for (int q = 0; q < Q; q++) {
-      const int c = c0 + 32 * q + lane;
-      if (c >= a.ds.n_cells) continue;
-      const float lse = mx[q] + logf(z[q]);
-      const float Ek = ek[q] / z[q], Em = em[q] / z[q];
-      const float pm = cb.pmb[q] - 8388608.0f;
-      const float pkm = cb.pdb[q] - 8388608.0f;
-      acc_lse += lse;
-      acc_n11 += Em;
-      acc_n01 += Ek - Em;
-      acc_n10 += pm - Em;
-      acc_n00 += pkm - Ek + Em;
-      if (a.posterior != nullptr) {
-        float *post = a.posterior + ((size_t)tree * a.ds.n_cells + c) * n;
+      // (against the maximum: r + log z would round a log of up to 72)
+      const float lse = mx + logf(z * expf(r - mx));
+      if (c0 + lane < a.ds.n_cells) {
+        const float Ed = ed / z, Em = em / z;
+        acc[0] += lse;
+        acc[1] += pd - Ed;
+        acc[2] += Ed;
+        acc[3] += pm - Em;
+        acc[4] += Em;
+      }
+      if constexpr (POST) {
+        // against the maximum, where the differences of the scores are exact
+        float zm = 0.0f;
         for (int j = 0; j < n; j++) {
-          uint32_t r[W32];
-          ld_row<W32>(rows + j * RS, r);
-          const float s = pair_score(masked_popc<W32>(cb.D[q], r),
-                                     masked_popc<W32>(cb.M[q], r), cb.pdb[q],
-                                     cb.pmb[q], l00, l01, l10, l11);
-          post[j] = expf(s - lse);
+          const float e = expf(mine[lane * tile + j] - mx);
+          zm += e;
+          mine[lane * tile + j] = e;
         }
+        const float inv = 1.0f / zm;
+        for (int j = 0; j < n; j++) mine[lane * tile + j] *= inv;
+        __syncwarp();
+        const int cells = min(32, a.ds.n_cells - c0);
+        float *post = a.posterior + ((size_t)tree * a.ds.n_cells + c0) * n;
+        // lane l starts at element l; 32 elements further is (n + l) / n cells
+        int cell = 0, j = lane;
+        while (j >= n) {
+          j -= n;
+          cell++;
+        }
+        for (int i = lane; i < cells * n; i += 32) {
+          post[i] = mine[cell * tile + j];
+          j += 32;
+          while (j >= n) {
+            j -= n;
+            cell++;
+          }
+        }
+        __syncwarp();
       }
     }
-  }
 #pragma unroll
-  for (int off = 16; off > 0; off >>= 1) {
-    acc_lse += __shfl_xor_sync(BBS_FULL_MASK, acc_lse, off);
-    acc_n00 += __shfl_xor_sync(BBS_FULL_MASK, acc_n00, off);
-    acc_n01 += __shfl_xor_sync(BBS_FULL_MASK, acc_n01, off);
-    acc_n10 += __shfl_xor_sync(BBS_FULL_MASK, acc_n10, off);
-    acc_n11 += __shfl_xor_sync(BBS_FULL_MASK, acc_n11, off);
+    for (int k = 0; k < 5; k++) {
+#pragma unroll
+      for (int off = 16; off > 0; off >>= 1)
+        acc[k] += __shfl_xor_sync(BBS_FULL_MASK, acc[k], off);
+      if (lane == 0) sums[slot][k] = acc[k];
+    }
   }
-  if (lane == 0) {
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    float t[5] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
+    for (int w = 0; w < 8; w++)
+      for (int k = 0; k < 5; k++) t[k] += sums[w][k];
     const double al = tb[0], be = tb[1];
-    a.logl[tree] = acc_lse;
+    a.logl[tree] = t[0];
     if (a.dalpha)
-      a.dalpha[tree] = (float)(-(double)acc_n00 / (1.0 - al) + (double)acc_n10 / al);
+      a.dalpha[tree] = (float)(-(double)t[1] / (1.0 - al) + (double)t[3] / al);
     if (a.dbeta)
-      a.dbeta[tree] = (float)((double)acc_n01 / be - (double)acc_n11 / (1.0 - be));
+      a.dbeta[tree] = (float)((double)t[2] / be - (double)t[4] / (1.0 - be));
   }
 }
 
