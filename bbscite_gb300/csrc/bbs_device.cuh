@@ -939,13 +939,22 @@ __device__ __forceinline__ void canonical_order(const uint32_t *rows, int n,
 }
 
 // The canonical order for counts inherited through a ring (rows of five to
-// eight words): the positions of canonical_order, each entry node | ppos
-// << 8 with ppos the order position of the node's parent, from `par`, the
-// tree's parent vector (the root, at position 0, gets 0).  Returns whether
-// every node lies fewer than kRing positions after its parent, so that the
-// parent's counts are still in the ring when the node is reached; where
-// not, ord still holds the canonical node order in its low bytes.  hist
-// doubles as the node -> position map (32 ceil(n / 32) >= n ints).
+// eight words): ord gets the nodes at the positions of canonical_order, and
+// hist, at position less one, an entry per node but the root that holds the
+// byte offsets the walk needs, so that a node costs it no address arithmetic
+// (`par` is the tree's parent vector; hist has 32 ceil(n / 32) >= n ints):
+//   bits 0-2   bit of the node in its byte of the gene table
+//   bit 5      the parent is the position before
+//   bits 7-12  offset of the parent's counts in the ring (position p in ring
+//              entry p + 1 mod kRing: pairs of positions start even)
+//   bits 23-27 node / 8, as an offset of 128 bytes above bit 16
+// Returns whether every node lies fewer than kRing positions after its
+// parent, so that the parent's counts are still in the ring when the node is
+// reached.
+inline constexpr uint32_t kRingBytes = 128u * kRing;
+__device__ __forceinline__ int ring_node(uint32_t o) {
+  return (int)((o >> 23 << 3) | (o & 7u));
+}
 template <int W32>
 __device__ __forceinline__ bool ring_order(const uint32_t *rows, int n,
                                            const uint8_t *par, uint16_t *ord,
@@ -1003,11 +1012,18 @@ __device__ __forceinline__ bool ring_order(const uint32_t *rows, int n,
     if (valid && (same & below) == 0) hist[dep[g]] += __popc(same);
     __syncwarp();
   }
-  // node -> position, then the entries with their parents' positions
+  // node -> position, then the entries
 #pragma unroll
   for (int g = 0; g < W32; g++) {
     const int x = 32 * g + lane;
     if (x < n) hist[x] = at[g];
+  }
+  __syncwarp();
+  int pp[W32];
+#pragma unroll
+  for (int g = 0; g < W32; g++) {
+    const int x = 32 * g + lane;
+    pp[g] = x < n - 1 ? hist[min((int)par[x], n - 1)] : 0;
   }
   __syncwarp();
   bool ok = true;
@@ -1015,9 +1031,13 @@ __device__ __forceinline__ bool ring_order(const uint32_t *rows, int n,
   for (int g = 0; g < W32; g++) {
     const int x = 32 * g + lane;
     if (x < n) {
-      const int pp = x == n - 1 ? 0 : hist[min((int)par[x], n - 1)];
-      ord[at[g]] = (uint16_t)(x | (pp << 8));
-      ok = ok && at[g] - pp < kRing;
+      ord[at[g]] = (uint16_t)x;
+      ok = ok && at[g] - pp[g] < kRing;
+      if (at[g] > 0)
+        hist[at[g] - 1] =
+            (int)(((uint32_t)x & 7u) | (pp[g] == at[g] - 1 ? 32u : 0u) |
+                  (((uint32_t)(pp[g] + 1) * 128u) & (kRingBytes - 128u)) |
+                  ((uint32_t)x >> 3 << 23));
     }
   }
   __syncwarp();
@@ -1171,63 +1191,106 @@ __device__ __noinline__ bool parents_match_rows(const uint32_t *rows, int n,
   return __all_sync(BBS_FULL_MASK, ok);
 }
 
-// Inherited counts of the nodes at order positions i and i + 1, all Q cells
-// at once (packed), for rows of five to eight words: the parents' counts
-// come from the ring (entries hold the parents' order positions,
-// ring_order), the increments from the gene table, and positions i and i + 1
-// are stored in the ring.  All four loads come first.  Why no load reads an overwritten entry: when the loads run,
-// positions up to i - 1 are stored (each lane reads and writes only its own
-// column, in program order).  A parent at position p < i was stored at
-// entry p % kRing, and the positions stored since, p + 1 .. i - 1, are
+// Inherited counts of the nodes at order positions i and i + 1, i odd, all Q
+// cells at once (packed), for rows of five to eight words: `o` holds their
+// entries (ring_order); the parents' counts come from the ring, the
+// increments from the gene table, and both positions are stored in the ring.
+// All four loads come first.  Why no load reads an overwritten entry: when
+// the loads run, positions up to i - 1 are stored (each lane reads and writes
+// only its own column, in program order).  A parent at position p < i was
+// stored at its entry, and the positions stored since, p + 1 .. i - 1, are
 // fewer than kRing (ring_order checked i + 1 - p < kRing), so none of them
 // maps to that entry.  A parent at position i, not stored yet, is taken
 // from the register.
-template <int Q, int NW = kPackWords<Q>>
-__device__ __forceinline__ void inherit_pair_ring(const SumCtx &sx, int i,
-                                                  int lane,
-                                                  uint32_t (&k0)[NW],
-                                                  uint32_t (&k1)[NW], int &j0,
-                                                  int &j1) {
-  const uint32_t o0 = sx.ord[i], o1 = sx.ord[i + 1];
-  j0 = (int)(o0 & 0xFF);
-  j1 = (int)(o1 & 0xFF);
-  const int p0 = (int)(o0 >> 8), p1 = (int)(o1 >> 8);
-  uint32_t a0[NW], a1[NW], g0[NW], g1[NW];
-  ld_pack<Q>(sx.ring, (p0 & (kRing - 1)) * 32 + lane, a0);
-  ld_pack<Q>(sx.ring, (p1 & (kRing - 1)) * 32 + lane, a1);
-  gene_inc<Q>(sx.gt, j0, lane, g0);
-  gene_inc<Q>(sx.gt, j1, lane, g1);
-#pragma unroll
-  for (int w = 0; w < NW; w++) {
-    k0[w] = a0[w] + g0[w];
-    k1[w] = (p1 == i ? k0[w] : a1[w]) + g1[w];
-  }
-  st_pack<Q>(sx.ring, (i & (kRing - 1)) * 32 + lane, k0);
-  st_pack<Q>(sx.ring, ((i + 1) & (kRing - 1)) * 32 + lane, k1);
+// With node and parent position in 16 bits most of the walk's some 36
+// instructions a pair were address arithmetic; these are some 21 (langevin
+// chains at 255 x 512: 109.4 -> 94.2 ms per 1000 steps of 1024 chains, bound
+// by the latency of 1.75 warps per scheduler, what shared memory takes).
+__device__ __forceinline__ uint2 ring_pair(const SumCtx &sx, int i) {
+  return *reinterpret_cast<const uint2 *>(sx.hist + i - 1);
+}
+
+__device__ __forceinline__ uint32_t ring_counts(const SumCtx &sx, uint32_t o,
+                                                int lane, uint32_t &g) {
+  const char *ring = reinterpret_cast<const char *>(sx.ring + lane);
+  const char *gt = reinterpret_cast<const char *>(sx.gt + lane);
+  g = *reinterpret_cast<const uint32_t *>(gt + (o >> 16));
+  return *reinterpret_cast<const uint32_t *>(ring + (o & (kRingBytes - 128u)));
+}
+
+// The node's bits of its gene-table word (the shift takes o's low five bits).
+__device__ __forceinline__ uint32_t ring_gene(uint32_t g, uint32_t o) {
+  return __funnelshift_r(g, 0u, o) & 0x01010101u;
 }
 
 template <int Q, int NW = kPackWords<Q>>
-__device__ __forceinline__ void inherit_one_ring(const SumCtx &sx, int i,
-                                                 int lane, uint32_t (&k)[NW],
-                                                 int &j) {
-  const uint32_t o = sx.ord[i];
-  j = (int)(o & 0xFF);
-  const int p = (int)(o >> 8);
-  uint32_t a[NW], g[NW];
-  ld_pack<Q>(sx.ring, (p & (kRing - 1)) * 32 + lane, a);
-  gene_inc<Q>(sx.gt, j, lane, g);
-#pragma unroll
-  for (int w = 0; w < NW; w++) k[w] = a[w] + g[w];
-  st_pack<Q>(sx.ring, (i & (kRing - 1)) * 32 + lane, k);
+__device__ __forceinline__ void inherit_pair_ring(const SumCtx &sx, uint2 o,
+                                                  int i, int lane,
+                                                  uint32_t (&k0)[NW],
+                                                  uint32_t (&k1)[NW]) {
+  static_assert(NW == 1, "wide rows take one or two cells per lane");
+  uint32_t g0, g1;
+  const uint32_t a0 = ring_counts(sx, o.x, lane, g0);
+  const uint32_t a1 = ring_counts(sx, o.y, lane, g1);
+  k0[0] = a0 + ring_gene(g0, o.x);
+  k1[0] = ((o.y & 32u) ? k0[0] : a1) + ring_gene(g1, o.y);
+  char *at = reinterpret_cast<char *>(sx.ring + lane) +
+             (((uint32_t)i + 1u) * 128u & (kRingBytes - 128u));
+  *reinterpret_cast<uint32_t *>(at) = k0[0];
+  *reinterpret_cast<uint32_t *>(at + 128) = k1[0];
+}
+
+// The node at position i, the last of the order.
+template <int Q, int NW = kPackWords<Q>>
+__device__ __forceinline__ void inherit_last_ring(const SumCtx &sx, uint32_t o,
+                                                  int lane,
+                                                  uint32_t (&k)[NW]) {
+  uint32_t g;
+  const uint32_t a = ring_counts(sx, o, lane, g);
+  k[0] = a + ring_gene(g, o);
+}
+
+// The pairs of positions from i = 1 on, each passed to f with its entries;
+// i ends at the last position where one is left over, else at n.  Counts are
+// one pair ahead of f's work and entries one pair ahead of the counts, which
+// hides the loads behind the previous pair's arithmetic; two pairs per
+// iteration, alternating between two register sets.  (Entries i + 5 and i + 6
+// of hist, i + 5 < n, may lie past the order's end and are then not used: i +
+// 5 is even, so the pair ends within hist's multiple of 32 ints.)
+template <int Q, typename F>
+__device__ __forceinline__ void walk_ring(const SumCtx &sx, int n, int lane,
+                                          int &i, F f) {
+  constexpr int NW = kPackWords<Q>;
+  if (i + 1 >= n) return;
+  uint32_t kA0[NW], kA1[NW], kB0[NW], kB1[NW];
+  uint2 oA = ring_pair(sx, i), oB = oA;
+  inherit_pair_ring<Q>(sx, oA, i, lane, kA0, kA1);
+  if (i + 3 < n) oB = ring_pair(sx, i + 2);
+#pragma unroll 1
+  for (; i + 5 < n; i += 4) {
+    const uint2 oC = ring_pair(sx, i + 4);
+    inherit_pair_ring<Q>(sx, oB, i + 2, lane, kB0, kB1);
+    f(kA0, oA.x, kA1, oA.y);
+    oA = oC;
+    const uint2 oD = ring_pair(sx, i + 6);
+    inherit_pair_ring<Q>(sx, oA, i + 4, lane, kA0, kA1);
+    f(kB0, oB.x, kB1, oB.y);
+    oB = oD;
+  }
+  if (i + 3 < n) {
+    inherit_pair_ring<Q>(sx, oB, i + 2, lane, kB0, kB1);
+    f(kA0, oA.x, kA1, oA.y);
+    f(kB0, oB.x, kB1, oB.y);
+    i += 4;
+  } else {
+    f(kA0, oA.x, kA1, oA.y);
+    i += 2;
+  }
 }
 
 // The root's zero counts, at order position 0.
-template <int Q, int NW = kPackWords<Q>>
 __device__ __forceinline__ void store_root(const SumCtx &sx, int lane) {
-  uint32_t zero[NW];
-#pragma unroll
-  for (int w = 0; w < NW; w++) zero[w] = 0u;
-  st_pack<Q>(sx.ring, lane, zero);
+  sx.ring[32 + lane] = 0u;
 }
 
 // The sum score's float work of two nodes, side by side in the halves of
@@ -1337,39 +1400,60 @@ __device__ __noinline__ Resum<Q> resum_cells(const uint32_t *rows, int n,
 // resum_cells for the ring: the counts inherited once more along the
 // order (the chunk's gene table is still in place), the same terms summed
 // in the same order as resum_cells, so the sums are those of the other
-// count sources.
+// count sources.  The lane's two cells go side by side in the halves of
+// paired registers, whether both are wanted or one: 24 instructions a node
+// (cell by cell behind a test of its bit, 40).
 template <int Q>
 __device__ __noinline__ Resum<Q> resum_cells_ring(int n, const SumCtx sx,
                                                   int lane, float c1,
-                                                  float c2, const QF<Q> base,
-                                                  unsigned bad) {
+                                                  float c2,
+                                                  const QF<Q> base) {
   constexpr int NW = kPackWords<Q>;
-  Resum<Q> o;
-#pragma unroll
-  for (int q = 0; q < Q; q++) o.z.v[q] = o.ed.v[q] = o.em.v[q] = 0.0f;
-  store_root<Q>(sx, lane);
+  static_assert(NW == 1, "wide rows take one or two cells per lane");
+  const float2 c1p = dup2(c1), c2p = dup2(c2), bias = dup2(8388608.0f);
+  const float2 b = make_float2(base.v[0], base.v[Q - 1]);
+  float2 z = make_float2(0.0f, 0.0f), ed = z, em = z;
+  auto add = [&](uint32_t k) {
+    const float2 fd = fsub2(make_float2(pack_d_biased(k, 0),
+                                        pack_d_biased(k, 1)), bias);
+    const float2 fm = fsub2(make_float2(pack_m_biased(k, 0),
+                                        pack_m_biased(k, 1)), bias);
+    const float2 t = ffma2(fd, c1p, ffma2(fm, c2p, b));
+    const float2 e = make_float2(ex2_approx(t.x), ex2_approx(t.y));
+    z = fadd2(z, e);
+    ed = ffma2(e, fd, ed);
+    em = ffma2(e, fm, em);
+  };
+  store_root(sx, lane);
+  add(0u);
+  int i = 1;
+  if (i + 1 < n) {
+    uint2 o = ring_pair(sx, 1);
 #pragma unroll 1
-  for (int i2 = 0; i2 < n; i2++) {
-    uint32_t k[NW];
-    if (i2 == 0) {
-#pragma unroll
-      for (int w = 0; w < NW; w++) k[w] = 0u;
-    } else {
-      int j;
-      inherit_one_ring<Q>(sx, i2, lane, k, j);
-    }
-#pragma unroll
-    for (int q = 0; q < Q; q++) {
-      if (!((bad >> q) & 1u)) continue;
-      const float fd = pack_d_biased(k[q >> 1], q) - 8388608.0f;
-      const float fm = pack_m_biased(k[q >> 1], q) - 8388608.0f;
-      const float e = ex2_approx(fmaf(fd, c1, fmaf(fm, c2, base.v[q])));
-      o.z.v[q] += e;
-      o.ed.v[q] = fmaf(e, fd, o.ed.v[q]);
-      o.em.v[q] = fmaf(e, fm, o.em.v[q]);
+    for (; i + 1 < n; i += 2) {
+      const uint2 next = i + 2 < n ? ring_pair(sx, i + 2) : o;
+      uint32_t k0[NW], k1[NW];
+      inherit_pair_ring<Q>(sx, o, i, lane, k0, k1);
+      add(k0[0]);
+      add(k1[0]);
+      o = next;
     }
   }
-  return o;
+  if (i < n) {
+    uint32_t k[NW];
+    inherit_last_ring<Q>(sx, (uint32_t)sx.hist[i - 1], lane, k);
+    add(k[0]);
+  }
+  Resum<Q> out;
+  out.z.v[0] = z.x;
+  out.ed.v[0] = ed.x;
+  out.em.v[0] = em.x;
+  if constexpr (Q > 1) {
+    out.z.v[1] = z.y;
+    out.ed.v[1] = ed.y;
+    out.em.v[1] = em.y;
+  }
+  return out;
 }
 
 // Lane sums of k and m at the chosen nodes of cells it loads itself.
@@ -1408,7 +1492,7 @@ __device__ __forceinline__ void sum_cells(const uint32_t *rows, int n,
     base2[q] = dup2(base[q]);
   }
   // the root (ord[0]) has no counted bits: t = base
-  if constexpr (RING) store_root<Q>(sx, lane);
+  if constexpr (RING) store_root(sx, lane);
 #pragma unroll
   for (int q = 0; q < Q; q++) {
     mx[q] = base[q];
@@ -1418,30 +1502,10 @@ __device__ __forceinline__ void sum_cells(const uint32_t *rows, int n,
   // the other nodes two at a time, in the two halves of paired registers
   int i = 1;
   if constexpr (RING) {
-    // counts one pair ahead of the float work, which hides the table's
-    // load latency behind the previous pair's arithmetic; two pairs per
-    // iteration, alternating between two register sets
-    if (i + 1 < n) {
-      uint32_t kA0[NW], kA1[NW], kB0[NW], kB1[NW];
-      int jA0, jA1, jB0, jB1;  // node numbers (the max score uses them)
-      inherit_pair_ring<Q>(sx, i, lane, kA0, kA1, jA0, jA1);
-#pragma unroll 1
-      for (; i + 5 < n; i += 4) {
-        inherit_pair_ring<Q>(sx, i + 2, lane, kB0, kB1, jB0, jB1);
-        sum_counts2<Q, NW>(kA0, kA1, c1p, c2p, base2, mx, z2, ed2, em2);
-        inherit_pair_ring<Q>(sx, i + 4, lane, kA0, kA1, jA0, jA1);
-        sum_counts2<Q, NW>(kB0, kB1, c1p, c2p, base2, mx, z2, ed2, em2);
-      }
-      if (i + 3 < n) {
-        inherit_pair_ring<Q>(sx, i + 2, lane, kB0, kB1, jB0, jB1);
-        sum_counts2<Q, NW>(kA0, kA1, c1p, c2p, base2, mx, z2, ed2, em2);
-        sum_counts2<Q, NW>(kB0, kB1, c1p, c2p, base2, mx, z2, ed2, em2);
-        i += 4;
-      } else {
-        sum_counts2<Q, NW>(kA0, kA1, c1p, c2p, base2, mx, z2, ed2, em2);
-        i += 2;
-      }
-    }
+    walk_ring<Q>(sx, n, lane, i, [&](const uint32_t(&k0)[NW], uint32_t,
+                                     const uint32_t(&k1)[NW], uint32_t) {
+      sum_counts2<Q, NW>(k0, k1, c1p, c2p, base2, mx, z2, ed2, em2);
+    });
   } else {
     // the order entries one pair ahead: the rows' addresses are known when
     // an iteration starts
@@ -1477,8 +1541,7 @@ __device__ __forceinline__ void sum_cells(const uint32_t *rows, int n,
     float fd[Q], fm[Q];
     if constexpr (RING) {
       uint32_t k[NW];
-      int j;
-      inherit_one_ring<Q>(sx, i, lane, k, j);
+      inherit_last_ring<Q>(sx, (uint32_t)sx.hist[i - 1], lane, k);
 #pragma unroll
       for (int q = 0; q < Q; q++) {
         fd[q] = pack_d_biased(k[q >> 1], q) - 8388608.0f;
@@ -1533,7 +1596,7 @@ __device__ __forceinline__ void sum_cells(const uint32_t *rows, int n,
     // more)
     Resum<Q> o;
     if constexpr (RING)
-      o = resum_cells_ring<Q>(n, sx, lane, c1, c2, b2, badm);
+      o = resum_cells_ring<Q>(n, sx, lane, c1, c2, b2);
     else
       o = resum_cells<W32, Q>(rows, n, cb, sx, lane, c1, c2, b2, badm);
 #pragma unroll
@@ -1682,7 +1745,7 @@ __device__ __forceinline__ void max_cells_ring(int n, const Cells<W32, Q> &cb,
   float2 pdb[Q], pmb[Q];
   {
     const int root = (int)(sx.ord[0] & 0xFF);
-    store_root<Q>(sx, lane);
+    store_root(sx, lane);
 #pragma unroll
     for (int q = 0; q < Q; q++) {
       best[q] = pair_score(0, 0, cb.pdb[q], cb.pmb[q], L.l00, L.l01, L.l10,
@@ -1693,31 +1756,16 @@ __device__ __forceinline__ void max_cells_ring(int n, const Cells<W32, Q> &cb,
     }
   }
   int i = 1;
-  if (i + 1 < n) {
-    uint32_t kA0[NW], kA1[NW], kB0[NW], kB1[NW];
-    int jA0, jA1, jB0, jB1;
-    inherit_pair_ring<Q>(sx, i, lane, kA0, kA1, jA0, jA1);
-#pragma unroll 1
-    for (; i + 5 < n; i += 4) {
-      inherit_pair_ring<Q>(sx, i + 2, lane, kB0, kB1, jB0, jB1);
-      max_update2<Q, NW>(kA0, jA0, kA1, jA1, pdb, pmb, L2, best, bj);
-      inherit_pair_ring<Q>(sx, i + 4, lane, kA0, kA1, jA0, jA1);
-      max_update2<Q, NW>(kB0, jB0, kB1, jB1, pdb, pmb, L2, best, bj);
-    }
-    if (i + 3 < n) {
-      inherit_pair_ring<Q>(sx, i + 2, lane, kB0, kB1, jB0, jB1);
-      max_update2<Q, NW>(kA0, jA0, kA1, jA1, pdb, pmb, L2, best, bj);
-      max_update2<Q, NW>(kB0, jB0, kB1, jB1, pdb, pmb, L2, best, bj);
-      i += 4;
-    } else {
-      max_update2<Q, NW>(kA0, jA0, kA1, jA1, pdb, pmb, L2, best, bj);
-      i += 2;
-    }
-  }
+  walk_ring<Q>(sx, n, lane, i, [&](const uint32_t(&k0)[NW], uint32_t o0,
+                                   const uint32_t(&k1)[NW], uint32_t o1) {
+    max_update2<Q, NW>(k0, ring_node(o0), k1, ring_node(o1), pdb, pmb, L2,
+                       best, bj);
+  });
   if (i < n) {
     uint32_t kk[NW];
-    int j;
-    inherit_one_ring<Q>(sx, i, lane, kk, j);
+    const uint32_t o = (uint32_t)sx.hist[i - 1];
+    const int j = ring_node(o);
+    inherit_last_ring<Q>(sx, o, lane, kk);
 #pragma unroll
     for (int q = 0; q < Q; q++) {
       const float s = pair_score_b(pack_d_biased(kk[q >> 1], q),

@@ -1434,7 +1434,7 @@ __global__ void __launch_bounds__(32 * kFewRanges * kFewGroups)
 // order fits the ring and its rates have exact codes (bbs_incr.cuh), each node
 // takes its parent's codes from the ring plus its gene's, some 20
 // instructions a node for 64 cells; otherwise masked popcounts, which run the
-// population-count pipe at its peak (255 x 512, 1500 trees: 735 us, now 230 us,
+// population-count pipe at its peak (255 x 512, 1500 trees: 735 us, now 225 us,
 // bound by the latency of the walk at three blocks per SM).
 template <int W32, bool ATTACH>
 __global__ void __launch_bounds__(128) score_walk_kernel(const ScoreArgs a) {
@@ -1451,6 +1451,10 @@ __global__ void __launch_bounds__(128) score_walk_kernel(const ScoreArgs a) {
   int *hist = reinterpret_cast<int *>(base + w.hist);
   uint32_t *ring = reinterpret_cast<uint32_t *>(base + w.warps + warp * w.per_warp);
   uint32_t *gt = ring + ring_bytes(Q) / 4;
+  SumCtx sx{};
+  sx.hist = hist;
+  sx.ring = ring;
+  sx.gt = gt;
   copy_rows_part<W32>(a.rows + (size_t)tree * n * RS, rows, n, WARPS, warp, lane);
   if (threadIdx.x < 2) sums[threadIdx.x] = 0;
   __syncthreads();
@@ -1515,41 +1519,41 @@ __global__ void __launch_bounds__(128) score_walk_kernel(const ScoreArgs a) {
       // T of both cells in one word; with attachments, keys T << 8 | 255 - j
       uint32_t best = (uint32_t)code.off * 0x10001u;
       uint32_t key0 = 0u, key1 = 0u;
-      auto see = [&](uint32_t t, int j) {
+      auto see = [&](uint32_t t, uint32_t o) {
         if constexpr (ATTACH) {
-          const uint32_t jj = 255u - (uint32_t)j;
+          const uint32_t jj = 255u - (uint32_t)ring_node(o);
           key0 = max(key0, __byte_perm(t, jj, 0x5104u));
           key1 = max(key1, __byte_perm(t, jj, 0x5324u));
         } else {
           best = __vmaxu2(best, t);
         }
       };
-      auto gene = [&](int j) {
-        uint32_t g[1];
-        gene_inc<Q>(gt, j, lane, g);
-        return (g[0] & 0x00010001u) * wd + ((g[0] >> 8) & 0x00010001u) * wm;
+      auto gene = [&](uint32_t g, uint32_t o) {
+        const uint32_t b = ring_gene(g, o);
+        return (b & 0x00010001u) * wd + ((b >> 8) & 0x00010001u) * wm;
       };
-      ring[lane] = best;
-      see(best, n - 1);
+      ring[32 + lane] = best;
+      see(best, (uint32_t)(n - 1) >> 3 << 23 | ((uint32_t)(n - 1) & 7u));
       int i = 1;
 #pragma unroll 2
       for (; i + 1 < n; i += 2) {
-        const uint32_t o0 = ord[i], o1 = ord[i + 1];
-        const int u0 = (int)(o0 & 0xFF), u1 = (int)(o1 & 0xFF);
-        const int p0 = (int)(o0 >> 8), p1 = (int)(o1 >> 8);
-        const uint32_t a0 = ring[(p0 & (kRing - 1)) * 32 + lane];
-        const uint32_t a1 = ring[(p1 & (kRing - 1)) * 32 + lane];
-        const uint32_t t0 = a0 + gene(u0);
-        const uint32_t t1 = (p1 == i ? t0 : a1) + gene(u1);
-        ring[(i & (kRing - 1)) * 32 + lane] = t0;
-        ring[((i + 1) & (kRing - 1)) * 32 + lane] = t1;
-        see(t0, u0);
-        see(t1, u1);
+        const uint2 o = ring_pair(sx, i);
+        uint32_t g0, g1;
+        const uint32_t a0 = ring_counts(sx, o.x, lane, g0);
+        const uint32_t a1 = ring_counts(sx, o.y, lane, g1);
+        const uint32_t t0 = a0 + gene(g0, o.x);
+        const uint32_t t1 = ((o.y & 32u) ? t0 : a1) + gene(g1, o.y);
+        const uint32_t at = (uint32_t)(i + 1) * 32u & (kRingBytes / 4 - 32u);
+        ring[at + lane] = t0;
+        ring[at + 32 + lane] = t1;
+        see(t0, o.x);
+        see(t1, o.y);
       }
       if (i < n) {
-        const uint32_t o = ord[i];
-        see(ring[((int)(o >> 8) & (kRing - 1)) * 32 + lane] + gene((int)(o & 0xFF)),
-            (int)(o & 0xFF));
+        const uint32_t o = (uint32_t)hist[i - 1];
+        uint32_t g;
+        const uint32_t t = ring_counts(sx, o, lane, g);
+        see(t + gene(g, o), o);
       }
 #pragma unroll
       for (int q = 0; q < Q; q++) {

@@ -404,6 +404,29 @@ def test_wide_row_ring_chains_replay_in_fp64(native, orc, G, Cn, launch):
                       final["dm"][ch]) <= 2
 
 
+@pytest.mark.parametrize("score", ["max", "sum"])
+@pytest.mark.parametrize("G", [128, 129, 130, 131, 255])
+def test_ring_walk_remainders_replay_in_fp64(native, orc, G, score):
+    """129 to 132 and 256 nodes: every remainder of the ring's loop of two
+    pairs, and order entries up to the end of their array."""
+    Cn = 70
+    m, _, _ = D.generate_dataset(3100 + G, G, Cn, 5e-4, 0.25, 0.08, 0.01)
+    mut, known = D.matrix_to_bits(m)
+    p = _headline_params(native, "langevin", 0.2, seed=0x51DF + G)
+    p.score_mode = getattr(native, "SCORE_" + score.upper())
+    chains, steps = 2, 60
+    rng = np.random.default_rng(G)
+    starts = np.stack([D.random_parent_vector(rng, G) for _ in range(chains)])
+    with native.Context(mut, known, Cn, G, p) as c:
+        c.init_chains(chains, starts)
+        c.set_launch(2, 1, 2)
+        tr = c.run(steps, trace=True)
+        final = c.chains()
+    for ch in range(chains):
+        assert replay(orc, native, m, p, starts[ch], tr[ch],
+                      final["dm"][ch]) <= 2
+
+
 @pytest.mark.parametrize("wpc", [1, 2])
 def test_headline_batch_equals_replayed_chains(native, orc, wpc):
     """The batched launch of the bench's headline shape -- one 95 x 96
