@@ -180,6 +180,14 @@ int launch_init(const InitArgs &a, int w32, bool sum, void *stream) {
 // 571 -> 184 us, 310 trees 571 -> 169 us.
 inline constexpr int kFewTrees = 304;
 
+// Many trees of rows of up to four words are walked (score_tree_kernel) from
+// this many nodes and cells on; below, finding the parents and the order costs
+// what the walk saves.  Calls for 4096 trees, masked popcounts and walk: 31 x
+// 250 128, 126 us; 31 x 96 118, 117; 63 x 64 136, 137; 63 x 96 150, 136; 95 x
+// 96 205, 184; 95 x 500 390, 268; 127 x 500 566, 351; for 320 trees 31 x 64 46,
+// 53; 63 x 96 56, 54; 127 x 64 60, 69; 127 x 96 74, 70.
+inline constexpr int kWalkNodes = 64, kWalkCells = 65;
+
 template <int W32, bool ATTACH>
 static int launch_score_t(const ScoreArgs &a, cudaStream_t s) {
   constexpr int RS = rs_of_w32(W32), WPB = 4, Q = 2;
@@ -195,10 +203,17 @@ static int launch_score_t(const ScoreArgs &a, cudaStream_t s) {
     if (e != cudaSuccess) return (int)e;
     score_walk_kernel<W32, ATTACH><<<a.n_trees, 128, smem, s>>>(a);
   } else {
+    const int blocks = (a.n_trees + WPB - 1) / WPB;
+    if (a.ds.n_nodes >= kWalkNodes && a.ds.n_cells >= kWalkCells) {
+      const size_t smem = WPB * (size_t)WalkLayout(a.ds.n_nodes, RS).bytes(1);
+      cudaError_t e = prepare_smem(score_tree_kernel<W32, ATTACH>, smem);
+      if (e != cudaSuccess) return (int)e;
+      score_tree_kernel<W32, ATTACH><<<blocks, WPB * 32, smem, s>>>(a);
+      return (int)cudaGetLastError();
+    }
     const size_t smem = WPB * rows;
     cudaError_t e = prepare_smem(score_kernel<W32, Q, ATTACH>, smem);
     if (e != cudaSuccess) return (int)e;
-    const int blocks = (a.n_trees + WPB - 1) / WPB;
     score_kernel<W32, Q, ATTACH><<<blocks, WPB * 32, smem, s>>>(a);
   }
   return (int)cudaGetLastError();

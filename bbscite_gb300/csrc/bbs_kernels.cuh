@@ -1314,9 +1314,9 @@ struct WalkLayout {
   }
 };
 
-// Scores of a batch, one warp per tree: many trees of rows of up to four
-// words, whose trees' parent vectors and orders would cost as much as they
-// save (95 x 96: 65 us for 4096 trees).
+// Scores of many trees by masked popcounts, one warp per tree: rows of up to
+// four words with few nodes or cells, where finding the parents and the order
+// of a walk would cost as much as it saves.
 template <int W32, int Q, bool ATTACH>
 __global__ void __launch_bounds__(128) score_kernel(const ScoreArgs a) {
   extern __shared__ __align__(16) uint32_t smem[];
@@ -1429,6 +1429,117 @@ __global__ void __launch_bounds__(32 * kFewRanges * kFewGroups)
   if (threadIdx.x == 0) write_score(a, tree, sums[0], sums[1], L, bt[3]);
 }
 
+// The parents of the tree with ancestor rows `rows` -- the deepest proper
+// ancestors -- by `threads` threads, a warp's or a block's: whether this
+// thread's nodes agree with them (rows that are not a tree's do not).
+template <int W32>
+__device__ __forceinline__ bool walk_parents(const uint32_t *rows, int n,
+                                             uint8_t *par, int *hist, int id,
+                                             int threads) {
+  constexpr int RS = rs_of_w32(W32);
+  for (int x = id; x < n; x += threads) {
+    uint32_t r[W32];
+    ld_row<W32>(rows + x * RS, r);
+    int pc = 0;
+#pragma unroll
+    for (int k = 0; k < W32; k++) pc += __popc(r[k]);
+    hist[x] = pc;
+  }
+  if (threads > 32) __syncthreads(); else __syncwarp();
+  bool ok = true;
+  for (int x = id; x < n; x += threads) {
+    uint32_t r[W32], q[W32];
+    ld_row<W32>(rows + x * RS, r);
+    // a tree's parent has one ancestor less
+    int p = x == n - 1 ? x : -1;
+#pragma unroll
+    for (int k = 0; k < W32; k++) {
+      uint32_t v = k == (x >> 5) ? r[k] & ~(1u << (x & 31)) : r[k];
+      while (v != 0u && p < 0) {
+        const int y = 32 * k + __ffs(v) - 1;
+        v &= v - 1u;
+        if (y < n && hist[y] == hist[x] - 1) p = y;
+      }
+    }
+    if (p < 0) {
+      ok = false;
+      p = n - 1;
+    }
+    par[x] = (uint8_t)p;
+    ld_row<W32>(rows + p * RS, q);
+#pragma unroll
+    for (int k = 0; k < W32; k++) {
+      const uint32_t own = k == (x >> 5) ? 1u << (x & 31) : 0u;
+      ok = ok && (x == n - 1 ? r[k] == own
+                             : r[k] == (q[k] | own) && (q[k] & own) == 0u);
+    }
+  }
+  return ok;
+}
+
+// The nodes with the highest codes of the lane's two cells, each node's codes
+// its parent's from the ring plus its gene's (sx: the order's entries in hist,
+// ring and gene table): the class sums and, with attachments, the nodes.
+template <bool ATTACH>
+__device__ __forceinline__ void walk_codes(const SumCtx &sx,
+                                           const MaxCode &code, int n,
+                                           int lane, int (&bj)[2], int &k,
+                                           int &m) {
+  const uint32_t wd = (uint32_t)(-code.s * code.P), wm = (uint32_t)(code.s * code.Q);
+  // T of both cells in one word; with attachments, keys T << 8 | 255 - j
+  uint32_t best = (uint32_t)code.off * 0x10001u;
+  uint32_t key0 = 0u, key1 = 0u;
+  auto see = [&](uint32_t t, uint32_t o) {
+    if constexpr (ATTACH) {
+      const uint32_t jj = 255u - (uint32_t)ring_node(o);
+      key0 = max(key0, __byte_perm(t, jj, 0x5104u));
+      key1 = max(key1, __byte_perm(t, jj, 0x5324u));
+    } else {
+      best = __vmaxu2(best, t);
+    }
+  };
+  auto gene = [&](uint32_t g, uint32_t o) {
+    const uint32_t b = ring_gene(g, o);
+    return (b & 0x00010001u) * wd + ((b >> 8) & 0x00010001u) * wm;
+  };
+  sx.ring[32 + lane] = best;
+  see(best, (uint32_t)(n - 1) >> 3 << 23 | ((uint32_t)(n - 1) & 7u));
+  int i = 1;
+#pragma unroll 2
+  for (; i + 1 < n; i += 2) {
+    const uint2 o = ring_pair(sx, i);
+    uint32_t g0, g1;
+    const uint32_t a0 = ring_counts(sx, o.x, lane, g0);
+    const uint32_t a1 = ring_counts(sx, o.y, lane, g1);
+    const uint32_t t0 = a0 + gene(g0, o.x);
+    const uint32_t t1 = ((o.y & 32u) ? t0 : a1) + gene(g1, o.y);
+    const uint32_t at = (uint32_t)(i + 1) * 32u & (kRingBytes / 4 - 32u);
+    sx.ring[at + lane] = t0;
+    sx.ring[at + 32 + lane] = t1;
+    see(t0, o.x);
+    see(t1, o.y);
+  }
+  if (i < n) {
+    const uint32_t o = (uint32_t)sx.hist[i - 1];
+    uint32_t g;
+    const uint32_t t = ring_counts(sx, o, lane, g);
+    see(t + gene(g, o), o);
+  }
+#pragma unroll
+  for (int q = 0; q < 2; q++) {
+    int d, mm;
+    if constexpr (ATTACH) {
+      const uint32_t key = q ? key1 : key0;
+      bj[q] = 255 - (int)(key & 0xFFu);
+      decode<true>(code, key >> 8, d, mm);
+    } else {
+      decode<true>(code, (best >> (16 * q)) & 0xFFFFu, d, mm);
+    }
+    k += d + mm;
+    m += mm;
+  }
+}
+
 // Scores of many trees with rows of five to eight words: one block per tree,
 // four warps over its chunks of 64 cells.  Where the rows are a tree whose
 // order fits the ring and its rates have exact codes (bbs_incr.cuh), each node
@@ -1460,44 +1571,7 @@ __global__ void __launch_bounds__(128) score_walk_kernel(const ScoreArgs a) {
   __syncthreads();
   const float *bt = a.beta_terms + 4 * (size_t)tree;
   const LogTable L{a.ds.l00, a.ds.l10, bt[1], bt[2]};
-  // parents: the deepest proper ancestor, checked against the rows
-  for (int x = threadIdx.x; x < n; x += blockDim.x) {
-    uint32_t r[W32];
-    ld_row<W32>(rows + x * RS, r);
-    int pc = 0;
-#pragma unroll
-    for (int k = 0; k < W32; k++) pc += __popc(r[k]);
-    hist[x] = pc;
-  }
-  __syncthreads();
-  bool ok = true;
-  for (int x = threadIdx.x; x < n; x += blockDim.x) {
-    uint32_t r[W32], q[W32];
-    ld_row<W32>(rows + x * RS, r);
-    // a tree's parent has one ancestor less
-    int p = x == n - 1 ? x : -1;
-#pragma unroll
-    for (int k = 0; k < W32; k++) {
-      uint32_t v = k == (x >> 5) ? r[k] & ~(1u << (x & 31)) : r[k];
-      while (v != 0u && p < 0) {
-        const int y = 32 * k + __ffs(v) - 1;
-        v &= v - 1u;
-        if (y < n && hist[y] == hist[x] - 1) p = y;
-      }
-    }
-    if (p < 0) {
-      ok = false;
-      p = n - 1;
-    }
-    par[x] = (uint8_t)p;
-    ld_row<W32>(rows + p * RS, q);
-#pragma unroll
-    for (int k = 0; k < W32; k++) {
-      const uint32_t own = k == (x >> 5) ? 1u << (x & 31) : 0u;
-      ok = ok && (x == n - 1 ? r[k] == own
-                             : r[k] == (q[k] | own) && (q[k] & own) == 0u);
-    }
-  }
+  bool ok = walk_parents<W32>(rows, n, par, hist, threadIdx.x, blockDim.x);
   ok = __syncthreads_and(ok);
   const MaxCode code =
       make_code(L.l00, L.l01, L.l10, L.l11, a.ds.max_d, a.ds.max_m, lane);
@@ -1508,7 +1582,6 @@ __global__ void __launch_bounds__(128) score_walk_kernel(const ScoreArgs a) {
   }
   __syncthreads();
   ok = ok && fits != 0;
-  const uint32_t wd = (uint32_t)(-code.s * code.P), wm = (uint32_t)(code.s * code.Q);
   int k = 0, m = 0;
   for (int c0 = 64 * warp; c0 < a.ds.n_cells; c0 += 64 * WARPS) {
     Cells<W32, Q> cb;
@@ -1516,58 +1589,7 @@ __global__ void __launch_bounds__(128) score_walk_kernel(const ScoreArgs a) {
     int bj[Q];
     if (ok) {
       build_gene_table<W32, Q>(cb, gt, n, lane);
-      // T of both cells in one word; with attachments, keys T << 8 | 255 - j
-      uint32_t best = (uint32_t)code.off * 0x10001u;
-      uint32_t key0 = 0u, key1 = 0u;
-      auto see = [&](uint32_t t, uint32_t o) {
-        if constexpr (ATTACH) {
-          const uint32_t jj = 255u - (uint32_t)ring_node(o);
-          key0 = max(key0, __byte_perm(t, jj, 0x5104u));
-          key1 = max(key1, __byte_perm(t, jj, 0x5324u));
-        } else {
-          best = __vmaxu2(best, t);
-        }
-      };
-      auto gene = [&](uint32_t g, uint32_t o) {
-        const uint32_t b = ring_gene(g, o);
-        return (b & 0x00010001u) * wd + ((b >> 8) & 0x00010001u) * wm;
-      };
-      ring[32 + lane] = best;
-      see(best, (uint32_t)(n - 1) >> 3 << 23 | ((uint32_t)(n - 1) & 7u));
-      int i = 1;
-#pragma unroll 2
-      for (; i + 1 < n; i += 2) {
-        const uint2 o = ring_pair(sx, i);
-        uint32_t g0, g1;
-        const uint32_t a0 = ring_counts(sx, o.x, lane, g0);
-        const uint32_t a1 = ring_counts(sx, o.y, lane, g1);
-        const uint32_t t0 = a0 + gene(g0, o.x);
-        const uint32_t t1 = ((o.y & 32u) ? t0 : a1) + gene(g1, o.y);
-        const uint32_t at = (uint32_t)(i + 1) * 32u & (kRingBytes / 4 - 32u);
-        ring[at + lane] = t0;
-        ring[at + 32 + lane] = t1;
-        see(t0, o.x);
-        see(t1, o.y);
-      }
-      if (i < n) {
-        const uint32_t o = (uint32_t)hist[i - 1];
-        uint32_t g;
-        const uint32_t t = ring_counts(sx, o, lane, g);
-        see(t + gene(g, o), o);
-      }
-#pragma unroll
-      for (int q = 0; q < Q; q++) {
-        int d, mm;
-        if constexpr (ATTACH) {
-          const uint32_t key = q ? key1 : key0;
-          bj[q] = 255 - (int)(key & 0xFFu);
-          decode<true>(code, key >> 8, d, mm);
-        } else {
-          decode<true>(code, (best >> (16 * q)) & 0xFFFFu, d, mm);
-        }
-        k += d + mm;
-        m += mm;
-      }
+      walk_codes<ATTACH>(sx, code, n, lane, bj, k, m);
       __syncwarp();
     } else {
       best_nodes<W32, Q>(rows, n, cb, L.l00, L.l01, L.l10, L.l11,
@@ -1591,6 +1613,64 @@ __global__ void __launch_bounds__(128) score_walk_kernel(const ScoreArgs a) {
   }
   __syncthreads();
   if (threadIdx.x == 0) write_score(a, tree, sums[0], sums[1], L, bt[3]);
+}
+
+// The same for rows of up to four words, one warp per tree (4096 trees at 95 x
+// 96: the call went from 255 to 240 us, at 95 x 500 from 390 to 268 us; the
+// rest is the copy of the trees).
+template <int W32, bool ATTACH>
+__global__ void __launch_bounds__(128) score_tree_kernel(const ScoreArgs a) {
+  extern __shared__ __align__(16) uint32_t smem[];
+  constexpr int RS = rs_of_w32(W32), Q = 2;
+  const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
+  const int tree = blockIdx.x * (blockDim.x >> 5) + wib;
+  if (tree >= a.n_trees) return;  // whole warp
+  const int n = a.ds.n_nodes;
+  const WalkLayout w(n, RS);
+  uint8_t *base = reinterpret_cast<uint8_t *>(smem) + wib * w.bytes(1);
+  uint32_t *rows = reinterpret_cast<uint32_t *>(base);
+  uint8_t *par = base + w.par;
+  uint16_t *ord = reinterpret_cast<uint16_t *>(base + w.ord);
+  SumCtx sx{};
+  sx.hist = reinterpret_cast<int *>(base + w.hist);
+  sx.ring = reinterpret_cast<uint32_t *>(base + w.warps);
+  sx.gt = sx.ring + ring_bytes(Q) / 4;
+  copy_rows<W32>(a.rows + (size_t)tree * n * RS, rows, n, lane);
+  __syncwarp();
+  const float *bt = a.beta_terms + 4 * (size_t)tree;
+  const LogTable L{a.ds.l00, a.ds.l10, bt[1], bt[2]};
+  const MaxCode code =
+      make_code(L.l00, L.l01, L.l10, L.l11, a.ds.max_d, a.ds.max_m, lane);
+  bool ok = code.usable && code.exact;
+  if (ok)
+    ok = __all_sync(BBS_FULL_MASK,
+                    walk_parents<W32>(rows, n, par, sx.hist, lane, 32)) &&
+         ring_order<W32>(rows, n, par, ord, sx.hist, lane);
+  int k = 0, m = 0;
+  for (int c0 = 0; c0 < a.ds.n_cells; c0 += 32 * Q) {
+    Cells<W32, Q> cb;
+    load_cells<W32, Q>(cb, a.ds, c0, 32, lane);
+    int bj[Q];
+    if (ok) {
+      build_gene_table<W32, Q>(cb, sx.gt, n, lane);
+      walk_codes<ATTACH>(sx, code, n, lane, bj, k, m);
+    } else {
+      best_nodes<W32, Q>(rows, n, cb, L.l00, L.l01, L.l10, L.l11,
+                         a.ds.neg_zero, bj);
+      counts_at<W32, Q>(rows, cb, bj, k, m);
+    }
+    if constexpr (ATTACH) {
+#pragma unroll
+      for (int q = 0; q < Q; q++) {
+        const int c = c0 + 32 * q + lane;
+        if (c < a.ds.n_cells)
+          a.attach[(size_t)tree * a.ds.n_cells + c] = (uint32_t)bj[q];
+      }
+    }
+  }
+  k = (int)__reduce_add_sync(BBS_FULL_MASK, (uint32_t)k);
+  m = (int)__reduce_add_sync(BBS_FULL_MASK, (uint32_t)m);
+  if (lane == 0) write_score(a, tree, k, m, L, bt[3]);
 }
 
 template <int W32>

@@ -100,3 +100,12 @@ def test_adjoint_and_posteriors_match_fp64(native, orc, G, Cn, trees):
         assert abs(db[t] - gb) <= 1e-4 * abs(gb) + 1e-3
         assert np.abs(post[t] - po).max() <= 1e-3
         np.testing.assert_allclose(post[t].sum(1), 1.0, rtol=1e-4)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("G,Cn", [(62, 65), (63, 64), (63, 65), (95, 97),
+                                  (127, 66)])
+def test_walked_trees_score_as_few_do(native, orc, G, Cn):
+    """Both sides of the sizes from which rows of up to four words are
+    walked, odd and even ends of the walk's pairs, and the most nodes."""
+    test_many_trees_score_as_few_do(native, orc, G, Cn)
