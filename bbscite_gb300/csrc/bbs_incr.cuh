@@ -457,12 +457,12 @@ __device__ __forceinline__ void class_deltas(const Table<W32, Q> &tab,
   }
 }
 
-// Adds the classes' changes to the table, or takes them back.
+// Adds the classes' changes to the table, or takes them back: the nodes of
+// list_nodes (nc of them, nv of the first class).
 template <int W32, int Q, int NW = kPackWords<Q>>
 __device__ __forceinline__ void apply_classes(const Table<W32, Q> &tab,
-                                              uint8_t *list,
-                                              const Delta &x,
-                                              const NodeSets<W32> &C,
+                                              const uint8_t *list, int nc,
+                                              int nv, const Delta &x,
                                               Packed<NW> dv, Packed<NW> dw,
                                               bool back, int lane) {
   auto swap_entries = [&]() {
@@ -473,8 +473,6 @@ __device__ __forceinline__ void apply_classes(const Table<W32, Q> &tab,
     tab.st((int)x.w, lane, a);
   };
   if (back && x.swap) swap_entries();
-  int nv;
-  const int nc = list_nodes<W32>(C, list, lane, nv);
   if (back) {
 #pragma unroll
     for (int i = 0; i < NW; i++) {
@@ -510,7 +508,9 @@ __device__ __noinline__ void take_back(const Table<W32, Q> tab, uint8_t *list,
                                        const Delta x, const NodeSets<W32> C,
                                        const Packed<NW> dv,
                                        const Packed<NW> dw, int lane) {
-  apply_classes<W32, Q>(tab, list, x, C, dv, dw, true, lane);
+  int nv;
+  const int nc = list_nodes<W32>(C, list, lane, nv);
+  apply_classes<W32, Q>(tab, list, nc, nv, x, dv, dw, true, lane);
 }
 
 // ------------------------------------------------------------------------
@@ -698,7 +698,8 @@ __device__ __noinline__ Resum1 resum_slot_table(const Table<W32, Q> tab,
 // sum_cells with the counts of every node in the table and the tree's
 // canonical order (ord): the same terms in the same pairs and
 // order, so the same sums.  The table's entries are all in place before the
-// loop, so its loads wait for nothing but the order.
+// loop, so its loads wait for nothing but the order.  ord + 1 is 8-byte
+// aligned and followed by three zeros (slot_sum).
 template <int W32, int Q>
 __device__ __forceinline__ void sum_cells_table(
     const Table<W32, Q> &tab, const uint16_t *ord, int n, const float (&pd)[Q], const float (&pm)[Q], const LogTable &L,
@@ -720,52 +721,56 @@ __device__ __forceinline__ void sum_cells_table(
     z2[q] = make_float2(ex2_approx(base[q]), 0.0f);
     ed2[q] = em2[q] = make_float2(0.0f, 0.0f);
   }
-  auto entry = [&](uint32_t o, uint32_t (&k)[NW]) {
-    tab.ld((int)(o & 0xFF), lane, k);
-  };
-  int i = 1;
-  if (i + 1 < n) {
-    // the table's loads one pair ahead of the float work, the order's two
-    uint32_t kA0[NW], kA1[NW], kB0[NW], kB1[NW];
-    const int last = n - 1;
-    entry(ord[i], kA0);
-    entry(ord[i + 1], kA1);
-    uint32_t o0 = ord[min(i + 2, last)], o1 = ord[min(i + 3, last)];
+  // Four nodes an iteration, in the pairs (1, 2), (3, 4), ... of the other
+  // count sources: their entries are loaded an iteration ahead of the float
+  // work and the order, four nodes a load, two ahead.  (96 nodes, one warp
+  // per scheduler, one and three cells per lane: 46 and 85 clocks a pair; one
+  // node a load and one pair ahead 58 and 95.)  Past the order's end stand
+  // zeros, past its last group that group again: loaded, not summed.
+  if (n > 1) {
+    const int last = (n - 2) >> 2;
+    auto order4 = [&](int g) {
+      return *reinterpret_cast<const uint2 *>(ord + 1 + 4 * min(g, last));
+    };
+    auto entries = [&](uint2 o, uint32_t (&k)[4][NW]) {
+      tab.ld((int)__byte_perm(o.x, 0u, 0x4440u), lane, k[0]);
+      tab.ld((int)__byte_perm(o.x, 0u, 0x4442u), lane, k[1]);
+      tab.ld((int)__byte_perm(o.y, 0u, 0x4440u), lane, k[2]);
+      tab.ld((int)__byte_perm(o.y, 0u, 0x4442u), lane, k[3]);
+    };
+    uint32_t k[4][NW];
+    entries(order4(0), k);
+    uint2 o = order4(1);
+    int left = n - 1;  // positions not summed yet
 #pragma unroll 1
-    for (; i + 5 < n; i += 4) {
-      entry(o0, kB0);
-      entry(o1, kB1);
-      o0 = ord[i + 4];
-      o1 = ord[i + 5];
-      sum_counts2<Q, NW>(kA0, kA1, c1p, c2p, base2, mx, z2, ed2, em2);
-      entry(o0, kA0);
-      entry(o1, kA1);
-      o0 = ord[min(i + 6, last)];
-      o1 = ord[min(i + 7, last)];
-      sum_counts2<Q, NW>(kB0, kB1, c1p, c2p, base2, mx, z2, ed2, em2);
-    }
-    sum_counts2<Q, NW>(kA0, kA1, c1p, c2p, base2, mx, z2, ed2, em2);
-    i += 2;
-    if (i + 1 < n) {
-      entry(o0, kB0);
-      entry(o1, kB1);
-      sum_counts2<Q, NW>(kB0, kB1, c1p, c2p, base2, mx, z2, ed2, em2);
-      i += 2;
-    }
-  }
-  if (i < n) {
-    uint32_t k[NW];
-    entry(ord[i], k);
+    for (int g = 2; left >= 4; left -= 4, g++) {
+      uint32_t next[4][NW];
+      entries(o, next);
+      o = order4(g);
+      sum_counts2<Q, NW>(k[0], k[1], c1p, c2p, base2, mx, z2, ed2, em2);
+      sum_counts2<Q, NW>(k[2], k[3], c1p, c2p, base2, mx, z2, ed2, em2);
 #pragma unroll
-    for (int q = 0; q < Q; q++) {
-      const float fd = pack_d_biased(k[q >> 1], q) - 8388608.0f;
-      const float fm = pack_m_biased(k[q >> 1], q) - 8388608.0f;
-      const float t = fmaf(fd, c1, fmaf(fm, c2, base[q]));
-      const float e = ex2_approx(t);
-      mx[q] = fmaxf(mx[q], t);
-      z2[q].x += e;
-      ed2[q].x = fmaf(e, fd, ed2[q].x);
-      em2[q].x = fmaf(e, fm, em2[q].x);
+      for (int b = 0; b < 4; b++)
+#pragma unroll
+        for (int w = 0; w < NW; w++) k[b][w] = next[b][w];
+    }
+    if (left >= 2) {
+      sum_counts2<Q, NW>(k[0], k[1], c1p, c2p, base2, mx, z2, ed2, em2);
+#pragma unroll
+      for (int w = 0; w < NW; w++) k[0][w] = k[2][w];
+    }
+    if (left & 1) {
+#pragma unroll
+      for (int q = 0; q < Q; q++) {
+        const float fd = pack_d_biased(k[0][q >> 1], q) - 8388608.0f;
+        const float fm = pack_m_biased(k[0][q >> 1], q) - 8388608.0f;
+        const float t = fmaf(fd, c1, fmaf(fm, c2, base[q]));
+        const float e = ex2_approx(t);
+        mx[q] = fmaxf(mx[q], t);
+        z2[q].x += e;
+        ed2[q].x = fmaf(e, fd, ed2[q].x);
+        em2[q].x = fmaf(e, fm, em2[q].x);
+      }
     }
   }
   float z[Q], ed[Q], em[Q];

@@ -57,8 +57,10 @@ __host__ __device__ __forceinline__ SlotSum slot_sum(uint8_t *slot, int n,
   o.par0 = p;
   o.par1 = p + n;
   p += align16(2 * n) + wic * sum_warp_bytes(n, w32, q, counts);
-  o.sx.ord = reinterpret_cast<uint16_t *>(p);
-  p += align16(2 * n);
+  // (rows of up to four words: position 1 on 8 bytes, as sum_cells_table reads
+  // it, and three zeros past the end)
+  o.sx.ord = reinterpret_cast<uint16_t *>(p) + (w32 <= 4 ? 3 : 0);
+  p += order_bytes(n, w32);
   o.sx.hist = reinterpret_cast<int *>(p);
   p += align16(4 * 32 * ((n + 31) / 32));
   if (counts && w32 <= 4) o.sx.cnt = reinterpret_cast<uint32_t *>(p);
@@ -551,6 +553,8 @@ __device__ __forceinline__ void run_chain_table(
   // table and, for the sum score, the order and cell sums follow it)
   bool tree_ok = false;
   bool ord_ok = false;  // ss.sx.ord is the current tree's order
+  if constexpr (SUM)
+    if (lane < 3) ss.sx.ord[n + lane] = 0;  // (read in groups of four)
   MaxCode code{};
   CellSums<Q> cs;
   float pd[Q], pm[Q];
@@ -620,6 +624,7 @@ __device__ __forceinline__ void run_chain_table(
     bbs_move_params mp{};
     bool related = false;
     bool classes = false;    // the proposal is described by classes
+    int nc = 0, nv = 0;      // their nodes (list), those of the first class
     bool built = false;      // prop holds the proposal's rows
     bool applied = false;    // the table holds the proposal's counts
     bool from_rows = false;  // scored from its rows
@@ -679,8 +684,7 @@ __device__ __forceinline__ void run_chain_table(
     }
     if (classes) {
       delta = move_classes<W32>(mp, related, D, C);
-      int nv;
-      const int nc = list_nodes<W32>(C, list, lane, nv);
+      nc = list_nodes<W32>(C, list, lane, nv);
       if constexpr (!SUM) {
         int sk = 0, sm = 0;
         // CH chunks of cells from chunk c on
@@ -765,7 +769,6 @@ __device__ __forceinline__ void run_chain_table(
             continue;  // rejected: the chain's state stays as it is
           }
         }
-        __syncwarp();  // the list is written again
         from_table = true;
         order = prop;
       }
@@ -786,7 +789,7 @@ __device__ __forceinline__ void run_chain_table(
     }
     if constexpr (SUM) {
       if (classes) {
-        apply_classes<W32, Q>(tab, list, delta, C, dv, dw, false, lane);
+        apply_classes<W32, Q>(tab, list, nc, nv, delta, dv, dw, false, lane);
         applied = true;
       }
     }
@@ -923,7 +926,8 @@ __device__ __forceinline__ void run_chain_table(
             for (int c = 0; c < chunks; c++) {
               const Table<W32, Q> tc = tab.chunk(c, n);
               if (chunks > 1) class_deltas<W32, Q>(tc, delta, lane, dv, dw);
-              apply_classes<W32, Q>(tc, list, delta, C, dv, dw, false, lane);
+              apply_classes<W32, Q>(tc, list, nc, nv, delta, dv, dw, false,
+                                    lane);
             }
           } else {
             cs = pcs;

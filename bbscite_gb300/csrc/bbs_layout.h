@@ -27,6 +27,12 @@ __host__ __device__ inline int gene_table_bytes(int n, int q) {
   return 4 * ((q + 1) / 2) * ((n + 7) / 8) * 32;
 }
 
+// The canonical node order; rows of up to four words with three entries
+// before and three after it (slot_sum).
+__host__ __device__ inline int order_bytes(int n, int w32) {
+  return align16(w32 <= 4 ? 2 * n + 12 : 2 * n);
+}
+
 // Per warp of a chain with the node-order scratch (every sum-score chain:
 // its order is canonical; every chain that inherits counts): the canonical
 // node order, its depth histogram and, with `counts`, the packed counts of
@@ -34,7 +40,7 @@ __host__ __device__ inline int gene_table_bytes(int n, int q) {
 // and gene table (wider rows).
 __host__ __device__ inline int sum_warp_bytes(int n, int w32, int q,
                                               bool counts) {
-  int b = align16(2 * n) + align16(4 * 32 * ((n + 31) / 32));
+  int b = order_bytes(n, w32) + align16(4 * 32 * ((n + 31) / 32));
   if (counts)
     b += w32 <= 4 ? align16(pack_table_bytes(n, q))
                   : align16(ring_bytes(q)) + align16(gene_table_bytes(n, q));
