@@ -872,19 +872,21 @@ struct SumCtx {
   uint32_t *gt;         // [ceil(n / 8)][32][NW]
 };
 
-// ord and hist of the tree with ancestor rows `rows`; the parent of each
-// node from `par` (0 where par is null).  Depth = ancestors - 1 = the
-// popcount of the node's row less one (a row holds the node and the root).
+// The canonical positions of the lane's nodes: by depth, then by node.  Depth =
+// ancestors - 1 = the popcount of the node's row less one (a row holds the node
+// and the root).  A group's nodes of one depth are counted by the first of
+// them, whose add returns how many lie in the groups before; no lane waits for
+// another group.  (Every node adding by itself, then a read and a write of the
+// counts group after group, took some 2000 clocks at 96 nodes.)
 template <int W32>
-__device__ __forceinline__ void canonical_order(const uint32_t *rows, int n,
-                                                const uint8_t *par,
-                                                uint16_t *ord, int *hist,
-                                                int lane) {
+__device__ __forceinline__ void depth_order(const uint32_t *rows, int n,
+                                            int *hist, int lane,
+                                            int (&at)[W32]) {
   constexpr int RS = rs_of_w32(W32);
   const int B = (n + 31) >> 5;  // node groups; bins per lane in the scan
   for (int i = lane; i < 32 * B; i += 32) hist[i] = 0;
-  __syncwarp();
-  int dep[W32];
+  int dep[W32], old[W32];
+  unsigned same[W32];
 #pragma unroll
   for (int g = 0; g < W32; g++) {
     const int x = 32 * g + lane;
@@ -895,11 +897,19 @@ __device__ __forceinline__ void canonical_order(const uint32_t *rows, int n,
       int pc = 0;
 #pragma unroll
       for (int k = 0; k < W32; k++) pc += __popc(a[k]);
-      dep[g] = pc - 1;
-      atomicAdd(&hist[pc - 1], 1);
+      dep[g] = max(pc - 1, 0);
     }
+    same[g] = __match_any_sync(BBS_FULL_MASK, dep[g]);
   }
   __syncwarp();
+  const unsigned below = (1u << lane) - 1u;
+#pragma unroll
+  for (int g = 0; g < W32; g++) {
+    old[g] = 0;
+    if (dep[g] >= 0 && (same[g] & below) == 0)
+      old[g] = atomicAdd(&hist[dep[g]], __popc(same[g]));
+    __syncwarp();
+  }
   // exclusive scan of the bins, lane l owning bins l*B .. l*B + B - 1
   int loc[W32], s = 0;
 #pragma unroll
@@ -922,20 +932,29 @@ __device__ __forceinline__ void canonical_order(const uint32_t *rows, int n,
       run += loc[k];
     }
   __syncwarp();
-  const unsigned below = (1u << lane) - 1u;
+#pragma unroll
+  for (int g = 0; g < W32; g++)
+    at[g] = __shfl_sync(BBS_FULL_MASK, old[g], __ffs(same[g]) - 1) +
+            __popc(same[g] & below) + (dep[g] >= 0 ? hist[dep[g]] : 0);
+  __syncwarp();
+}
+
+// ord of the tree with ancestor rows `rows`; the parent of each node from
+// `par` (0 where par is null).
+template <int W32>
+__device__ __forceinline__ void canonical_order(const uint32_t *rows, int n,
+                                                const uint8_t *par,
+                                                uint16_t *ord, int *hist,
+                                                int lane) {
+  int at[W32];
+  depth_order<W32>(rows, n, hist, lane, at);
 #pragma unroll
   for (int g = 0; g < W32; g++) {
     const int x = 32 * g + lane;
-    const bool valid = x < n;
-    const unsigned same = __match_any_sync(BBS_FULL_MASK, valid ? dep[g] : -1);
-    if (valid) {
-      const int pos = hist[dep[g]] + __popc(same & below);
-      ord[pos] = (uint16_t)(x | ((par != nullptr ? (int)par[x] : 0) << 8));
-    }
-    __syncwarp();
-    if (valid && (same & below) == 0) hist[dep[g]] += __popc(same);
-    __syncwarp();
+    if (x < n)
+      ord[at[g]] = (uint16_t)(x | ((par != nullptr ? (int)par[x] : 0) << 8));
   }
+  __syncwarp();
 }
 
 // The canonical order for counts inherited through a ring (rows of five to
@@ -959,59 +978,8 @@ template <int W32>
 __device__ __forceinline__ bool ring_order(const uint32_t *rows, int n,
                                            const uint8_t *par, uint16_t *ord,
                                            int *hist, int lane) {
-  constexpr int RS = rs_of_w32(W32);
-  const int B = (n + 31) >> 5;
-  for (int i = lane; i < 32 * B; i += 32) hist[i] = 0;
-  __syncwarp();
-  int dep[W32], at[W32];
-#pragma unroll
-  for (int g = 0; g < W32; g++) {
-    const int x = 32 * g + lane;
-    dep[g] = -1;
-    at[g] = 0;
-    if (x < n) {
-      uint32_t a[W32];
-      ld_row<W32>(rows + x * RS, a);
-      int pc = 0;
-#pragma unroll
-      for (int k = 0; k < W32; k++) pc += __popc(a[k]);
-      dep[g] = pc - 1;
-      atomicAdd(&hist[pc - 1], 1);
-    }
-  }
-  __syncwarp();
-  int loc[W32], s = 0;
-#pragma unroll
-  for (int k = 0; k < W32; k++) {
-    loc[k] = k < B ? hist[lane * B + k] : 0;
-    s += loc[k];
-  }
-  int incl = s;
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const int v = __shfl_up_sync(BBS_FULL_MASK, incl, o);
-    if (lane >= o) incl += v;
-  }
-  int run = incl - s;
-  __syncwarp();
-#pragma unroll
-  for (int k = 0; k < W32; k++)
-    if (k < B) {
-      hist[lane * B + k] = run;
-      run += loc[k];
-    }
-  __syncwarp();
-  const unsigned below = (1u << lane) - 1u;
-#pragma unroll
-  for (int g = 0; g < W32; g++) {
-    const int x = 32 * g + lane;
-    const bool valid = x < n;
-    const unsigned same = __match_any_sync(BBS_FULL_MASK, valid ? dep[g] : -1);
-    if (valid) at[g] = hist[dep[g]] + __popc(same & below);
-    __syncwarp();
-    if (valid && (same & below) == 0) hist[dep[g]] += __popc(same);
-    __syncwarp();
-  }
+  int at[W32];
+  depth_order<W32>(rows, n, hist, lane, at);
   // node -> position, then the entries
 #pragma unroll
   for (int g = 0; g < W32; g++) {

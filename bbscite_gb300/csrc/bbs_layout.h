@@ -151,11 +151,19 @@ __host__ __device__ inline int wide_slot_bytes(int n, int rs, int wpc, int w32,
          wpc * wide_part_bytes(q, chunks, ns);
 }
 
+inline constexpr int kFewCells = 12;
+
 // The plan of a launch of `slots` chain slots per block, its largest dataset
 // of n nodes and n_cells cells.  Where the tables do not fit a block, or a
 // sum-score chain's cells of rows of up to four words do not fit one chunk,
 // the cells are streamed as before (such launches are bound by their masked
 // popcounts).
+// Nor does the sum score of at most 32 nodes and kFewCells cells take one:
+// nearly every proposal is accepted, so the bound rejects little, and the sum
+// over so few nodes costs less than following the table (1000 steps of 750
+// Langevin chains, every node and table: 8 x 4 2.28, 3.54 ms; 8 x 9 2.27, 3.07;
+// 20 x 9 2.83, 3.48; 8 x 16 2.28, 2.57; at fixed rates 8 x 9 2.12, 1.80; 20 x 9
+// 2.70, 2.28; 8 x 16 2.12, 1.54.  From 33 nodes on the table is no slower).
 // Rows of five to eight words take a table when `wide`: max-score chains at
 // fixed rates that have codes (after a change of rates the table would have to
 // be made again).  It is in shared memory where that leaves an SM four warps;
@@ -189,7 +197,7 @@ inline TablePlan plan_tables(int n, int w32, int n_cells, int q, int wpc,
   }
   const TablePlan p{0, false, slots * slot_bytes(n, rs, wpc, sum, w32, q, false),
                     n, 0};
-  if (sum && chunks > 1) return p;
+  if (sum && (chunks > 1 || (w32 == 1 && n_cells <= kFewCells))) return p;
   const bool inc = wpc == 1 && one_dataset && chunks == 1;
   const int smem =
       inc ? chain_launch_smem(n, n_cells, q, wpc, slots, sum)

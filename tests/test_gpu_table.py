@@ -89,6 +89,36 @@ def test_untraced_chains_equal_traced_ones(native, score, move, G, Cn, q):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("move", ["beta_walk", "langevin"])
+@pytest.mark.parametrize("G,Cn", [(8, 12), (8, 13), (31, 12), (31, 13),
+                                  (32, 12), (62, 9), (127, 4)])
+def test_few_cells_give_the_same_in_company(native, move, G, Cn):
+    """Sum-score chains of few cells alone, on either side of the sizes that
+    take a table, and in a launch with a larger dataset, which decides for
+    both; n - 1 nodes with every remainder of the sum's groups of four."""
+    sets, params = [], []
+    for k, (g, c) in enumerate([(G, Cn), (G, 40)]):
+        mut, known = _setup(g, c, 5 + k)
+        sets.append((mut, known, c, g))
+        params.append(native.default_params(
+            alpha_mean=1e-2, beta_mean=0.3, seed=31 + k, prob_beta_change=0.15,
+            score_mode=native.SCORE_SUM,
+            error_move=getattr(native, "ERROR_" + move.upper())))
+    got = []
+    for who in ([0], [0, 1]):
+        with native.Batch([sets[k] for k in who],
+                          [params[k] for k in who]) as b:
+            b.init_chains(4)
+            b.set_launch(2, 4, 1)
+            for steps in (1, 50, 300):
+                b.run(steps)
+            got.append(b.best(0))
+    assert got[0]["score"] == got[1]["score"]
+    assert got[0]["alpha"] == got[1]["alpha"]
+    assert (got[0]["dm"] == got[1]["dm"]).all()
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("shape", [(1, 4, 0, 1), (4, 2, 1, 1), (2, 4, 0, 4)])
 def test_mixed_batches_equal_their_datasets_alone(native, shape):
     """Datasets of one launch with one to eight chunks of cells."""
