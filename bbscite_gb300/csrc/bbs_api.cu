@@ -954,8 +954,6 @@ int bbs_get_sizes(const bbs_ctx *c, uint32_t *n_cells, uint32_t *n_genes,
 
 namespace {
 
-// One-warp chains per block (1-8; they share the block's increment table)
-// that keep the most warps resident on an SM; ties keep the smaller block.
 TablePlan chain_plan(const bbs_ctx *c, int q, int wpc, int cpb) {
   return plan_tables((int)c->n_nodes, w32_of_nodes((int)c->n_nodes),
                      (int)c->n_cells, q, wpc, cpb, c->md.score_mode != 0, true,
@@ -963,12 +961,28 @@ TablePlan chain_plan(const bbs_ctx *c, int q, int wpc, int cpb) {
                      c->smem_sm);
 }
 
+// Shared memory a shape is accepted by: the plan's, and the slots' with the
+// counts of every node where a pass takes all cells, which blocks of as many
+// chains have to hold whether or not they end up with a table.
+int shape_smem(const bbs_ctx *c, int q, int wpc, int cpb) {
+  return std::max(chain_plan(c, q, wpc, cpb).smem,
+                  chain_launch_smem((int)c->n_nodes, (int)c->n_cells, q, wpc,
+                                    cpb, c->md.score_mode != 0));
+}
+
+// Resident warps per SM of blocks of cpb chains of wpc warps.
+int resident_warps(const bbs_ctx *c, int q, int wpc, int cpb) {
+  return chain_resident_warps(shape_smem(c, q, wpc, cpb), wpc * cpb,
+                              chain_regs(q, chain_plan(c, q, wpc, cpb).chunks > 0),
+                              c->smem_sm, c->smem_block, c->smem_reserved);
+}
+
+// One-warp chains per block (1-8; they share the block's increment table)
+// that keep the most warps resident on an SM; ties keep the smaller block.
 int pick_chains_per_block(const bbs_ctx *c, int q) {
   int best = 1, best_warps = 0;
   for (int cpb = 1; cpb * 32 <= chain_max_threads(q); cpb++) {
-    const int smem = chain_plan(c, q, 1, cpb).smem;
-    const int w = chain_resident_warps(smem, cpb, q, c->smem_sm, c->smem_block,
-                                       c->smem_reserved);
+    const int w = resident_warps(c, q, 1, cpb);
     if (w > best_warps) {
       best_warps = w;
       best = cpb;
@@ -977,12 +991,11 @@ int pick_chains_per_block(const bbs_ctx *c, int q) {
   return best;
 }
 
-// Launch shape without timing: split the cells over up to four warps per
-// chain when there are too few chains to give every scheduler ~3 warps,
-// preferring shapes that leave no cell slots empty.
-void default_launch(bbs_ctx *c) {
-  const int groups = (int)((c->n_cells + 31) / 32);
-  const int qmax = w32_of_nodes((int)c->n_nodes) > 4 ? 2 : kMaxQ;
+// Launch shape without timing, rows of five to eight words: split the cells
+// over up to four warps per chain when there are too few chains to give every
+// scheduler ~3 warps, preferring shapes that leave no cell slots empty.
+void default_wide_launch(bbs_ctx *c) {
+  const int groups = (int)((c->n_cells + 31) / 32), qmax = 2;
   double best = 1e30;
   for (int wpc = 1; wpc <= 4; wpc++) {
     const int q = std::max(1, (groups + wpc - 1) / wpc);
@@ -1002,6 +1015,70 @@ void default_launch(bbs_ctx *c) {
     c->q = qmax;
   }
   c->cpb = c->wpc == 1 ? pick_chains_per_block(c, c->q) : 1;
+}
+
+// Launch shape without timing, rows of up to four words.  With a table a step
+// is bound by its own latency, nearly the same for one cell per lane as for
+// four, until an SM holds more than a warp per scheduler; so the fewest rounds
+// of resident chains win, then the shorter step.  An estimate of
+//   rounds   of resident chains, between whole rounds and their fraction,
+//   step     the latency of one: more for the sum score's exact sums with three
+//            or four cells per lane, for further chunks of cells, and without a
+//            table (every node by popcounts),
+//   crowd    what each warp per scheduler beyond the first adds.
+// Fitted to 8 to 3000 chains of 20 to 127 genes and 24 to 400 cells.  Shapes as
+// (cells per lane, warps, chains per block), by the rule of wide rows, used for
+// all before, and by this one, ms: max score, 400 steps, 8 chains at 63 x 64
+// (1, 2, 1) 0.73, (2, 1, 1) 0.67; 750 at 95 x 96 (1, 3, 1) 2.29, (3, 1, 5) 1.14;
+// sum score, 400 steps, 750 at 95 x 128 (1, 4, 1) 3.62, (2, 2, 1) 2.43; 200
+// steps, 3000 at 95 x 128 (4, 1, 8), which has no room for tables, 14.7, (2, 2,
+// 1) 3.7.
+void default_launch(bbs_ctx *c) {
+  if (w32_of_nodes((int)c->n_nodes) > 4) {
+    default_wide_launch(c);
+    return;
+  }
+  const bool sum = c->md.score_mode != 0;
+  // (error moves of the max score are scored from the rows)
+  const bool errors = !sum && c->md.mp.cum_beta > 0.0f;
+  const int groups = (int)((c->n_cells + 31) / 32);
+  const double n = c->n_nodes, chains = c->n_chains;
+  double best = 1e30;
+  c->q = c->wpc = c->cpb = 1;
+  for (int wpc = 1; wpc <= 4; wpc++)
+    for (int q = 1; q <= kMaxQ; q++) {
+      // (no warp and no cell slot that would stay empty)
+      if ((q - 1) * wpc >= groups || (wpc - 1) * q >= groups) continue;
+      const int passes = (groups + q * wpc - 1) / (q * wpc);
+      for (int cpb = 1; cpb == 1 || (wpc == 1 && 32 * cpb <= chain_max_threads(q));
+           cpb++) {
+        const int warps = resident_warps(c, q, wpc, cpb);
+        if (warps == 0) continue;
+        const int per_block = wpc * cpb;
+        const double blocks = std::ceil(chains / cpb);
+        const double full = blocks / ((double)(warps / per_block) * c->n_sms);
+        const double rounds =
+            std::max(1.0, 0.75 * std::ceil(full) + 0.25 * full);
+        const double held = std::min(
+            (double)warps, std::ceil(blocks / c->n_sms) * per_block);
+        const double shared = 0.5 * (std::ceil(held / 4.0) + held / 4.0);
+        const double crowd =
+            1.0 + (sum ? 0.25 * q : 0.45) * std::max(0.0, shared - 1.0);
+        double step = q == 1 ? 1.04 : q == 2 ? 1.0 : q == 3 ? 1.04 : 1.07;
+        if (sum && q > 2) step = 1.0 + n / 96.0 * (q == 3 ? 0.4 : 0.75);
+        if (errors) step *= 1.0 + n / 96.0 * 0.25 * std::max(0, q * passes - 2);
+        step *= chain_plan(c, q, wpc, cpb).chunks > 0
+                    ? 1.0 + 0.25 * std::min(1.0, n / 64.0) * (passes - 1)
+                    : (1.0 + n / 24.0) * passes;
+        const double est = rounds * step * crowd;
+        if (est < best) {
+          best = est;
+          c->q = q;
+          c->wpc = wpc;
+          c->cpb = cpb;
+        }
+      }
+    }
 }
 
 size_t tree_words(const bbs_ctx *c, uint32_t n_trees) {
@@ -1087,7 +1164,7 @@ int start_run(bbs_ctx *c, uint32_t n_steps, const bbs_raw_move *d_moves,
               bbs_step_trace *d_trace) {
   {
     const int cpb = c->wpc > 1 ? 1 : c->cpb;
-    const int smem = chain_plan(c, c->q, c->wpc, cpb).smem;
+    const int smem = shape_smem(c, c->q, c->wpc, cpb);
     if (32 * c->wpc * cpb > chain_max_threads(c->q) || smem > c->smem_block)
       return fail(BBS_ERR_SIZE,
                   "launch shape (%d cells per lane, %d warps per chain, %d "
@@ -1282,7 +1359,7 @@ int bbs_autotune(bbs_ctx *c, uint32_t probe_steps, float *best_ms) {
         for (int cpb : {1, 2, 4, 7, 8}) {
           if (wpc > 1 && cpb > 1) continue;
           if (32 * wpc * cpb > chain_max_threads(q)) continue;
-          if (chain_plan(c, q, wpc, cpb).smem > c->smem_block)
+          if (shape_smem(c, q, wpc, cpb) > c->smem_block)
             continue;  // too large a block
           c->q = q;
           c->wpc = wpc;
@@ -2163,8 +2240,17 @@ bool batch_reserve_tables(bbs_batch *b) {
 // bounds by group_wpb).  Checked before a run launches anything.
 bool batch_shape_fits(const bbs_batch *b) {
   for (const auto &grp : b->groups) {
-    const int smem = group_plan(b, grp).smem;
-    if (smem > b->smem_block) return false;
+    // (the plan's, and the slots' with counts as for one context's chains)
+    const int q = group_q(b, grp), slots = group_wpb(b, grp) / b->wpc;
+    const bool counts =
+        grp.w32 > 4 ||
+        (grp.only_ds >= 0 &&
+         inherits_counts(grp.w32, grp.max_cells, 32 * b->wpc * q));
+    const int smem =
+        slots * slot_bytes(grp.max_nodes, rs_of_w32(grp.w32), b->wpc,
+                           b->sum || counts, grp.w32, q, counts) +
+        bbs::table_bytes(grp.max_nodes, grp.w32, q, b->wpc, counts);
+    if (std::max(smem, group_plan(b, grp).smem) > b->smem_block) return false;
   }
   return true;
 }

@@ -97,7 +97,8 @@ __host__ __device__ constexpr int chain_blocks(int w32, int q, bool tab) {
   if (tab) return w32 > 4 ? 1 : (q == 1 ? 3 : (q == 2 ? 2 : 1));
   return q == 1 ? 4 : (q == 2 ? 3 : 1);
 }
-__host__ __device__ constexpr int chain_regs(int q) {
+__host__ __device__ constexpr int chain_regs(int q, bool tab) {
+  if (tab) return q == 1 ? 168 : 255;
   return q == 1 ? 128 : (q == 2 ? 168 : 255);
 }
 
@@ -209,12 +210,12 @@ inline TablePlan plan_tables(int n, int w32, int n_cells, int q, int wpc,
 // Resident warps per SM of such a launch (blocks of warps_per_block
 // warps), from the SM's shared memory (smem_sm bytes, reserved_per_block
 // of them taken by each block, at most smem_block per block) and registers.
-inline int chain_resident_warps(int smem, int warps_per_block, int q,
-                                int smem_sm, int smem_block,
-                                int reserved_per_block) {
+inline int chain_resident_warps(int smem, int warps_per_block,
+                                int regs_per_thread, int smem_sm,
+                                int smem_block, int reserved_per_block) {
   if (smem > smem_block) return 0;
   const int by_smem = smem_sm / (smem + reserved_per_block);
-  const int regs = (chain_regs(q) + 7) & ~7;
+  const int regs = (regs_per_thread + 7) & ~7;
   const int by_regs = 65536 / (regs * 32 * warps_per_block);
   const int blocks = by_smem < by_regs ? by_smem : by_regs;
   return blocks * warps_per_block;

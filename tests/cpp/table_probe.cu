@@ -50,7 +50,9 @@ int main() {
               const bbs::TablePlan p = bbs::plan_tables(
                   n, w32, cells, q, wpc, slots, sum != 0, false, true, kBlock,
                   kBlock + 1024);
-              const bool fits = slots * sb <= kBlock && !(sum && chunks > 1);
+              const bool few = w32 == 1 && cells <= bbs::kFewCells;
+              const bool fits =
+                  slots * sb <= kBlock && !(sum && (chunks > 1 || few));
               if (p.inc || p.chunks != (fits ? chunks : 0) ||
                   p.smem != slots * (fits ? sb
                                           : bbs::slot_bytes(n, rs, wpc,
