@@ -440,9 +440,11 @@ struct Piece {
 // On GB300 the copy engines read and write pageable memory through the host's
 // page tables: 6.3 MB take 48 us in and 42 us out (38 and 41 us pinned),
 // while the memcpy into or out of the mirror alone runs at 19 GB/s, 320 us.
-// A copy of its own costs some microseconds whatever its size, the memcpy of
-// 64 KB about three.
-constexpr size_t kDirectBytes = 64 * 1024;
+// A copy of its own costs some microseconds whatever its size: calls on trees
+// of 80 nodes and 14 cells, through the mirror and direct, took 46.0 and 49.0
+// us with 160 KB of rows, 52.0 and 55.4 with 256 KB, 59.2 and 58.3 with 384 KB,
+// 68.1 and 61.4 with 512 KB.
+constexpr size_t kDirectBytes = 256 * 1024;
 
 // Pieces of the context's scratch for one call of a host-buffer entry point
 // (bbs_score_trees, bbs_apply_moves, bbs_sumscore_grad).  The call adds up
@@ -955,10 +957,11 @@ int bbs_get_sizes(const bbs_ctx *c, uint32_t *n_cells, uint32_t *n_genes,
 namespace {
 
 TablePlan chain_plan(const bbs_ctx *c, int q, int wpc, int cpb) {
-  return plan_tables((int)c->n_nodes, w32_of_nodes((int)c->n_nodes),
-                     (int)c->n_cells, q, wpc, cpb, c->md.score_mode != 0, true,
-                     wide_tables(c->ds, c->md, c->terms), c->smem_block,
-                     c->smem_sm);
+  const int w32 = w32_of_nodes((int)c->n_nodes);
+  return plan_tables((int)c->n_nodes, w32, (int)c->n_cells, q, wpc, cpb,
+                     c->md.score_mode != 0, true,
+                     w32 > 4 && wide_tables(c->ds, c->md, c->terms),
+                     c->smem_block, c->smem_sm);
 }
 
 // Shared memory a shape is accepted by: the plan's, and the slots' with the

@@ -1,5 +1,5 @@
 """The calls on host buffers give the same results whether an array crosses
-through the pinned mirror (up to 64 KB) or straight from the caller's memory:
+through the pinned mirror (small arrays) or straight from the caller's memory:
 a batch equals its trees taken a few at a time."""
 import numpy as np
 import pytest
