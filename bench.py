@@ -846,8 +846,9 @@ def run_ours(args) -> None:
             "per_chain_step": popc_step,
             "note": "32-bit POPC of the masked-popcount formulation "
                     "(cells x nodes x 2 x ceil(genes/32)); the benched "
-                    "kernels inherit counts and issue none of them in the "
-                    "node loop, so this is work done, not a pipe's use"},
+                    "kernels read proposals off a table of every node and "
+                    "issue none of them, so this is work done, not a pipe's "
+                    "use"},
     }
 
     # end to end through the C ABI with host buffers (batched+adjoint)
