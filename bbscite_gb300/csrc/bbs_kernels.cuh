@@ -1551,8 +1551,9 @@ __device__ __forceinline__ void walk_codes(const SumCtx &sx,
 // order fits the ring and its rates have exact codes (bbs_incr.cuh), each node
 // takes its parent's codes from the ring plus its gene's, some 20
 // instructions a node for 64 cells; otherwise masked popcounts, which run the
-// population-count pipe at its peak (255 x 512, 1500 trees: 735 us, now 225 us,
-// bound by the latency of the walk at three blocks per SM).
+// population-count pipe at its peak (255 x 512, 1500 trees: 735 us, walked 230
+// us, and another 9 us less a call with offsets in the order's entries; bound by
+// the latency of the walk at three blocks per SM).
 template <int W32, bool ATTACH>
 __global__ void __launch_bounds__(128) score_walk_kernel(const ScoreArgs a) {
   extern __shared__ __align__(16) uint32_t smem[];

@@ -599,9 +599,9 @@ def run_beyond_caps(N, chains, steps, flush, torch, warm=20000, early=1500):
     regime of nearly all of a 1,000,000-step run.  The rate after `early`
     steps is reported too: there the sum score still sums many cells a
     second time, while their best attachment lies far below the bound it is
-    taken against.  Launch shapes are tuned after `early` steps.  Both
-    forms inherit counts through the ring (rows of eight words); the
-    roofline is the issue slots, from the warp instructions per chain-step
+    taken against.  Launch shapes are tuned after `early` steps.  The sum
+    score walks the ring (rows of eight words), the max score reads a
+    table; the roofline is the issue slots, from the warp instructions per chain-step
     of the committed ncu summary (captured after `warm` steps)."""
     from bbscite_gb300 import data as D
     G, Cn = 255, 512

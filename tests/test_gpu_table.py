@@ -179,3 +179,43 @@ def test_wide_max_chains_equal_traced_ones(native, G, Cn, launch):
             got.append((c.chains(), c.best(), c.save_chains()))
     assert got[0][2] == got[1][2]
     assert got[0][1]["score"] == got[1][1]["score"]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("score", ["max", "sum"])
+@pytest.mark.parametrize("G,Cn,chains", [(8, 70, 700), (31, 96, 40),
+                                         (63, 200, 3), (95, 96, 1200),
+                                         (127, 130, 400), (127, 400, 5)])
+def test_default_shapes_give_the_chains_of_one_warp(native, score, G, Cn,
+                                                    chains):
+    """The shape chosen without tuning, few and many chains, one and more
+    passes over the cells, leaves every chain as one-warp blocks of one cell
+    per lane do."""
+    mut, known = _setup(G, Cn, 7)
+    p = native.default_params(alpha_mean=1e-2, beta_mean=0.3, seed=41,
+                              prob_beta_change=0.1,
+                              score_mode=getattr(native,
+                                                 "SCORE_" + score.upper()))
+    images = []
+    for shape in (None, (1, 1, 1)):
+        with native.Context(mut, known, Cn, G, p) as c:
+            c.init_chains(chains)
+            if shape:
+                c.set_launch(*shape)
+            c.run(40)
+            images.append(c.save_chains())
+    assert images[0] == images[1]
+
+
+@pytest.mark.gpu
+def test_blocks_whose_counts_do_not_fit_are_refused(native):
+    """Eight chains of 96 nodes and 96 cells at three cells per lane have no
+    room for their counts, although they would without a table."""
+    mut, known = _setup(95, 96, 7)
+    with native.Context(mut, known, 96, 95) as c:
+        c.init_chains(8)
+        c.set_launch(3, 1, 8)
+        with pytest.raises(native.BbsError):
+            c.run(10)
+        c.set_launch(3, 1, 7)
+        c.run(10)
