@@ -2204,6 +2204,23 @@ int batch_build_groups(bbs_batch *b) {
   return BBS_OK;
 }
 
+// Cells per lane of a batch nobody tunes.  Sum-score chains read proposals off
+// a table only where their cells fit one pass, so up to 128 cells get as many
+// cells per lane as that takes, unless smaller datasets would be most of the
+// work.  600 steps with two and with that many cells per lane, ms: 2844 chains
+// at 105 x 81 46.7, 16.0; 20 at 20 x 70 2.74, 0.76; 300 at 127 x 128 (300 steps)
+// 10.2, 2.1.  Max-score tables take several passes.
+int default_cells_per_lane(const bbs_batch *b) {
+  uint32_t lo = UINT32_MAX, hi = 0;
+  for (uint32_t d = 0; d < b->n_datasets; d++) {
+    if (b->n_genes[d] + 1 > 128) continue;
+    const uint32_t g = (b->n_cells[d] + 31) / 32;
+    lo = std::min(lo, g);
+    hi = std::max(hi, g);
+  }
+  return b->sum && hi > 2 && hi <= (uint32_t)kMaxQ && 2 * lo >= hi ? (int)hi : 2;
+}
+
 // Cells per lane of a launch group: 1 or 2 above 128 nodes.
 int group_q(const bbs_batch *b, const bbs_batch::Group &grp) {
   return grp.w32 > 4 ? std::min(b->q, 2) : b->q;
@@ -2363,6 +2380,7 @@ int bbs_batch_create(bbs_batch **out, uint32_t n_datasets,
     b->n_cells.assign(n_cells, n_cells + n_datasets);
     b->n_genes.assign(n_genes, n_genes + n_datasets);
     b->sum = sum;
+    b->q = default_cells_per_lane(b);
     cudaGetDevice(&b->device);
     cudaDeviceGetAttribute(&b->n_sms, cudaDevAttrMultiProcessorCount, b->device);
     cudaDeviceGetAttribute(&b->smem_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor,

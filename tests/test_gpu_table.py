@@ -219,3 +219,26 @@ def test_blocks_whose_counts_do_not_fit_are_refused(native):
             c.run(10)
         c.set_launch(3, 1, 7)
         c.run(10)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("G,Cn", [(20, 64), (20, 65), (63, 97), (127, 128),
+                                  (40, 129)])
+def test_untuned_sum_batches_equal_their_chains_alone(native, G, Cn):
+    """Two, three and four cells per lane by default, and more cells than one
+    pass takes."""
+    mut, known = _setup(G, Cn, 9)
+    p = native.default_params(alpha_mean=1e-2, beta_mean=0.3, seed=43,
+                              prob_beta_change=0.1,
+                              score_mode=native.SCORE_SUM)
+    with native.Batch([(mut, known, Cn, G)], p) as b:
+        b.init_chains(6)
+        b.run(120)
+        batch = b.best(0)
+    with native.Context(mut, known, Cn, G, p) as c:
+        c.init_chains(6)
+        c.set_launch(1, 1, 1)
+        c.run(120)
+        one = c.best()
+    assert one["score"] == batch["score"]
+    assert (one["dm"] == batch["dm"]).all()
