@@ -867,6 +867,8 @@ __device__ __forceinline__ float entry_shift(const uint32_t (&a)[NW],
 }
 
 inline constexpr float kBoundUnit = 4096.0f;  // 2^-12 of a base-2 log
+inline constexpr float kFlushed = 3.0092655e-36f;  // 2^-118: 128 terms of 2^-126
+                                                   // and as much again
 
 // Adds upper bounds of a proposal's sum score and max score over one chunk of
 // this warp's cells, relative to the current tree, to up: up[0] bounds sum_c log2(z'_c / z_c),
@@ -874,6 +876,10 @@ inline constexpr float kBoundUnit = 4096.0f;  // 2^-12 of a base-2 log
 // 1 / kBoundUnit.  eps bounds the relative rounding of a term against its
 // shifted form.  Sums of up to 128 terms are good to 2^-17 of the largest
 // partial sum, so a cell's remainder z - zo is taken with 2^-15 z on top.
+// Terms below 2^-126 were flushed to zero, in zo and in z; kFlushed covers them,
+// for the nodes that move and for those that stay: where a cell's best node
+// moves far away, the exact sum takes the others against their own maximum and
+// counts them again.
 template <int W32, int Q, int NW = kPackWords<Q>>
 __device__ __forceinline__ void bound_proposal(
     const Table<W32, Q> &tab, const Delta &x, const uint8_t *list, int nv, int nc,
@@ -910,8 +916,7 @@ __device__ __forceinline__ void bound_proposal(
 #pragma unroll
       for (int q = 0; q < Q; q++) {
         rest[q] -= zo[q];
-        // terms below 2^-126 were flushed to zero: at most 2^-118 together
-        z1[q] = fmaf(zo[q] + 3.0092655e-36f, ex2_approx(hv[q]), z1[q]);
+        z1[q] = fmaf(zo[q] + kFlushed, ex2_approx(hv[q]), z1[q]);
         gain[q] = fmaxf(gain[q], mo[q] + hv[q]);
       }
     }
@@ -921,7 +926,8 @@ __device__ __forceinline__ void bound_proposal(
   float s = 0.0f, g = 0.0f;
 #pragma unroll
   for (int q = 0; q < Q; q++) {
-    const float left = fmaxf(rest[q], 0.0f) + 3.0517578e-05f * cs.z[q];
+    const float left =
+        fmaxf(rest[q], 0.0f) + fmaf(3.0517578e-05f, cs.z[q], kFlushed);
     const float zu = fmaf(z1[q], 1.0f + eps, left);
     // the largest exponent left is at most the current one and at most the
     // logarithm of what is left of the sum

@@ -242,3 +242,45 @@ def test_untuned_sum_batches_equal_their_chains_alone(native, G, Cn):
         one = c.best()
     assert one["score"] == batch["score"]
     assert (one["dm"] == batch["dm"]).all()
+
+
+@pytest.mark.gpu
+def test_the_sum_scores_bound_is_a_bound(tmp_path):
+    """Proposals bounded and summed by the chain kernels' own functions, at
+    cells far below their reference and nodes at the end of the range of
+    normal floats (tests/cpp/bound_probe.cu)."""
+    from bbscite_gb300 import build as B
+    exe = str(tmp_path / "bound_probe")
+    subprocess.run([B.nvcc(), *B.ARCH, "-O3", "-std=c++17", "-I" + B.INCLUDE,
+                    "-I" + B.CSRC,
+                    os.path.join(ROOT, "tests", "cpp", "bound_probe.cu"),
+                    "-o", exe], check=True, capture_output=True)
+    r = subprocess.run([exe, "far"], capture_output=True, text=True,
+                       timeout=300)
+    assert r.returncode == 0, r.stdout
+    assert r.stdout.startswith("bound ok "), r.stdout
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("move", ["beta_walk", "langevin"])
+@pytest.mark.parametrize("G,Cn,q,alpha", [(95, 96, 3, 1e-4), (95, 96, 3, 1e-5),
+                                          (111, 60, 2, 1e-4),
+                                          (126, 128, 4, 1e-5)])
+def test_first_steps_at_small_rates_equal_traced_ones(native, move, G, Cn, q,
+                                                      alpha):
+    """Random trees and rates far below them: the first steps pass cells whose
+    best node lies far below their reference."""
+    mut, known = _setup(G, Cn, 5)
+    p = native.default_params(
+        alpha_mean=alpha, beta_mean=0.3, seed=59, prob_beta_change=0.05,
+        score_mode=native.SCORE_SUM,
+        error_move=getattr(native, "ERROR_" + move.upper()))
+    got = []
+    for trace in (False, True):
+        with native.Context(mut, known, Cn, G, p) as c:
+            c.init_chains(1000)
+            c.set_launch(q, 1, 1)
+            for steps in (30, 100):
+                c.run(steps, trace=trace)
+            got.append(c.save_chains())
+    assert got[0] == got[1]
