@@ -937,10 +937,16 @@ __device__ __forceinline__ void bound_proposal(
       g += top - cs.mx[q];
     }
   }
-  // rounded up; beyond +-8000 per lane the sum saturates upwards (inf and
-  // NaN end there too: such a proposal is not rejected)
-  s = s < 8000.0f && g < 8000.0f ? fmaxf(s, -8000.0f) : 8000.0f;
-  g = g < 8000.0f ? fmaxf(g, -8000.0f) : 8000.0f;
+  // rounded up, and down to -8000 at most, which is still above the lane's sum.
+  // A lane above 8000 (cells of rates far below those of real data; inf and NaN
+  // end there too) has no bound, and with it the proposal has none
+  const bool high = !(s < 8000.0f && g < 8000.0f);
+  if (__any_sync(BBS_FULL_MASK, high)) {
+    up[0] = up[1] = INFINITY;
+    return;
+  }
+  s = fmaxf(s, -8000.0f);
+  g = fmaxf(g, -8000.0f);
   up[0] += (float)__reduce_add_sync(BBS_FULL_MASK, __float2int_ru(s * kBoundUnit) + 1);
   up[1] += (float)__reduce_add_sync(BBS_FULL_MASK, __float2int_ru(g * kBoundUnit) + 1);
 }

@@ -5,6 +5,8 @@
 //   far   one cell whose best node, 100 to 116 powers of two below the cell's
 //         reference, moves away, while the other nodes lie about where a term
 //         leaves the range of normal floats (2^-126)
+//   high  one lane whose cells gain more than the bound counts, beside lanes
+//         that lose less than that
 #include <cmath>
 #include <cstdint>
 #include <cstdio>
@@ -195,12 +197,40 @@ void far_cases(std::vector<Case> &cases) {
     cases.push_back(far_case(logs(1.0e-4, 0.3), 32, 58, 1, 41, 0, 40, others, false));
 }
 
+// Four cells per lane, a node moved from one branch to another: lane 0's cells
+// have 60 of their 120 mutations in either, `lose` other lanes' lose `down`.
+Case high_case(int lose, int down) {
+  const bbs::LogTable L = logs(1.0e-20, 0.2);
+  Case c = empty_case(4, 8, 128, L);
+  for (int q = 0; q < 4; q++)
+    for (int lane = 0; lane < 32; lane++) {
+      const size_t at = (size_t)q * 32 + lane;
+      const bool gains = lane == 0, loses = lane > 0 && lane <= lose;
+      c.pm[at] = gains || loses ? 120.0f : 0.0f;
+      c.entry[(size_t)0 * 128 + at] = field(0, gains ? 60 : loses ? 120 : 0);
+      c.entry[(size_t)1 * 128 + at] = field(0, gains ? 60 : 0);
+      c.entry[(size_t)2 * 128 + at] = field(0, loses ? down : 0);
+    }
+  c.x.a0 = 1;
+  c.x.b0 = 2;
+  c.x.a1 = c.x.b1 = 7;
+  c.list = {0};
+  c.nv = c.nc = 1;
+  return c;
+}
+
+void high_cases(std::vector<Case> &cases) {
+  for (int lose : {0, 1, 31})
+    for (int down : {1, 60}) cases.push_back(high_case(lose, down));
+}
+
 }  // namespace
 
 int main(int argc, char **argv) {
   const std::string kind = argc > 1 ? argv[1] : "";
   std::vector<Case> cases;
   if (kind == "far") far_cases(cases);
+  if (kind == "high") high_cases(cases);
   if (cases.empty()) return 2;
 
   // everything in one allocation each

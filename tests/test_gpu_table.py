@@ -245,17 +245,19 @@ def test_untuned_sum_batches_equal_their_chains_alone(native, G, Cn):
 
 
 @pytest.mark.gpu
-def test_the_sum_scores_bound_is_a_bound(tmp_path):
+@pytest.mark.parametrize("kind", ["far", "high"])
+def test_the_sum_scores_bound_is_a_bound(tmp_path, kind):
     """Proposals bounded and summed by the chain kernels' own functions, at
-    cells far below their reference and nodes at the end of the range of
-    normal floats (tests/cpp/bound_probe.cu)."""
+    cells far below their reference with nodes at the end of the range of
+    normal floats, and at gains beyond what a lane counts
+    (tests/cpp/bound_probe.cu)."""
     from bbscite_gb300 import build as B
     exe = str(tmp_path / "bound_probe")
     subprocess.run([B.nvcc(), *B.ARCH, "-O3", "-std=c++17", "-I" + B.INCLUDE,
                     "-I" + B.CSRC,
                     os.path.join(ROOT, "tests", "cpp", "bound_probe.cu"),
                     "-o", exe], check=True, capture_output=True)
-    r = subprocess.run([exe, "far"], capture_output=True, text=True,
+    r = subprocess.run([exe, kind], capture_output=True, text=True,
                        timeout=300)
     assert r.returncode == 0, r.stdout
     assert r.stdout.startswith("bound ok "), r.stdout
