@@ -6,13 +6,18 @@
 
 namespace bbs {
 
+// Lets a kernel take `smem` bytes of dynamic shared memory: its limit has to be
+// raised where they and its static ones (at most 4 KB in any kernel) are more
+// than 48 KB together.
 template <typename K>
 inline cudaError_t prepare_smem(K kernel, size_t smem) {
-  if (smem > 48 * 1024)
-    return cudaFuncSetAttribute(kernel,
-                                cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)smem);
-  return cudaSuccess;
+  if (smem <= 44 * 1024) return cudaSuccess;
+  cudaFuncAttributes at;
+  const cudaError_t e = cudaFuncGetAttributes(&at, kernel);
+  if (e != cudaSuccess || smem + at.sharedSizeBytes <= 48 * 1024) return e;
+  return cudaFuncSetAttribute(kernel,
+                              cudaFuncAttributeMaxDynamicSharedMemorySize,
+                              (int)smem);
 }
 
 // Persistent launch.  wpc == 1: blocks of `cpb` one-warp chains; wpc > 1:

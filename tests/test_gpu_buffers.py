@@ -109,3 +109,11 @@ def test_walked_trees_score_as_few_do(native, orc, G, Cn):
     """Both sides of the sizes from which rows of up to four words are
     walked, odd and even ends of the walk's pairs, and the most nodes."""
     test_many_trees_score_as_few_do(native, orc, G, Cn)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("G,Cn", [(91, 100), (92, 128), (174, 64)])
+def test_posteriors_whose_tiles_nearly_fill_48_kb(native, orc, G, Cn):
+    """The tile alone below 48 KB, with the kernel's static shared memory
+    above."""
+    test_adjoint_and_posteriors_match_fp64(native, orc, G, Cn, 3)
