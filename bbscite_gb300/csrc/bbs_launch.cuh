@@ -7,17 +7,26 @@
 namespace bbs {
 
 // Lets a kernel take `smem` bytes of dynamic shared memory: its limit has to be
-// raised where they and its static ones (at most 4 KB in any kernel) are more
-// than 48 KB together.
+// raised where they and its static ones (far below 4 KB in every kernel) are
+// more than 48 KB together.  The limit is the kernel's in the whole process, so
+// it only ever goes to the most a block may have: set to what a call needs, it
+// would take another thread's room between its call here and its launch.
 template <typename K>
 inline cudaError_t prepare_smem(K kernel, size_t smem) {
   if (smem <= 44 * 1024) return cudaSuccess;
   cudaFuncAttributes at;
-  const cudaError_t e = cudaFuncGetAttributes(&at, kernel);
-  if (e != cudaSuccess || smem + at.sharedSizeBytes <= 48 * 1024) return e;
+  cudaError_t e = cudaFuncGetAttributes(&at, kernel);
+  if (e != cudaSuccess || smem <= (size_t)at.maxDynamicSharedSizeBytes) return e;
+  int device = 0, block = 0;
+  e = cudaGetDevice(&device);
+  if (e == cudaSuccess)
+    e = cudaDeviceGetAttribute(&block, cudaDevAttrMaxSharedMemoryPerBlockOptin,
+                               device);
+  if (e != cudaSuccess) return e;
+  if (smem + at.sharedSizeBytes > (size_t)block) return cudaErrorInvalidValue;
   return cudaFuncSetAttribute(kernel,
                               cudaFuncAttributeMaxDynamicSharedMemorySize,
-                              (int)smem);
+                              block - (int)at.sharedSizeBytes);
 }
 
 // Persistent launch.  wpc == 1: blocks of `cpb` one-warp chains; wpc > 1:

@@ -5,6 +5,8 @@ error is kept per thread, so two contexts and a batch driven from three
 threads at the same time (ctypes releases the GIL during each call) give
 exactly the results of the same runs one after another.
 """
+import os
+import subprocess
 import threading
 
 import numpy as np
@@ -86,3 +88,70 @@ def test_contexts_on_three_threads_match_sequential_runs(native):
         np.testing.assert_array_equal(dm_p, dm_s)
         assert s_p == s_s
     assert all("gene count 300" in m for m in par[3]), set(par[3])
+
+
+@pytest.mark.parametrize("sizes", [(224, 255), (103, 126)])
+def test_scoring_threads_of_different_sizes_leave_each_other_alone(native,
+                                                                   sizes):
+    """Scores and posteriors from two threads, their sizes in the same row
+    width: the calls run the same kernels and ask for different amounts of
+    shared memory."""
+    rng = np.random.default_rng(3)
+    jobs = []
+    for G in sizes:
+        m, _, _ = D.generate_dataset(40 + G, G, 70, 1e-3, 0.2, 0.1, 0.02)
+        mut, known = D.matrix_to_bits(m)
+        pv = [D.random_parent_vector(rng, G) for _ in range(320)]
+        jobs.append((G, mut, known, np.stack(
+            [native.parent_to_matrix(p)[1] for p in pv])))
+    calls = 400
+
+    def work(G, mut, known, dms, n):
+        out = None
+        with native.Context(mut, known, 70, G) as c:
+            for _ in range(n):
+                s, counts, at = c.score_trees(dms, 0.2, attach=True)
+                l, da, db, post = c.sumscore_grad(dms[:3], 1e-3, 0.2,
+                                                  posterior=True)
+                got = [s, counts, at, l, da, db, post]
+                if out is None:
+                    out = got
+                for x, y in zip(got, out):
+                    np.testing.assert_array_equal(x, y)
+        return out
+
+    alone = [work(*j, 1) for j in jobs]
+    together, errs = [None, None], []
+    start = threading.Barrier(2)
+
+    def wrap(i):
+        try:
+            start.wait(timeout=60)
+            together[i] = work(*jobs[i], calls)
+        except BaseException as exc:  # reported on the main thread
+            errs.append(exc)
+    threads = [threading.Thread(target=wrap, args=(i,)) for i in (0, 1)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join(timeout=300)
+    assert not errs, errs
+    assert all(not t.is_alive() for t in threads)
+    for a, b in zip(alone, together):
+        for x, y in zip(a, b):
+            np.testing.assert_array_equal(x, y)
+
+
+def test_a_kernels_limit_is_never_lowered(tmp_path):
+    """The order in which two threads' calls may reach a kernel's limit of
+    shared memory, one after the other (tests/cpp/limit_probe.cu)."""
+    from bbscite_gb300 import build as B
+    exe = str(tmp_path / "limit_probe")
+    src = os.path.join(os.path.dirname(os.path.abspath(__file__)), "cpp",
+                       "limit_probe.cu")
+    subprocess.run([B.nvcc(), *B.ARCH, "-std=c++17", "-I" + B.INCLUDE,
+                    "-I" + B.CSRC, src, "-o", exe], check=True,
+                   capture_output=True)
+    r = subprocess.run([exe], capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stdout
+    assert r.stdout.startswith("limits ok"), r.stdout
