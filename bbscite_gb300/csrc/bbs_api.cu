@@ -2067,6 +2067,7 @@ struct bbs_batch {
   unsigned int *d_counters = nullptr;
   int *d_status = nullptr;
   int q = 2, wpb = 4, merge = 0;
+  bool q_set = false;  // cells per lane set by the caller or the tuner
   int wpc = 1;  // warps per chain (above 1 a block is one chain)
   // graph of the current shape and step count
   cudaGraphExec_t graph = nullptr;
@@ -2155,6 +2156,8 @@ struct BatchCheckpointHeader {
 static_assert(sizeof(BatchCheckpointHeader) == 72, "batch checkpoint header layout");
 constexpr char kBatchCheckpointMagic[8] = {'B', 'B', 'S', 'B', 'A', 'T', 'C', 'H'};
 
+void settle_cells_per_lane(bbs_batch *b);
+
 // Launch groups for the current shape: one per row width (exact, or the
 // even width of its row stride with merge), chains costliest first.
 int batch_build_groups(bbs_batch *b) {
@@ -2201,6 +2204,7 @@ int batch_build_groups(bbs_batch *b) {
     b->side.push_back(s);
     b->side_ev.push_back(ev);
   }
+  settle_cells_per_lane(b);
   return BBS_OK;
 }
 
@@ -2273,6 +2277,14 @@ bool batch_shape_fits(const bbs_batch *b) {
     if (std::max(smem, group_plan(b, grp).smem) > b->smem_block) return false;
   }
   return true;
+}
+
+// The default cells per lane, or two where a block of the warps that the caller
+// asked for has no room for that many.
+void settle_cells_per_lane(bbs_batch *b) {
+  if (b->q_set) return;
+  b->q = default_cells_per_lane(b);
+  if (!batch_shape_fits(b)) b->q = 2;
 }
 
 // Issues one run: zero the work counters, then one launch per group on its
@@ -2577,6 +2589,7 @@ int bbs_batch_set_launch(bbs_batch *b, int q, int wpb, int merge) {
     return fail(BBS_ERR_INPUT, "warps per block must be in [1, %d]",
                 kMaxBlockThreads / 32);
   if (q) b->q = q;
+  b->q_set = b->q_set || q != 0;
   if (wpb) b->wpb = wpb;
   if (merge >= 0 && merge != b->merge) {
     b->merge = merge ? 1 : 0;
@@ -2585,6 +2598,7 @@ int bbs_batch_set_launch(bbs_batch *b, int q, int wpb, int merge) {
       if (r != BBS_OK) return r;
     }
   }
+  settle_cells_per_lane(b);
   if (b->graph) cudaGraphExecDestroy(b->graph);
   b->graph = nullptr;
   return BBS_OK;
@@ -2603,6 +2617,7 @@ int bbs_batch_set_chain_warps(bbs_batch *b, int warps_per_chain) {
   if (warps_per_chain < 1 || warps_per_chain > 4)
     return fail(BBS_ERR_INPUT, "warps per chain must be 1, 2, 3 or 4");
   b->wpc = warps_per_chain;
+  settle_cells_per_lane(b);
   if (b->graph) cudaGraphExecDestroy(b->graph);
   b->graph = nullptr;
   return BBS_OK;

@@ -286,3 +286,27 @@ def test_first_steps_at_small_rates_equal_traced_ones(native, move, G, Cn, q,
                 c.run(steps, trace=trace)
             got.append(c.save_chains())
     assert got[0] == got[1]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("G,Cn,warps,chain_warps", [
+    (95, 96, 8, 1), (127, 128, 6, 1), (127, 128, 7, 1), (127, 96, 4, 4)])
+def test_untuned_sum_batches_take_any_warps(native, G, Cn, warps, chain_warps):
+    """Warps set without cells per lane: where as many cells per lane as a pass
+    takes leave the block no room, two do."""
+    mut, known = _setup(G, Cn, 9)
+    p = native.default_params(alpha_mean=1e-2, beta_mean=0.3, seed=43,
+                              prob_beta_change=0.1,
+                              score_mode=native.SCORE_SUM)
+    got = []
+    for shape in (None, (warps, chain_warps)):
+        with native.Batch([(mut, known, Cn, G)], p) as b:
+            if shape:
+                b.set_launch(warps_per_block=warps)
+            b.init_chains(10)
+            if shape:
+                b.set_chain_warps(chain_warps)
+                assert b.launch()[0] == 2
+            b.run(60)
+            got.append(b.save_chains())
+    assert got[0] == got[1]
