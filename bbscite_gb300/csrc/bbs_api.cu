@@ -245,6 +245,11 @@ struct TableBuf {
   }
 };
 
+// Cells per lane, warps per chain and chains per block of the chain kernel.
+struct LaunchShape {
+  int q = 1, wpc = 1, cpb = 1;
+};
+
 struct bbs_ctx {
   int device = 0, n_sms = 0;
   int smem_sm = 0, smem_block = 0, smem_reserved = 0;  // per SM / block
@@ -268,6 +273,8 @@ struct bbs_ctx {
   int *h_cancel = nullptr;        // mapped pinned flag
   int *d_cancel = nullptr;
   int q = 1, wpc = 1, cpb = 1;  // chain-kernel launch shape
+  unsigned set = 0;             // which of them the caller set (kSet...)
+  LaunchShape spread;           // the shape without tables (settle_launch)
   bool running = false;
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
   float last_ms = 0.0f;
@@ -973,6 +980,12 @@ int shape_smem(const bbs_ctx *c, int q, int wpc, int cpb) {
                                     cpb, c->md.score_mode != 0));
 }
 
+// Whether blocks of a shape may be launched.
+bool shape_fits(const bbs_ctx *c, int q, int wpc, int cpb) {
+  return 32 * wpc * cpb <= chain_max_threads(q) &&
+         shape_smem(c, q, wpc, cpb) <= c->smem_block;
+}
+
 // Resident warps per SM of blocks of cpb chains of wpc warps.
 int resident_warps(const bbs_ctx *c, int q, int wpc, int cpb) {
   return chain_resident_warps(shape_smem(c, q, wpc, cpb), wpc * cpb,
@@ -980,25 +993,18 @@ int resident_warps(const bbs_ctx *c, int q, int wpc, int cpb) {
                               c->smem_sm, c->smem_block, c->smem_reserved);
 }
 
-// One-warp chains per block (1-8; they share the block's increment table)
-// that keep the most warps resident on an SM; ties keep the smaller block.
-int pick_chains_per_block(const bbs_ctx *c, int q) {
-  int best = 1, best_warps = 0;
-  for (int cpb = 1; cpb * 32 <= chain_max_threads(q); cpb++) {
-    const int w = resident_warps(c, q, 1, cpb);
-    if (w > best_warps) {
-      best_warps = w;
-      best = cpb;
-    }
-  }
-  return best;
-}
-
 // Launch shape without timing, rows of five to eight words: split the cells
 // over up to four warps per chain when there are too few chains to give every
-// scheduler ~3 warps, preferring shapes that leave no cell slots empty.
-void default_wide_launch(bbs_ctx *c) {
-  const int groups = (int)((c->n_cells + 31) / 32), qmax = 2;
+// scheduler ~3 warps, preferring shapes that leave no cell slots empty; blocks
+// of as many one-warp chains (1-8) as keep the most warps resident on an SM,
+// the smaller block on ties.  Without `table` the warps are counted for blocks
+// that hold counts and no table.
+LaunchShape spread_launch(const bbs_ctx *c, bool table) {
+  const int groups = (int)((c->n_cells + 31) / 32);
+  const int qmax = w32_of_nodes((int)c->n_nodes) > 4 ? 2 : kMaxQ;
+  LaunchShape o;
+  o.q = qmax;  // very wide datasets: chunks of qmax per lane
+  o.wpc = 4;
   double best = 1e30;
   for (int wpc = 1; wpc <= 4; wpc++) {
     const int q = std::max(1, (groups + wpc - 1) / wpc);
@@ -1009,15 +1015,26 @@ void default_wide_launch(bbs_ctx *c) {
     const double est = waste / occ * (1.0 + 0.1 * (wpc - 1));
     if (est < best) {
       best = est;
-      c->wpc = wpc;
-      c->q = q;
+      o.wpc = wpc;
+      o.q = q;
     }
   }
-  if (best >= 1e30) {  // very wide datasets: chunks of qmax per lane
-    c->wpc = 4;
-    c->q = qmax;
+  if (o.wpc > 1) return o;
+  int best_warps = 0;
+  for (int cpb = 1; cpb * 32 <= chain_max_threads(o.q); cpb++) {
+    const int w =
+        table ? resident_warps(c, o.q, 1, cpb)
+              : chain_resident_warps(
+                    chain_launch_smem((int)c->n_nodes, (int)c->n_cells, o.q, 1,
+                                      cpb, c->md.score_mode != 0),
+                    cpb, chain_regs(o.q, false), c->smem_sm, c->smem_block,
+                    c->smem_reserved);
+    if (w > best_warps) {
+      best_warps = w;
+      o.cpb = cpb;
+    }
   }
-  c->cpb = c->wpc == 1 ? pick_chains_per_block(c, c->q) : 1;
+  return o;
 }
 
 // Launch shape without timing, rows of up to four words.  With a table a step
@@ -1036,18 +1053,15 @@ void default_wide_launch(bbs_ctx *c) {
 // sum score, 400 steps, 750 at 95 x 128 (1, 4, 1) 3.62, (2, 2, 1) 2.43; 200
 // steps, 3000 at 95 x 128 (4, 1, 8), which has no room for tables, 14.7, (2, 2,
 // 1) 3.7.
-void default_launch(bbs_ctx *c) {
-  if (w32_of_nodes((int)c->n_nodes) > 4) {
-    default_wide_launch(c);
-    return;
-  }
+LaunchShape default_launch(const bbs_ctx *c) {
+  if (w32_of_nodes((int)c->n_nodes) > 4) return spread_launch(c, true);
   const bool sum = c->md.score_mode != 0;
   // (error moves of the max score are scored from the rows)
   const bool errors = !sum && c->md.mp.cum_beta > 0.0f;
   const int groups = (int)((c->n_cells + 31) / 32);
   const double n = c->n_nodes, chains = c->n_chains;
   double best = 1e30;
-  c->q = c->wpc = c->cpb = 1;
+  LaunchShape o;
   for (int wpc = 1; wpc <= 4; wpc++)
     for (int q = 1; q <= kMaxQ; q++) {
       // (no warp and no cell slot that would stay empty)
@@ -1076,12 +1090,34 @@ void default_launch(bbs_ctx *c) {
         const double est = rounds * step * crowd;
         if (est < best) {
           best = est;
-          c->q = q;
-          c->wpc = wpc;
-          c->cpb = cpb;
+          o = {q, wpc, cpb};
         }
       }
     }
+  return o;
+}
+
+// The shape the caller set, its other numbers from the default.  Such a mix need
+// not fit a block -- eight chains per block at the default of two cells per
+// lane, say; the numbers then follow the rule that spreads the cells over warps
+// (c->spread), whose mixes were accepted before chains had tables.
+constexpr unsigned kSetCells = 1, kSetWarps = 2, kSetChains = 4;
+void settle_launch(bbs_ctx *c, const LaunchShape &rest) {
+  if (!(c->set & kSetCells)) c->q = rest.q;
+  if (!(c->set & kSetWarps)) c->wpc = rest.wpc;
+  if (!(c->set & kSetChains)) c->cpb = rest.cpb;
+  if (c->wpc > 1) c->cpb = 1;
+  if (shape_fits(c, c->q, c->wpc, c->cpb)) return;
+  c->q = c->spread.q;
+  c->wpc = c->spread.wpc;
+  c->cpb = c->spread.cpb;
+}
+
+// New chains: the default shape.
+void reset_launch(bbs_ctx *c) {
+  c->set = 0;
+  c->spread = spread_launch(c, false);
+  settle_launch(c, default_launch(c));
 }
 
 size_t tree_words(const bbs_ctx *c, uint32_t n_trees) {
@@ -1154,7 +1190,7 @@ int bbs_init_chains(bbs_ctx *c, uint32_t n_chains, const uint32_t *parents) {
     int r = le != 0 ? cuda_fail(le, "init kernel launch")
                     : sync_stream(c, "init kernel");
     if (r != BBS_OK) free_chains(c);
-    default_launch(c);
+    reset_launch(c);
     return r;
   } catch (...) {
     return fail(BBS_ERR_ALLOC, "allocation failed in bbs_init_chains");
@@ -1168,7 +1204,7 @@ int start_run(bbs_ctx *c, uint32_t n_steps, const bbs_raw_move *d_moves,
   {
     const int cpb = c->wpc > 1 ? 1 : c->cpb;
     const int smem = shape_smem(c, c->q, c->wpc, cpb);
-    if (32 * c->wpc * cpb > chain_max_threads(c->q) || smem > c->smem_block)
+    if (!shape_fits(c, c->q, c->wpc, cpb))
       return fail(BBS_ERR_SIZE,
                   "launch shape (%d cells per lane, %d warps per chain, %d "
                   "chains per block) needs %d bytes of shared memory and %d "
@@ -1307,10 +1343,15 @@ int bbs_set_launch(bbs_ctx *c, int cells_per_lane, int warps_per_chain,
   if (chains_per_block < 0 || 32 * chains_per_block > kMaxBlockThreads)
     return fail(BBS_ERR_INPUT, "chains per block must be in [1, %d]",
                 kMaxBlockThreads / 32);
-  if (cells_per_lane) c->q = cells_per_lane;
-  if (warps_per_chain) c->wpc = warps_per_chain;
-  if (chains_per_block) c->cpb = chains_per_block;
+  if (cells_per_lane) c->q = c->spread.q = cells_per_lane;
+  if (warps_per_chain) c->wpc = c->spread.wpc = warps_per_chain;
+  if (chains_per_block) c->cpb = c->spread.cpb = chains_per_block;
   if (c->wpc > 1) c->cpb = 1;
+  if (c->spread.wpc > 1) c->spread.cpb = 1;
+  c->set |= (cells_per_lane ? kSetCells : 0) | (warps_per_chain ? kSetWarps : 0) |
+            (chains_per_block ? kSetChains : 0);
+  // (bbs_init_chains starts anew)
+  if (c->n_chains) settle_launch(c, default_launch(c));
   return BBS_OK;
 }
 
@@ -1361,9 +1402,7 @@ int bbs_autotune(bbs_ctx *c, uint32_t probe_steps, float *best_ms) {
         if (wpc * q > groups + 1) continue;  // mostly empty cell slots
         for (int cpb : {1, 2, 4, 7, 8}) {
           if (wpc > 1 && cpb > 1) continue;
-          if (32 * wpc * cpb > chain_max_threads(q)) continue;
-          if (shape_smem(c, q, wpc, cpb) > c->smem_block)
-            continue;  // too large a block
+          if (!shape_fits(c, q, wpc, cpb)) continue;  // too large a block
           c->q = q;
           c->wpc = wpc;
           c->cpb = cpb;
@@ -1392,6 +1431,8 @@ int bbs_autotune(bbs_ctx *c, uint32_t probe_steps, float *best_ms) {
     c->q = bq;
     c->wpc = bw;
     c->cpb = bb;
+    c->spread = {bq, bw, bb};
+    c->set = kSetCells | kSetWarps | kSetChains;
     const int r = sync_stream(c, "autotune restore");
     if (best_ms) *best_ms = best;
     return r;
@@ -1657,7 +1698,7 @@ int bbs_load_chains(bbs_ctx *c, const void *buf, size_t size) {
       return cuda_fail((int)e, "bbs_load_chains");
     }
     c->n_chains = hd.n_chains;
-    default_launch(c);
+    reset_launch(c);
     return BBS_OK;
   } catch (...) {
     return fail(BBS_ERR_ALLOC, "allocation failed in bbs_load_chains");

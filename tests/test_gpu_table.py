@@ -310,3 +310,28 @@ def test_untuned_sum_batches_take_any_warps(native, G, Cn, warps, chain_warps):
             b.run(60)
             got.append(b.save_chains())
     assert got[0] == got[1]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("G,Cn,chains,part", [
+    (63, 64, 8, dict(chains_per_block=8)),
+    (20, 33, 1024, dict(chains_per_block=6)),
+    (95, 96, 1024, dict(cells_per_lane=1)),
+    (111, 128, 40, dict(warps_per_chain=4)),
+])
+def test_parts_of_a_shape_are_accepted(native, G, Cn, chains, part):
+    """A shape of which the caller sets a part runs, whatever the default for
+    the rest."""
+    mut, known = _setup(G, Cn, 9)
+    for score in (native.SCORE_MAX, native.SCORE_SUM):
+        p = native.default_params(alpha_mean=1e-3, beta_mean=0.2, seed=43,
+                                  score_mode=score)
+        got = []
+        for kw in ({}, part):
+            with native.Context(mut, known, Cn, G, p) as c:
+                c.init_chains(chains)
+                if kw:
+                    c.set_launch(**kw)
+                c.run(20)
+                got.append(c.save_chains())
+        assert got[0] == got[1]
