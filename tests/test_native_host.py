@@ -257,3 +257,17 @@ def test_random_trees_fit_the_ring():
     assert worst < 64, worst
     star = np.full(256, 255, dtype=np.int64)
     assert _ring_distance(star) >= 64
+
+
+def test_a_build_leaves_little_behind(native):
+    """Both libraries and what is kept beside them stay far below the 640 MB
+    that a build once left: whoever copies the tree copies them too."""
+    from bbscite_gb300 import build as B
+    total = 0
+    for path in (B.LIB, B.LIB_CHECKED, B.BUILD, B.BUILD_CHECKED):
+        if os.path.isfile(path):
+            total += os.path.getsize(path)
+        for folder, _, files in os.walk(path):
+            total += sum(os.path.getsize(os.path.join(folder, f))
+                         for f in files)
+    assert total < 250e6, total
