@@ -870,6 +870,10 @@ inline constexpr float kBoundUnit = 4096.0f;  // 2^-12 of a base-2 log
 inline constexpr float kFlushed = 3.0092655e-36f;  // 2^-118: 128 terms of 2^-126
                                                    // and as much again
 
+__device__ __forceinline__ int lane_bound(float s) {
+  return __float2int_ru((s < 8192.0f ? fmaxf(s, -64.0f) : 8192.0f) * kBoundUnit) + 1;
+}
+
 // Adds upper bounds of a proposal's sum score and max score over one chunk of
 // this warp's cells, relative to the current tree, to up: up[0] bounds sum_c log2(z'_c / z_c),
 // up[1] bounds sum_c (largest exponent' - largest exponent), in units of
@@ -937,18 +941,16 @@ __device__ __forceinline__ void bound_proposal(
       g += top - cs.mx[q];
     }
   }
-  // rounded up, and down to -8000 at most, which is still above the lane's sum.
-  // A lane above 8000 (cells of rates far below those of real data; inf and NaN
-  // end there too) has no bound, and with it the proposal has none
-  const bool high = !(s < 8000.0f && g < 8000.0f);
-  if (__any_sync(BBS_FULL_MASK, high)) {
-    up[0] = up[1] = INFINITY;
-    return;
-  }
-  s = fmaxf(s, -8000.0f);
-  g = fmaxf(g, -8000.0f);
-  up[0] += (float)__reduce_add_sync(BBS_FULL_MASK, __float2int_ru(s * kBoundUnit) + 1);
-  up[1] += (float)__reduce_add_sync(BBS_FULL_MASK, __float2int_ru(g * kBoundUnit) + 1);
+  // Rounded up.  A lane loses 15 a cell at most (what is left is at least 2^-15
+  // z): -64 is still above it.  Upwards 8192, where inf and NaN end too, would
+  // be no bound; but no other lanes bring such a lane's sum back below 4096, and
+  // a warp above that has no bound (the rates are far below those of real data),
+  // nor has the proposal then.
+  const int si = __reduce_add_sync(BBS_FULL_MASK, lane_bound(s));
+  const int gi = __reduce_add_sync(BBS_FULL_MASK, lane_bound(g));
+  constexpr int most = 4096 * (int)kBoundUnit;
+  up[0] += si < most ? (float)si : INFINITY;
+  up[1] += gi < most ? (float)gi : INFINITY;
 }
 
 }  // namespace bbs
