@@ -601,13 +601,21 @@ uint64_t fnv1a_of(uint64_t h, const T &v) {
   return fnv1a(h, &v, sizeof(T));
 }
 
-// Whether chains with rows of five to eight words may take a table
-// (plan_tables): the max score at fixed rates that have codes.
-bool wide_tables(const DatasetDev &ds, const ModelDev &md, const float *terms) {
-  return md.score_mode == 0 && md.mp.cum_beta == 0.0f &&
-         make_code_host(terms[2], terms[4], terms[3], terms[5], ds.max_d,
-                        ds.max_m)
-             .usable;
+// Whether max-score chains with rows of five to eight words, `load` of them per
+// SM, take a table (plan_tables): codes at fixed rates that decide every proposal,
+// and where those they leave open are not too dear to score from the rows.  300
+// steps, ms, with codes that tie somewhere and through the ring: 64, 256 and 800
+// chains at 150 x 100 3.0, 3.5, 10.2 and 4.7, 5.1, 5.8; 256 at 180 x 100 4.3, 5.8;
+// at 200 x 150 8.5 to 9.8, 5.7 (exact codes 1.9); 128 at 255 x 512 17 to 20, 8.3
+// (2.7).
+bool wide_tables(const DatasetDev &ds, const ModelDev &md, const float *terms,
+                 double load) {
+  if (md.score_mode != 0 || md.mp.cum_beta != 0.0f) return false;
+  const MaxCode k = make_code_host(terms[2], terms[4], terms[3], terms[5],
+                                   ds.max_d, ds.max_m);
+  const bool cheap =
+      load <= 2.0 && ds.n_nodes * ((ds.n_cells + 31) / 32) <= 750;
+  return k.usable && (k.exact || cheap);
 }
 
 // Device bytes of the global tables of a launch: its blocks are at most what
@@ -967,7 +975,9 @@ TablePlan chain_plan(const bbs_ctx *c, int q, int wpc, int cpb) {
   const int w32 = w32_of_nodes((int)c->n_nodes);
   return plan_tables((int)c->n_nodes, w32, (int)c->n_cells, q, wpc, cpb,
                      c->md.score_mode != 0, true,
-                     w32 > 4 && wide_tables(c->ds, c->md, c->terms),
+                     w32 > 4 && wide_tables(c->ds, c->md, c->terms,
+                                            (double)c->n_chains /
+                                                std::max(1, c->n_sms)),
                      c->smem_block, c->smem_sm);
 }
 
@@ -2231,7 +2241,9 @@ int batch_build_groups(bbs_batch *b) {
       if ((int)b->chain_ds[u] != g.only_ds) g.only_ds = -1;
     for (uint32_t d = 0; d < b->n_datasets && w > 4; d++)
       if (key[d] == w)
-        g.wide = g.wide && wide_tables(b->ds[d], b->md[d], &b->terms[8 * d]);
+        g.wide = g.wide && wide_tables(b->ds[d], b->md[d], &b->terms[8 * d],
+                                       (double)g.units.size() /
+                                           std::max(1, b->n_sms));
     BBS_CUDA(cudaMalloc(&g.d_units, sizeof(uint32_t) * g.units.size()), "cudaMalloc");
     BBS_CUDA(cudaMemcpy(g.d_units, g.units.data(), sizeof(uint32_t) * g.units.size(),
                         cudaMemcpyHostToDevice), "cudaMemcpy");

@@ -335,3 +335,58 @@ def test_parts_of_a_shape_are_accepted(native, G, Cn, chains, part):
                 c.run(20)
                 got.append(c.save_chains())
         assert got[0] == got[1]
+
+
+def _ms_a_run(native, mut, known, Cn, G, chains, steps, runs=1, launch=None,
+              **kw):
+    """Device time of `runs` runs of `steps` steps, the least of several."""
+    p = native.default_params(seed=5, **kw)
+    with native.Context(mut, known, Cn, G, p) as c:
+        c.init_chains(chains)
+        if launch:
+            c.set_launch(*launch)
+        c.run(500)
+        times = []
+        for _ in range(5):
+            t = 0.0
+            for _ in range(runs):
+                c.run(steps)
+                t += c.last_run_ms()
+            times.append(t)
+    return min(times)
+
+
+# rates whose codes tie at every sixth count: log(1 - alpha) - log(beta) is a
+# sixth of log(1 - beta) - log(alpha)
+TIES = dict(alpha_mean=0.000511870, beta_mean=0.3)
+
+
+@pytest.mark.gpu
+def test_wide_chains_with_codes_that_tie_cost_no_more_than_the_ring(native):
+    """255 x 512 at rates whose codes tie, against the same chains with error
+    moves that never come, which take the ring."""
+    mut, known = _setup(255, 512, 7)
+    ties = _ms_a_run(native, mut, known, 512, 255, 128, 100, **TIES)
+    ring = _ms_a_run(native, mut, known, 512, 255, 128, 100,
+                     prob_beta_change=1e-6, **TIES)
+    assert ties <= 1.3 * ring, (ties, ring)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("G,Cn,launch", [
+    (150, 100, (1, 4, 1)),   # codes, the proposals they leave from the rows
+    (200, 150, (2, 3, 1)),   # the ring
+])
+def test_wide_chains_with_codes_that_tie_equal_traced_ones(native, G, Cn,
+                                                           launch):
+    mut, known = _setup(G, Cn, 7)
+    p = native.default_params(seed=31, **TIES)
+    got = []
+    for trace in (False, True):
+        with native.Context(mut, known, Cn, G, p) as c:
+            c.init_chains(5)
+            c.set_launch(*launch)
+            for steps in (2, 60, 200):
+                c.run(steps, trace=trace)
+            got.append(c.save_chains())
+    assert got[0] == got[1]
