@@ -273,6 +273,7 @@ struct bbs_ctx {
   int *h_cancel = nullptr;        // mapped pinned flag
   int *d_cancel = nullptr;
   int q = 1, wpc = 1, cpb = 1;  // chain-kernel launch shape
+  Tables tables = Tables::codes;  // of max-score chains
   unsigned set = 0;             // which of them the caller set (kSet...)
   LaunchShape spread;           // the shape without tables (settle_launch)
   bool running = false;
@@ -601,21 +602,30 @@ uint64_t fnv1a_of(uint64_t h, const T &v) {
   return fnv1a(h, &v, sizeof(T));
 }
 
-// Whether max-score chains with rows of five to eight words, `load` of them per
-// SM, take a table (plan_tables): codes at fixed rates that decide every proposal,
-// and where those they leave open are not too dear to score from the rows.  300
-// steps, ms, with codes that tie somewhere and through the ring: 64, 256 and 800
-// chains at 150 x 100 3.0, 3.5, 10.2 and 4.7, 5.1, 5.8; 256 at 180 x 100 4.3, 5.8;
-// at 200 x 150 8.5 to 9.8, 5.7 (exact codes 1.9); 128 at 255 x 512 17 to 20, 8.3
-// (2.7).
-bool wide_tables(const DatasetDev &ds, const ModelDev &md, const float *terms,
+// What max-score chains read proposals off, `load` of them per SM.  With rows of
+// five to eight words: codes at fixed rates that decide every proposal, and where
+// those they leave open are not too dear to score from the rows.  300 steps, ms,
+// with codes that tie somewhere and through the ring: 64, 256 and 800 chains at
+// 150 x 100 3.0, 3.5, 10.2 and 4.7, 5.1, 5.8; 256 at 180 x 100 4.3, 5.8; at 200 x
+// 150 8.5 to 9.8, 5.7 (exact codes 1.9); 128 at 255 x 512 17 to 20, 8.3 (2.7).
+Tables tables_of(const DatasetDev &ds, const ModelDev &md, const float *terms,
                  double load) {
-  if (md.score_mode != 0 || md.mp.cum_beta != 0.0f) return false;
-  const MaxCode k = make_code_host(terms[2], terms[4], terms[3], terms[5],
-                                   ds.max_d, ds.max_m);
-  const bool cheap =
-      load <= 2.0 && ds.n_nodes * ((ds.n_cells + 31) / 32) <= 750;
-  return k.usable && (k.exact || cheap);
+  if (md.score_mode != 0) return Tables::none;
+  const float pb = md.mp.cum_beta;
+  const bool wide = ds.n_nodes > 128;
+  if (wide && pb != 0.0f) return Tables::none;
+  CodeQuality codes{true, true, 0, 1};
+  if (pb == 0.0f) {
+    const MaxCode k = make_code_host(terms[2], terms[4], terms[3], terms[5],
+                                     ds.max_d, ds.max_m);
+    codes = {k.usable, k.exact, k.ties,
+             std::max(1, std::min(ds.max_d, ds.max_m))};
+    const bool cheap = load <= 2.0 &&
+                       ds.n_nodes * ((ds.n_cells + 31) / 32) <= 750;
+    if (wide)
+      return k.usable && (k.exact || cheap) ? Tables::codes : Tables::none;
+  }
+  return max_score_tables(ds.n_nodes, ds.n_cells, load, pb, codes);
 }
 
 // Device bytes of the global tables of a launch: its blocks are at most what
@@ -971,14 +981,12 @@ int bbs_get_sizes(const bbs_ctx *c, uint32_t *n_cells, uint32_t *n_genes,
 
 namespace {
 
-TablePlan chain_plan(const bbs_ctx *c, int q, int wpc, int cpb) {
+TablePlan chain_plan(const bbs_ctx *c, int q, int wpc, int cpb,
+                     bool any = true) {
   const int w32 = w32_of_nodes((int)c->n_nodes);
   return plan_tables((int)c->n_nodes, w32, (int)c->n_cells, q, wpc, cpb,
                      c->md.score_mode != 0, true,
-                     w32 > 4 && wide_tables(c->ds, c->md, c->terms,
-                                            (double)c->n_chains /
-                                                std::max(1, c->n_sms)),
-                     c->smem_block, c->smem_sm);
+                     c->tables != Tables::none, c->smem_block, c->smem_sm, any);
 }
 
 // Shared memory a shape is accepted by: the plan's, and the slots' with the
@@ -1126,6 +1134,8 @@ void settle_launch(bbs_ctx *c, const LaunchShape &rest) {
 // New chains: the default shape.
 void reset_launch(bbs_ctx *c) {
   c->set = 0;
+  c->tables = tables_of(c->ds, c->md, c->terms,
+                        (double)c->n_chains / std::max(1, c->n_sms));
   c->spread = spread_launch(c, false);
   settle_launch(c, default_launch(c));
 }
@@ -1240,14 +1250,14 @@ int start_run(bbs_ctx *c, uint32_t n_steps, const bbs_raw_move *d_moves,
   {
     const int cpb = c->wpc > 1 ? 1 : c->cpb;
     TablePlan p = chain_plan(c, c->q, c->wpc, cpb);
-    // replays and traces of rows of five to eight words go through the ring
+    // replays and traces of rows of five to eight words go through the ring, and
+    // have no kernels for tables of counts
     const bool rec = d_moves != nullptr || d_trace != nullptr;
-    if ((rec && c->n_nodes > 128) ||
+    if ((rec && (c->n_nodes > 128 || c->tables == Tables::counts)) ||
         !c->table.reserve(table_bytes(p, cpb, c->n_chains, c->n_sms,
                                       c->smem_sm)))
-      p = TablePlan{0, false,
-                    chain_launch_smem((int)c->n_nodes, (int)c->n_cells, c->q,
-                                      c->wpc, cpb, c->md.score_mode != 0), 0, 0};
+      p = chain_plan(c, c->q, c->wpc, cpb, false);
+    a.by_counts = c->tables == Tables::counts ? 1 : 0;
     a.chunks = p.chunks;
     a.with_inc = p.inc ? 1 : 0;
     a.smem = p.smem;
@@ -2110,7 +2120,7 @@ struct bbs_batch {
   struct Group {
     int w32 = 0, max_nodes = 0, max_cells = 0;
     int only_ds = -1;  // the group's dataset when it has only one
-    bool wide = true;  // every dataset may take tables of wide rows
+    Tables tables = Tables::codes;  // of max-score chains
     std::vector<uint32_t> units;
     uint32_t *d_units = nullptr;
   };
@@ -2239,11 +2249,20 @@ int batch_build_groups(bbs_batch *b) {
     g.only_ds = (int)b->chain_ds[g.units[0]];
     for (const uint32_t u : g.units)
       if ((int)b->chain_ds[u] != g.only_ds) g.only_ds = -1;
-    for (uint32_t d = 0; d < b->n_datasets && w > 4; d++)
-      if (key[d] == w)
-        g.wide = g.wide && wide_tables(b->ds[d], b->md[d], &b->terms[8 * d],
-                                       (double)g.units.size() /
-                                           std::max(1, b->n_sms));
+    // rows of five to eight words: a table where it suits every dataset; else
+    // the choice of most (the kernels run the others too)
+    uint32_t votes[3] = {0, 0, 0}, datasets = 0;
+    const double load = (double)g.units.size() / std::max(1, b->n_sms);
+    for (uint32_t d = 0; d < b->n_datasets; d++) {
+      if (key[d] != w) continue;
+      datasets++;
+      votes[(int)tables_of(b->ds[d], b->md[d], &b->terms[8 * d], load)]++;
+    }
+    g.tables = 2 * votes[0] > datasets || (w > 4 && votes[0] > 0)
+                   ? Tables::none
+               : votes[(int)Tables::counts] > votes[(int)Tables::codes]
+                   ? Tables::counts
+                   : Tables::codes;
     BBS_CUDA(cudaMalloc(&g.d_units, sizeof(uint32_t) * g.units.size()), "cudaMalloc");
     BBS_CUDA(cudaMemcpy(g.d_units, g.units.data(), sizeof(uint32_t) * g.units.size(),
                         cudaMemcpyHostToDevice), "cudaMemcpy");
@@ -2292,10 +2311,12 @@ int group_wpb(const bbs_batch *b, const bbs_batch::Group &grp) {
   return std::min(b->wpb, chain_max_threads(group_q(b, grp)) / 32);
 }
 
-TablePlan group_plan(const bbs_batch *b, const bbs_batch::Group &grp) {
+TablePlan group_plan(const bbs_batch *b, const bbs_batch::Group &grp,
+                     bool any = true) {
   return plan_tables(grp.max_nodes, grp.w32, grp.max_cells, group_q(b, grp),
                      b->wpc, group_wpb(b, grp) / b->wpc, b->sum,
-                     grp.only_ds >= 0, grp.wide, b->smem_block, b->smem_sm);
+                     grp.only_ds >= 0, grp.tables != Tables::none,
+                     b->smem_block, b->smem_sm, any);
 }
 
 // The groups' global tables, one after the other in b->table; before a
@@ -2389,10 +2410,10 @@ int batch_issue(bbs_batch *b, uint32_t n_steps) {
                                              b->n_sms, b->smem_sm)
                                : 0;
     if (table_at + tb > b->table.cap)
-      p = TablePlan{0, false, chain_launch_smem(grp.max_nodes, grp.max_cells, q,
-                                                b->wpc, slots, b->sum), 0, 0};
+      p = group_plan(b, grp, false);
     a.chunks = p.chunks;
     a.with_inc = p.inc ? 1 : 0;
+    a.by_counts = grp.tables == Tables::counts ? 1 : 0;
     a.smem = p.smem;
     a.ns = p.ns;
     a.table = b->table.p + table_at / 4;

@@ -55,13 +55,14 @@ struct MaxCode {
   int P, Q, s, au, bu, off;
   uint32_t invP, invQ;  // floor(2^32 / P) + 1: quotients of x < 2^24
   float margin;
+  int ties;  // denominators up to dmax that come that close
   bool usable, exact;
 };
 
 // Neighbouring fractions al / bl < |c1| / |c2| < au / bu, found so far.
 struct Neighbours {
   int al = 0, bl = 1, au = 1, bu = 0;
-  bool exact = true;
+  int ties = 0;
   __host__ __device__ void below(int a, int b) {
     if (a * bl > al * b || (a * bl == al * b && b < bl)) {
       al = a;
@@ -80,7 +81,7 @@ struct Neighbours {
     int a = (int)fminf(floorf((float)b * (a1 / a2)), (float)mmax);
     const float x = (float)b * a1;
     if (a < mmax && (float)(a + 1) * a2 - x <= margin) a++;
-    exact = exact && fabsf(x - (float)a * a2) > margin;
+    ties += fabsf(x - (float)a * a2) > margin ? 0 : 1;
     below(a, b);
     if (a < mmax) above(a + 1, b);
   }
@@ -119,7 +120,8 @@ __host__ __device__ inline void code_end(MaxCode &k, const Neighbours &f,
   // neighbours in lowest terms; near-ties sorted inconsistently are not
   k.usable = k.usable && f.au * f.bl - f.al * f.bu == 1 &&
              k.P * dmax + k.Q * mmax <= 65535;
-  k.exact = k.exact && f.exact;
+  k.ties = f.ties;
+  k.exact = k.exact && f.ties == 0;
   k.invP = 0xFFFFFFFFu / (uint32_t)k.P + 1u;
   k.invQ = 0xFFFFFFFFu / (uint32_t)k.Q + 1u;
 }
@@ -144,7 +146,7 @@ inline __device__ __noinline__ MaxCode make_code(float l00, float l01,
     f.below(xa, xb);
     f.above(ya, yb);
   }
-  f.exact = __all_sync(BBS_FULL_MASK, f.exact);
+  f.ties = (int)__reduce_add_sync(BBS_FULL_MASK, (unsigned)f.ties);
   code_end(k, f, dmax, mmax);
   return k;
 }
@@ -649,6 +651,82 @@ __device__ __forceinline__ void scan_codes(const Table<W32, Q> &tab, int n,
       if (nv > 0) o = __vmaxu2(o, tv[c * NW + i] + dv[c].k[i]);
       if (nc > nv) o = __vmaxu2(o, tw[c * NW + i] + dw[c].k[i]);
     }
+}
+
+// The max score over a table of counts: lane sums of k and m at each cell's best
+// node by its reference-order score at the rates of L, the first in node order
+// (best_nodes); of the current tree or, with nc > 0 nodes in list, of the
+// proposal x, to whose counts the table goes and back.  For chains whose codes
+// do not exist, tie at many nodes or would be made anew too often; out of line,
+// as the others' steps need the room.
+template <int W32, int Q, int NW = kPackWords<Q>>
+__device__ __noinline__ int2 scan_counts(const Table<W32, Q> tab,
+                                         const DatasetDev *ds,
+                                         const LogTable L, int chunks, int wpc,
+                                         int wic, int lane,
+                                         const uint8_t *list, int nc, int nv,
+                                         const Delta x) {
+  const int n = ds->n_nodes;
+  const LogTable2 L2 = log_table2(L, ds->neg_zero);
+  int sk = 0, sm = 0;
+#pragma unroll 1
+  for (int c = 0; c < chunks; c++) {
+    const Table<W32, Q> tc = tab.chunk(c, n);
+    Packed<NW> dv, dw;
+    if (nc > 0) {
+      class_deltas<W32, Q>(tc, x, lane, dv, dw);
+      apply_classes<W32, Q>(tc, list, nc, nv, x, dv, dw, false, lane);
+    }
+    float best[Q];
+    uint32_t at[Q];  // the best node's entry
+    float2 pdb[Q], pmb[Q];
+    {
+      Cells<W32, Q> cb;
+      load_cells<W32, Q>(cb, *ds, 32 * (wpc * Q * c + wic), 32 * wpc, lane);
+      uint32_t k[NW];
+      tc.ld(0, lane, k);
+#pragma unroll
+      for (int q = 0; q < Q; q++) {
+        pdb[q] = dup2(cb.pdb[q]);
+        pmb[q] = dup2(cb.pmb[q]);
+        at[q] = k[q >> 1];
+        best[q] = pair_score_b(pack_d_biased(at[q], q), pack_m_biased(at[q], q),
+                               cb.pdb[q], cb.pmb[q], L.l00, L.l01, L.l10,
+                               L.l11);
+      }
+    }
+    // (past the end the last node again, whose score is not above itself)
+#pragma unroll 1
+    for (int j = 1; j < n; j += 2) {
+      uint32_t a[NW], b[NW];
+      tc.ld(j, lane, a);
+      tc.ld(min(j + 1, n - 1), lane, b);
+#pragma unroll
+      for (int q = 0; q < Q; q++) {
+        const uint32_t u = a[q >> 1], v = b[q >> 1];
+        const float2 s = pair_score_b2(
+            make_float2(pack_d_biased(u, q), pack_d_biased(v, q)),
+            make_float2(pack_m_biased(u, q), pack_m_biased(v, q)), pdb[q],
+            pmb[q], L2);
+        at[q] = s.x > best[q] ? u : at[q];
+        best[q] = s.x > best[q] ? s.x : best[q];
+        at[q] = s.y > best[q] ? v : at[q];
+        best[q] = s.y > best[q] ? s.y : best[q];
+      }
+    }
+#pragma unroll
+    for (int q = 0; q < Q; q++) {
+      const int d = (int)((at[q] >> (16 * (q & 1))) & 0xFFu),
+                m = (int)((at[q] >> (16 * (q & 1) + 8)) & 0xFFu);
+      sk += d + m;
+      sm += m;
+    }
+    if (nc > 0)
+      apply_classes<W32, Q>(tc, list, nc, nv, x, dv, dw, true, lane);
+  }
+  sk = (int)__reduce_add_sync(BBS_FULL_MASK, (uint32_t)sk);
+  sm = (int)__reduce_add_sync(BBS_FULL_MASK, (uint32_t)sm);
+  return make_int2(sk, sm);
 }
 
 // ------------------------------------------------------------------------

@@ -106,6 +106,7 @@ struct RunArgs {
   int *status;                // device status word (0 = ok, 1 = cancelled)
   int wpc;                    // warps per chain (cells split over them)
   int chunks;                 // table of every node (TablePlan); 0: none
+  int by_counts;              // 1: max-score tables hold counts, not codes
   int with_inc;               // 1: increment tables after the slots
   int smem;                   // dynamic shared memory of the plan
   int ns;                     // nodes of the table in shared memory
@@ -132,6 +133,7 @@ struct BatchArgs {
   int table_ds;              // the launch's only dataset, or -1
   int chunks;                // table of every node (TablePlan); 0: none
   int with_inc;              // 1: increment tables (one dataset only)
+  int by_counts;             // 1: max-score tables hold counts, not codes
   int smem;                  // dynamic shared memory of the plan
   int ns;                    // nodes of the table in shared memory
   uint32_t *table;           // the others' entries, per slot of the launch

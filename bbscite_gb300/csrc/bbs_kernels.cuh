@@ -520,7 +520,7 @@ __device__ __noinline__ void propose_tree_call(
 // Bound at 95 x 96 (1024 one-warp chains, 1.8 warps per scheduler) by the
 // latency of one step's serial chain -- draw, descendant sets, table loads,
 // reductions -- no longer by the node loop's instructions.
-template <int W32, int Q, bool SUM>
+template <int W32, int Q, bool SUM, bool COUNTS>
 __device__ __forceinline__ void run_chain_table(
     const DatasetDev &ds, const ModelDev &md, uint32_t chain_id,
     uint32_t *g, uint32_t *gbest, uint64_t *lhash, float *lbeta, int K,
@@ -530,6 +530,7 @@ __device__ __forceinline__ void run_chain_table(
     const SlotSum &ss, const Table<W32, Q> tab, int chunks, int wpc, int wic,
     int lane) {
   constexpr int NW = kPackWords<Q>;
+  constexpr bool CODES = !SUM && !COUNTS;
   const int n = ds.n_nodes;
   const bool multi = wpc > 1;
   const int stride = 32 * wpc, c0 = 32 * wic;
@@ -638,11 +639,11 @@ __device__ __forceinline__ void run_chain_table(
         tree_ok = parents_match_rows<W32>(cur, n, cpar, lane);
       }
       fresh_rows = fresh_table = false;
-      if constexpr (!SUM)
+      if constexpr (CODES)
         code = make_code(L.l00, L.l01, L.l10, L.l11, ds.max_d, ds.max_m, lane);
-      else
+      else if constexpr (SUM)
         tolerances();
-      if (!tree_ok || (!SUM && !code.usable)) continue;
+      if (!tree_ok || (CODES && !code.usable)) continue;
       from_table = SUM;
       order = cur;
     } else if (!err_move) {
@@ -651,7 +652,7 @@ __device__ __forceinline__ void run_chain_table(
         mp = realize_classes<W32>(cur, cpar, n, raw, lane, D.v, D.w, related,
                                   general, corr);
       }
-      if constexpr (!SUM) general = general || !code.usable;
+      if constexpr (CODES) general = general || !code.usable;
       if (general) {
         corr = 1.0f;
         const Realized R = realize_move<W32>(cur, n, beta, raw, lane, D.v, D.w);
@@ -685,7 +686,11 @@ __device__ __forceinline__ void run_chain_table(
     if (classes) {
       delta = move_classes<W32>(mp, related, D, C);
       nc = list_nodes<W32>(C, list, lane, nv);
-      if constexpr (!SUM) {
+      if constexpr (COUNTS) {
+        const int2 km = scan_counts<W32, Q>(tab, &ds, L, chunks, wpc, wic, lane,
+                                            list, nc, nv, delta);
+        ev = finish_max(ds, L, prior, km.x, km.y, wpc, wic, lane, part, i & 1);
+      } else if constexpr (CODES) {
         int sk = 0, sm = 0;
         // CH chunks of cells from chunk c on
         auto read_off = [&](auto CHT, int c) {
@@ -777,6 +782,12 @@ __device__ __forceinline__ void run_chain_table(
     } else if (SUM && err_move && tree_ok) {
       from_table = true;
       if (!ord_ok) order = cur;
+    } else if (COUNTS && err_move && tree_ok) {
+      if constexpr (COUNTS) {
+        const int2 km = scan_counts<W32, Q>(tab, &ds, PL, chunks, wpc, wic,
+                                            lane, list, 0, 0, delta);
+        ev = finish_max(ds, PL, pprior, km.x, km.y, wpc, wic, lane, part, i & 1);
+      }
     } else if (!fresh) {
       from_rows = true;
     }
@@ -799,8 +810,8 @@ __device__ __forceinline__ void run_chain_table(
       canonical_order<W32>(order, n, fresh ? cpar : nullptr, ss.sx.ord,
                            ss.sx.hist, lane);
     if (fresh) {
-      const int off = SUM ? 0 : code.off, wd = SUM ? 1 : -code.s * code.P,
-                wm = SUM ? 256 : code.s * code.Q;
+      const int off = CODES ? code.off : 0, wd = CODES ? -code.s * code.P : 1,
+                wm = CODES ? code.s * code.Q : 256;
       if (ss.sx.inc != nullptr)
         fill_table_inherit<Q>(ss.sx, n, lane, off, wd, wm);
       else
@@ -927,13 +938,14 @@ __device__ __forceinline__ void run_chain_table(
           if constexpr (!SUM) {
             for (int c = 0; c < chunks; c++) {
               const Table<W32, Q> tc = tab.chunk(c, n);
-              if (chunks > 1) class_deltas<W32, Q>(tc, delta, lane, dv, dw);
+              if (COUNTS || chunks > 1)
+                class_deltas<W32, Q>(tc, delta, lane, dv, dw);
               apply_classes<W32, Q>(tc, list, nc, nv, delta, dv, dw, false,
                                     lane);
             }
           } else {
             cs = pcs;
-                ord_ok = true;
+            ord_ok = true;
           }
 #ifdef BBS_CHECKED
           device_check(parents_match_rows<W32>(cur, n, cpar, lane), status,
@@ -945,9 +957,9 @@ __device__ __forceinline__ void run_chain_table(
       } else if (tree_ok) {
         if constexpr (SUM) {
           cs = pcs;
-            tolerances();
+          tolerances();
         } else {
-          fresh_table = true;
+          fresh_table = CODES;
         }
       }
     } else if (applied) {
@@ -1004,20 +1016,21 @@ __device__ __forceinline__ Table<W32, Q> wide_table(uint8_t *slot_base, int n,
 }
 
 // Launch bounds of each variant (bbs_layout.h).
-template <int W32, int Q, bool TAB>
+template <int W32, int Q, int TAB>
 struct ChainBounds {
   static constexpr int threads = chain_max_threads(Q);
-  static constexpr int min_blocks = chain_blocks(W32, Q, TAB);
+  static constexpr int min_blocks = chain_blocks(W32, Q, TAB != 0);
 };
 
 // One dataset: chains 0..n_chains-1, one warp per chain (blocks of `cpb`
 // chains) or wpc warps per chain (the block is one chain).  REC: recorded
 // moves and/or a step trace (replays and tests); without them the move and
 // trace paths compile away.
-// TAB: proposals are read off a table (a.chunks > 0), else every node is
-// evaluated; kernels of their own, so that neither carries the other's code
-// and registers.
-template <int W32, int Q, bool SUM, bool REC, bool TAB>
+// TAB: 1 or 2, proposals are read off a table (a.chunks > 0), of counts for 2;
+// 0, every node is evaluated.  Kernels of their own, so that none carries
+// another's code and registers (with codes and counts in one, 20 x 24 took 11 %
+// longer and 63 x 64 4 %).
+template <int W32, int Q, bool SUM, bool REC, int TAB>
 __global__ void __launch_bounds__((ChainBounds<W32, Q, TAB>::threads),
                                   (ChainBounds<W32, Q, TAB>::min_blocks))
     mcmc_kernel(const RunArgs a) {
@@ -1031,12 +1044,12 @@ __global__ void __launch_bounds__((ChainBounds<W32, Q, TAB>::threads),
   const int slot = wib / wpc, wic = wib - slot * wpc;
   const int n = a.ds.n_nodes;
   // the launcher's plan, for the whole block
-  const bool inc = a.with_inc != 0, ring = W32 > 4 && !TAB;
-  constexpr bool wide = W32 > 4 && TAB;
-  constexpr bool scratch = SUM || W32 > 4 || TAB;
+  const bool inc = a.with_inc != 0, ring = W32 > 4 && TAB == 0;
+  constexpr bool wide = W32 > 4 && TAB != 0;
+  constexpr bool scratch = SUM || W32 > 4 || TAB != 0;
   const int sb =
       wide ? wide_slot_bytes(n, RS, wpc, W32, Q, a.chunks, a.ns)
-      : TAB && !inc ? table_slot_bytes(n, RS, wpc, W32, Q, a.chunks)
+      : TAB != 0 && !inc ? table_slot_bytes(n, RS, wpc, W32, Q, a.chunks)
                     : slot_bytes(n, RS, wpc, scratch, W32, Q, inc || ring);
   uint8_t *slot_base = reinterpret_cast<uint8_t *>(smem) + (size_t)slot * sb;
   uint32_t *buf0 = reinterpret_cast<uint32_t *>(slot_base);
@@ -1048,7 +1061,7 @@ __global__ void __launch_bounds__((ChainBounds<W32, Q, TAB>::threads),
   SlotSum ss{};
   if (scratch) ss = slot_sum(slot_base, n, RS, wpc, wic, W32, Q, inc || ring);
   Table<W32, Q> tab{};
-  if constexpr (TAB) {
+  if constexpr (TAB != 0) {
     if constexpr (wide) {
       tab = wide_table<W32, Q>(slot_base, n, RS, wpc, wic, a.chunks, a.ns,
                                a.table, blockIdx.x * cpb + slot);
@@ -1078,8 +1091,8 @@ __global__ void __launch_bounds__((ChainBounds<W32, Q, TAB>::threads),
     uint32_t *best = a.best_rows + (size_t)chain * K * n * RS;
     uint64_t *lhash = K > 1 ? a.list_hash + (size_t)chain * K : nullptr;
     float *lbeta = K > 1 ? a.list_beta + (size_t)chain * K : nullptr;
-    if constexpr (TAB)
-      run_chain_table<W32, Q, SUM>(
+    if constexpr (TAB != 0)
+      run_chain_table<W32, Q, SUM, TAB == 2>(
           a.ds, a.md, (uint32_t)chain, rows, best, lhash, lbeta, K,
           a.states + chain, moves, trace, a.n_steps, a.cancel, a.status, buf0,
           buf1, part, sflag, pbuf, ss, tab, a.chunks, wpc, wic, lane);
@@ -1093,7 +1106,7 @@ __global__ void __launch_bounds__((ChainBounds<W32, Q, TAB>::threads),
 
 // One work unit of the batched launch: chain `chain` of dataset `d`, run
 // by the wpc warps of its slot (warp wic of them).
-template <int W32, int Q, bool SUM, bool TAB>
+template <int W32, int Q, bool SUM, int TAB>
 __device__ __forceinline__ void batch_unit(const BatchArgs &b,
                                            const DatasetDev &ds,
                                            const ModelDev &md, uint32_t chain,
@@ -1109,13 +1122,13 @@ __device__ __forceinline__ void batch_unit(const BatchArgs &b,
   // Philox key: the chain's number within its dataset, so a dataset's
   // chains draw the same moves here as in a one-dataset run.
   const uint32_t local = chain - d * (uint32_t)b.chains_per_dataset;
-  if constexpr (TAB) {
+  if constexpr (TAB != 0) {
     // (this dataset's chunks and nodes: a launch's largest dataset sizes the
     // slots)
     const int span = 32 * wpc * Q;
     Table<W32, Q> tab = slot_tab;
     tab.ns = min(tab.ns, ds.n_nodes);
-    run_chain_table<W32, Q, SUM>(
+    run_chain_table<W32, Q, SUM, TAB == 2>(
         ds, md, local, b.rows + off, b.best_rows + off, nullptr, nullptr, 1,
         b.states + chain, nullptr, nullptr, b.n_steps, b.cancel, b.status, buf0,
         buf1, part, sflag, pbuf, ss, tab, (ds.n_cells + span - 1) / span, wpc,
@@ -1134,7 +1147,7 @@ __device__ __forceinline__ void batch_unit(const BatchArgs &b,
 // slot and takes its chains together).
 // MULTI: chains of b.wpc > 1 warps; without it every chain is one warp,
 // known at compile time.
-template <int W32, int Q, bool SUM, bool MULTI, bool TAB>
+template <int W32, int Q, bool SUM, bool MULTI, int TAB>
 __global__ void __launch_bounds__((ChainBounds<W32, Q, TAB>::threads),
                                   (W32 > 4 ? 1
                                            : ChainBounds<W32, Q, TAB>::min_blocks))
@@ -1146,12 +1159,12 @@ __global__ void __launch_bounds__((ChainBounds<W32, Q, TAB>::threads),
   const int wpc = MULTI ? b.wpc : 1;
   const int slot = wib / wpc, wic = wib - slot * wpc;
   // the host's plan, the same in every thread
-  const bool inc = b.with_inc != 0, ring = W32 > 4 && !TAB;
-  constexpr bool wide = W32 > 4 && TAB;
-  constexpr bool scratch = SUM || W32 > 4 || TAB;
+  const bool inc = b.with_inc != 0, ring = W32 > 4 && TAB == 0;
+  constexpr bool wide = W32 > 4 && TAB != 0;
+  constexpr bool scratch = SUM || W32 > 4 || TAB != 0;
   const int sb =
       wide ? wide_slot_bytes(b.max_nodes, RS, wpc, W32, Q, b.chunks, b.ns)
-      : TAB && !inc
+      : TAB != 0 && !inc
           ? table_slot_bytes(b.max_nodes, RS, wpc, W32, Q, b.chunks)
           : slot_bytes(b.max_nodes, RS, wpc, scratch, W32, Q, inc || ring);
   uint8_t *slot_base = reinterpret_cast<uint8_t *>(smem) + (size_t)slot * sb;
@@ -1168,7 +1181,7 @@ __global__ void __launch_bounds__((ChainBounds<W32, Q, TAB>::threads),
   if (scratch)
     ss = slot_sum(slot_base, b.max_nodes, RS, wpc, wic, W32, Q, inc || ring);
   Table<W32, Q> tab{};
-  if constexpr (TAB) {
+  if constexpr (TAB != 0) {
     if constexpr (wide) {
       tab = wide_table<W32, Q>(
           slot_base, b.max_nodes, RS, wpc, wic, b.chunks, b.ns, b.table,

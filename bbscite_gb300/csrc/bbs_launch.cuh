@@ -32,7 +32,7 @@ inline cudaError_t prepare_smem(K kernel, size_t smem) {
 // Persistent launch.  wpc == 1: blocks of `cpb` one-warp chains; wpc > 1:
 // blocks of one chain of wpc warps.  As many blocks as chains need, capped
 // at what stays resident; each block then walks its chain slots.
-template <int W32, int Q, bool SUM, bool REC, bool TAB>
+template <int W32, int Q, bool SUM, bool REC, int TAB>
 int launch_mcmc_k(const RunArgs &a, int cpb, int n_sms, cudaStream_t s) {
   if (a.wpc > 1) cpb = 1;
   const int threads = 32 * a.wpc * cpb;
@@ -56,15 +56,19 @@ int launch_mcmc_t(const RunArgs &a, int cpb, int n_sms, cudaStream_t s) {
   // (rows of five to eight words replay and trace through the ring)
   // (and the sum score keeps it)
   if constexpr (W32 <= 4 || (!REC && !SUM))
-    if (a.chunks > 0)
-      return launch_mcmc_k<W32, Q, SUM, REC, true>(a, cpb, n_sms, s);
-  return launch_mcmc_k<W32, Q, SUM, REC, false>(a, cpb, n_sms, s);
+    if (a.chunks > 0) {
+      if constexpr (W32 <= 4 && !REC && !SUM)
+        if (a.by_counts)
+          return launch_mcmc_k<W32, Q, SUM, REC, 2>(a, cpb, n_sms, s);
+      return launch_mcmc_k<W32, Q, SUM, REC, 1>(a, cpb, n_sms, s);
+    }
+  return launch_mcmc_k<W32, Q, SUM, REC, 0>(a, cpb, n_sms, s);
 }
 
 // Work-list launch: enough resident slots to fill the GPU, never more than
 // there are units.  Blocks of wpb one-warp slots (b.wpc == 1), or of one
 // slot of wpb == b.wpc warps.
-template <int W32, int Q, bool SUM, bool MULTI, bool TAB>
+template <int W32, int Q, bool SUM, bool MULTI, int TAB>
 int launch_batch_k(const BatchArgs &b, int wpb, int n_sms, cudaStream_t s) {
   const int threads = 32 * wpb;
   if (threads > chain_max_threads(Q)) return (int)cudaErrorInvalidConfiguration;
@@ -89,9 +93,13 @@ int launch_batch_k(const BatchArgs &b, int wpb, int n_sms, cudaStream_t s) {
 template <int W32, int Q, bool SUM, bool MULTI>
 int launch_batch_t(const BatchArgs &b, int wpb, int n_sms, cudaStream_t s) {
   if constexpr (W32 <= 4 || !SUM)
-    if (b.chunks > 0)
-      return launch_batch_k<W32, Q, SUM, MULTI, true>(b, wpb, n_sms, s);
-  return launch_batch_k<W32, Q, SUM, MULTI, false>(b, wpb, n_sms, s);
+    if (b.chunks > 0) {
+      if constexpr (W32 <= 4 && !SUM)
+        if (b.by_counts)
+          return launch_batch_k<W32, Q, SUM, MULTI, 2>(b, wpb, n_sms, s);
+      return launch_batch_k<W32, Q, SUM, MULTI, 1>(b, wpb, n_sms, s);
+    }
+  return launch_batch_k<W32, Q, SUM, MULTI, 0>(b, wpb, n_sms, s);
 }
 
 // One unit per row width: launches with recorded moves or a trace (REC) or

@@ -2,6 +2,8 @@
 // kernels carve their dynamic shared memory by and the host launchers
 // request (host and device code).
 #pragma once
+#include <algorithm>
+
 #include "bbs_internal.h"
 
 namespace bbs {
@@ -154,6 +156,43 @@ __host__ __device__ inline int wide_slot_bytes(int n, int rs, int wpc, int w32,
 
 inline constexpr int kFewCells = 12;
 
+// What the chains of a launch read proposals off.
+enum class Tables { none, codes, counts };
+
+// The choice for max-score chains of up to 128 nodes: `load` chains per SM, error
+// moves a share pb of all, the rates' codes (where pb is 0).
+//   none    Few nodes and cells: an evaluation from the rows costs less than
+//           following the table does, the more so the more often rates change,
+//           which makes codes and table anew, and the more chains share an SM.
+//   counts  Otherwise, where rates change so often that codes do not pay, and at
+//           fixed rates without codes or with codes that leave many proposals to
+//           an evaluation from the rows: the table holds counts, and a proposal
+//           scores every node from them.
+//   codes   The rest.
+// A step, us, by rows / codes / counts, error moves 1 in 11 (Langevin): 2432 chains
+// of 8 x 24 2.0 / 6.0 / 4.9, 1216 of 32 x 64 4.3 / 4.8 / 4.5, 608 of 95 x 96
+// 10.5 / 5.8 / 8.2; 1 in 2: 608 of 95 x 96 10.8 / 12.1 / 8.4.  Over 4 to 127
+// genes, 8 to 256 cells, 8 to 2432 chains and none to half of the moves the choice
+// took 1 % longer than the best of the three; codes alone, 26 %.
+struct CodeQuality {
+  bool usable, exact;
+  int ties, most;  // of the denominators that tie, and how many could
+};
+inline Tables max_score_tables(int n, int n_cells, double load, float pb,
+                               const CodeQuality &codes) {
+  const int work = n * ((n_cells + 31) / 32);
+  const bool poor = pb == 0.0f && (!codes.usable || 3 * codes.ties >= codes.most);
+  const double crowd = 1.0 + std::min(load, 8.0) / 4.0;
+  if (work <= (poor ? 112.0 : std::min(112.0, (5.0 + 270.0 * pb) * crowd)))
+    return Tables::none;
+  if (poor || (pb == 0.0f && !codes.exact && (n > 64 || work > 192)))
+    return Tables::counts;
+  const float often = load < 1.0 || (n_cells > 128 && n >= 64) ? 0.4f
+                      : load >= 4.0 && n <= 64 && n_cells <= 128 ? 0.12f
+                                                                 : 0.2f;
+  return pb > often ? Tables::counts : Tables::codes;
+}
+
 // The plan of a launch of `slots` chain slots per block, its largest dataset
 // of n nodes and n_cells cells.  Where the tables do not fit a block, or a
 // sum-score chain's cells of rows of up to four words do not fit one chunk,
@@ -165,23 +204,23 @@ inline constexpr int kFewCells = 12;
 // Langevin chains, every node and table: 8 x 4 2.28, 3.54 ms; 8 x 9 2.27, 3.07;
 // 20 x 9 2.83, 3.48; 8 x 16 2.28, 2.57; at fixed rates 8 x 9 2.12, 1.80; 20 x 9
 // 2.70, 2.28; 8 x 16 2.12, 1.54.  From 33 nodes on the table is no slower).
-// Rows of five to eight words take a table when `wide`: max-score chains at
-// fixed rates that have codes (after a change of rates the table would have to
-// be made again).  It is in shared memory where that leaves an SM four warps;
-// else one chain per SM keeps as many nodes there as fit (255 x 512: 216 of
-// 256), the others in global memory.  The sum score keeps the ring: half of
-// its proposals are accepted in the runs measured (255 x 512) and then summed
+// Max-score chains take one where `max_table` says so.  With rows of five to
+// eight words it is in shared memory where that leaves an SM four warps; else
+// one chain per SM keeps as many nodes there as fit (255 x 512: 216 of 256),
+// the others in global memory.  The sum score keeps the ring at that width: half
+// of its proposals are accepted in the runs measured (255 x 512) and then summed
 // over every node, which with a table was slower (200 x 150: 17 M against
 // 22 M chain-steps/s).
 inline TablePlan plan_tables(int n, int w32, int n_cells, int q, int wpc,
-                             int slots, bool sum, bool one_dataset, bool wide,
-                             int smem_block, int smem_sm) {
+                             int slots, bool sum, bool one_dataset,
+                             bool max_table, int smem_block, int smem_sm,
+                             bool any_table = true) {
   const int rs = rs_of_w32(w32), span = 32 * wpc * q;
   const int chunks = (n_cells + span - 1) / span;
   if (w32 > 4) {
     const TablePlan ring{0, false,
                          chain_launch_smem(n, n_cells, q, wpc, slots, sum), 0, 0};
-    if (!wide || sum) return ring;
+    if (!max_table || sum || !any_table) return ring;
     auto smem_of = [&](int ns) {
       return slots * wide_slot_bytes(n, rs, wpc, w32, q, chunks, ns);
     };
@@ -198,7 +237,9 @@ inline TablePlan plan_tables(int n, int w32, int n_cells, int q, int wpc,
   }
   const TablePlan p{0, false, slots * slot_bytes(n, rs, wpc, sum, w32, q, false),
                     n, 0};
-  if (sum && (chunks > 1 || (w32 == 1 && n_cells <= kFewCells))) return p;
+  if (!any_table ||
+      (sum ? chunks > 1 || (w32 == 1 && n_cells <= kFewCells) : !max_table))
+    return p;
   const bool inc = wpc == 1 && one_dataset && chunks == 1;
   const int smem =
       inc ? chain_launch_smem(n, n_cells, q, wpc, slots, sum)

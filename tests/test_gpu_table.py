@@ -390,3 +390,79 @@ def test_wide_chains_with_codes_that_tie_equal_traced_ones(native, G, Cn,
                 c.run(steps, trace=trace)
             got.append(c.save_chains())
     assert got[0] == got[1]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("share", [0.0, 1.0, 50.0])
+@pytest.mark.parametrize("move", ["beta_walk", "langevin"])
+@pytest.mark.parametrize("G,Cn,launch", [
+    (127, 33, (1, 2, 1)),    # the most nodes, a last cell of its own
+    (126, 64, (2, 1, 2)),    # an odd number of nodes
+    (95, 97, (2, 1, 1)),     # two chunks, the last of one cell
+    (63, 200, (1, 2, 1)),    # four chunks
+    (112, 128, (1, 4, 1)),   # four warps
+])
+def test_chains_on_tables_of_counts_equal_traced_ones(native, share, move, G,
+                                                      Cn, launch):
+    """Error moves as many as tree moves and fifty times as many, and none at
+    rates without codes: tables of counts against evaluations from the rows."""
+    mut, known = _setup(G, Cn, 5)
+    p = native.default_params(
+        alpha_mean=1e-2 if share else 0.5, beta_mean=0.3 if share else 0.5,
+        seed=29, prob_beta_change=share,
+        error_move=getattr(native, "ERROR_" + move.upper()))
+    got = []
+    for trace in (False, True):
+        with native.Context(mut, known, Cn, G, p) as c:
+            c.init_chains(8)
+            c.set_launch(*launch)
+            for steps in (3, 37, 300):
+                c.run(steps, trace=trace)
+            got.append(c.save_chains())
+    assert got[0] == got[1]
+
+
+@pytest.mark.gpu
+def test_mixed_batches_on_tables_of_counts_equal_their_datasets_alone(native):
+    """A launch group most of whose datasets are better off with counts runs
+    the others on counts too."""
+    sizes = [(100, 90), (120, 64), (127, 200), (97, 40)]
+    data = [_setup(G, Cn, 9 + i) + (Cn, G) for i, (G, Cn) in enumerate(sizes)]
+    params = [native.default_params(alpha_mean=1e-2, beta_mean=0.3,
+                                    prob_beta_change=0.1 if i == 1 else 2.0,
+                                    error_move=native.ERROR_RANDOM_WALK,
+                                    seed=70 + i) for i in range(len(sizes))]
+    with native.Batch(data, params) as b:
+        b.init_chains(5)
+        b.run(150)
+        best = [b.best(d) for d in range(len(sizes))]
+    for d, (G, Cn) in enumerate(sizes):
+        with native.Context(*data[d], params[d]) as c:
+            c.init_chains(5)
+            c.set_launch(1, 1, 1)
+            c.run(150)
+            one, alpha = c.best(), c.best_alpha()
+        assert alpha == best[d]["alpha"]
+        for k in ("score", "beta"):
+            assert one[k] == best[d][k]
+        assert (one["dm"] == best[d]["dm"]).all()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("G,Cn,chains,launch,share,most", [
+    # many small chains: a step with one error move in eleven, and without
+    (8, 24, 2432, None, 0.1, 1.5),
+    # error moves as many as tree moves
+    (95, 96, 1024, (3, 1, 7), 1.0, 4.8),
+])
+def test_error_moves_cost_what_they_should(native, G, Cn, chains, launch, share,
+                                           most):
+    """Against the same chains at fixed rates."""
+    mut, known = _setup(G, Cn, 5)
+    kw = dict(alpha_mean=1e-2, beta_mean=0.2)
+    fixed = _ms_a_run(native, mut, known, Cn, G, chains, 200, launch=launch,
+                      **kw)
+    moved = _ms_a_run(native, mut, known, Cn, G, chains, 200, launch=launch,
+                      prob_beta_change=share,
+                      error_move=native.ERROR_LANGEVIN, **kw)
+    assert moved <= most * fixed, (moved, fixed)
