@@ -628,6 +628,18 @@ Tables tables_of(const DatasetDev &ds, const ModelDev &md, const float *terms,
   return max_score_tables(ds.n_nodes, ds.n_cells, load, pb, codes);
 }
 
+// Runs of so few steps that making a table costs more than it saves.  One step of
+// 1024 chains at 95 x 96, batched: max score 61 us with a table, 31 without, sum
+// score 56 and 29; two steps 67 and 53, 65 and 47, but with a table filled from
+// the block's increments max-score chains gain from the second on (one context,
+// 35 and 46).  Rows of five to eight words, 1, 2 and 4 steps of 128 chains at 255 x
+// 512 133, 146 and 166 us, through the ring 61, 88 and 143; of 256 at 200 x 150,
+// all in shared memory, 72, 79 and 94, through the ring 45, 64 and 101.
+bool too_few_steps(uint32_t steps, int w32, const TablePlan &p, bool sum) {
+  const uint32_t few = w32 > 4 ? (p.global ? 6 : 3) : !sum && p.inc ? 1 : 2;
+  return p.chunks > 0 && steps <= few;
+}
+
 // Device bytes of the global tables of a launch: its blocks are at most what
 // the chains need and what is resident.
 size_t table_bytes(const TablePlan &p, int slots, size_t n_chains, int n_sms,
@@ -1253,7 +1265,9 @@ int start_run(bbs_ctx *c, uint32_t n_steps, const bbs_raw_move *d_moves,
     // replays and traces of rows of five to eight words go through the ring, and
     // have no kernels for tables of counts
     const bool rec = d_moves != nullptr || d_trace != nullptr;
-    if ((rec && (c->n_nodes > 128 || c->tables == Tables::counts)) ||
+    if (too_few_steps(n_steps, w32_of_nodes((int)c->n_nodes), p,
+                      c->md.score_mode != 0) ||
+        (rec && (c->n_nodes > 128 || c->tables == Tables::counts)) ||
         !c->table.reserve(table_bytes(p, cpb, c->n_chains, c->n_sms,
                                       c->smem_sm)))
       p = chain_plan(c, c->q, c->wpc, cpb, false);
@@ -2409,7 +2423,7 @@ int batch_issue(bbs_batch *b, uint32_t n_steps) {
     const size_t tb = p.global ? table_bytes(p, slots, grp.units.size(),
                                              b->n_sms, b->smem_sm)
                                : 0;
-    if (table_at + tb > b->table.cap)
+    if (table_at + tb > b->table.cap || too_few_steps(n_steps, grp.w32, p, b->sum))
       p = group_plan(b, grp, false);
     a.chunks = p.chunks;
     a.with_inc = p.inc ? 1 : 0;

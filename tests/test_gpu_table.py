@@ -466,3 +466,36 @@ def test_error_moves_cost_what_they_should(native, G, Cn, chains, launch, share,
                       prob_beta_change=share,
                       error_move=native.ERROR_LANGEVIN, **kw)
     assert moved <= most * fixed, (moved, fixed)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("steps,most", [(1, 1.4), (4, 1.2)])
+def test_short_runs_make_no_table_for_a_few_steps(native, steps, most):
+    """Runs of a few steps at 255 x 512, against chains that take the ring."""
+    mut, known = _setup(255, 512, 7)
+    kw = dict(alpha_mean=1e-3, beta_mean=0.2)
+    table = _ms_a_run(native, mut, known, 512, 255, 128, steps, 40, **kw)
+    ring = _ms_a_run(native, mut, known, 512, 255, 128, steps, 40,
+                     prob_beta_change=1e-6, **kw)
+    assert table <= most * ring, (table, ring)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("score", ["max", "sum"])
+@pytest.mark.parametrize("G,Cn,launch", [(63, 64, (2, 1, 2)), (95, 97, (2, 1, 1)),
+                                         (200, 40, (2, 1, 1)),
+                                         (255, 512, (2, 4, 1))])
+def test_short_runs_equal_one_long_one(native, score, G, Cn, launch):
+    mut, known = _setup(G, Cn, 5)
+    p = native.default_params(alpha_mean=1e-3, beta_mean=0.2, seed=29,
+                              score_mode=getattr(native,
+                                                 "SCORE_" + score.upper()))
+    got = []
+    for runs in ([36], [1, 2, 3, 4, 6, 7, 13]):
+        with native.Context(mut, known, Cn, G, p) as c:
+            c.init_chains(6)
+            c.set_launch(*launch)
+            for steps in runs:
+                c.run(steps)
+            got.append(c.save_chains())
+    assert got[0] == got[1]
