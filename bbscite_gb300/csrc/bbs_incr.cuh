@@ -7,7 +7,9 @@
 // reads a proposal off it:
 //   - max score: the table holds integer codes that order a cell's nodes as
 //     their scores do (MaxCode), 16 bits per cell; a proposal's best nodes
-//     are the maxima over the unchanged nodes and the two shifted classes;
+//     are the maxima over the unchanged nodes and the two shifted classes.
+//     Where rates change often, or have no codes, it holds the counts, and a
+//     proposal scores every node from them (scan_counts);
 //   - sum score (rows of up to four words): the table holds the counts.  A
 //     proposal is first bounded from above by the terms that move (two
 //     exponentials per class and cell); only one that the bound does not
@@ -653,9 +655,9 @@ __device__ __forceinline__ void scan_codes(const Table<W32, Q> &tab, int n,
     }
 }
 
-// The max score over a table of counts: lane sums of k and m at each cell's best
-// node by its reference-order score at the rates of L, the first in node order
-// (best_nodes); of the current tree or, with nc > 0 nodes in list, of the
+// The max score over a table of counts: lane sums of k and m at each cell's
+// best node by its reference-order score at the rates of L, the first in node
+// order (best_nodes); of the current tree or, with nc > 0 nodes in list, of the
 // proposal x, to whose counts the table goes and back.  For chains whose codes
 // do not exist, tie at many nodes or would be made anew too often; out of line,
 // as the others' steps need the room.
@@ -732,6 +734,10 @@ __device__ __noinline__ int2 scan_counts(const Table<W32, Q> tab,
 // ------------------------------------------------------------------------
 // Sum score
 // ------------------------------------------------------------------------
+// Terms below 2^-126 are flushed to zero: 2^-118 is above 128 of them and as
+// much again.
+inline constexpr float kFlushed = 3.0092655e-36f;
+
 // What the bound keeps of the current tree, for the lane's Q cells: the
 // exponents' offset, the sum of the terms and its reciprocal, and the
 // largest exponent (all against the reference the sum was taken against).
@@ -780,9 +786,9 @@ __device__ __noinline__ Resum1 resum_slot_table(const Table<W32, Q> tab,
 // aligned and followed by three zeros (slot_sum).
 template <int W32, int Q>
 __device__ __forceinline__ void sum_cells_table(
-    const Table<W32, Q> &tab, const uint16_t *ord, int n, const float (&pd)[Q], const float (&pm)[Q], const LogTable &L,
-    int c0, int stride, int lane, int n_cells, long long (&acc)[6],
-    CellSums<Q> &cs) {
+    const Table<W32, Q> &tab, const uint16_t *ord, int n, const float (&pd)[Q],
+    const float (&pm)[Q], const LogTable &L, int c0, int stride, int lane,
+    int n_cells, long long (&acc)[6], CellSums<Q> &cs) {
   constexpr int NW = kPackWords<Q>;
   const float c1 = (L.l01 - L.l00) * kLog2E;
   const float c2 = (L.l11 - L.l10) * kLog2E;
@@ -945,23 +951,23 @@ __device__ __forceinline__ float entry_shift(const uint32_t (&a)[NW],
 }
 
 inline constexpr float kBoundUnit = 4096.0f;  // 2^-12 of a base-2 log
-inline constexpr float kFlushed = 3.0092655e-36f;  // 2^-118: 128 terms of 2^-126
-                                                   // and as much again
 
+// A lane's sum as an integer not below it, in units of 1 / kBoundUnit; 8192,
+// where inf and NaN end too, for a larger one.
 __device__ __forceinline__ int lane_bound(float s) {
-  return __float2int_ru((s < 8192.0f ? fmaxf(s, -64.0f) : 8192.0f) * kBoundUnit) + 1;
+  s = s < 8192.0f ? fmaxf(s, -64.0f) : 8192.0f;
+  return __float2int_ru(s * kBoundUnit) + 1;
 }
 
 // Adds upper bounds of a proposal's sum score and max score over one chunk of
-// this warp's cells, relative to the current tree, to up: up[0] bounds sum_c log2(z'_c / z_c),
-// up[1] bounds sum_c (largest exponent' - largest exponent), in units of
-// 1 / kBoundUnit.  eps bounds the relative rounding of a term against its
-// shifted form.  Sums of up to 128 terms are good to 2^-17 of the largest
-// partial sum, so a cell's remainder z - zo is taken with 2^-15 z on top.
-// Terms below 2^-126 were flushed to zero, in zo and in z; kFlushed covers them,
-// for the nodes that move and for those that stay: where a cell's best node
-// moves far away, the exact sum takes the others against their own maximum and
-// counts them again.
+// this warp's cells, relative to the current tree, to up: up[0] bounds sum_c
+// log2(z'_c / z_c), up[1] bounds sum_c (largest exponent' - largest exponent),
+// in units of 1 / kBoundUnit.  eps bounds the relative rounding of a term
+// against its shifted form.  Sums of up to 128 terms are good to 2^-17 of the
+// largest partial sum, so a cell's remainder z - zo is taken with 2^-15 z on
+// top.  kFlushed, on zo and on z, covers the flushed terms of the nodes that
+// move and of those that stay: where a cell's best node moves far away, the
+// exact sum takes the others against their own maximum and counts them again.
 template <int W32, int Q, int NW = kPackWords<Q>>
 __device__ __forceinline__ void bound_proposal(
     const Table<W32, Q> &tab, const Delta &x, const uint8_t *list, int nv, int nc,
@@ -986,7 +992,7 @@ __device__ __forceinline__ void bound_proposal(
       }
       z1[q] = 0.0f;
       gain[q] = -INFINITY;
-      rest[q] = cs.z[q];
+      rest[q] = cs.z[q] + kFlushed;
     }
   }
 #pragma unroll 1
@@ -1008,8 +1014,7 @@ __device__ __forceinline__ void bound_proposal(
   float s = 0.0f, g = 0.0f;
 #pragma unroll
   for (int q = 0; q < Q; q++) {
-    const float left =
-        fmaxf(rest[q], 0.0f) + fmaf(3.0517578e-05f, cs.z[q], kFlushed);
+    const float left = fmaxf(rest[q], 0.0f) + 3.0517578e-05f * cs.z[q];
     const float zu = fmaf(z1[q], 1.0f + eps, left);
     // the largest exponent left is at most the current one and at most the
     // logarithm of what is left of the sum
@@ -1019,11 +1024,10 @@ __device__ __forceinline__ void bound_proposal(
       g += top - cs.mx[q];
     }
   }
-  // Rounded up.  A lane loses 15 a cell at most (what is left is at least 2^-15
-  // z): -64 is still above it.  Upwards 8192, where inf and NaN end too, would
-  // be no bound; but no other lanes bring such a lane's sum back below 4096, and
-  // a warp above that has no bound (the rates are far below those of real data),
-  // nor has the proposal then.
+  // A lane loses 15 a cell at most (what is left is at least 2^-15 z), so that
+  // lane_bound's -64 is not below it.  Its 8192 is no bound; but no other lanes
+  // bring that sum back below 4096, and a warp above 4096 has no bound (the
+  // rates are far below those of real data), nor has the proposal then.
   const int si = __reduce_add_sync(BBS_FULL_MASK, lane_bound(s));
   const int gi = __reduce_add_sync(BBS_FULL_MASK, lane_bound(g));
   constexpr int most = 4096 * (int)kBoundUnit;
