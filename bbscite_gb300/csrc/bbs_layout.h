@@ -116,14 +116,16 @@ __host__ __device__ inline int chain_launch_smem(int n, int n_cells, int q,
          table_bytes(n, w32, q, wpc, counts);
 }
 
-// Rows of up to four words: the table of every node that proposals are read
-// off (bbs_incr.cuh).
+// The table of every node that proposals are read off (bbs_incr.cuh).
 //   chunks  chunks of 32 wpc q cells the table holds (0: no table, the cells
 //           are streamed); the sum score takes one.
-//   inc     the block's increment tables come with it, which refill the table
-//           after the rates of a chain change: one-warp chains of one dataset
-//           in one chunk share one (the layout with `counts` above).  Other
-//           launches fill their tables from the rows and keep the room.
+//   inc     rows of up to four words: the block's increment tables come with
+//           it, which fill it, and again after a chain's rates change its codes:
+//           one-warp chains of one dataset in one chunk share one (the layout
+//           with `counts` above).  Other launches fill their tables from the
+//           rows and keep the room.
+//   ns, global  rows of five to eight words: what of it is in shared memory and
+//           what in global memory.
 struct TablePlan {
   int chunks;
   bool inc;
@@ -159,8 +161,8 @@ inline constexpr int kFewCells = 12;
 // What the chains of a launch read proposals off.
 enum class Tables { none, codes, counts };
 
-// The choice for max-score chains of up to 128 nodes: `load` chains per SM, error
-// moves a share pb of all, the rates' codes (where pb is 0).
+// The choice for max-score chains of up to 128 nodes: `load` chains per SM,
+// error moves a share pb of all, the rates' codes (where pb is 0).
 //   none    Few nodes and cells: an evaluation from the rows costs less than
 //           following the table does, the more so the more often rates change,
 //           which makes codes and table anew, and the more chains share an SM.
@@ -169,11 +171,12 @@ enum class Tables { none, codes, counts };
 //           an evaluation from the rows: the table holds counts, and a proposal
 //           scores every node from them.
 //   codes   The rest.
-// A step, us, by rows / codes / counts, error moves 1 in 11 (Langevin): 2432 chains
-// of 8 x 24 2.0 / 6.0 / 4.9, 1216 of 32 x 64 4.3 / 4.8 / 4.5, 608 of 95 x 96
-// 10.5 / 5.8 / 8.2; 1 in 2: 608 of 95 x 96 10.8 / 12.1 / 8.4.  Over 4 to 127
-// genes, 8 to 256 cells, 8 to 2432 chains and none to half of the moves the choice
-// took 1 % longer than the best of the three; codes alone, 26 %.
+// A step, us, by rows / codes / counts, one move in eleven an error move
+// (Langevin): 2432 chains of 8 x 24 2.0 / 5.8 / 4.8, 608 of 32 x 64 3.5 / 2.8 /
+// 3.3, 608 of 95 x 96 10.4 / 5.7 / 7.8; one in two: 608 of 95 x 96 10.8 / 14.7
+// / 8.1.  Fitted to chains past their first thousands of steps, 4 to 127 genes,
+// 8 to 256 cells, 8 to 2432 chains, none to half of the moves: the choice takes
+// 1 % longer than the best of the three on average, codes alone 28 %.
 struct CodeQuality {
   bool usable, exact;
   int ties, most;  // of the denominators that tie, and how many could
@@ -182,35 +185,35 @@ inline Tables max_score_tables(int n, int n_cells, double load, float pb,
                                const CodeQuality &codes) {
   const int work = n * ((n_cells + 31) / 32);
   const bool poor = pb == 0.0f && (!codes.usable || 3 * codes.ties >= codes.most);
-  const double crowd = 1.0 + std::min(load, 8.0) / 4.0;
-  if (work <= (poor ? 112.0 : std::min(112.0, (5.0 + 270.0 * pb) * crowd)))
+  const double crowd = 1.0 + 0.35 * std::max(0.0, std::min(load, 8.0) - 1.0);
+  const double base = pb == 0.0f && load > 12.0 ? 17.0 : 5.0;
+  if (work <= (poor ? 100.0 : std::min(100.0, base + 190.0 * pb * crowd)))
     return Tables::none;
   if (poor || (pb == 0.0f && !codes.exact && (n > 64 || work > 192)))
     return Tables::counts;
-  const float often = load < 1.0 || (n_cells > 128 && n >= 64) ? 0.4f
+  const float often = load < 1.0 || (n_cells > 128 && n >= 64) ? 0.25f
                       : load >= 4.0 && n <= 64 && n_cells <= 128 ? 0.12f
                                                                  : 0.2f;
   return pb > often ? Tables::counts : Tables::codes;
 }
 
-// The plan of a launch of `slots` chain slots per block, its largest dataset
-// of n nodes and n_cells cells.  Where the tables do not fit a block, or a
-// sum-score chain's cells of rows of up to four words do not fit one chunk,
-// the cells are streamed as before (such launches are bound by their masked
-// popcounts).
-// Nor does the sum score of at most 32 nodes and kFewCells cells take one:
-// nearly every proposal is accepted, so the bound rejects little, and the sum
-// over so few nodes costs less than following the table (1000 steps of 750
-// Langevin chains, every node and table: 8 x 4 2.28, 3.54 ms; 8 x 9 2.27, 3.07;
-// 20 x 9 2.83, 3.48; 8 x 16 2.28, 2.57; at fixed rates 8 x 9 2.12, 1.80; 20 x 9
-// 2.70, 2.28; 8 x 16 2.12, 1.54.  From 33 nodes on the table is no slower).
-// Max-score chains take one where `max_table` says so.  With rows of five to
-// eight words it is in shared memory where that leaves an SM four warps; else
-// one chain per SM keeps as many nodes there as fit (255 x 512: 216 of 256),
-// the others in global memory.  The sum score keeps the ring at that width: half
-// of its proposals are accepted in the runs measured (255 x 512) and then summed
-// over every node, which with a table was slower (200 x 150: 17 M against
-// 22 M chain-steps/s).
+// The plan of a launch of `slots` chain slots per block, its largest dataset of
+// n nodes and n_cells cells.  Where the tables do not fit a block, or a
+// sum-score chain's cells of rows of up to four words do not fit one chunk, the
+// cells are streamed as before (such launches are bound by their masked
+// popcounts). Nor does the sum score of at most 32 nodes and kFewCells cells
+// take one: nearly every proposal is accepted, so the bound rejects little, and
+// the sum over so few nodes costs less than following the table (1000 steps of
+// 750 Langevin chains, every node and table: 8 x 4 2.28, 3.54 ms; 8 x 9 2.27,
+// 3.07; 20 x 9 2.83, 3.48; 8 x 16 2.28, 2.57; at fixed rates 8 x 9 2.12, 1.80;
+// 20 x 9 2.70, 2.28; 8 x 16 2.12, 1.54.  From 33 nodes on the table is no
+// slower). Max-score chains take one where `max_table` says so.  With rows of
+// five to eight words it is in shared memory where that leaves an SM four
+// warps; else one chain per SM keeps as many nodes there as fit (255 x 512: 216
+// of 256), the others in global memory.  The sum score keeps the ring at that
+// width: half of its proposals are accepted in the runs measured (255 x 512)
+// and then summed over every node, which with a table was slower (200 x 150: 17
+// M against 22 M chain-steps/s).
 inline TablePlan plan_tables(int n, int w32, int n_cells, int q, int wpc,
                              int slots, bool sum, bool one_dataset,
                              bool max_table, int smem_block, int smem_sm,
