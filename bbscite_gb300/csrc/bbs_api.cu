@@ -602,12 +602,13 @@ uint64_t fnv1a_of(uint64_t h, const T &v) {
   return fnv1a(h, &v, sizeof(T));
 }
 
-// What max-score chains read proposals off, `load` of them per SM.  With rows of
-// five to eight words: codes at fixed rates that decide every proposal, and where
-// those they leave open are not too dear to score from the rows.  300 steps, ms,
-// with codes that tie somewhere and through the ring: 64, 256 and 800 chains at
-// 150 x 100 3.0, 3.5, 10.2 and 4.7, 5.1, 5.8; 256 at 180 x 100 4.3, 5.8; at 200 x
-// 150 8.5 to 9.8, 5.7 (exact codes 1.9); 128 at 255 x 512 17 to 20, 8.3 (2.7).
+// What max-score chains read proposals off, `load` of them per SM.  With rows
+// of five to eight words: codes at fixed rates that decide every proposal, and
+// where those they leave open are not too dear to score from the rows.  300
+// steps, ms, with codes that tie somewhere and through the ring: 64, 256 and
+// 800 chains at 150 x 100 3.0, 3.5, 10.2 and 4.7, 5.1, 5.8; 256 at 180 x 100
+// 4.3, 5.8; at 200 x 150 8.5 to 9.8, 5.7 (exact codes 1.9); 128 at 255 x 512 17
+// to 20, 8.3 (2.7).
 Tables tables_of(const DatasetDev &ds, const ModelDev &md, const float *terms,
                  double load) {
   if (md.score_mode != 0) return Tables::none;
@@ -628,13 +629,14 @@ Tables tables_of(const DatasetDev &ds, const ModelDev &md, const float *terms,
   return max_score_tables(ds.n_nodes, ds.n_cells, load, pb, codes);
 }
 
-// Runs of so few steps that making a table costs more than it saves.  One step of
-// 1024 chains at 95 x 96, batched: max score 61 us with a table, 31 without, sum
-// score 56 and 29; two steps 67 and 53, 65 and 47, but with a table filled from
-// the block's increments max-score chains gain from the second on (one context,
-// 35 and 46).  Rows of five to eight words, 1, 2 and 4 steps of 128 chains at 255 x
-// 512 133, 146 and 166 us, through the ring 61, 88 and 143; of 256 at 200 x 150,
-// all in shared memory, 72, 79 and 94, through the ring 45, 64 and 101.
+// Runs of so few steps that making a table costs more than it saves.  One step
+// of 1024 chains at 95 x 96, batched: max score 61 us with a table, 31 without,
+// sum score 56 and 29; two steps 67 and 53, 65 and 47, but with a table filled
+// from the block's increments max-score chains gain from the second on (one
+// context, 35 and 46).  Rows of five to eight words, 1, 2 and 4 steps of 128
+// chains at 255 x 512 133, 146 and 166 us, through the ring 61, 88 and 143; of
+// 256 at 200 x 150, all in shared memory, 72, 79 and 94, through the ring 45,
+// 64 and 101.
 bool too_few_steps(uint32_t steps, int w32, const TablePlan &p, bool sum) {
   const uint32_t few = w32 > 4 ? (p.global ? 6 : 3) : !sum && p.inc ? 1 : 2;
   return p.chunks > 0 && steps <= few;
@@ -1079,10 +1081,10 @@ LaunchShape spread_launch(const bbs_ctx *c, bool table) {
 // Fitted to 8 to 3000 chains of 20 to 127 genes and 24 to 400 cells.  Shapes as
 // (cells per lane, warps, chains per block), by the rule of wide rows, used for
 // all before, and by this one, ms: max score, 400 steps, 8 chains at 63 x 64
-// (1, 2, 1) 0.73, (2, 1, 1) 0.67; 750 at 95 x 96 (1, 3, 1) 2.29, (3, 1, 5) 1.14;
-// sum score, 400 steps, 750 at 95 x 128 (1, 4, 1) 3.62, (2, 2, 1) 2.43; 200
-// steps, 3000 at 95 x 128 (4, 1, 8), which has no room for tables, 14.7, (2, 2,
-// 1) 3.7.
+// (1, 2, 1) 0.73, (2, 1, 1) 0.67; 750 at 95 x 96 (1, 3, 1) 2.29, (3, 1, 5)
+// 1.14; sum score, 400 steps, 750 at 95 x 128 (1, 4, 1) 3.62, (2, 2, 1) 2.43;
+// 200 steps, 3000 at 95 x 128 (4, 1, 8), which has no room for tables, 14.7,
+// (2, 2, 1) 3.7.
 LaunchShape default_launch(const bbs_ctx *c) {
   if (w32_of_nodes((int)c->n_nodes) > 4) return spread_launch(c, true);
   const bool sum = c->md.score_mode != 0;
@@ -1127,10 +1129,10 @@ LaunchShape default_launch(const bbs_ctx *c) {
   return o;
 }
 
-// The shape the caller set, its other numbers from the default.  Such a mix need
-// not fit a block -- eight chains per block at the default of two cells per
-// lane, say; the numbers then follow the rule that spreads the cells over warps
-// (c->spread), whose mixes were accepted before chains had tables.
+// The shape the caller set, its other numbers from the default.  Such a mix
+// need not fit a block -- eight chains per block at the default of two cells
+// per lane, say; the numbers then follow the rule that spreads the cells over
+// warps (c->spread), whose mixes were accepted before chains had tables.
 constexpr unsigned kSetCells = 1, kSetWarps = 2, kSetChains = 4;
 void settle_launch(bbs_ctx *c, const LaunchShape &rest) {
   if (!(c->set & kSetCells)) c->q = rest.q;
@@ -1262,8 +1264,8 @@ int start_run(bbs_ctx *c, uint32_t n_steps, const bbs_raw_move *d_moves,
   {
     const int cpb = c->wpc > 1 ? 1 : c->cpb;
     TablePlan p = chain_plan(c, c->q, c->wpc, cpb);
-    // replays and traces of rows of five to eight words go through the ring, and
-    // have no kernels for tables of counts
+    // replays and traces of rows of five to eight words go through the ring,
+    // and have no kernels for tables of counts
     const bool rec = d_moves != nullptr || d_trace != nullptr;
     if (too_few_steps(n_steps, w32_of_nodes((int)c->n_nodes), p,
                       c->md.score_mode != 0) ||
@@ -2298,8 +2300,8 @@ int batch_build_groups(bbs_batch *b) {
 // a table only where their cells fit one pass, so up to 128 cells get as many
 // cells per lane as that takes, unless smaller datasets would be most of the
 // work.  600 steps with two and with that many cells per lane, ms: 2844 chains
-// at 105 x 81 46.7, 16.0; 20 at 20 x 70 2.74, 0.76; 300 at 127 x 128 (300 steps)
-// 10.2, 2.1.  Max-score tables take several passes.
+// at 105 x 81 46.7, 16.0; 20 at 20 x 70 2.74, 0.76; 300 at 127 x 128 (300
+// steps) 10.2, 2.1.  Max-score tables take several passes.
 int default_cells_per_lane(const bbs_batch *b) {
   uint32_t lo = UINT32_MAX, hi = 0;
   for (uint32_t d = 0; d < b->n_datasets; d++) {

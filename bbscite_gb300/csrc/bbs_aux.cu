@@ -174,10 +174,10 @@ int launch_init(const InitArgs &a, int w32, bool sum, void *stream) {
   }
 }
 
-// Up to this many trees a block scores one tree (score_few_kernel): about two
-// blocks of 16 warps per SM.  Calls on either side of it, before and now: 300
-// trees at 95 x 96 79 -> 59 us, 310 trees 87 -> 77 us; 300 trees at 255 x 512
-// 571 -> 184 us, 310 trees 571 -> 169 us.
+// Up to this many trees a block scores one tree (score_few_kernel): two blocks
+// of 16 warps on each of GB300's 152 SMs.  Calls on either side of it, before
+// and now: 300 trees at 95 x 96 79 -> 59 us, 310 trees 87 -> 77 us; 300 trees
+// at 255 x 512 571 -> 184 us, 310 trees 571 -> 169 us.
 inline constexpr int kFewTrees = 304;
 
 // Many trees of rows of up to four words are walked (score_tree_kernel) from

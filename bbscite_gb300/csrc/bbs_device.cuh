@@ -1589,15 +1589,11 @@ __device__ __forceinline__ void sum_cells(const uint32_t *rows, int n,
   }
 }
 
-// This warp's part of the sum score and expected counts (fixed point,
-// warp-reduced), its terms added in the canonical order (sx.ord, built
-// here).  Inherited counts serve cells held in registers when sx brings the
-// parent vector, the count table and the increment table.
-// The masked-popcount node loop, out of line: it serves only streamed cells
-// and mixed launch groups (rows of up to four words), trees whose order
-// does not fit the ring or whose parent vector is not known (wider rows),
-// and keeping one copy of it outside the chain kernels leaves the
-// inherited-count loops and the step code small.
+// The masked-popcount node loop, out of line: it serves chains without a table
+// and proposals that are not followed in one (rows of up to four words), trees
+// whose order does not fit the ring or whose parent vector is not known (wider
+// rows), and keeping one copy of it outside the chain kernels leaves the ring's
+// loops and the step code small.
 struct Acc6 {
   long long v[6];
 };
@@ -1616,6 +1612,10 @@ __device__ __noinline__ Acc6 sum_cells_popc(const uint32_t *rows, int n,
   return o;
 }
 
+// This warp's part of the sum score and expected counts (fixed point,
+// warp-reduced), its terms added in the canonical order (sx.ord, built here):
+// counts through the ring for rows of five to eight words where sx brings the
+// tree's parent vector, masked popcounts otherwise.
 template <int W32, int Q>
 __device__ __forceinline__ void sum_part(const uint32_t *rows, int n,
                                          const DatasetDev &ds,
@@ -1666,13 +1666,13 @@ __device__ __forceinline__ void sum_part(const uint32_t *rows, int n,
   acc[5] = warp_sum_ll(acc[5]);
 }
 
-// Max score with counts through the ring: the nodes in the canonical order
-// with their counts found one pair ahead as for the sum score, each node's score in the reference's
-// order, and the first maximum in node-index order -- an equal score at a
-// lower index wins, which is what std::max over the nodes in index order
-// keeps (src/TreeScorer.hpp:187-193) -- so the chosen nodes are those of
-// best_nodes.  The ring no longer holds every node at the end: the class
-// counts at the chosen nodes are the caller's masked popcounts.
+// Max score with counts through the ring: the nodes in the canonical order with
+// their counts found one pair ahead as for the sum score, each node's score in
+// the reference's order, and the first maximum in node-index order -- an equal
+// score at a lower index wins, which is what std::max over the nodes in index
+// order keeps (src/TreeScorer.hpp:187-193) -- so the chosen nodes are those of
+// best_nodes.  The ring no longer holds every node at the end: the class counts
+// at the chosen nodes are the caller's masked popcounts.
 __device__ __forceinline__ void max_select(float s, int j, float &best,
                                            int &bj) {
   const bool up = s > best || (s == best && j < bj);

@@ -4,9 +4,15 @@
 //                 A chain is one warp, or `wpc` warps that split its cells
 //                 (the block is then that one chain).  The chain's current
 //                 and proposed ancestor rows are double-buffered in shared
-//                 memory; cell rows stay in registers (or are re-read per
-//                 chunk for wide datasets).
-//   score_kernel  TreeScorer::logscore_tree over a batch (warp per tree).
+//                 memory.  Proposals are read off a table of every node of the
+//                 current tree (bbs_incr.cuh), or every node is evaluated, the
+//                 cell rows loaded for each evaluation.
+//   batch_kernel  the same over many datasets, from a work list.
+//   init_kernel   the chains' initial states.
+//   score_*       TreeScorer::logscore_tree over a batch: score_few_kernel a
+//                 block per tree; score_walk_kernel and score_tree_kernel, a
+//                 block or a warp per tree, codes inherited along the tree;
+//                 score_kernel, a warp per tree, masked popcounts.
 //   apply_kernel  realize_raw_move_sample + update ctor over a batch.
 //   grad_kernel   sum-over-attachments score with its fused adjoint.
 #pragma once
@@ -515,11 +521,12 @@ __device__ __noinline__ void propose_tree_call(
                     lane);
 }
 
-// run_chain with the table of bbs_incr.cuh in ss.sx.cnt (rows of up to four
-// words; `chunks` chunks of the warp's cells, one for the sum score).
-// Bound at 95 x 96 (1024 one-warp chains, 1.8 warps per scheduler) by the
-// latency of one step's serial chain -- draw, descendant sets, table loads,
-// reductions -- no longer by the node loop's instructions.
+// run_chain with a table of bbs_incr.cuh: `chunks` chunks of the warp's cells
+// in tab, one for the sum score, which holds counts (rows of up to four words).
+// Max score chains hold codes or, with COUNTS, counts (up to four words). Bound
+// at 95 x 96 (1024 one-warp chains, 1.8 warps per scheduler) by the latency of
+// one step's serial chain -- draw, descendant sets, table loads, reductions --
+// no longer by the node loop's instructions.
 template <int W32, int Q, bool SUM, bool COUNTS>
 __device__ __forceinline__ void run_chain_table(
     const DatasetDev &ds, const ModelDev &md, uint32_t chain_id,
@@ -1562,11 +1569,11 @@ __device__ __forceinline__ void walk_codes(const SumCtx &sx,
 // Scores of many trees with rows of five to eight words: one block per tree,
 // four warps over its chunks of 64 cells.  Where the rows are a tree whose
 // order fits the ring and its rates have exact codes (bbs_incr.cuh), each node
-// takes its parent's codes from the ring plus its gene's, some 20
-// instructions a node for 64 cells; otherwise masked popcounts, which run the
+// takes its parent's codes from the ring plus its gene's, some 20 instructions
+// a node for 64 cells; otherwise masked popcounts, which run the
 // population-count pipe at its peak (255 x 512, 1500 trees: 735 us, walked 230
-// us, and another 9 us less a call with offsets in the order's entries; bound by
-// the latency of the walk at three blocks per SM).
+// us, and another 9 us less a call with offsets in the order's entries; bound
+// by the latency of the walk at three blocks per SM).
 template <int W32, bool ATTACH>
 __global__ void __launch_bounds__(128) score_walk_kernel(const ScoreArgs a) {
   extern __shared__ __align__(16) uint32_t smem[];
@@ -1735,8 +1742,9 @@ __global__ void __launch_bounds__(128) apply_kernel(const ApplyArgs a) {
 // softmax-weighted sums of d and m; a cell whose maximum lies more than 80
 // below r is summed again against its maximum.  An online maximum per term,
 // as before, took both sides of a branch and two exponentials for most nodes
-// (4096 trees at 95 x 96: 110 us, now 85 us, bound by instruction issue).  The expected class counts give dlogL /
-// dtheta = sum_c sum_k E_pi[n_k] dl_k / dtheta.
+// (4096 trees at 95 x 96: 110 us, now 85 us, bound by instruction issue).  The
+// expected class counts give dlogL / dtheta = sum_c sum_k E_pi[n_k] dl_k /
+// dtheta.
 // With posteriors a warp keeps its cells' scores in shared memory (`tile`
 // floats per cell) and writes the 32 cells' rows as one contiguous piece; a
 // store per lane and node went to 32 lines each (50 trees at 61 x 201: 83 ->

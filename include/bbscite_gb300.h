@@ -207,7 +207,8 @@ BBS_API int bbs_cancel(bbs_ctx *ctx);
  * cells per lane per chunk (1-4; 1-2 above 128 nodes), warps per chain
  * (1-4; the cells are split over them) and chains per block (one-warp
  * chains only: 1-4, or 1-8 with 3-4 cells per lane; a run with a larger
- * block fails).  0 keeps a value.  bbs_init_chains picks a default. */
+ * block fails).  0 keeps a value; one that was never set may still change
+ * with the others, so that the shape fits.  bbs_init_chains picks a default. */
 BBS_API int bbs_set_launch(bbs_ctx *ctx, int cells_per_lane,
                            int warps_per_chain, int chains_per_block);
 BBS_API int bbs_get_launch(const bbs_ctx *ctx, int *cells_per_lane,
@@ -318,7 +319,8 @@ BBS_API int bbs_batch_last_run_ms(const bbs_batch *batch, float *ms);
 /* Launch shape: cells per lane (1-4; 1-2 above 128 nodes) and warps per
  * block (1-8; a launch group with 1-2 cells per lane takes at most 4, and
  * a block too large for its shared memory fails the run with
- * BBS_ERR_SIZE);
+ * BBS_ERR_SIZE).  0 keeps a value; cells per lane that were never set follow
+ * the warps, so that the block fits;
  * merge_rows != 0 runs trees of an odd number of 32-bit row words (1, 3,
  * 5, 7) with the next even width, which has the same row stride (one
  * launch per pair of widths instead of two). */
