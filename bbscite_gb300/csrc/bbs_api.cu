@@ -604,25 +604,30 @@ uint64_t fnv1a_of(uint64_t h, const T &v) {
 
 // What max-score chains read proposals off, `load` of them per SM.  With rows
 // of five to eight words: codes at fixed rates that decide every proposal, and
-// where those they leave open are not too dear to score from the rows.  300
-// steps, ms, with codes that tie somewhere and through the ring: 64, 256 and
-// 800 chains at 150 x 100 3.0, 3.5, 10.2 and 4.7, 5.1, 5.8; 256 at 180 x 100
-// 4.3, 5.8; at 200 x 150 8.5 to 9.8, 5.7 (exact codes 1.9); 128 at 255 x 512 17
-// to 20, 8.3 (2.7).
+// where those they leave open are not too dear to score from the rows.  500
+// steps, ms, after 8,000, with codes that tie somewhere and through the ring:
+// 64 and 800 chains at 150 x 100 3.5 to 4.1, 11.4 to 14.1 and 7.9, 9.6; 256 at
+// 130 x 200 4.2 to 5.4, 6.8; at 200 x 150 9.3 to 11.3, 9.6 (exact codes 2.7);
+// 64 at 160 x 400 7.0, 9.8; 1024 at 255 x 100 61 to 63, 23; 128 at 255 x 512
+// after 6,000 19 to 23, 13.9 (3.9).
 Tables tables_of(const DatasetDev &ds, const ModelDev &md, const float *terms,
                  double load) {
   if (md.score_mode != 0) return Tables::none;
   const float pb = md.mp.cum_beta;
   const bool wide = ds.n_nodes > 128;
   if (wide && pb != 0.0f) return Tables::none;
-  CodeQuality codes{true, true, 0, 1};
+  CodeQuality codes{true, 0, 1};
   if (pb == 0.0f) {
     const MaxCode k = make_code_host(terms[2], terms[4], terms[3], terms[5],
                                      ds.max_d, ds.max_m);
-    codes = {k.usable, k.exact, k.ties,
-             std::max(1, std::min(ds.max_d, ds.max_m))};
-    const bool cheap = load <= 2.0 &&
-                       ds.n_nodes * ((ds.n_cells + 31) / 32) <= 750;
+    // denominators whose fractions stay within the counts of a cell
+    const float ratio =
+        std::abs(terms[4] - terms[2]) / std::abs(terms[5] - terms[3]);
+    codes = {k.usable, k.ties,
+             k.usable ? (int)std::min((float)ds.max_d, (float)ds.max_m / ratio)
+                      : 0};
+    const bool cheap =
+        load * ds.n_nodes * ((ds.n_cells + 31) / 32) <= 1600.0;
     if (wide)
       return k.usable && (k.exact || cheap) ? Tables::codes : Tables::none;
   }
@@ -633,12 +638,16 @@ Tables tables_of(const DatasetDev &ds, const ModelDev &md, const float *terms,
 // of 1024 chains at 95 x 96, batched: max score 61 us with a table, 31 without,
 // sum score 56 and 29; two steps 67 and 53, 65 and 47, but with a table filled
 // from the block's increments max-score chains gain from the second on (one
-// context, 35 and 46).  Rows of five to eight words, 1, 2 and 4 steps of 128
-// chains at 255 x 512 133, 146 and 166 us, through the ring 61, 88 and 143; of
-// 256 at 200 x 150, all in shared memory, 72, 79 and 94, through the ring 45,
-// 64 and 101.
+// context, 35 and 46); of 512 chains at 20 x 24, four steps, max score 24 and
+// 17, sum score 27 and 20, sixteen 39 and 37, 46 and 49.  Rows of five to eight
+// words, 1, 2 and 4 steps of 128 chains at 255 x 512 133, 146 and 166 us,
+// through the ring 61, 88 and 143; of 256 at 200 x 150, all in shared memory,
+// 72, 79 and 94, through the ring 45, 64 and 101.
 bool too_few_steps(uint32_t steps, int w32, const TablePlan &p, bool sum) {
-  const uint32_t few = w32 > 4 ? (p.global ? 6 : 3) : !sum && p.inc ? 1 : 2;
+  const uint32_t few = w32 > 4          ? (p.global ? 6 : 3)
+                       : w32 == 1       ? 8
+                       : !sum && p.inc ? 1
+                                        : 2;
   return p.chunks > 0 && steps <= few;
 }
 

@@ -167,9 +167,10 @@ enum class Tables { none, codes, counts };
 //           following the table does, the more so the more often rates change,
 //           which makes codes and table anew, and the more chains share an SM.
 //   counts  Otherwise, where rates change so often that codes do not pay, and at
-//           fixed rates without codes or with codes that leave many proposals to
-//           an evaluation from the rows: the table holds counts, and a proposal
-//           scores every node from them.
+//           fixed rates without codes or with codes that tie at most counts (a
+//           ratio of the log differences like 1 or 1/2) and so leave many
+//           proposals to an evaluation from the rows: the table holds counts,
+//           and a proposal scores every node from them.
 //   codes   The rest.
 // A step, us, by rows / codes / counts, one move in eleven an error move
 // (Langevin): 2432 chains of 8 x 24 2.0 / 5.8 / 4.8, 608 of 32 x 64 3.5 / 2.8 /
@@ -178,19 +179,18 @@ enum class Tables { none, codes, counts };
 // 8 to 256 cells, 8 to 2432 chains, none to half of the moves: the choice takes
 // 1 % longer than the best of the three on average, codes alone 28 %.
 struct CodeQuality {
-  bool usable, exact;
+  bool usable;
   int ties, most;  // of the denominators that tie, and how many could
 };
 inline Tables max_score_tables(int n, int n_cells, double load, float pb,
                                const CodeQuality &codes) {
   const int work = n * ((n_cells + 31) / 32);
-  const bool poor = pb == 0.0f && (!codes.usable || 3 * codes.ties >= codes.most);
+  const bool poor = pb == 0.0f && (!codes.usable || 5 * codes.ties >= 2 * codes.most);
   const double crowd = 1.0 + 0.35 * std::max(0.0, std::min(load, 8.0) - 1.0);
   const double base = pb == 0.0f && load > 12.0 ? 17.0 : 5.0;
   if (work <= (poor ? 100.0 : std::min(100.0, base + 190.0 * pb * crowd)))
     return Tables::none;
-  if (poor || (pb == 0.0f && !codes.exact && (n > 64 || work > 192)))
-    return Tables::counts;
+  if (poor) return Tables::counts;
   const float often = load < 1.0 || (n_cells > 128 && n >= 64) ? 0.25f
                       : load >= 4.0 && n <= 64 && n_cells <= 128 ? 0.12f
                                                                  : 0.2f;
