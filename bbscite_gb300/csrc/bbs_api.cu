@@ -638,14 +638,15 @@ Tables tables_of(const DatasetDev &ds, const ModelDev &md, const float *terms,
 // of 1024 chains at 95 x 96, batched: max score 61 us with a table, 31 without,
 // sum score 56 and 29; two steps 67 and 53, 65 and 47, but with a table filled
 // from the block's increments max-score chains gain from the second on (one
-// context, 35 and 46); of 512 chains at 20 x 24, four steps, max score 24 and
-// 17, sum score 27 and 20, sixteen 39 and 37, 46 and 49.  Rows of five to eight
-// words, 1, 2 and 4 steps of 128 chains at 255 x 512 133, 146 and 166 us,
-// through the ring 61, 88 and 143; of 256 at 200 x 150, all in shared memory,
-// 72, 79 and 94, through the ring 45, 64 and 101.
+// context, 35 and 46).  Up to 32 nodes, 4 and 8 steps, us, max score, then sum:
+// 512 chains at 20 x 24 23, 29 and 17, 24; 27, 34 and 20, 30; 64 at 25 x 100 18,
+// 23 and 16, 25; 22, 27 and 21, 35.  Rows of five to eight words, 1, 2 and 4
+// steps of 128 chains at 255 x 512 133, 146 and 166, through the ring 61, 88 and
+// 143; of 256 at 200 x 150, all in shared memory, 72, 79 and 94, through the
+// ring 45, 64 and 101.
 bool too_few_steps(uint32_t steps, int w32, const TablePlan &p, bool sum) {
-  const uint32_t few = w32 > 4          ? (p.global ? 6 : 3)
-                       : w32 == 1       ? 8
+  const uint32_t few = w32 > 4         ? (p.global ? 6 : 3)
+                       : w32 == 1      ? 4
                        : !sum && p.inc ? 1
                                         : 2;
   return p.chunks > 0 && steps <= few;
