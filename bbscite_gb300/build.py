@@ -12,7 +12,7 @@ Outputs (git-ignored):
 Translation units are compiled in parallel; nothing is rebuilt when the
 library is newer than every source.  The objects go once they are linked, and
 the checked library's device code is compressed for size (at some 6 ms per unit
-when its first kernel loads): 178 MB are left of a build, not 634.
+when its first kernel loads): some 200 MB are left of a build, not 634.
 """
 from __future__ import annotations
 
